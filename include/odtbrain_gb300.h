@@ -197,6 +197,56 @@ odt_status odt_bpp3d_execute_timed(const odt_bpp3d_plan *plan,
 odt_status odt_bpp3d_launch_count(const odt_bpp3d_plan *plan,
                                   int64_t *launches);
 
+/* ---- Opposite views ------------------------------------------------------
+ * Rotating by phi + pi is rotating the filtered slab by pi about y and then
+ * by phi, and a rotation by pi maps the slab's grid onto itself.  So two views
+ * phi and phi + pi can share the backward transforms and the resampling: the
+ * second view's spectrum, of the mirrored projection, is added to the first's
+ * before the transforms.  A unit is one view or two opposite ones:
+ *   views     device, num_units*2 int32: the first view's angle index and the
+ *             opposite one's (or -1); every angle appears exactly once
+ *   geometry  device, num_units*6 doubles: the first views' rotations
+ * The caller pairs only views whose in/out decisions agree: for every output
+ * (z, x), inside the domain for the second view exactly where the first
+ * view's coordinates are inside it.
+ * ODT_ERR_UNSUPPORTED for plans about a tilted axis, filter or kz_phase tables
+ * that are not even in kx, and workspace limits too small for one unit. */
+typedef struct odt_bpp3d_units {
+    int32_t num_units;
+    int32_t reserved;
+    const int32_t *views;
+    const double *geometry;
+} odt_bpp3d_units;
+
+/* Bytes of device workspace odt_bpp3d_execute_pairs and
+ * odt_bpp3d_adjoint_pairs need (adjoint_bytes may be NULL). */
+odt_status odt_bpp3d_pair_workspace_size(const odt_bpp3d_plan *plan,
+                                         int32_t num_units, uint64_t *bytes,
+                                         uint64_t *adjoint_bytes);
+
+/* odt_bpp3d_execute_gain over units of opposite views (gain and angle_gain
+ * may be NULL).  With `timing` it waits for the stream and fills it like
+ * odt_bpp3d_execute_timed. */
+odt_status odt_bpp3d_execute_pairs(const odt_bpp3d_plan *plan,
+                                   const odt_bpp3d_units *units,
+                                   const void *sino, const double *weights,
+                                   const float *gain, const void *angle_gain,
+                                   void *volume, void *workspace, void *stream,
+                                   odt_stage_timing *timing);
+
+/* odt_bpp3d_adjoint over units of opposite views. */
+odt_status odt_bpp3d_adjoint_pairs(const odt_bpp3d_plan *plan,
+                                   const odt_bpp3d_units *units,
+                                   const void *sino, const double *weights,
+                                   const float *gain, const void *angle_gain,
+                                   const void *vol_grad, void *sino_grad,
+                                   float *gain_grad, void *angle_gain_grad,
+                                   void *workspace, void *stream);
+
+/* Number of kernel launches one odt_bpp3d_execute_pairs makes. */
+odt_status odt_bpp3d_pair_launch_count(const odt_bpp3d_plan *plan,
+                                       int32_t num_units, int64_t *launches);
+
 /* Bytes of the library's static device scratch used by
  * odt_bpp3d_execute_noalloc. */
 #define ODT_NOALLOC_SCRATCH_BYTES (64ull << 20)

@@ -23,7 +23,7 @@ import numpy as np
 from . import _geometry as geom
 from . import _native
 from ._alg3d import (_WS_DEFAULT, _device_for, _get_plan, _get_tables,
-                     _is_tensor, _torch)
+                     _is_tensor, _pairing, _torch)
 
 
 class Backprop2D:
@@ -60,7 +60,8 @@ class Backprop2D:
 
         def build_tables():
             return (geom.compute_angle_weights_1d(angles) if weight_angles
-                    else None, geom.rotation_2d_geometry(angles, ln), None)
+                    else None, geom.rotation_2d_geometry(angles, ln), None,
+                    ln)
         tkey = (device.index, "2d", angles.dtype.str, angles.shape,
                 angles.tobytes(), ln, bool(weight_angles))
         key = ("2d", device.index, A, ln, g["lN"], g["padl"], pad_mode,
@@ -91,9 +92,11 @@ class Backprop2D:
 
         with torch.cuda.device(device):
             self.plan = _get_plan(key, build_desc)
-            self.weights, self.geometry, _ = _get_tables(tkey, build_tables)
-            self.workspace = torch.empty(max(self.plan.workspace_bytes, 1),
-                                         device=device, dtype=torch.uint8)
+            self.weights, self.geometry, _, units = _get_tables(tkey,
+                                                                build_tables)
+            self._units, ws_bytes, _ = _pairing(self.plan, units)
+            self.workspace = torch.empty(max(ws_bytes, 1), device=device,
+                                         dtype=torch.uint8)
 
     def __call__(self, sino, out=None, check=True):
         """Reconstruct from a device sinogram (A, ln); returns the (ln, ln)
@@ -114,20 +117,30 @@ class Backprop2D:
             raise ValueError("out must be a contiguous %s tensor of shape "
                              "%s" % (vdtype, (ln, ln)))
         stream = torch.cuda.current_stream(self.device)
-        self.plan.execute(
-            ctypes.c_void_p(sino.data_ptr()),
-            ctypes.c_void_p(self.weights.data_ptr()
-                            if self.weights is not None else 0),
-            ctypes.c_void_p(self.geometry.data_ptr()),
-            ctypes.c_void_p(out.data_ptr()),
-            ctypes.c_void_p(self.workspace.data_ptr()),
-            ctypes.c_void_p(stream.cuda_stream))
+        self._execute(sino, out, stream)
         if check:
             self.plan.read_status(ctypes.c_void_p(stream.cuda_stream))
         return out
 
+    def _execute(self, sino, out, stream, timed=False):
+        sptr = ctypes.c_void_p(sino.data_ptr())
+        wptr = ctypes.c_void_p(self.weights.data_ptr()
+                               if self.weights is not None else 0)
+        optr = ctypes.c_void_p(out.data_ptr())
+        ws = ctypes.c_void_p(self.workspace.data_ptr())
+        handle = ctypes.c_void_p(stream.cuda_stream)
+        if self._units is not None:
+            return self.plan.execute_pairs(self._units.struct, sptr, wptr,
+                                           None, None, optr, ws, handle,
+                                           timed)
+        run = self.plan.execute_timed if timed else self.plan.execute
+        return run(sptr, wptr, ctypes.c_void_p(self.geometry.data_ptr()),
+                   optr, ws, handle)
+
     @property
     def launches_per_call(self):
+        if self._units is not None:
+            return self.plan.pair_launches(self._units.num)
         return self.plan.launches_per_execute
 
     def timed(self, sino, out=None):
@@ -140,14 +153,7 @@ class Backprop2D:
             out = torch.empty((ln, ln), device=self.device, dtype=vdtype)
         self(sino, out=out, check=False)  # argument checks, warm tables
         stream = torch.cuda.current_stream(self.device)
-        t = self.plan.execute_timed(
-            ctypes.c_void_p(sino.data_ptr()),
-            ctypes.c_void_p(self.weights.data_ptr()
-                            if self.weights is not None else 0),
-            ctypes.c_void_p(self.geometry.data_ptr()),
-            ctypes.c_void_p(out.data_ptr()),
-            ctypes.c_void_p(self.workspace.data_ptr()),
-            ctypes.c_void_p(stream.cuda_stream))
+        t = self._execute(sino, out, stream, timed=True)
         self.plan.read_status(ctypes.c_void_p(stream.cuda_stream))
         return t
 

@@ -43,6 +43,12 @@ _TABLE_CACHE = collections.OrderedDict()
 _TABLE_CACHE_SIZE = 8
 
 
+# Units per angle up to which opposite views are paired.  A unit of two views
+# costs @@ of a single one (256^3 columns), so pairing pays from the first
+# few pairs; the share leaves out sets with stray accidental pairs.
+_PAIR_SHARE = 0.9
+
+
 def _torch():
     import torch
     return torch
@@ -95,10 +101,25 @@ def _pad_mode(padding, padval):
     return _native.ODT_PAD_RAMP, complex(padval)
 
 
+class _Units:
+    """The opposite views of an angle set as odt_bpp3d_units, with the device
+    arrays it points to."""
+
+    def __init__(self, views, geometry, device):
+        torch = _torch()
+        self.num = len(views)
+        self.views = torch.from_numpy(views).to(device)
+        self.geometry = torch.from_numpy(np.ascontiguousarray(
+            geometry[views[:, 0]], dtype=np.float64)).to(device)
+        self.struct = _native.Bpp3dUnits(self.num, 0, self.views.data_ptr(),
+                                         self.geometry.data_ptr())
+
+
 def _get_tables(key, build):
-    """(weights, geometry, taxis) for `key`: `build()` returns the host
-    weights (or None), the geometry and the tilted axis; the device tensors
-    are cached and must not be modified."""
+    """(weights, geometry, taxis, units) for `key`: `build()` returns the
+    host weights (or None), the geometry, the tilted axis and the length of
+    the plane whose opposite views may be paired (or None); the device
+    tensors are cached and must not be modified."""
     with _PLAN_LOCK:
         hit = _TABLE_CACHE.get(key)
         if hit is not None:
@@ -106,17 +127,33 @@ def _get_tables(key, build):
             return hit
     torch = _torch()
     device = torch.device("cuda", key[0])
-    weights, geometry, taxis = build()
+    weights, geometry, taxis, plane = build()
+    units = None
+    if plane is not None:
+        views = geom.opposite_units(geometry, plane)
+        if len(views) <= _PAIR_SHARE * len(geometry):
+            units = _Units(views, geometry, device)
     dw = (torch.from_numpy(np.ascontiguousarray(weights, dtype=np.float64))
           .to(device) if weights is not None else None)
     dg = torch.from_numpy(np.ascontiguousarray(geometry, dtype=np.float64)) \
         .to(device)
-    hit = (dw, dg, taxis)
+    hit = (dw, dg, taxis, units)
     with _PLAN_LOCK:
         _TABLE_CACHE[key] = hit
         while len(_TABLE_CACHE) > _TABLE_CACHE_SIZE:
             _TABLE_CACHE.popitem(last=False)
     return hit
+
+
+def _pairing(plan, units):
+    """(units or None, workspace bytes, adjoint workspace bytes or None) of
+    an execution of `plan`: over `units` of opposite views where the plan can
+    pair them, else over single angles."""
+    sizes = plan.pair_workspace_bytes(units.num) if units is not None \
+        else None
+    if sizes is None:
+        return None, plan.workspace_bytes, None
+    return (units,) + sizes
 
 
 def _get_plan(key, build_desc):
@@ -183,21 +220,23 @@ class Backprop3D:
             def build_tables():
                 return (geom.compute_angle_weights_1d(angles)
                         if weight_angles else None,
-                        geom.rotation_y_geometry(angles, lnx, lnx), None)
+                        geom.rotation_y_geometry(angles, lnx, lnx), None, lnx)
             tkey = (device.index, "y", angles.dtype.str, angles.shape,
                     angles.tobytes(), lnx, bool(weight_angles))
         else:
             kind = _native.ODT_GEOM_AFFINE3D
 
             def build_tables():
-                return geom.tilted_geometry(angles, tilted_axis,
-                                            weight_angles, (lnx, lny, lnx))
+                return geom.tilted_geometry(
+                    angles, tilted_axis, weight_angles,
+                    (lnx, lny, lnx)) + (None,)
             tkey = (device.index, "tilted", angles.dtype.str, angles.shape,
                     angles.tobytes(), np.asarray(tilted_axis,
                                                  dtype=np.float64).tobytes(),
                     lnx, lny, bool(weight_angles))
         with torch.cuda.device(device):
-            dweights, dgeometry, taxis = _get_tables(tkey, build_tables)
+            dweights, dgeometry, taxis, units = _get_tables(tkey,
+                                                            build_tables)
         in_dtype = {"complex64": _native.ODT_INPUT_C64,
                     "complex128": _native.ODT_INPUT_C128}[str(input_dtype)
                                                          .replace("torch.",
@@ -243,12 +282,16 @@ class Backprop3D:
                 self.weights = torch.from_numpy(np.ascontiguousarray(
                     user_weights, dtype=np.float64)).to(self.device)
             self.geometry = dgeometry
-            self.workspace = torch.empty(max(self.plan.workspace_bytes, 1),
+            self._units, ws_bytes, self._adjoint_bytes = _pairing(self.plan,
+                                                                  units)
+            self.workspace = torch.empty(max(ws_bytes, 1),
                                          device=self.device,
                                          dtype=torch.uint8)
 
     @property
     def launches_per_call(self):
+        if self._units is not None:
+            return self.plan.pair_launches(self._units.num)
         return self.plan.launches_per_execute
 
     def volume_shape(self):
@@ -292,10 +335,21 @@ class Backprop3D:
         torch = _torch()
         with torch.cuda.device(self.device):
             out, stream, args = self._args(sino, out)
-            self.plan.execute(*args)
+            self._execute(args)
             if check:
                 self.plan.read_status(ctypes.c_void_p(stream.cuda_stream))
         return out
+
+    def _execute(self, args, gptr=None, aptr=None, timed=False):
+        sino, weights, geometry, volume, workspace, stream = args
+        if self._units is not None:
+            return self.plan.execute_pairs(self._units.struct, sino, weights,
+                                           gptr, aptr, volume, workspace,
+                                           stream, timed)
+        if timed:
+            return self.plan.execute_timed(*args)
+        return self.plan.execute_gain(sino, weights, geometry, gptr, aptr,
+                                      volume, workspace, stream)
 
     def forward_gain(self, sino, gain=None, angle_gain=None, out=None,
                      check=True):
@@ -310,8 +364,7 @@ class Backprop3D:
             aptr = ctypes.c_void_p(
                 self._check_angle_gain(angle_gain).data_ptr()
                 if angle_gain is not None else 0)
-            self.plan.execute_gain(args[0], args[1], args[2], gptr, aptr,
-                                   args[3], args[4], args[5])
+            self._execute(args, gptr, aptr)
             if check:
                 self.plan.read_status(ctypes.c_void_p(stream.cuda_stream))
         return out
@@ -365,6 +418,8 @@ class Backprop3D:
             raise ValueError("vol_grad must be complex64 of the volume shape")
         vol_grad = vol_grad.contiguous()
         ws_bytes = self.plan.adjoint_workspace_bytes()
+        if self._units is not None:
+            ws_bytes = self._adjoint_bytes
         ws = torch.empty(max(ws_bytes, 1), device=self.device,
                          dtype=torch.uint8)
         sgrad = (torch.empty(self.shape, device=self.device,
@@ -389,10 +444,14 @@ class Backprop3D:
         def ptr(t):
             return ctypes.c_void_p(t.data_ptr() if t is not None else 0)
         with torch.cuda.device(self.device):
-            self.plan.adjoint(
-                sptr, ptr(self.weights), ptr(self.geometry), gptr, aptr,
-                ptr(vol_grad), ptr(sgrad), ptr(ggrad), ptr(aggrad), ptr(ws),
-                ctypes.c_void_p(stream.cuda_stream))
+            rest = (gptr, aptr, ptr(vol_grad), ptr(sgrad), ptr(ggrad),
+                    ptr(aggrad), ptr(ws), ctypes.c_void_p(stream.cuda_stream))
+            if self._units is not None:
+                self.plan.adjoint_pairs(self._units.struct, sptr,
+                                        ptr(self.weights), *rest)
+            else:
+                self.plan.adjoint(sptr, ptr(self.weights),
+                                  ptr(self.geometry), *rest)
             self.plan.read_status(ctypes.c_void_p(stream.cuda_stream))
         del ws
         if need_angle_gain:
@@ -405,7 +464,7 @@ class Backprop3D:
         torch = _torch()
         with torch.cuda.device(self.device):
             out, stream, args = self._args(sino, out)
-            t = self.plan.execute_timed(*args)
+            t = self._execute(args, timed=True)
             self.plan.read_status(ctypes.c_void_p(stream.cuda_stream))
         return t
 

@@ -85,6 +85,75 @@ def rotation_y_geometry(angles, nz, nx):
     return out
 
 
+def opposite_units(geometry, n):
+    """Opposite views of a set of plane rotations (A, 6) of an n x n plane:
+    an int32 array (U, 2) of (angle, opposite angle or -1) in which every
+    angle appears once.
+
+    Views phi and phi + pi resample with coordinates c and n-1-c, so they can
+    share one slab (the CUDA stages' header has the construction) -- as long
+    as both make the same in/out decisions.  Those are strict comparisons of
+    FP64 coordinates with 0 and n-1; c and n-1-c agree to about 1e-13, so
+    views are paired when no output's coordinate lies within 1e-9 of the
+    boundary, or when both matrices' entries are 0 or +-1 and the coordinates
+    therefore exact.
+    """
+    geometry = np.asarray(geometry)
+    A = geometry.shape[0]
+    theta = np.arctan2(geometry[:, 1], geometry[:, 0]) % (2 * np.pi)
+    order = np.argsort(theta, kind="stable")
+    srt = theta[order]
+    # the first view at or after the opposite direction (a tolerance before
+    # it, wrapping around)
+    opp = (theta + np.pi - 1e-9) % (2 * np.pi)
+    at = order[np.searchsorted(srt, opp) % A]
+    ok = np.all(np.abs(geometry[:, :4] + geometry[at, :4]) < 1e-12, axis=1)
+    partner = np.full(A, -1)
+    for a in np.flatnonzero(ok):
+        b = at[a]
+        if partner[a] < 0 and partner[b] < 0 and b != a:
+            partner[a], partner[b] = b, a
+    first = np.flatnonzero((partner < 0) | (np.arange(A) < partner))
+    paired = first[partner[first] >= 0]
+    apart = paired[~(_clear_of_boundary(geometry[paired], n)
+                     | (_quarter_turn(geometry[paired])
+                        & _quarter_turn(geometry[partner[paired]])))]
+    views = np.stack([first, partner[first]], axis=1)
+    views[np.isin(first, apart), 1] = -1
+    alone = np.stack([partner[apart], np.full(len(apart), -1)], axis=1)
+    return np.ascontiguousarray(np.concatenate([views, alone]),
+                                dtype=np.int32)
+
+
+def _quarter_turn(geometry):
+    """Per angle: the rotation is an exact multiple of a quarter turn."""
+    m = geometry[:, :4]
+    return np.all((m == 0) | (np.abs(m) == 1), axis=1)
+
+
+def _clear_of_boundary(geometry, n):
+    """Per angle: no output (oz, ox) of the n x n plane has a coordinate
+    within 1e-9 of 0 or n-1."""
+    m = geometry[:, :4]
+    oz = np.arange(n)
+    clear = np.ones(geometry.shape[0], dtype=bool)
+    for axis in (0, 1):
+        m1 = m[:, 2 * axis + 1, None]
+        base = geometry[:, 4 + axis, None] + m[:, 2 * axis, None] * oz
+        inv = 1 / np.where(m1 == 0, 1e-300, m1)
+        for edge in (0.0, n - 1.0):
+            # the row's distance to the edge at the integer ox nearest to
+            # its crossing
+            d = edge - base
+            ox = d * inv
+            np.rint(ox, out=ox)
+            np.clip(ox, 0, n - 1, out=ox)
+            ox *= m1
+            d -= ox
+            clear &= np.abs(d, out=d).min(axis=1) > 1e-9
+    return clear
+
+
 # ------------------------------------------------------------- tilted path
 def norm_vec(vector):
     """Unit vector along ``vector`` (length-3)."""

@@ -36,6 +36,10 @@ EXPORTED_SYMBOLS = (
     "odt_bpp3d_launch_count",
     "odt_bpp3d_execute_noalloc",
     "odt_bpp3d_execute_gain",
+    "odt_bpp3d_pair_workspace_size",
+    "odt_bpp3d_execute_pairs",
+    "odt_bpp3d_adjoint_pairs",
+    "odt_bpp3d_pair_launch_count",
     "odt_bpp3d_adjoint_workspace_size",
     "odt_bpp3d_adjoint",
     "odt_bpp3d_read_status",
@@ -95,6 +99,12 @@ class Bpp3dDesc(ctypes.Structure):
         ("workspace_limit", ctypes.c_uint64),
         ("z_shift", ctypes.c_double),
     ]
+
+
+class Bpp3dUnits(ctypes.Structure):
+    """odt_bpp3d_units: units of opposite views (device pointers)."""
+    _fields_ = [("num_units", ctypes.c_int32), ("reserved", ctypes.c_int32),
+                ("views", ctypes.c_void_p), ("geometry", ctypes.c_void_p)]
 
 
 class MlpParams(ctypes.Structure):
@@ -201,6 +211,16 @@ def lib():
         L.odt_bpp3d_execute_noalloc.argtypes = [vp, vp, vp, vp, vp, vp]
         L.odt_bpp3d_execute_gain.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp,
                                              vp]
+        L.odt_bpp3d_pair_workspace_size.argtypes = [
+            vp, ctypes.c_int32, ctypes.POINTER(ctypes.c_uint64),
+            ctypes.POINTER(ctypes.c_uint64)]
+        L.odt_bpp3d_execute_pairs.argtypes = [
+            vp, ctypes.POINTER(Bpp3dUnits)] + [vp] * 7 + [
+                ctypes.POINTER(StageTiming)]
+        L.odt_bpp3d_adjoint_pairs.argtypes = [
+            vp, ctypes.POINTER(Bpp3dUnits)] + [vp] * 10
+        L.odt_bpp3d_pair_launch_count.argtypes = [
+            vp, ctypes.c_int32, ctypes.POINTER(ctypes.c_int64)]
         L.odt_bpp3d_adjoint_workspace_size.argtypes = [
             vp, ctypes.POINTER(ctypes.c_uint64)]
         L.odt_bpp3d_adjoint.argtypes = [vp] * 12
@@ -249,6 +269,9 @@ def lib():
                      "odt_bpp3d_angle_batch", "odt_bpp3d_execute",
                      "odt_bpp3d_execute_timed", "odt_bpp3d_launch_count",
                      "odt_bpp3d_execute_noalloc", "odt_bpp3d_execute_gain",
+                     "odt_bpp3d_pair_workspace_size",
+                     "odt_bpp3d_execute_pairs", "odt_bpp3d_adjoint_pairs",
+                     "odt_bpp3d_pair_launch_count",
                      "odt_bpp3d_adjoint_workspace_size", "odt_bpp3d_adjoint",
                      "odt_bpp3d_read_status", "odt_bpp3d_plan_destroy",
                      "odt_mlp_gain_forward", "odt_mlp_store_size",
@@ -357,6 +380,44 @@ class Plan:
                                           vgrad_ptr, sgrad_ptr, ggrad_ptr,
                                           aggrad_ptr, workspace_ptr,
                                           stream_handle))
+
+    def pair_workspace_bytes(self, num_units):
+        """(workspace, adjoint workspace) bytes of an execution over
+        `num_units` units of opposite views, or None if the plan cannot pair
+        views (its tables, or a workspace limit too small)."""
+        ws, adj = ctypes.c_uint64(), ctypes.c_uint64()
+        st = lib().odt_bpp3d_pair_workspace_size(
+            self._h, int(num_units), ctypes.byref(ws), ctypes.byref(adj))
+        if st == ODT_ERR_UNSUPPORTED:
+            return None
+        check(st)
+        return int(ws.value), int(adj.value)
+
+    def pair_launches(self, num_units):
+        n = ctypes.c_int64()
+        check(lib().odt_bpp3d_pair_launch_count(self._h, int(num_units),
+                                                ctypes.byref(n)))
+        return int(n.value)
+
+    def execute_pairs(self, units, sino_ptr, weights_ptr, gain_ptr,
+                      again_ptr, volume_ptr, workspace_ptr, stream_handle,
+                      timed=False):
+        t = StageTiming() if timed else None
+        with self._lock:
+            check(lib().odt_bpp3d_execute_pairs(
+                self._h, ctypes.byref(units), sino_ptr, weights_ptr,
+                gain_ptr, again_ptr, volume_ptr, workspace_ptr,
+                stream_handle, ctypes.byref(t) if timed else None))
+        return t.as_dict() if timed else None
+
+    def adjoint_pairs(self, units, sino_ptr, weights_ptr, gain_ptr,
+                      again_ptr, vgrad_ptr, sgrad_ptr, ggrad_ptr, aggrad_ptr,
+                      workspace_ptr, stream_handle):
+        with self._lock:
+            check(lib().odt_bpp3d_adjoint_pairs(
+                self._h, ctypes.byref(units), sino_ptr, weights_ptr,
+                gain_ptr, again_ptr, vgrad_ptr, sgrad_ptr, ggrad_ptr,
+                aggrad_ptr, workspace_ptr, stream_handle))
 
     def read_status(self, stream_handle):
         check(lib().odt_bpp3d_read_status(self._h, stream_handle))

@@ -19,6 +19,13 @@
 // FFT and vice versa; the transpose of the x-prefilter boundary terms
 // collects two weighted sums of the cotangent and scatters them onto the
 // four samples outside the crop.
+//
+// Opposite views (units of two angles, see stages.cu): both views' spectra
+// take their gradient from the shared slab's Z_p, the second one against the
+// propagator of its own plane nz-1-p,
+//   conj(e^(i w (c - z_p))) Z_p = conj(e^(i w c)) e^(i w z_p) Z_p,  c = 2 zshift - 1,
+// so one propagator recurrence serves both and the constant factor is applied
+// when the sum is complete.  The second view's row gradients are mirrored.
 #include "odt_fft.cuh"
 #include "odt_internal.cuh"
 #include "odt_stage_util.cuh"
@@ -116,8 +123,8 @@ __global__ void __launch_bounds__(LPC * L::TPL) k_adj_rows(StageParams P, L line
 }
 
 // Columns: forward FFT along y of the zero-padded cotangent column of every
-// plane, accumulated against the conjugate propagator into Qg[a][ky][kx].
-template <class L, int KX>
+// plane, accumulated against the conjugate propagator into Qg[slot][ky][kx].
+template <class L, int KX, bool PAIR>
 __global__ void __launch_bounds__(KX * L::TPL) k_adj_columns(StageParams P, L line, const float2 *Tg, float2 *Qg,
                                                              int q0, int qn, int ppc)
 {
@@ -146,6 +153,8 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_columns(StageParams P, L li
     const bool pf = P.order >= 2;
     __syncthreads();
     float2 E[L::SLOTS], Q[L::SLOTS];
+    float2 R[PAIR ? L::SLOTS : 1];  // the opposite view's sum, without its constant factor
+    const float copp = 2.f * P.zshift - 1.f;
     int flip = 0;
     int cur_a = -1;
     auto flush = [&](int a) {
@@ -153,9 +162,15 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_columns(StageParams P, L li
         for (int r = 0; r < L::SLOTS; ++r) {
             const int ky = j + r * L::TPL;
             if (colok && ky < n) {
-                float2 *d = Qg + ((size_t)a * n + ky) * lNx + kx;
+                float2 *d = Qg + ((size_t)(PAIR ? 2 * a : a) * n + ky) * lNx + kx;
                 atomicAdd(&d->x, Q[r].x);
                 atomicAdd(&d->y, Q[r].y);
+                if (PAIR) {
+                    d += (size_t)n * lNx;
+                    const float2 o = cmul_conj(R[r], expi_phase(P.tab.wsplit[(size_t)ky * lNx + kx], copp));
+                    atomicAdd(&d->x, o.x);
+                    atomicAdd(&d->y, o.y);
+                }
             }
         }
     };
@@ -173,6 +188,8 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_columns(StageParams P, L li
             for (int r = 0; r < L::SLOTS; ++r) {
                 const int ky = j + r * L::TPL;
                 Q[r] = make_float2(0.f, 0.f);
+                if (PAIR)
+                    R[r] = make_float2(0.f, 0.f);
                 if (colok && ky < n) {
                     const size_t k = (size_t)ky * lNx + kx;
                     E[r] = expi_phase(P.tab.wsplit[k], zp);
@@ -261,8 +278,18 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_columns(StageParams P, L li
                 }
                 cz.x = fmaf(b.x, v[r].x, fmaf(b.y, v[r].y, cz.x));
                 cz.y = fmaf(b.x, v[r].y, fmaf(-b.y, v[r].x, cz.y));
+                if (PAIR) {
+                    // the opposite view's terms, alpha and beta exchanged
+                    const float2 al = P.tab.alpha[k], be = P.tab.beta[k];
+                    b = make_float2(fmaf(zh, al.x, zl * be.x), fmaf(zh, al.y, zl * be.y));
+                    b = cmul_conj(b, expi_phase(P.tab.wsplit[k], copp));
+                    R[r].x = fmaf(b.x, v[r].x, fmaf(b.y, v[r].y, R[r].x));
+                    R[r].y = fmaf(b.x, v[r].y, fmaf(-b.y, v[r].x, R[r].y));
+                }
             }
             Q[r] = Q[r] + cz;
+            if (PAIR)
+                R[r] = cfma(e, v[r], R[r]);
             if (ky < n)
                 E[r] = cmul(E[r], stp[ky * KX + c]);
         }
@@ -289,7 +316,17 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_spectrum(StageParams P, L l
     const int kx = blockIdx.x * KX + c;
     const bool colok = kx < P.lNx;
     const int lNx = P.lNx;
-    const int a = blockIdx.y;
+    const int sl = blockIdx.y;  // spectrum slot
+    int a = sl;
+    bool mirrored = false;
+    if (P.units) {
+        const int2 u = P.units[sl >> 1];
+        mirrored = sl & 1;
+        a = mirrored ? u.y : u.x;
+        if (a < 0)
+            return;  // no opposite view (uniform over the CTA)
+    }
+    const int kg = (mirrored && kx) ? lNx - kx : kx;  // the gains' column
     __syncthreads();
     int flip = 0;
     float2 X[L::SLOTS];
@@ -298,7 +335,7 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_spectrum(StageParams P, L l
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
             const int ky = j + r * L::TPL;
-            X[r] = (colok && ky < n) ? rowspec[((size_t)a * n + ky) * lNx + kx] : make_float2(0.f, 0.f);
+            X[r] = (colok && ky < n) ? rowspec[((size_t)sl * n + ky) * lNx + kx] : make_float2(0.f, 0.f);
         }
         line.template run<-1, true>(X, j, buf0 + c, buf1 + c, KX, tw, flip);
     }
@@ -309,15 +346,16 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_spectrum(StageParams P, L l
         v[r] = make_float2(0.f, 0.f);
         if (colok && ky < n) {
             const size_t k = (size_t)ky * lNx + kx;
-            const float2 q = Qg[((size_t)a * n + ky) * lNx + kx];
+            const float2 q = Qg[((size_t)sl * n + ky) * lNx + kx];
             const float2 G = P.tab.G[k];
-            const float gk = P.gain ? P.gain[k] : 1.f;
-            const size_t ak = (size_t)a * n * lNx + k;
+            const size_t gk0 = (size_t)ky * lNx + kg;
+            const float gk = P.gain ? P.gain[gk0] : 1.f;
+            const size_t ak = (size_t)a * n * lNx + gk0;
             const float2 ga = P.again ? P.again[ak] : make_float2(1.f, 0.f);
             if (dgain) {
                 // d/dg of G g ga X: Re(conj(G ga X) q)
                 const float2 gx = cmul(cmul(G, ga), X[r]);
-                atomicAdd(dgain + k, gx.x * q.x + gx.y * q.y);
+                atomicAdd(dgain + gk0, gx.x * q.x + gx.y * q.y);
             }
             if (dagain) {
                 // d/d(ga) of G g ga X: conj(G g X) q
@@ -336,14 +374,14 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_spectrum(StageParams P, L l
     for (int r = 0; r < L::SLOTS; ++r) {
         const int ky = j + r * L::TPL;
         if (ky < n)
-            W[((size_t)a * n + ky) * lNx + kx] = v[r];
+            W[((size_t)sl * n + ky) * lNx + kx] = v[r];
     }
 }
 
 // Rows: full backward FFT along x of W -> the cotangent of the padded plane.
 template <class L, int LPC>
 __global__ void __launch_bounds__(LPC * L::TPL) k_adj_rows_full(StageParams P, L line, const float2 *W, float2 *Pg,
-                                                                int nb)
+                                                                int nslots)
 {
     extern __shared__ float2 smem[];
     const int n = line.size();  // lNx
@@ -352,7 +390,7 @@ __global__ void __launch_bounds__(LPC * L::TPL) k_adj_rows_full(StageParams P, L
     copy_twiddles<L>(tw, P.tab.twx, n);
     const int l = threadIdx.x / L::TPL, j = threadIdx.x % L::TPL;
     const long long lid = (long long)blockIdx.x * LPC + l;
-    const bool valid = lid < (long long)nb * P.lNy;
+    const bool valid = lid < (long long)nslots * P.lNy;
     const float2 *src = W + (size_t)(valid ? lid : 0) * n;
     float2 v[L::SLOTS];
 #pragma unroll
@@ -397,19 +435,33 @@ __device__ __forceinline__ void pad_transpose_axis(const PadAxis &ax, int i, F &
     }
 }
 
-__global__ void k_adj_pad(StageParams P, const float2 *Pg, const double *weights, int nb, float2 *dsino)
+__global__ void k_adj_pad(StageParams P, const float2 *Pg, const double *weights, int nslots, float2 *dsino)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
-    const int a = blockIdx.z;
-    if (x >= P.nx || a >= nb)
+    const int sl = blockIdx.z;  // spectrum slot
+    if (x >= P.nx || sl >= nslots)
         return;
+    int a = sl;
+    bool mirrored = false;
+    if (P.units) {
+        const int2 u = P.units[sl >> 1];
+        mirrored = sl & 1;
+        a = mirrored ? u.y : u.x;
+        if (a < 0)
+            return;
+    }
     const PadAxis ay{P.ny, P.padyl, P.lNy - P.ny - P.padyl, P.pad_mode};
     const PadAxis axx{P.nx, P.padxl, P.lNx - P.nx - P.padxl, P.pad_mode};
-    const float2 *plane = Pg + (size_t)a * P.lNy * P.lNx;
+    const float2 *plane = Pg + (size_t)sl * P.lNy * P.lNx;
     float2 acc = make_float2(0.f, 0.f);
     pad_transpose_axis(ay, y, [&](int Y, float cy) {
         pad_transpose_axis(axx, x, [&](int X, float cx) {
+            if (mirrored) {
+                X = 2 * P.padxl + P.nx - 1 - X;
+                X += X < 0 ? P.lNx : 0;
+                X -= X >= P.lNx ? P.lNx : 0;
+            }
             const float2 g = plane[(size_t)Y * P.lNx + X];
             const float cc = cy * cx;
             acc.x = fmaf(cc, g.x, acc.x);
@@ -449,7 +501,11 @@ static cudaError_t set_adj_attrs(int n)
                              (int)smem_adj_rows<L>(n));
     if (e != cudaSuccess)
         return e;
-    e = cudaFuncSetAttribute(k_adj_columns<L, Cfg<L>::KX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_adj_columns<L, Cfg<L>::KX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem_adj_cols<L>(n));
+    if (e != cudaSuccess)
+        return e;
+    e = cudaFuncSetAttribute(k_adj_columns<L, Cfg<L>::KX, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem_adj_cols<L>(n));
     if (e != cudaSuccess)
         return e;
@@ -483,42 +539,46 @@ cudaError_t launch_adj_columns(const StageParams &P, const float2 *Tg, float2 *Q
         using L = decltype(line);
         constexpr int KX = Cfg<L>::KX;
         dim3 grid((P.lNx + KX - 1) / KX, (qn + kAdjPlanesPerBlock - 1) / kAdjPlanesPerBlock);
-        k_adj_columns<L, KX><<<grid, KX * L::TPL, smem_adj_cols<L>(line.n), s>>>(P, line, Tg, Qg, q0, qn,
-                                                                                kAdjPlanesPerBlock);
+        if (P.units)
+            k_adj_columns<L, KX, true>
+                <<<grid, KX * L::TPL, smem_adj_cols<L>(line.n), s>>>(P, line, Tg, Qg, q0, qn, kAdjPlanesPerBlock);
+        else
+            k_adj_columns<L, KX, false>
+                <<<grid, KX * L::TPL, smem_adj_cols<L>(line.n), s>>>(P, line, Tg, Qg, q0, qn, kAdjPlanesPerBlock);
         return cudaGetLastError();
     });
 }
 
 cudaError_t launch_adj_spectrum(const StageParams &P, const float2 *rowspec, const float2 *Qg, float *dgain,
-                                float2 *dagain, float2 *W, int nb, cudaStream_t s)
+                                float2 *dagain, float2 *W, int nslots, cudaStream_t s)
 {
     return with_line(P.lNy, [&](auto line) {
         using L = decltype(line);
         constexpr int KX = Cfg<L>::KX;
-        dim3 grid((P.lNx + KX - 1) / KX, nb);
+        dim3 grid((P.lNx + KX - 1) / KX, nslots);
         k_adj_spectrum<L, KX><<<grid, KX * L::TPL, smem_adj_cols<L>(line.n), s>>>(P, line, rowspec, Qg, dgain,
                                                                                  dagain, W);
         return cudaGetLastError();
     });
 }
 
-cudaError_t launch_adj_rows_full(const StageParams &P, const float2 *W, float2 *Pg, int nb, cudaStream_t s)
+cudaError_t launch_adj_rows_full(const StageParams &P, const float2 *W, float2 *Pg, int nslots, cudaStream_t s)
 {
     return with_line(P.lNx, [&](auto line) {
         using L = decltype(line);
         constexpr int LPC = Cfg<L>::LPC;
-        const long long lines = (long long)nb * P.lNy;
+        const long long lines = (long long)nslots * P.lNy;
         k_adj_rows_full<L, LPC><<<(unsigned)((lines + LPC - 1) / LPC), LPC * L::TPL, smem_adj_rows<L>(line.n),
-                                  s>>>(P, line, W, Pg, nb);
+                                  s>>>(P, line, W, Pg, nslots);
         return cudaGetLastError();
     });
 }
 
-cudaError_t launch_adj_pad(const StageParams &P, const float2 *Pg, const double *weights, int nb, float2 *dsino,
+cudaError_t launch_adj_pad(const StageParams &P, const float2 *Pg, const double *weights, int nslots, float2 *dsino,
                            cudaStream_t s)
 {
-    dim3 grid((P.nx + 127) / 128, P.ny, nb);
-    k_adj_pad<<<grid, 128, 0, s>>>(P, Pg, weights, nb, dsino);
+    dim3 grid((P.nx + 127) / 128, P.ny, nslots);
+    k_adj_pad<<<grid, 128, 0, s>>>(P, Pg, weights, nslots, dsino);
     return cudaGetLastError();
 }
 

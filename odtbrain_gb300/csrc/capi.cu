@@ -206,15 +206,24 @@ int odt::set_error(int status, const char *msg)
     return (int)fail((odt_status)status, msg ? msg : "");
 }
 
+namespace {
+// Batching and workspace of an execution over `units` slabs.
+struct Layout {
+    int units, batch;  // slabs (angles, or units of opposite views), slabs per batch
+    int spu;           // spectrum slots per slab: 1, or 2 with opposite views
+    int jobs;          // (slab, plane) jobs per column/row launch
+    size_t off_rowspec, off_T, off_T2, off_Tab, off_slab, off_comp, off_rot, ws_bytes;
+    size_t off_Qg, off_W, off_Pg, off_vT, adj_ws_bytes;  // adjoint-only regions after ws_bytes
+};
+}  // namespace
+
 struct odt_bpp3d_plan {
     odt_bpp3d_desc d;
     int device;      // CUDA device the tables, events and stream belong to
     int nz;
-    int batch;       // angles per batch
-    int jobs;        // (angle, plane) jobs per column/row launch
     int ydefer;      // the row stage adds the y-prefilter terms (StageParams::ydefer)
-    size_t off_rowspec, off_T, off_T2, off_Tab, off_slab, off_comp, off_rot, ws_bytes;
-    size_t off_Qg, off_W, off_Pg, off_vT, adj_ws_bytes;  // adjoint-only regions after ws_bytes
+    int even;        // filter and propagator phase are even in kx (opposite views can be paired)
+    Layout lay;      // one angle per slab
     double bx_ca, bx_cb, by_ca, by_cb;  // one-pole solve in the adjoint's form
     int npoles;                         // prefilter poles: 0, 1 or 2
     float kx_solve[16], ky_solve[16];   // boundary_matrix of x and y lines
@@ -296,8 +305,99 @@ StageParams stage_params(const odt_bpp3d_plan *p)
     P.again = nullptr;
     P.status = p->d_status;
     P.ydefer = p->ydefer;
-    P.yedge_off = p->ydefer ? (long long)p->jobs * d.ny * d.pad_nx : 0;
+    P.units = nullptr;
+    P.yedge_off = p->ydefer ? (long long)p->lay.jobs * d.ny * d.pad_nx : 0;
     return P;
+}
+
+// The largest batch of slabs (and column-stage chunk) whose workspace fits
+// the plan's limit; one slab per batch with a shrunken chunk where none does.
+Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
+{
+    const odt_bpp3d_desc &d = p->d;
+    const int lNy = d.pad_ny, lNx = d.pad_nx, nz = p->nz, np = p->npoles;
+    const bool tilted = d.geometry == ODT_GEOM_AFFINE3D;
+    const size_t plane_row_bytes = (size_t)d.ny * lNx * 8;           // one job's column-stage output
+    const size_t edge_row_bytes = p->ydefer ? (size_t)4 * np * lNx * 8 : 0;  // its y-prefilter edge samples
+    // one coefficient slab [z][x][ypitch] (the adjoint's slab gradients
+    // [y][z][x] fit too)
+    const size_t slab_bytes = (size_t)nz * odt::yaxis_slab_pitch(d.ny) * d.nx * 8;
+    const size_t rowspec_bytes = (size_t)spu * lNy * lNx * 8;        // one slab's row spectra
+    const size_t tab_bytes = np ? (size_t)2 * np * d.ny * lNx * 8 : 0;  // one slab's z-boundary rows
+    const size_t vol_bytes = (size_t)nz * d.ny * d.nx * 8;           // compensation buffer
+    const uint64_t limit = d.workspace_limit ? d.workspace_limit : kDefaultWorkspace;
+    // chunk buffers take at most a quarter of the limit, so tight limits
+    // (save_memory) keep room for a batch of slabs
+    const uint64_t plane_budget = std::min<uint64_t>(kPlaneBudget, limit / 4);
+    // and at most 1024 planes (where the gain levels off), so small planes do
+    // not take memory for nothing
+    const size_t jobs_cap = std::max<size_t>(16, std::min<size_t>(1024, plane_budget / 2 / plane_row_bytes));
+    auto layout = [&](int batch, size_t jobs) -> Layout {
+        Layout y{};
+        y.units = units;
+        y.batch = batch;
+        y.spu = spu;
+        y.jobs = (int)jobs;
+        const int nbatches = (units + batch - 1) / batch;
+        size_t w = 0;
+        y.off_rowspec = w; w = align_up(w + (size_t)batch * rowspec_bytes);
+        y.off_T = w; w = align_up(w + jobs * (plane_row_bytes + edge_row_bytes));
+        y.off_T2 = w; w = align_up(w + jobs * (plane_row_bytes + edge_row_bytes));
+        y.off_Tab = w; w = align_up(w + (size_t)batch * tab_bytes);
+        y.off_slab = w; w = align_up(w + (size_t)batch * slab_bytes);
+        y.off_comp = w; w = align_up(w + (nbatches > 1 ? vol_bytes : 0));
+        y.off_rot = w;
+        w = align_up(w + odt::rotate_scratch_bytes(batch, d.ny, d.nx, nz, tilted ? 1 : 0));
+        y.ws_bytes = w;
+        const size_t spec_b = (size_t)batch * rowspec_bytes;
+        y.off_Qg = w; w = align_up(w + spec_b);
+        y.off_W = w; w = align_up(w + spec_b);
+        y.off_Pg = w; w = align_up(w + spec_b);
+        // the volume gradient in the [z][x][y] order (y-axis adjoint)
+        y.off_vT = w; w = align_up(w + vol_bytes);
+        y.adj_ws_bytes = w;
+        return y;
+    };
+    auto jobs_for = [&](int batch) {
+        size_t jobs = std::min((size_t)batch * nz, jobs_cap);
+        return jobs >= 16 ? jobs / 16 * 16 : jobs;
+    };
+    int best = 0;
+    for (int lo = 1, hi = units; lo <= hi;) {  // ws grows with the batch
+        const int mid = lo + (hi - lo) / 2;
+        if (layout(mid, jobs_for(mid)).ws_bytes <= limit) {
+            best = mid;
+            lo = mid + 1;
+        } else {
+            hi = mid - 1;
+        }
+    }
+    // a single batch needs no compensation buffer, so it can fit when a
+    // slightly smaller batch does not
+    if (best < units && layout(units, jobs_for(units)).ws_bytes <= limit)
+        best = units;
+    if (best > 0)
+        return layout(best, jobs_for(best));
+    // one slab per batch; shrink the column-stage chunk toward the limit
+    size_t jobs = jobs_for(1);
+    while (jobs > 1 && layout(1, jobs).ws_bytes > limit)
+        jobs = jobs > 16 ? jobs - 16 : jobs - 1;
+    return layout(1, jobs);
+}
+
+// The layout of an execution over units of opposite views; an error when the
+// plan cannot pair views.
+odt_status pair_layout(const odt_bpp3d_plan *plan, int num_units, Layout *y)
+{
+    if (!plan->even)
+        return fail(ODT_ERR_UNSUPPORTED, "opposite views need the rotation about y and tables even in kx");
+    if (num_units < 1 || num_units > plan->d.num_angles)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "need 1 <= num_units <= num_angles");
+    *y = make_layout(plan, num_units, 2);
+    const uint64_t limit = plan->d.workspace_limit ? plan->d.workspace_limit : kDefaultWorkspace;
+    if (y->ws_bytes > limit)
+        return fail(ODT_ERR_UNSUPPORTED, "the workspace limit holds no unit of opposite views");
+    return ODT_OK;
 }
 
 odt_status validate(const odt_bpp3d_desc *d)
@@ -544,95 +644,29 @@ odt_status odt_bpp3d_plan_create(const odt_bpp3d_desc *desc, odt_bpp3d_plan **ou
     p->tab.zpow = (const float *)(base + oZ);
     p->d_status = (int *)(base + oSt);
 
-    // ---- batching: the largest angle batch (and column-stage chunk) whose
-    // workspace fits the limit
     // tilted path, order >= 2: the column stage leaves the y-prefilter
     // terms to the row stage and stores each job's raw edge samples (4 np
     // rows) after the chunk's jobs
-    p->jobs = 0;
+    p->lay = Layout{};
     p->ydefer = 0;
     {
         const StageParams G = stage_params(p);
         p->ydefer = (tilted && pf && !odt::single_row_plan(G)) ? 1 : 0;
     }
-    const size_t plane_row_bytes = (size_t)d.ny * lNx * 8;           // one job's column-stage output
-    const size_t edge_row_bytes = p->ydefer ? (size_t)4 * np * lNx * 8 : 0;  // its y-prefilter edge samples
-    // one angle's coefficient slab [z][x][ypitch] (the adjoint's slab
-    // gradients [y][z][x] fit too)
-    const size_t slab_bytes = (size_t)nz * odt::yaxis_slab_pitch(d.ny) * d.nx * 8;
-    const size_t rowspec_bytes = (size_t)lNy * lNx * 8;              // one angle's row spectra
-    const size_t tab_bytes = pf ? (size_t)2 * np * d.ny * lNx * 8 : 0;  // one angle's z-boundary rows
-    const size_t vol_bytes = (size_t)nz * d.ny * d.nx * 8;           // compensation buffer
-    const uint64_t limit = d.workspace_limit ? d.workspace_limit : kDefaultWorkspace;
-    // chunk buffers take at most a quarter of the limit, so tight limits
-    // (save_memory) keep room for a batch of angles
-    const uint64_t plane_budget = std::min<uint64_t>(kPlaneBudget, limit / 4);
-    // and at most 1024 planes (where the gain levels off), so small planes do
-    // not take memory for nothing
-    const size_t jobs_cap = std::max<size_t>(16, std::min<size_t>(1024, plane_budget / 2 / plane_row_bytes));
-    auto layout = [&](int batch, size_t jobs, bool commit) -> size_t {
-        const int nbatches = (d.num_angles + batch - 1) / batch;
-        size_t w = 0;
-        const size_t o_rowspec = w; w = align_up(w + (size_t)batch * rowspec_bytes);
-        const size_t o_T = w; w = align_up(w + jobs * (plane_row_bytes + edge_row_bytes));
-        const size_t o_T2 = w; w = align_up(w + jobs * (plane_row_bytes + edge_row_bytes));
-        const size_t o_Tab = w; w = align_up(w + (size_t)batch * tab_bytes);
-        const size_t o_slab = w; w = align_up(w + (size_t)batch * slab_bytes);
-        const size_t o_comp = w; w = align_up(w + (nbatches > 1 ? vol_bytes : 0));
-        const size_t o_rot = w;
-        w = align_up(w + odt::rotate_scratch_bytes(batch, d.ny, d.nx, nz, tilted ? 1 : 0));
-        if (commit) {
-            p->batch = batch;
-            p->jobs = (int)jobs;
-            p->off_rowspec = o_rowspec;
-            p->off_T = o_T;
-            p->off_T2 = o_T2;
-            p->off_Tab = o_Tab;
-            p->off_slab = o_slab;
-            p->off_comp = o_comp;
-            p->off_rot = o_rot;
-            p->ws_bytes = w;
-        }
-        return w;
-    };
-    auto jobs_for = [&](int batch) {
-        size_t jobs = std::min((size_t)batch * nz, jobs_cap);
-        return jobs >= 16 ? jobs / 16 * 16 : jobs;
-    };
-    int best = 0;
-    for (int lo = 1, hi = d.num_angles; lo <= hi;) {  // ws grows with the batch
-        const int mid = lo + (hi - lo) / 2;
-        if (layout(mid, jobs_for(mid), false) <= limit) {
-            best = mid;
-            lo = mid + 1;
-        } else {
-            hi = mid - 1;
-        }
-    }
-    // a single batch needs no compensation buffer, so it can fit when a
-    // slightly smaller batch does not
-    if (best < d.num_angles && layout(d.num_angles, jobs_for(d.num_angles), false) <= limit)
-        best = d.num_angles;
-    if (best > 0) {
-        layout(best, jobs_for(best), true);
-    } else {
-        // one angle per batch; shrink the column-stage chunk toward the limit
-        size_t jobs = jobs_for(1);
-        while (jobs > 1 && layout(1, jobs, false) > limit)
-            jobs = jobs > 16 ? jobs - 16 : jobs - 1;
-        layout(1, jobs, true);
-    }
+    p->lay = make_layout(p, d.num_angles, 1);
 
-    {
-        const size_t spec_b = (size_t)p->batch * lNy * lNx * 8;
-        size_t w = p->ws_bytes;
-        p->off_Qg = w; w = align_up(w + spec_b);
-        p->off_W = w; w = align_up(w + spec_b);
-        p->off_Pg = w; w = align_up(w + spec_b);
-        // the volume gradient in the [z][x][y] order (y-axis adjoint)
-        p->off_vT = w; w = align_up(w + (size_t)nz * d.ny * d.nx * 8);
-        p->adj_ws_bytes = w;
-    }
+    // opposite views share a slab through the mirrored spectrum, which needs
+    // tables even in kx (true of the reference's filters about y)
+    p->even = tilted ? 0 : 1;
+    for (int ky = 0; p->even && ky < lNy; ++ky)
+        for (int kx = 1; kx < lNx - kx; ++kx) {
+            const size_t k = (size_t)ky * lNx + kx, m = (size_t)ky * lNx + (lNx - kx);
+            if (desc->kz_phase[k] != desc->kz_phase[m] || desc->filter[2 * k] != desc->filter[2 * m] ||
+                desc->filter[2 * k + 1] != desc->filter[2 * m + 1]) {
+                p->even = 0;
+                break;
+            }
+        }
 
     p->col_slots = 0;
     StageParams P = stage_params(p);
@@ -667,7 +701,7 @@ odt_status odt_bpp3d_workspace_size(const odt_bpp3d_plan *plan, uint64_t *bytes)
 {
     if (!plan || !bytes)
         return fail(ODT_ERR_INVALID_ARGUMENT, "NULL argument");
-    *bytes = plan->ws_bytes;
+    *bytes = plan->lay.ws_bytes;
     return ODT_OK;
 }
 
@@ -675,7 +709,7 @@ odt_status odt_bpp3d_angle_batch(const odt_bpp3d_plan *plan, int32_t *batch)
 {
     if (!plan || !batch)
         return fail(ODT_ERR_INVALID_ARGUMENT, "NULL argument");
-    *batch = plan->batch;
+    *batch = plan->lay.batch;
     return ODT_OK;
 }
 
@@ -725,11 +759,13 @@ struct LaunchTimer {
     }
 };
 
-odt_status run_plan(const odt_bpp3d_plan *plan, const void *sino, const double *weights, const double *geometry,
-                    const float *gain, const void *again, void *volume, void *workspace, void *stream,
-                    odt_stage_timing *timing)
+// One execution: `units` NULL is one angle per slab (geometry per angle),
+// otherwise the device list of opposite views with one geometry per unit.
+odt_status run_plan(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *units, const void *sino,
+                    const double *weights, const double *geometry, const float *gain, const void *again,
+                    void *volume, void *workspace, void *stream, odt_stage_timing *timing)
 {
-    if (!plan || !sino || !geometry || !volume || (!workspace && plan->ws_bytes))
+    if (!sino || !geometry || !volume || (!workspace && lay.ws_bytes))
         return fail(ODT_ERR_INVALID_ARGUMENT, "NULL pointer argument");
     if (((uintptr_t)workspace % kAlign) != 0)
         return fail(ODT_ERR_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
@@ -742,15 +778,15 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const void *sino, const double *
     P.gain = gain;
     const size_t spec_elems = (size_t)plan->d.pad_ny * plan->d.pad_nx;
     char *ws = (char *)workspace;
-    float2 *rowspec = (float2 *)(ws + plan->off_rowspec);
-    float2 *T = (float2 *)(ws + plan->off_T);
-    float2 *Tab = (float2 *)(ws + plan->off_Tab);
-    float2 *slab = (float2 *)(ws + plan->off_slab);
-    float2 *comp = (float2 *)(ws + plan->off_comp);
-    void *rot_scratch = ws + plan->off_rot;
+    float2 *rowspec = (float2 *)(ws + lay.off_rowspec);
+    float2 *T = (float2 *)(ws + lay.off_T);
+    float2 *Tab = (float2 *)(ws + lay.off_Tab);
+    float2 *slab = (float2 *)(ws + lay.off_slab);
+    float2 *comp = (float2 *)(ws + lay.off_comp);
+    void *rot_scratch = ws + lay.off_rot;
     const size_t in_elem = d.input_dtype == ODT_INPUT_C128 ? 16 : 8;
     const int geo_stride = d.geometry == ODT_GEOM_AFFINE3D ? 12 : 6;
-    const int nbatches = (d.num_angles + plan->batch - 1) / plan->batch;
+    const int nbatches = (lay.units + lay.batch - 1) / lay.batch;
     const double plane_in = (double)d.ny * d.nx, spec = (double)d.pad_ny * d.pad_nx;
     const double vol = (double)plan->nz * d.ny * d.nx;
     const double out_elem = d.onlyreal ? 4.0 : 8.0;
@@ -759,22 +795,29 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const void *sino, const double *
     LaunchTimer lt(timing, s);
     cudaError_t e;
     for (int b = 0; b < nbatches; ++b) {
-        const int a0 = b * plan->batch;
-        const int nb = std::min(plan->batch, d.num_angles - a0);
-        const char *sino_b = (const char *)sino + (size_t)a0 * d.ny * d.nx * in_elem;
-        P.again = again ? (const float2 *)again + (size_t)a0 * spec_elems : nullptr;
+        const int a0 = b * lay.batch;  // first slab of the batch
+        const int nb = std::min(lay.batch, lay.units - a0);
+        const int ns = nb * lay.spu;   // spectrum slots
+        const char *sino_b = (const char *)sino;
+        const double *w_b = weights;
+        if (units) {
+            P.units = units + a0;
+            P.again = (const float2 *)again;
+        } else {
+            sino_b += (size_t)a0 * d.ny * d.nx * in_elem;
+            w_b = weights ? weights + a0 : nullptr;
+            P.again = again ? (const float2 *)again + (size_t)a0 * spec_elems : nullptr;
+        }
         lt.begin(ODT_STAGE_ROWS_FORWARD);
-        e = odt::launch_rows_forward(P, sino_b, weights ? weights + a0 : nullptr, nb, rowspec, s);
+        e = odt::launch_rows_forward(P, sino_b, w_b, ns, rowspec, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "rows_forward launch");
-        lt.end(nb * (plane_in * in_elem + spec * 8.0));
-        if (d.intp_order >= 2) {
-            lt.begin(ODT_STAGE_COLUMNS_PROPAGATE);
-            e = odt::launch_columns_boundary(P, rowspec, Tab, nb, s);
-            if (e != cudaSuccess)
-                return cuda_fail(e, "columns_boundary launch");
-            lt.end(0.0);
-        }
+        lt.end(ns * (plane_in * in_elem + spec * 8.0));
+        lt.begin(ODT_STAGE_COLUMNS_PROPAGATE);
+        e = odt::launch_columns_spectrum(P, rowspec, Tab, nb, s);
+        if (e != cudaSuccess)
+            return cuda_fail(e, "columns_spectrum launch");
+        lt.end(0.0);
         const int total = nb * plan->nz;
         if (odt::single_row_plan(P)) {
             // single-row planes: the column stage is the identity and runs
@@ -783,16 +826,16 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const void *sino, const double *
             e = odt::launch_rows_line(P, rowspec, Tab, slab, 0, total, s);
             if (e != cudaSuccess)
                 return cuda_fail(e, "rows_line launch");
-            lt.end(nb * spec * 8.0 + (double)total * plane_in * 8.0);
+            lt.end(ns * spec * 8.0 + (double)total * plane_in * 8.0);
         } else if (timing) {
             // per-stage timing: the stages one after the other on one stream
-            for (int q0 = 0; q0 < total; q0 += plan->jobs) {
-                const int qn = std::min(plan->jobs, total - q0);
+            for (int q0 = 0; q0 < total; q0 += lay.jobs) {
+                const int qn = std::min(lay.jobs, total - q0);
                 lt.begin(ODT_STAGE_COLUMNS_PROPAGATE);
                 e = odt::launch_columns_propagate(P, rowspec, T, q0, qn, s);
                 if (e != cudaSuccess)
                     return cuda_fail(e, "columns_propagate launch");
-                lt.end((double)qn / plan->nz * spec * 8.0);
+                lt.end((double)qn / plan->nz * lay.spu * spec * 8.0);
                 lt.begin(ODT_STAGE_ROWS_INVERSE);
                 e = odt::launch_rows_inverse(P, T, Tab, slab, q0, qn, s);
                 if (e != cudaSuccess)
@@ -802,13 +845,13 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const void *sino, const double *
         } else {
             // chunk pipeline: columns(k) on s into buffer k%2 after rows(k-2)
             // released it; rows(k) on s2 after columns(k)
-            float2 *Tb[2] = {T, (float2 *)(ws + plan->off_T2)};
+            float2 *Tb[2] = {T, (float2 *)(ws + lay.off_T2)};
             cudaStream_t s2 = plan->s2;
             if ((e = cudaEventRecord(plan->ev_fork, s)) || (e = cudaStreamWaitEvent(s2, plan->ev_fork, 0)))
                 return cuda_fail(e, "stream fork");
             int k = 0;
-            for (int q0 = 0; q0 < total; q0 += plan->jobs, ++k) {
-                const int qn = std::min(plan->jobs, total - q0);
+            for (int q0 = 0; q0 < total; q0 += lay.jobs, ++k) {
+                const int qn = std::min(lay.jobs, total - q0);
                 const int buf = k & 1;
                 if (k >= 2 && (e = cudaStreamWaitEvent(s, plan->ev_row[buf], 0)))
                     return cuda_fail(e, "stream wait");
@@ -863,14 +906,49 @@ extern "C" {
 odt_status odt_bpp3d_execute(const odt_bpp3d_plan *plan, const void *sino, const double *weights,
                              const double *geometry, void *volume, void *workspace, void *stream)
 {
-    return run_plan(plan, sino, weights, geometry, nullptr, nullptr, volume, workspace, stream, nullptr);
+    if (!plan)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "NULL pointer argument");
+    return run_plan(plan, plan->lay, nullptr, sino, weights, geometry, nullptr, nullptr, volume, workspace, stream,
+                    nullptr);
 }
 
 odt_status odt_bpp3d_execute_gain(const odt_bpp3d_plan *plan, const void *sino, const double *weights,
                                   const double *geometry, const float *gain, const void *angle_gain,
                                   void *volume, void *workspace, void *stream)
 {
-    return run_plan(plan, sino, weights, geometry, gain, angle_gain, volume, workspace, stream, nullptr);
+    if (!plan)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "NULL pointer argument");
+    return run_plan(plan, plan->lay, nullptr, sino, weights, geometry, gain, angle_gain, volume, workspace, stream,
+                    nullptr);
+}
+
+odt_status odt_bpp3d_pair_workspace_size(const odt_bpp3d_plan *plan, int32_t num_units, uint64_t *bytes,
+                                         uint64_t *adjoint_bytes)
+{
+    if (!plan || !bytes)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "NULL argument");
+    Layout y;
+    const odt_status st = pair_layout(plan, num_units, &y);
+    if (st != ODT_OK)
+        return st;
+    *bytes = y.ws_bytes;
+    if (adjoint_bytes)
+        *adjoint_bytes = y.adj_ws_bytes;
+    return ODT_OK;
+}
+
+odt_status odt_bpp3d_execute_pairs(const odt_bpp3d_plan *plan, const odt_bpp3d_units *units, const void *sino,
+                                   const double *weights, const float *gain, const void *angle_gain, void *volume,
+                                   void *workspace, void *stream, odt_stage_timing *timing)
+{
+    if (!plan || !units || !units->views)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "NULL pointer argument");
+    Layout y;
+    const odt_status st = pair_layout(plan, units->num_units, &y);
+    if (st != ODT_OK)
+        return st;
+    return run_plan(plan, y, (const int2 *)units->views, sino, weights, units->geometry, gain, angle_gain, volume,
+                    workspace, stream, timing);
 }
 
 odt_status odt_bpp3d_adjoint_workspace_size(const odt_bpp3d_plan *plan, uint64_t *bytes)
@@ -879,16 +957,16 @@ odt_status odt_bpp3d_adjoint_workspace_size(const odt_bpp3d_plan *plan, uint64_t
         return fail(ODT_ERR_INVALID_ARGUMENT, "NULL argument");
     if (plan->d.intp_order > 3)
         return fail(ODT_ERR_UNSUPPORTED, "the adjoint is implemented for spline orders 0..3");
-    *bytes = plan->adj_ws_bytes;
+    *bytes = plan->lay.adj_ws_bytes;
     return ODT_OK;
 }
 
-odt_status odt_bpp3d_adjoint(const odt_bpp3d_plan *plan, const void *sino, const double *weights,
-                             const double *geometry, const float *gain, const void *angle_gain,
-                             const void *vol_grad, void *sino_grad, float *gain_grad, void *angle_gain_grad,
-                             void *workspace, void *stream)
+static odt_status run_adjoint(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *units, const void *sino,
+                              const double *weights, const double *geometry, const float *gain,
+                              const void *angle_gain, const void *vol_grad, void *sino_grad, float *gain_grad,
+                              void *angle_gain_grad, void *workspace, void *stream)
 {
-    if (!plan || !geometry || !vol_grad || !workspace)
+    if (!geometry || !vol_grad || !workspace)
         return fail(ODT_ERR_INVALID_ARGUMENT, "NULL pointer argument");
     if (!sino_grad && !gain_grad && !angle_gain_grad)
         return ODT_OK;
@@ -910,19 +988,19 @@ odt_status odt_bpp3d_adjoint(const odt_bpp3d_plan *plan, const void *sino, const
     StageParams P = stage_params(plan);
     P.gain = gain;
     char *ws = (char *)workspace;
-    float2 *rowspec = (float2 *)(ws + plan->off_rowspec);
-    float2 *T = (float2 *)(ws + plan->off_T);
-    float2 *slab = (float2 *)(ws + plan->off_slab);
-    float2 *Qg = (float2 *)(ws + plan->off_Qg);
-    float2 *W = (float2 *)(ws + plan->off_W);
-    float2 *Pg = (float2 *)(ws + plan->off_Pg);
+    float2 *rowspec = (float2 *)(ws + lay.off_rowspec);
+    float2 *T = (float2 *)(ws + lay.off_T);
+    float2 *slab = (float2 *)(ws + lay.off_slab);
+    float2 *Qg = (float2 *)(ws + lay.off_Qg);
+    float2 *W = (float2 *)(ws + lay.off_W);
+    float2 *Pg = (float2 *)(ws + lay.off_Pg);
     const size_t in_elem = d.input_dtype == ODT_INPUT_C128 ? 16 : 8;
     const size_t spec = (size_t)d.pad_ny * d.pad_nx;
-    const int nbatches = (d.num_angles + plan->batch - 1) / plan->batch;
+    const int nbatches = (lay.units + lay.batch - 1) / lay.batch;
     cudaError_t e;
     const float2 *vg = (const float2 *)vol_grad;
     if (!tilted) {
-        float2 *vT = (float2 *)(ws + plan->off_vT);
+        float2 *vT = (float2 *)(ws + lay.off_vT);
         e = odt::launch_volume_zxy(vg, vT, plan->nz, d.ny, d.nx, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "volume transpose launch");
@@ -934,8 +1012,11 @@ odt_status odt_bpp3d_adjoint(const odt_bpp3d_plan *plan, const void *sino, const
             return cuda_fail(e, "cudaMemsetAsync");
     }
     for (int b = 0; b < nbatches; ++b) {
-        const int a0 = b * plan->batch;
-        const int nb = std::min(plan->batch, d.num_angles - a0);
+        const int u0 = b * lay.batch;  // first slab of the batch
+        const int nb = std::min(lay.batch, lay.units - u0);
+        const int ns = nb * lay.spu;   // spectrum slots
+        const int a0 = units ? 0 : u0; // angle that the per-angle arrays start at
+        P.units = units ? units + u0 : nullptr;
         P.again = angle_gain ? (const float2 *)angle_gain + (size_t)a0 * spec : nullptr;
         RotParams R;
         R.ny = d.ny;
@@ -948,21 +1029,21 @@ odt_status odt_bpp3d_adjoint(const odt_bpp3d_plan *plan, const void *sino, const
         R.onlyreal = 0;
         R.status = plan->d_status;
         e = odt::launch_rotate_adjoint(R, d.intp_order, tilted ? 1 : 0, vg,
-                                       geometry + (size_t)a0 * geo_stride, slab, ws + plan->off_rot, s);
+                                       geometry + (size_t)u0 * geo_stride, slab, ws + lay.off_rot, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "rotate_adjoint launch");
         if (gain_grad || angle_gain_grad) {
             const char *sino_b = (const char *)sino + (size_t)a0 * d.ny * d.nx * in_elem;
-            e = odt::launch_rows_forward(P, sino_b, weights ? weights + a0 : nullptr, nb, rowspec, s);
+            e = odt::launch_rows_forward(P, sino_b, weights ? weights + a0 : nullptr, ns, rowspec, s);
             if (e != cudaSuccess)
                 return cuda_fail(e, "rows_forward launch");
         }
-        e = cudaMemsetAsync(Qg, 0, (size_t)nb * spec * sizeof(float2), s);
+        e = cudaMemsetAsync(Qg, 0, (size_t)ns * spec * sizeof(float2), s);
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaMemsetAsync");
         const int total = nb * plan->nz;
-        for (int q0 = 0; q0 < total; q0 += plan->jobs) {
-            const int qn = std::min(plan->jobs, total - q0);
+        for (int q0 = 0; q0 < total; q0 += lay.jobs) {
+            const int qn = std::min(lay.jobs, total - q0);
             e = odt::launch_adj_rows(P, slab, T, q0, qn, s);
             if (e != cudaSuccess)
                 return cuda_fail(e, "adj_rows launch");
@@ -972,14 +1053,14 @@ odt_status odt_bpp3d_adjoint(const odt_bpp3d_plan *plan, const void *sino, const
         }
         e = odt::launch_adj_spectrum(P, rowspec, Qg, gain_grad,
                                      angle_gain_grad ? (float2 *)angle_gain_grad + (size_t)a0 * spec : nullptr, W,
-                                     nb, s);
+                                     ns, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "adj_spectrum launch");
         if (sino_grad) {
-            e = odt::launch_adj_rows_full(P, W, Pg, nb, s);
+            e = odt::launch_adj_rows_full(P, W, Pg, ns, s);
             if (e != cudaSuccess)
                 return cuda_fail(e, "adj_rows_full launch");
-            e = odt::launch_adj_pad(P, Pg, weights ? weights + a0 : nullptr, nb,
+            e = odt::launch_adj_pad(P, Pg, weights ? weights + a0 : nullptr, ns,
                                     (float2 *)sino_grad + (size_t)a0 * d.ny * d.nx, s);
             if (e != cudaSuccess)
                 return cuda_fail(e, "adj_pad launch");
@@ -988,36 +1069,76 @@ odt_status odt_bpp3d_adjoint(const odt_bpp3d_plan *plan, const void *sino, const
     return ODT_OK;
 }
 
+odt_status odt_bpp3d_adjoint(const odt_bpp3d_plan *plan, const void *sino, const double *weights,
+                             const double *geometry, const float *gain, const void *angle_gain,
+                             const void *vol_grad, void *sino_grad, float *gain_grad, void *angle_gain_grad,
+                             void *workspace, void *stream)
+{
+    if (!plan)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "NULL pointer argument");
+    return run_adjoint(plan, plan->lay, nullptr, sino, weights, geometry, gain, angle_gain, vol_grad, sino_grad,
+                       gain_grad, angle_gain_grad, workspace, stream);
+}
+
+odt_status odt_bpp3d_adjoint_pairs(const odt_bpp3d_plan *plan, const odt_bpp3d_units *units, const void *sino,
+                                   const double *weights, const float *gain, const void *angle_gain,
+                                   const void *vol_grad, void *sino_grad, float *gain_grad, void *angle_gain_grad,
+                                   void *workspace, void *stream)
+{
+    if (!plan || !units || !units->views)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "NULL pointer argument");
+    Layout y;
+    const odt_status st = pair_layout(plan, units->num_units, &y);
+    if (st != ODT_OK)
+        return st;
+    return run_adjoint(plan, y, (const int2 *)units->views, sino, weights, units->geometry, gain, angle_gain,
+                       vol_grad, sino_grad, gain_grad, angle_gain_grad, workspace, stream);
+}
+
 odt_status odt_bpp3d_execute_timed(const odt_bpp3d_plan *plan, const void *sino, const double *weights,
                                    const double *geometry, void *volume, void *workspace, void *stream,
                                    odt_stage_timing *timing)
 {
     if (!timing)
         return fail(ODT_ERR_INVALID_ARGUMENT, "timing is NULL");
-    return run_plan(plan, sino, weights, geometry, nullptr, nullptr, volume, workspace, stream, timing);
+    if (!plan)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "NULL pointer argument");
+    return run_plan(plan, plan->lay, nullptr, sino, weights, geometry, nullptr, nullptr, volume, workspace, stream,
+                    timing);
+}
+
+static int64_t count_launches(const odt_bpp3d_plan *plan, const Layout &lay)
+{
+    int64_t n = 0;
+    for (int b = 0; b * lay.batch < lay.units; ++b) {
+        const int64_t total = (int64_t)std::min(lay.batch, lay.units - b * lay.batch) * plan->nz;
+        if (odt::single_row_plan(stage_params(plan)))
+            n += 4;  // row spectra, filtered spectra, fused column + row stage, resampling
+        else
+            n += 3 + 2 * ((total + lay.jobs - 1) / lay.jobs);
+        if (plan->d.geometry == ODT_GEOM_Y_AXIS)
+            n += 1;  // per-(slab, tile) geometry setup
+    }
+    return n;
 }
 
 odt_status odt_bpp3d_launch_count(const odt_bpp3d_plan *plan, int64_t *launches)
 {
     if (!plan || !launches)
         return fail(ODT_ERR_INVALID_ARGUMENT, "NULL argument");
-    const int A = plan->d.num_angles;
-    const int nbatches = (A + plan->batch - 1) / plan->batch;
-    int64_t n = 0;
-    for (int b = 0; b < nbatches; ++b) {
-        const int nb = std::min(plan->batch, A - b * plan->batch);
-        const int64_t total = (int64_t)nb * plan->nz;
-        if (odt::single_row_plan(stage_params(plan)))
-            n += 3;  // row spectra, fused column + row stage, resampling
-        else
-            n += 2 + 2 * ((total + plan->jobs - 1) / plan->jobs);
-        if (plan->d.intp_order >= 2)
-            n += 1;  // z-prefilter boundary columns
-        if (plan->d.geometry == ODT_GEOM_Y_AXIS)
-            n += 1;  // per-(angle, tile) geometry setup
-    }
-    *launches = n;
+    *launches = count_launches(plan, plan->lay);
     return ODT_OK;
+}
+
+odt_status odt_bpp3d_pair_launch_count(const odt_bpp3d_plan *plan, int32_t num_units, int64_t *launches)
+{
+    if (!plan || !launches)
+        return fail(ODT_ERR_INVALID_ARGUMENT, "NULL argument");
+    Layout y;
+    const odt_status st = pair_layout(plan, num_units, &y);
+    if (st == ODT_OK)
+        *launches = count_launches(plan, y);
+    return st;
 }
 
 odt_status odt_bpp3d_read_status(const odt_bpp3d_plan *plan, void *stream)
@@ -1122,12 +1243,12 @@ extern "C" odt_status odt_bpp3d_execute_noalloc(const odt_bpp3d_plan *plan, cons
 {
     if (!plan)
         return fail(ODT_ERR_INVALID_ARGUMENT, "NULL plan");
-    if (plan->ws_bytes > ODT_NOALLOC_SCRATCH_BYTES) {
+    if (plan->lay.ws_bytes > ODT_NOALLOC_SCRATCH_BYTES) {
         char buf[200];
         snprintf(buf, sizeof buf,
                  "plan needs %llu bytes of scratch, the static scratch holds %llu; create the plan with "
                  "workspace_limit <= %llu",
-                 (unsigned long long)plan->ws_bytes, (unsigned long long)ODT_NOALLOC_SCRATCH_BYTES,
+                 (unsigned long long)plan->lay.ws_bytes, (unsigned long long)ODT_NOALLOC_SCRATCH_BYTES,
                  (unsigned long long)ODT_NOALLOC_SCRATCH_BYTES);
         return fail(ODT_ERR_INVALID_ARGUMENT, buf);
     }
@@ -1151,5 +1272,6 @@ extern "C" odt_status odt_bpp3d_execute_noalloc(const odt_bpp3d_plan *plan, cons
         }
         scratch = g_noalloc_addr[dev];
     }
-    return run_plan(plan, sino, weights, geometry, nullptr, nullptr, volume, scratch, stream, nullptr);
+    return run_plan(plan, plan->lay, nullptr, sino, weights, geometry, nullptr, nullptr, volume, scratch, stream,
+                    nullptr);
 }

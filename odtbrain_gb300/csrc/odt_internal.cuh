@@ -72,7 +72,12 @@ struct StageParams {
     FilterTables tab;
     const float *gain;   // optional real per-frequency gain [lNy*lNx] (NULL: 1)
     const float2 *again; // optional complex per-angle gain [A][lNy*lNx], this
-                         // batch's first angle at again (NULL: 1)
+                         // batch's first angle at again (NULL: 1); with
+                         // units the first of all angles
+    // Opposite views (stages.cu): the batch's units, (angle, opposite angle
+    // or -1) each, numbered over all angles; spectra then hold two slots per
+    // unit.  NULL: one angle per unit, numbered within the batch.
+    const int2 *units;
     int *status;
     // Tilted path, order >= 2 (ydefer = 1): the column stage leaves the
     // y-prefilter boundary terms to the row stage and stores the raw y-line samples around the crop's ends, 4
@@ -98,21 +103,23 @@ struct RotParams {
 };
 
 // Launchers (stream-ordered; return cudaGetLastError()).
-cudaError_t launch_rows_forward(const StageParams &P, const void *sino_batch, const double *weights_batch,
-                                int nb, float2 *rowspec, cudaStream_t s);
-cudaError_t launch_columns_propagate(const StageParams &P, const float2 *rowspec, float2 *T, int q0, int qn,
+// Row spectra of a batch's slots (angles, or two per unit).  sino and
+// weights start at the batch's first angle, with units at angle 0.
+cudaError_t launch_rows_forward(const StageParams &P, const void *sino, const double *weights, int nslots,
+                                float2 *rowspec, cudaStream_t s);
+// Row spectra -> filtered spectra, in place, and (order >= 2) the
+// z-prefilter boundary rows Tab[unit][2 poles][ny][lNx].
+cudaError_t launch_columns_spectrum(const StageParams &P, float2 *rowspec, float2 *Tab, int nunits, cudaStream_t s);
+cudaError_t launch_columns_propagate(const StageParams &P, const float2 *spec, float2 *T, int q0, int qn,
                                      cudaStream_t s);
-// z-prefilter boundary columns of a batch (order >= 2): Tab[a][2][ny][lNx].
-cudaError_t launch_columns_boundary(const StageParams &P, const float2 *rowspec, float2 *Tab, int nb,
-                                    cudaStream_t s);
 // Single-row planes (lNy == ny == 1, slab pitch 1): the column and row
-// stages fused in one launch over jobs [q0, q0 + qn), from the row spectra.
+// stages fused in one launch over jobs [q0, q0 + qn), from the filtered spectra.
 bool single_row_plan(const StageParams &P);
 // Square power-of-two padded planes (N >= 256) cropped to their centred
 // half (ny = nx = N/2 from N/4): the column and row stages then run
 // kernels whose crop and edge positions are compile-time constants.
 bool half_crop(const StageParams &P);
-cudaError_t launch_rows_line(const StageParams &P, const float2 *rowspec, const float2 *Tab, float2 *slab, int q0,
+cudaError_t launch_rows_line(const StageParams &P, const float2 *spec, const float2 *Tab, float2 *slab, int q0,
                              int qn, cudaStream_t s);
 cudaError_t launch_rows_inverse(const StageParams &P, const float2 *T, const float2 *Tab, float2 *slab, int q0,
                                 int qn, cudaStream_t s);
@@ -140,10 +147,12 @@ cudaError_t launch_volume_zxy(const float2 *vol, float2 *vol_zxy, int nz, int ny
 cudaError_t configure_rotate_adjoint_kernels();
 cudaError_t launch_adj_rows(const StageParams &P, const float2 *sgrad, float2 *Tg, int q0, int qn, cudaStream_t s);
 cudaError_t launch_adj_columns(const StageParams &P, const float2 *Tg, float2 *Qg, int q0, int qn, cudaStream_t s);
+// The last three take spectrum slots (angles, or two per unit); with units
+// dagain, weights and dsino start at angle 0, otherwise at the batch's first.
 cudaError_t launch_adj_spectrum(const StageParams &P, const float2 *rowspec, const float2 *Qg, float *dgain,
-                                float2 *dagain, float2 *W, int nb, cudaStream_t s);
-cudaError_t launch_adj_rows_full(const StageParams &P, const float2 *W, float2 *Pg, int nb, cudaStream_t s);
-cudaError_t launch_adj_pad(const StageParams &P, const float2 *Pg, const double *weights, int nb, float2 *dsino,
+                                float2 *dagain, float2 *W, int nslots, cudaStream_t s);
+cudaError_t launch_adj_rows_full(const StageParams &P, const float2 *W, float2 *Pg, int nslots, cudaStream_t s);
+cudaError_t launch_adj_pad(const StageParams &P, const float2 *Pg, const double *weights, int nslots, float2 *dsino,
                            cudaStream_t s);
 bool line_size_supported(int n);
 

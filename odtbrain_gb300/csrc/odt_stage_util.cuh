@@ -235,19 +235,12 @@ inline size_t smem_rows_half(int n)
 {
     return (size_t)(2 * Cfg<L>::LPC * xslots<false>(n) + tw_slots(n) + EDGE_SLOTS * Cfg<L>::LPC) * sizeof(float2);
 }
-// k_columns_propagate of half-crop plans: smem_cols plus the third-pass
-// twiddle table.
-template <class L>
-inline size_t smem_cols_half(int n)
-{
-    return (size_t)(2 * Cfg<L>::KX * xslots<true>(n) + Cfg<L>::KX * n + tw_slots2(n) + EDGE_SLOTS * Cfg<L>::KX) *
-           sizeof(float2);
-}
+// k_columns_spectrum: the exchange buffers, the twiddle table and the edge
+// samples.
 template <class L>
 inline size_t smem_cols(int n)
 {
-    return (size_t)(2 * Cfg<L>::KX * xslots<true>(n) + Cfg<L>::KX * n + tw_slots(n) + EDGE_SLOTS * Cfg<L>::KX) *
-           sizeof(float2);
+    return (size_t)(2 * Cfg<L>::KX * xslots<true>(n) + tw_slots(n) + EDGE_SLOTS * Cfg<L>::KX) * sizeof(float2);
 }
 
 // Calls fn(line) with the line type for length n.

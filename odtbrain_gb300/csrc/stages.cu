@@ -5,11 +5,12 @@
 //   pad -> forward 2D FFT -> *prefactor/(lNx*lNy) -> for every z plane p:
 //   *exp(i km (M-1) z_p) -> unnormalised backward 2D FFT -> crop.
 //
-// GB300 decomposition (three kernels, all lines in registers):
+// GB300 decomposition (four kernels, all lines in registers):
 //   rows_forward       padded+weighted rows, forward FFT along x
-//   columns_propagate  forward FFT along y, filter multiply, then for a run
-//                      of z planes: propagator (exact anchor + complex
-//                      recurrence), backward FFT along y, crop in y
+//   columns_spectrum   forward FFT along y, filter multiply (in place), and
+//                      the z-prefilter boundary rows
+//   columns_propagate  for a run of z planes: propagator (exact anchor +
+//                      complex recurrence), backward FFT along y, crop in y
 //   rows_inverse       backward FFT along x, crop in x -> coefficient slab
 //
 // The B-spline prefilter that scipy.ndimage applies before resampling
@@ -22,6 +23,18 @@
 // prefiltered axis (folded into the filter table G), z gets per-frequency
 // boundary terms (alpha, beta tables), and x (and y) get per-line boundary
 // terms computed from four samples just outside the crop.
+//
+// Opposite views.  Rotating by phi + pi is rotating the slab by pi about y
+// and then by phi, and a rotation by pi maps the slab grid onto itself: plane
+// p to nz-1-p, column x to nx-1-x.  So two views phi and phi + pi (a "unit")
+// share one slab: with the second view's padded rows mirrored about the
+// crop's centre (columns m -> 2 padxl + nx-1 - m, modulo lNx) its spectrum X'
+// is the one of the mirrored view, and with z_(nz-1-p) = 2 zshift - 1 - z_p
+// plane p of the shared slab is the backward transform of
+//   G X e^(i w z_p) + G X' e^(i w (2 zshift - 1 - z_p)).
+// Both terms are formed before the transforms, so one backward 2D transform
+// per plane and one resampling serve two views.  256^3 from 200 views of a
+// full circle: step 54.2 -> @@ ms.
 #include <algorithm>
 #include <type_traits>
 
@@ -40,10 +53,6 @@ constexpr bool kColumnStepRegs = true;
 constexpr bool kColumnTw2 = true;
 // Planes between exact propagator anchors within a column CTA's run.
 constexpr int kReanchorPlanes = 32;
-// The half-crop column kernel's shared memory (smem_cols_half) has one
-// [n][KX] region, which holds the filtered spectrum because the steps are
-// in registers.
-static_assert(kColumnStepRegs, "smem_cols_half assumes register-held propagator steps");
 // Column CTAs that run through up to 256 planes of an angle, re-anchoring
 // the propagator every kReanchorPlanes planes: power-of-two columns of
 // 64-thread lines with the steps in registers (4 columns per CTA, the
@@ -52,8 +61,7 @@ static_assert(kColumnStepRegs, "smem_cols_half assumes register-held propagator 
 // 64 22.8, 128 22.4, 256 22.2 ms.  The other column kernels keep runs of
 // at most kReanchorPlanes planes (one exact anchor each): the 512-thread
 // CTAs of 256-point columns lost 30 % with longer runs (one wave of long
-// CTAs), and the generic kernel's extra shared memory for the re-anchoring
-// cost more than the longer runs saved.
+// CTAs).
 template <class L, int KX, bool HALF>
 constexpr bool long_runs()
 {
@@ -73,9 +81,11 @@ constexpr bool column_regs()
 // ---------------------------------------------------------------------------
 // (a) rows: pad + weight + forward FFT along x.
 // rowspec[a][y][kx], a in the batch, y over the padded height.
+// P.units: slot 2u is unit u's first view, slot 2u+1 its opposite view with
+// the padded row mirrored (left unwritten when there is none).
 template <class L, int LPC>
 __global__ void __launch_bounds__(LPC * L::TPL) k_rows_forward(StageParams P, L line, const void *sino,
-                                                               const double *weights, int nb, float2 *rowspec)
+                                                               const double *weights, int nslots, float2 *rowspec)
 {
     extern __shared__ float2 smem[];
     const int n = line.size();
@@ -84,17 +94,31 @@ __global__ void __launch_bounds__(LPC * L::TPL) k_rows_forward(StageParams P, L 
     copy_twiddles<L>(tw, P.tab.twx, n);
     const int l = threadIdx.x / L::TPL, j = threadIdx.x % L::TPL;
     const int lid = (int)blockIdx.x * LPC + l;
-    const int nlines = nb * P.lNy;
-    const bool valid = lid < nlines;
-    const int a = valid ? lid / P.lNy : 0;
-    const int y = valid ? lid - a * P.lNy : 0;
-    const double w = weights ? weights[a] : 1.0;
-    const size_t arow = (size_t)a * P.ny * P.nx;
+    const int nlines = nslots * P.lNy;
+    bool valid = lid < nlines;
+    const int slot = valid ? lid / P.lNy : 0;
+    const int y = valid ? lid - slot * P.lNy : 0;
+    int a = slot;
+    bool mirrored = false;
+    if (P.units) {
+        const int2 u = P.units[slot >> 1];
+        mirrored = slot & 1;
+        a = mirrored ? u.y : u.x;
+        valid = valid && a >= 0;
+    }
+    const double w = (weights && valid) ? weights[a] : 1.0;
+    const size_t arow = (size_t)(valid ? a : 0) * P.ny * P.nx;
     float2 v[L::SLOTS];
 #pragma unroll
     for (int r = 0; r < L::SLOTS; ++r) {
-        const int x = j + r * L::TPL;
-        v[r] = (valid && x < n) ? padded_sample(P, sino, arow, w, y, x) : make_float2(0.f, 0.f);
+        int x = j + r * L::TPL;
+        const bool in = valid && x < n;
+        if (mirrored) {
+            x = 2 * P.padxl + P.nx - 1 - x;
+            x += x < 0 ? n : 0;
+            x -= x >= n ? n : 0;
+        }
+        v[r] = in ? padded_sample(P, sino, arow, w, y, x) : make_float2(0.f, 0.f);
     }
     __syncthreads();
     int flip = 0;
@@ -114,30 +138,32 @@ __global__ void __launch_bounds__(LPC * L::TPL) k_rows_forward(StageParams P, L 
 // Column helpers shared by the two column kernels.  A CTA owns KX adjacent
 // spectrum columns kx; thread (c, j) holds rows ky = j + r*TPL of column c.
 
-// Column kx of angle a's row spectra, forward FFT along y, times the filter
-// table G (which includes the prefilter particular factors).
+// Column kx of the row spectra of one slot, forward FFT along y, times the
+// filter table G (which includes the prefilter particular factors) and the
+// gains.  `kg` is the column whose gains apply (the mirrored one for an
+// opposite view), `again` the view's own gain map.
 template <class L, int KX>
-__device__ __forceinline__ void column_spectrum(const StageParams &P, const L &line, const float2 *rowspec, int a,
-                                                int kx, bool colok, int c, int j, float2 *buf0, float2 *buf1,
-                                                const float2 *tw, int &flip, float2 (&v)[L::SLOTS])
+__device__ __forceinline__ void column_spectrum(const StageParams &P, const L &line, const float2 *spec, int kx,
+                                                int kg, const float2 *again, bool colok, int c, int j, float2 *buf0,
+                                                float2 *buf1, const float2 *tw, int &flip, float2 (&v)[L::SLOTS])
 {
     const int n = line.size();
 #pragma unroll
     for (int r = 0; r < L::SLOTS; ++r) {
         const int ky = j + r * L::TPL;
-        v[r] = (colok && ky < n) ? rowspec[((size_t)a * n + ky) * P.lNx + kx] : make_float2(0.f, 0.f);
+        v[r] = (colok && ky < n) ? spec[(size_t)ky * P.lNx + kx] : make_float2(0.f, 0.f);
     }
     line.template run<-1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
 #pragma unroll
     for (int r = 0; r < L::SLOTS; ++r) {
         const int ky = j + r * L::TPL;
         if (colok && ky < n) {
-            const size_t k = (size_t)ky * P.lNx + kx;
-            v[r] = cmul(v[r], P.tab.G[k]);
+            const size_t row = (size_t)ky * P.lNx;
+            v[r] = cmul(v[r], P.tab.G[row + kx]);
             if (P.gain)
-                v[r] = cscale(v[r], P.gain[k]);
-            if (P.again)
-                v[r] = cmul(v[r], P.again[(size_t)a * P.lNy * P.lNx + k]);
+                v[r] = cscale(v[r], P.gain[row + kg]);
+            if (again)
+                v[r] = cmul(v[r], again[row + kg]);
         } else {
             v[r] = make_float2(0.f, 0.f);
         }
@@ -279,18 +305,23 @@ __device__ __forceinline__ void column_inverse_store_half(const StageParams &P, 
 }
 
 // ---------------------------------------------------------------------------
-// (b0) z-prefilter boundary columns, once per angle (order >= 2).  The
-// prefiltered propagator of plane p is E_p + alpha z^p + beta z^(nz-1-p);
-// by linearity the alpha and beta parts are transformed once here
-// (Tab[a][0] = column transform of G*alpha, Tab[a][1] of G*beta) and the row
-// stage adds z^p Tab[a][0] + z^(nz-1-p) Tab[a][1] to the first and last
-// planes' rows.
-template <class L, int KX, int YF>
-__global__ void __launch_bounds__(KX * L::TPL) k_columns_boundary(StageParams P, L line, const float2 *rowspec,
-                                                                  float2 *Tab)
+// (b0) filtered spectra, once per view: forward FFT along y of the row
+// spectra times the filter and the gains, written back in place, and (order
+// >= 2) the z-prefilter boundary rows of the unit.  The prefiltered
+// propagator of plane p is E_p + alpha z^p + beta z^(nz-1-p); by linearity
+// the alpha and beta parts are transformed once here (Tab[u][0] = column
+// transform of G X alpha, Tab[u][1] of G X beta) and the row stage adds
+// z^p Tab[u][0] + z^(nz-1-p) Tab[u][1] to the first and last planes' rows.
+// The opposite view of a unit (PAIR) enters with alpha and beta exchanged:
+// its plane p is plane nz-1-p of its own slab.
+// The column kernel used to redo this transform at the head of every run of
+// planes and keep its result in shared memory for the re-anchoring; read
+// from here (16 bytes per element and 32 planes) that shared memory is free.
+template <class L, int KX, int YF, bool PAIR>
+__global__ void __launch_bounds__(KX * L::TPL) k_columns_spectrum(StageParams P, L line, float2 *rowspec, float2 *Tab)
 {
     if (!group_active<KX>(P, blockIdx.x * KX))
-        return;  // all-zero columns: the row stage never reads them
+        return;  // all-zero columns: no later stage reads them
     extern __shared__ float2 smem[];
     const int n = line.size();
     const int ls = xslots<true>(n);
@@ -299,34 +330,65 @@ __global__ void __launch_bounds__(KX * L::TPL) k_columns_boundary(StageParams P,
     const int c = threadIdx.x % KX, j = threadIdx.x / KX;
     const int kx = blockIdx.x * KX + c;
     const bool colok = kx < P.lNx;
-    const int a = blockIdx.y;
+    const int u = blockIdx.y;
+    const size_t K = (size_t)P.lNy * P.lNx;
     __syncthreads();
     int flip = 0;
-    float2 g[L::SLOTS];
-    column_spectrum<L, KX>(P, line, rowspec, a, kx, colok, c, j, buf0, buf1, tw, flip, g);
-    const int np = P.npoles;
-    const size_t K = (size_t)P.lNy * P.lNx;
+    float2 g[L::SLOTS], h[L::SLOTS];
+    const int2 views = PAIR ? P.units[u] : make_int2(u, -1);
+    float2 *spec = rowspec + (size_t)(PAIR ? 2 * u : u) * K;
+    column_spectrum<L, KX>(P, line, spec, kx, kx, P.again ? P.again + views.x * K : nullptr, colok, c, j, buf0, buf1,
+                           tw, flip, g);
+    if constexpr (PAIR) {
+        if (views.y >= 0) {  // uniform over the CTA
+            column_spectrum<L, KX>(P, line, spec + K, kx, kx ? P.lNx - kx : 0,
+                                   P.again ? P.again + views.y * K : nullptr, colok, c, j, buf0, buf1, tw, flip, h);
+        } else {
+#pragma unroll
+            for (int r = 0; r < L::SLOTS; ++r)
+                h[r] = make_float2(0.f, 0.f);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < L::SLOTS; ++r) {
+        const int ky = j + r * L::TPL;
+        if (colok && ky < n) {
+            spec[(size_t)ky * P.lNx + kx] = g[r];
+            if (PAIR)
+                spec[K + (size_t)ky * P.lNx + kx] = h[r];
+        }
+    }
+    const int np = P.npoles;  // 0 below order 2
 #pragma unroll 1
     for (int t = 0; t < 2 * np; ++t) {
-        const float2 *tab = t < np ? P.tab.alpha + t * K : P.tab.beta + (t - np) * K;
+        const int i = t < np ? t : t - np;
+        const float2 *tab = (t < np ? P.tab.alpha : P.tab.beta) + i * K;
+        const float2 *opp = (t < np ? P.tab.beta : P.tab.alpha) + i * K;
         float2 v[L::SLOTS];
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
             const int ky = j + r * L::TPL;
-            v[r] = (colok && ky < n) ? cmul(g[r], tab[(size_t)ky * P.lNx + kx]) : make_float2(0.f, 0.f);
+            v[r] = make_float2(0.f, 0.f);
+            if (colok && ky < n) {
+                const size_t k = (size_t)ky * P.lNx + kx;
+                v[r] = cmul(g[r], tab[k]);
+                if (PAIR)
+                    v[r] = cfma(h[r], opp[k], v[r]);
+            }
         }
         column_inverse_store<L, KX, YF>(P, line, v, c, j, colok, buf0, buf1, tw, edge, flip,
-                                        Tab + ((size_t)(a * 2 * np + t) * P.ny) * P.lNx + kx);
+                                        Tab + ((size_t)(u * 2 * np + t) * P.ny) * P.lNx + kx);
     }
 }
 
-// (b1) columns: for the z planes of jobs q in [q0, q0+qn) (q = a*nz + p):
-// propagator (exact anchor, then a complex recurrence whose per-element step
-// lives in shared memory), backward FFT along y, crop.  Output
-// T[q-q0][y][kx], y over the cropped height.
-template <class L, int KX, bool HALF, int YF>
+// (b1) columns: for the z planes of jobs q in [q0, q0+qn) (q = u*nz + p):
+// the filtered spectrum times the propagator (exact anchor, then a complex
+// recurrence), backward FFT along y, crop.  Output T[q-q0][y][kx], y over
+// the cropped height.  PAIR: the unit's opposite view is added with its own
+// propagator (the header comment), which the conjugate step advances.
+template <class L, int KX, bool HALF, int YF, bool PAIR>
 __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX * L::TPL <= 512) ? 2 : 1))
-    k_columns_propagate(StageParams P, L line, const float2 *rowspec, float2 *T, int q0, int qn, int ppc)
+    k_columns_propagate(StageParams P, L line, const float2 *spec, float2 *T, int q0, int qn, int ppc)
 {
     if (!group_active<KX>(P, blockIdx.x * KX))
         return;  // all-zero columns: the row stage never reads them
@@ -340,13 +402,7 @@ __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX *
     const int n = line.size();  // lNy
     const int ls = xslots<true>(n);
     float2 *buf0 = smem, *buf1 = smem + KX * ls, *tw = smem + 2 * KX * ls;
-    float2 *edge = tw + (TW2 ? tw_slots2(n) : tw_slots(n)); // [KX][EDGE_SLOTS]
-    float2 *stp = edge + EDGE_SLOTS * KX;  // [n][KX] propagator step per element
-    // long runs: [n][KX] the filtered spectrum G X of the current angle,
-    // for the exact re-anchoring every kReanchorPlanes planes (in the step
-    // region: the steps live in registers)
-    constexpr bool REANCHOR = long_runs<L, KX, HALF>();
-    float2 *gx = stp;
+    float2 *stp = tw + (TW2 ? tw_slots2(n) : tw_slots(n));  // [n][KX] propagator step (not STEP_REGS)
     if constexpr (TW2)
         copy_twiddles2<L>(tw, P.tab.twy, n);
     else
@@ -355,80 +411,89 @@ __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX *
     const int kx = blockIdx.x * KX + c;
     const bool colok = kx < P.lNx;
     const int lNx = P.lNx, nz = P.nz, ny = P.ny;
+    const size_t K = (size_t)n * lNx;
     const int qb = q0 + blockIdx.y * ppc;
     const int qe = min(q0 + qn, qb + ppc);
     float2 St[L::SLOTS];  // STEP_REGS: exp(i w) of this thread's elements
-    if constexpr (STEP_REGS) {
 #pragma unroll
-        for (int r = 0; r < L::SLOTS; ++r)  // (columns beyond lNx: never stored)
-            St[r] = colok ? P.tab.step[(size_t)(j + r * L::TPL) * lNx + kx] : make_float2(1.f, 0.f);
+    for (int r = 0; r < L::SLOTS; ++r) {  // (columns beyond lNx: never stored)
+        const int ky = j + r * L::TPL;
+        const float2 t = (colok && ky < n) ? P.tab.step[(size_t)ky * lNx + kx] : make_float2(1.f, 0.f);
+        if constexpr (STEP_REGS)
+            St[r] = t;
+        else if (ky < n)
+            stp[ky * KX + c] = t;  // read back only by this thread
     }
     __syncthreads();
 
-    float2 V[L::SLOTS];  // G * exp(i w z_p) for this thread's elements
+    float2 V[L::SLOTS];                    // G X exp(i w z_p) for this thread's elements
+    float2 W[PAIR ? L::SLOTS : 1];         // the opposite view's
     int flip = 0;
     // tilted generic crops: the edge samples this thread holds (fixed)
     unsigned long long eheld = 0;
     if constexpr (!HALF && YF > 0 && L::SLOTS <= 8)
         eheld = edge_holdings<L, YF>(P, n, j);
-    int cur_a = -1;
+    int cur_u = -1;
     int since = 0;  // planes advanced by the recurrence since the last exact anchor
-    int a = qb / nz, p = qb % nz;
+    int u = qb / nz, p = qb % nz;
     for (int q = qb; q < qe; ++q, ++p) {
         if (p == nz) {
             p = 0;
-            ++a;
+            ++u;
         }
-        if (a != cur_a || (REANCHOR && since == kReanchorPlanes)) {
-            // exact anchor at the first plane of an angle, and again every
+        if (u != cur_u || since == kReanchorPlanes) {
+            // exact anchor at the first plane of a unit, and again every
             // kReanchorPlanes planes: the FP32 recurrence drifts by about one
             // rounding per plane (measured on the 256^3 workload: rel-L2 to
             // the FP64 oracle 3.5e-7 with anchors every 32 planes, 1.6e-6
             // with one anchor per 256-plane run)
-            const bool fresh = a != cur_a;
-            if (fresh)
-                column_spectrum<L, KX>(P, line, rowspec, a, kx, colok, c, j, buf0, buf1, tw, flip, V);
             const float zp = (float)p - 0.5f * (float)nz + P.zshift;
+            const float zo = 2.f * P.zshift - 1.f - zp;  // the opposite view's plane
+            const float2 *su = spec + (size_t)(PAIR ? 2 * u : u) * K;
 #pragma unroll
             for (int r = 0; r < L::SLOTS; ++r) {
                 const int ky = j + r * L::TPL;
+                V[r] = make_float2(0.f, 0.f);
+                if (PAIR)
+                    W[r] = make_float2(0.f, 0.f);
                 if (colok && ky < n) {
                     const size_t k = (size_t)ky * lNx + kx;
-                    if (fresh) {
-                        if (REANCHOR)
-                            gx[ky * KX + c] = V[r];  // read back only by this thread
-                        if (!STEP_REGS)
-                            stp[ky * KX + c] = P.tab.step[k];
-                    } else if (REANCHOR) {
-                        V[r] = gx[ky * KX + c];
-                    }
-                    V[r] = cmul(V[r], expi_phase(P.tab.wsplit[k], zp));
+                    const float2 w = P.tab.wsplit[k];
+                    V[r] = cmul(su[k], expi_phase(w, zp));
+                    if (PAIR)
+                        W[r] = cmul(su[K + k], expi_phase(w, zo));
                 }
             }
-            cur_a = a;
+            cur_u = u;
             since = 0;
         }
         ++since;
         float2 v[L::SLOTS];
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
-            v[r] = V[r];
             const int ky = j + r * L::TPL;
-            if constexpr (STEP_REGS)
-                V[r] = cmul(V[r], St[r]);  // (ky < n: a power-of-two line)
-            else if (HALF || ky < n)  // half-crop plans: a power-of-two line, ky < n
-                V[r] = cmul(V[r], stp[ky * KX + c]);
+            v[r] = PAIR ? V[r] + W[r] : V[r];
+            if (STEP_REGS || HALF || ky < n) {  // (power-of-two lines: ky < n)
+                float2 st;
+                if constexpr (STEP_REGS)
+                    st = St[r];
+                else
+                    st = stp[ky * KX + c];
+                V[r] = cmul(V[r], st);
+                if (PAIR)
+                    W[r] = cmul_conj(W[r], st);
+            }
         }
         if constexpr (HALF)  // (tilted: the y-prefilter terms go to the row stage)
             column_inverse_store_half<L, KX, YF, TW2, (YF > 0)>(
-                P, line, v, c, j, buf0, buf1, tw, edge, flip, T + (size_t)(q - q0) * (L::N / 2) * L::N + kx,
+                P, line, v, c, j, buf0, buf1, tw, nullptr, flip, T + (size_t)(q - q0) * (L::N / 2) * L::N + kx,
                 T + P.yedge_off + (size_t)(q - q0) * 4 * (YF > 0 ? YF : 1) * L::N + kx);
         else if constexpr (YF > 0)  // (tilted: the y-prefilter terms go to the row stage)
             column_inverse_store<L, KX, YF, TW2, true>(
-                P, line, v, c, j, colok, buf0, buf1, tw, edge, flip, T + (size_t)(q - q0) * ny * lNx + kx,
+                P, line, v, c, j, colok, buf0, buf1, tw, nullptr, flip, T + (size_t)(q - q0) * ny * lNx + kx,
                 T + P.yedge_off + (size_t)(q - q0) * 4 * YF * lNx + kx, eheld);
         else
-            column_inverse_store<L, KX, YF, TW2>(P, line, v, c, j, colok, buf0, buf1, tw, edge, flip,
+            column_inverse_store<L, KX, YF, TW2>(P, line, v, c, j, colok, buf0, buf1, tw, nullptr, flip,
                                              T + (size_t)(q - q0) * ny * lNx + kx);
     }
 }
@@ -847,18 +912,19 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
 
 // (b1+b2) single-row planes (lNy == ny == 1, slab pitch 1: the 2D
 // reconstruction): the column transforms are the identity, so a job's row
-// is the row spectrum times the filter table (and gains) and the propagator
-// of its plane, formed here instead of in a column stage.  A CTA takes RG
+// is the filtered spectrum (k_spectrum_line) times the propagator of its
+// plane, formed here instead of in a column stage (PAIR: plus the opposite
+// view's, see the header comment).  A CTA takes RG
 // consecutive jobs as groups of LPC lines (one job per line).  With one
 // line per group the propagator is anchored exactly at the CTA's first job
-// (and wherever the angle changes) and advanced plane by plane with the
+// (and wherever the unit changes) and advanced plane by plane with the
 // complex step exp(i w), as in k_columns_propagate; with several lines per
 // group every line is anchored exactly.  Then per line the z-boundary rows
 // of its plane, the backward FFT along x, the x-prefilter boundary terms,
 // and the cropped row stored contiguously at slab[a][p][x].
-template <class L, int LPC, int NP>
+template <class L, int LPC, int NP, bool PAIR>
 __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 3 : 1)
-    k_rows_line(StageParams P, L line, const float2 *rowspec, const float2 *Tab, float2 *slab, int q0, int qn)
+    k_rows_line(StageParams P, L line, const float2 *spec, const float2 *Tab, float2 *slab, int q0, int qn)
 {
     constexpr int RG = rows_per_cta<LPC>(), G = RG / LPC;
     extern __shared__ float2 smem[];
@@ -872,7 +938,9 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 3 : 1)
     const bool pf = P.order >= 2;
     const int qbase = (int)blockIdx.x * RG;
     const int GV = min(G, (qn - qbase + LPC - 1) / LPC);  // groups holding a job
-    float2 W[L::SLOTS];  // LPC == 1: the next plane's propagated spectrum
+    // LPC == 1: the next plane's propagated spectrum, of the first and the
+    // opposite view
+    float2 V[L::SLOTS], W[PAIR ? L::SLOTS : 1];
     int cur_a = -1;
     __syncthreads();  // twiddles
 #pragma unroll 1
@@ -882,33 +950,35 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 3 : 1)
         const int q = q0 + (valid ? qrel : 0);
         const int a = q / nz, p = q - a * nz;
         float2 v[L::SLOTS];
-        if (LPC == 1 && a == cur_a) {
-#pragma unroll
-            for (int r = 0; r < L::SLOTS; ++r) {
-                const int x = j + r * L::TPL;
-                v[r] = W[r];
-                if (column_active(P, x))
-                    W[r] = cmul(W[r], P.tab.step[x]);
-            }
-        } else {
+        if (LPC > 1 || a != cur_a) {
             const float zp = (float)p - 0.5f * (float)nz + P.zshift;
+            const float zo = 2.f * P.zshift - 1.f - zp;
+            const float2 *su = spec + (size_t)(PAIR ? 2 * a : a) * n;
 #pragma unroll
             for (int r = 0; r < L::SLOTS; ++r) {
                 const int x = j + r * L::TPL;
-                float2 b = make_float2(0.f, 0.f);
+                V[r] = make_float2(0.f, 0.f);
+                if (PAIR)
+                    W[r] = make_float2(0.f, 0.f);
                 if (valid && column_active(P, x)) {
-                    b = cmul(rowspec[(size_t)a * n + x], P.tab.G[x]);
-                    if (P.gain)
-                        b = cscale(b, P.gain[x]);
-                    if (P.again)
-                        b = cmul(b, P.again[(size_t)a * n + x]);
-                    b = cmul(b, expi_phase(P.tab.wsplit[x], zp));
+                    const float2 w = P.tab.wsplit[x];
+                    V[r] = cmul(su[x], expi_phase(w, zp));
+                    if (PAIR)
+                        W[r] = cmul(su[n + x], expi_phase(w, zo));
                 }
-                v[r] = b;
-                if (LPC == 1)
-                    W[r] = column_active(P, x) ? cmul(b, P.tab.step[x]) : b;
             }
             cur_a = a;
+        }
+#pragma unroll
+        for (int r = 0; r < L::SLOTS; ++r) {
+            const int x = j + r * L::TPL;
+            v[r] = PAIR ? V[r] + W[r] : V[r];
+            if (LPC == 1 && column_active(P, x)) {
+                const float2 st = P.tab.step[x];
+                V[r] = cmul(V[r], st);
+                if (PAIR)
+                    W[r] = cmul_conj(W[r], st);
+            }
         }
         if (valid && pf) {
             constexpr int np = NP;
@@ -978,29 +1048,42 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 3 : 1)
     }
 }
 
-// (b0) z-prefilter boundary columns for single-row planes: the column
-// transforms are the identity, Tab[a][t][kx] = spectrum * G * (alpha, beta).
-__global__ void __launch_bounds__(256) k_columns_boundary_line(StageParams P, const float2 *rowspec, float2 *Tab,
-                                                               int nb)
+// (b0) k_columns_spectrum for single-row planes, whose column transforms are
+// the identity.  One thread per (unit, kx).
+__global__ void __launch_bounds__(256) k_spectrum_line(StageParams P, float2 *rowspec, float2 *Tab, int nunits)
 {
     const int lNx = P.lNx;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)nb * lNx)
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= (long long)nunits * lNx)
         return;
-    const int a = (int)(i / lNx), kx = (int)(i - (long long)a * lNx);
-    float2 b = make_float2(0.f, 0.f);
-    if (column_active(P, kx)) {
-        b = cmul(rowspec[(size_t)a * lNx + kx], P.tab.G[kx]);
+    const int u = (int)(id / lNx), kx = (int)(id - (long long)u * lNx);
+    const int2 views = P.units ? P.units[u] : make_int2(u, -1);
+    float2 *spec = rowspec + (size_t)(P.units ? 2 * u : u) * lNx + kx;
+    auto filtered = [&](float2 x, int a, int kg) {
+        x = cmul(x, P.tab.G[kx]);
         if (P.gain)
-            b = cscale(b, P.gain[kx]);
+            x = cscale(x, P.gain[kg]);
         if (P.again)
-            b = cmul(b, P.again[(size_t)a * lNx + kx]);
-    }
+            x = cmul(x, P.again[(size_t)a * lNx + kg]);
+        return x;
+    };
+    const bool act = column_active(P, kx);
+    const float2 zero = make_float2(0.f, 0.f);
+    const float2 g = act ? filtered(spec[0], views.x, kx) : zero;
+    const float2 h = (act && views.y >= 0) ? filtered(spec[lNx], views.y, kx ? lNx - kx : 0) : zero;
+    spec[0] = g;
+    if (P.units)
+        spec[lNx] = h;
     const int np = P.npoles;
-    const size_t K = (size_t)P.lNy * lNx;
     for (int i = 0; i < np; ++i) {
-        Tab[(size_t)(a * 2 * np + i) * lNx + kx] = cmul(b, P.tab.alpha[i * K + kx]);
-        Tab[(size_t)(a * 2 * np + np + i) * lNx + kx] = cmul(b, P.tab.beta[i * K + kx]);
+        const float2 al = P.tab.alpha[(size_t)i * lNx + kx], be = P.tab.beta[(size_t)i * lNx + kx];
+        float2 ta = cmul(g, al), tb = cmul(g, be);
+        if (P.units) {
+            ta = cfma(h, be, ta);
+            tb = cfma(h, al, tb);
+        }
+        Tab[(size_t)(u * 2 * np + i) * lNx + kx] = ta;
+        Tab[(size_t)(u * 2 * np + np + i) * lNx + kx] = tb;
     }
 }
 
@@ -1023,13 +1106,16 @@ static int planes_per_cta(const StageParams &P, int qn, bool long_run)
     return std::min(long_run ? 256 : kReanchorPlanes, std::max(4, ppc));
 }
 
-// Shared memory of the generic-crop column kernel: power-of-two columns of
-// 512 or more carry the third-pass twiddle table and the filtered-spectrum
-// region as the half-crop kernel does.
-template <class L>
+// Shared memory of the column kernel: the exchange buffers, the twiddle
+// tables and, where the propagator steps are not in registers, the steps.
+template <class L, bool HALF>
 static size_t smem_cols_prop(int n)
 {
-    return (column_regs<L, Cfg<L>::KX, false>() && pow2_len<L>() >= 512) ? smem_cols_half<L>(n) : smem_cols<L>(n);
+    constexpr int KX = Cfg<L>::KX;
+    constexpr bool regs = column_regs<L, KX, HALF>();
+    const bool tw2 = regs && kColumnTw2 && pow2_len<L>() >= 512;
+    return (size_t)(2 * KX * xslots<true>(n) + (tw2 ? tw_slots2(n) : tw_slots(n)) + (regs ? 0 : KX * n)) *
+           sizeof(float2);
 }
 
 // Calls fn(std::integral_constant<int, V>) for V = v (one of 0, 1, 2), so a
@@ -1057,24 +1143,34 @@ static int row_poles(const StageParams &P)
 }
 
 template <class L>
-static cudaError_t rows_forward_impl(const StageParams &P, L line, const void *sino, const double *w, int nb,
+static cudaError_t rows_forward_impl(const StageParams &P, L line, const void *sino, const double *w, int nslots,
                                      float2 *out, cudaStream_t s)
 {
     constexpr int LPC = Cfg<L>::LPC;
-    const long long lines = (long long)nb * P.lNy;
+    const long long lines = (long long)nslots * P.lNy;
     const unsigned grid = (unsigned)((lines + LPC - 1) / LPC);
-    k_rows_forward<L, LPC><<<grid, LPC * L::TPL, smem_rows<L>(line.n), s>>>(P, line, sino, w, nb, out);
+    k_rows_forward<L, LPC><<<grid, LPC * L::TPL, smem_rows<L>(line.n), s>>>(P, line, sino, w, nslots, out);
     return cudaGetLastError();
 }
 
 template <class L>
-static cudaError_t boundary_impl(const StageParams &P, L line, const float2 *rowspec, float2 *Tab, int nb,
+static cudaError_t spectrum_impl(const StageParams &P, L line, float2 *rowspec, float2 *Tab, int nunits,
                                  cudaStream_t s)
 {
     constexpr int KX = Cfg<L>::KX;
-    dim3 grid((P.lNx + KX - 1) / KX, nb);
+    dim3 grid((P.lNx + KX - 1) / KX, nunits);
     return with_poles(column_poles(P), [&](auto yf) {
-        k_columns_boundary<L, KX, decltype(yf)::value>
+        constexpr int YF = decltype(yf)::value;
+        if constexpr (YF == 0) {  // (units: y-axis plans only, no y-prefilter)
+            if (P.units) {
+                k_columns_spectrum<L, KX, YF, true>
+                    <<<grid, KX * L::TPL, smem_cols<L>(line.n), s>>>(P, line, rowspec, Tab);
+                return cudaGetLastError();
+            }
+        }
+        if (P.units)
+            return cudaErrorInvalidValue;
+        k_columns_spectrum<L, KX, YF, false>
             <<<grid, KX * L::TPL, smem_cols<L>(line.n), s>>>(P, line, rowspec, Tab);
         return cudaGetLastError();
     });
@@ -1096,28 +1192,38 @@ constexpr int half_groups()
 {
     return Cfg<L>::LPC >= 16 ? 1 : 16 / Cfg<L>::LPC;
 }
-template <class L>
-static cudaError_t columns_impl(const StageParams &P, L line, const float2 *rowspec, float2 *T, int q0, int qn,
-                                cudaStream_t s)
+template <class L, bool HALF, int YF, bool PAIR>
+static cudaError_t columns_launch(const StageParams &P, L line, const float2 *spec, float2 *T, int q0, int qn,
+                                  cudaStream_t s)
 {
     constexpr int KX = Cfg<L>::KX;
-    bool half = false;
-    if constexpr (half_line<L>())
-        half = half_crop(P);
-    const int ppc = planes_per_cta<KX>(P, qn, half ? long_runs<L, KX, true>() : long_runs<L, KX, false>());
+    const int ppc = planes_per_cta<KX>(P, qn, long_runs<L, KX, HALF>());
     dim3 grid((P.lNx + KX - 1) / KX, (qn + ppc - 1) / ppc);
+    k_columns_propagate<L, KX, HALF, YF, PAIR>
+        <<<grid, KX * L::TPL, smem_cols_prop<L, HALF>(line.n), s>>>(P, line, spec, T, q0, qn, ppc);
+    return cudaGetLastError();
+}
+template <class L>
+static cudaError_t columns_impl(const StageParams &P, L line, const float2 *spec, float2 *T, int q0, int qn,
+                                cudaStream_t s)
+{
     return with_poles(column_poles(P), [&](auto yf) {
         constexpr int YF = decltype(yf)::value;
         if constexpr (half_line<L>()) {
             if (half_crop(P)) {
-                k_columns_propagate<L, KX, true, YF>
-                    <<<grid, KX * L::TPL, smem_cols_half<L>(line.n), s>>>(P, line, rowspec, T, q0, qn, ppc);
-                return cudaGetLastError();
+                if constexpr (YF == 0) {
+                    if (P.units)
+                        return columns_launch<L, true, YF, true>(P, line, spec, T, q0, qn, s);
+                }
+                return P.units ? cudaErrorInvalidValue
+                               : columns_launch<L, true, YF, false>(P, line, spec, T, q0, qn, s);
             }
         }
-        k_columns_propagate<L, KX, false, YF>
-            <<<grid, KX * L::TPL, smem_cols_prop<L>(line.n), s>>>(P, line, rowspec, T, q0, qn, ppc);
-        return cudaGetLastError();
+        if constexpr (YF == 0) {
+            if (P.units)
+                return columns_launch<L, false, YF, true>(P, line, spec, T, q0, qn, s);
+        }
+        return P.units ? cudaErrorInvalidValue : columns_launch<L, false, YF, false>(P, line, spec, T, q0, qn, s);
     });
 }
 
@@ -1176,16 +1282,27 @@ static cudaError_t set_smem_attrs_np(int n)
                                  (int)(smem_rows<L>(n) + smem_rows_y<L, NP, true>(n)));
         if (e != cudaSuccess)
             return e;
-        e = cudaFuncSetAttribute(k_rows_line<L, Cfg<L>::LPC, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_rows<L>(n));
+        e = cudaFuncSetAttribute(k_rows_line<L, Cfg<L>::LPC, NP, false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows<L>(n));
+        if (e != cudaSuccess)
+            return e;
+        e = cudaFuncSetAttribute(k_rows_line<L, Cfg<L>::LPC, NP, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows<L>(n));
         if (e != cudaSuccess)
             return e;
     }
     if constexpr (half_line<L>()) {
-        e = cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, true, NP>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols_half<L>(n));
+        e = cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, true, NP, false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols_prop<L, true>(n));
         if (e != cudaSuccess)
             return e;
+        if constexpr (NP == 0) {
+            e = cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, true, NP, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem_cols_prop<L, true>(n));
+            if (e != cudaSuccess)
+                return e;
+        }
         if constexpr (NP >= 1) {
             e = cudaFuncSetAttribute(k_rows_inverse_half<L, Cfg<L>::LPC, half_groups<L>(), NP, false>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows_half<L>(n));
@@ -1198,12 +1315,23 @@ static cudaError_t set_smem_attrs_np(int n)
                 return e;
         }
     }
-    e = cudaFuncSetAttribute(k_columns_boundary<L, Cfg<L>::KX, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_cols<L>(n));
+    if constexpr (NP == 0) {
+        e = cudaFuncSetAttribute(k_columns_spectrum<L, Cfg<L>::KX, NP, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols<L>(n));
+        if (e != cudaSuccess)
+            return e;
+        e = cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, false, NP, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem_cols_prop<L, false>(n));
+        if (e != cudaSuccess)
+            return e;
+    }
+    e = cudaFuncSetAttribute(k_columns_spectrum<L, Cfg<L>::KX, NP, false>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols<L>(n));
     if (e != cudaSuccess)
         return e;
-    return cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, false, NP>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols_prop<L>(n));
+    return cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, false, NP, false>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols_prop<L, false>(n));
 }
 
 template <class L>
@@ -1233,8 +1361,8 @@ int columns_slots(const StageParams &P)
     const cudaError_t e = with_line(P.lNy, [&](auto line) {
         using L = decltype(line);
         constexpr int KX = Cfg<L>::KX;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_columns_propagate<L, KX, false, 0>,
-                                                             KX * L::TPL, smem_cols_prop<L>(line.n));
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_columns_propagate<L, KX, false, 0, false>,
+                                                             KX * L::TPL, smem_cols_prop<L, false>(line.n));
     });
     return e == cudaSuccess ? per * sms : 0;
 }
@@ -1255,18 +1383,18 @@ cudaError_t configure_kernels(const StageParams &P)
     return with_line(P.lNy, [&](auto line) { return set_smem_attrs<decltype(line)>(line.n); });
 }
 
-cudaError_t launch_rows_forward(const StageParams &P, const void *sino_batch, const double *weights_batch, int nb,
+cudaError_t launch_rows_forward(const StageParams &P, const void *sino, const double *weights, int nslots,
                                 float2 *rowspec, cudaStream_t s)
 {
     return with_line(P.lNx, [&](auto line) {
-        return rows_forward_impl(P, line, sino_batch, weights_batch, nb, rowspec, s);
+        return rows_forward_impl(P, line, sino, weights, nslots, rowspec, s);
     });
 }
 
-cudaError_t launch_columns_propagate(const StageParams &P, const float2 *rowspec, float2 *T, int q0, int qn,
+cudaError_t launch_columns_propagate(const StageParams &P, const float2 *spec, float2 *T, int q0, int qn,
                                      cudaStream_t s)
 {
-    return with_line(P.lNy, [&](auto line) { return columns_impl(P, line, rowspec, T, q0, qn, s); });
+    return with_line(P.lNy, [&](auto line) { return columns_impl(P, line, spec, T, q0, qn, s); });
 }
 
 bool half_crop(const StageParams &P)
@@ -1281,7 +1409,7 @@ bool single_row_plan(const StageParams &P)
     return P.lNy == 1 && P.ny == 1 && P.padyl == 0 && P.ypitch == 1;
 }
 
-cudaError_t launch_rows_line(const StageParams &P, const float2 *rowspec, const float2 *Tab, float2 *slab, int q0,
+cudaError_t launch_rows_line(const StageParams &P, const float2 *spec, const float2 *Tab, float2 *slab, int q0,
                              int qn, cudaStream_t s)
 {
     return with_line(P.lNx, [&](auto line) {
@@ -1291,8 +1419,12 @@ cudaError_t launch_rows_line(const StageParams &P, const float2 *rowspec, const 
         return with_poles(row_poles(P), [&](auto np) {
             constexpr int NP = decltype(np)::value;
             if constexpr (NP >= 1) {
-                k_rows_line<L, LPC, NP>
-                    <<<grid, LPC * L::TPL, smem_rows<L>(line.n), s>>>(P, line, rowspec, Tab, slab, q0, qn);
+                if (P.units)
+                    k_rows_line<L, LPC, NP, true>
+                        <<<grid, LPC * L::TPL, smem_rows<L>(line.n), s>>>(P, line, spec, Tab, slab, q0, qn);
+                else
+                    k_rows_line<L, LPC, NP, false>
+                        <<<grid, LPC * L::TPL, smem_rows<L>(line.n), s>>>(P, line, spec, Tab, slab, q0, qn);
                 return cudaGetLastError();
             } else {
                 return cudaErrorInvalidValue;
@@ -1301,15 +1433,14 @@ cudaError_t launch_rows_line(const StageParams &P, const float2 *rowspec, const 
     });
 }
 
-cudaError_t launch_columns_boundary(const StageParams &P, const float2 *rowspec, float2 *Tab, int nb,
-                                    cudaStream_t s)
+cudaError_t launch_columns_spectrum(const StageParams &P, float2 *rowspec, float2 *Tab, int nunits, cudaStream_t s)
 {
     if (single_row_plan(P)) {
-        const long long n = (long long)nb * P.lNx;
-        k_columns_boundary_line<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, rowspec, Tab, nb);
+        const long long n = (long long)nunits * P.lNx;
+        k_spectrum_line<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, rowspec, Tab, nunits);
         return cudaGetLastError();
     }
-    return with_line(P.lNy, [&](auto line) { return boundary_impl(P, line, rowspec, Tab, nb, s); });
+    return with_line(P.lNy, [&](auto line) { return spectrum_impl(P, line, rowspec, Tab, nunits, s); });
 }
 
 cudaError_t launch_rows_inverse(const StageParams &P, const float2 *T, const float2 *Tab, float2 *slab, int q0,
