@@ -527,8 +527,9 @@ odt_status odt_bpp3d_plan_create(const odt_bpp3d_desc *desc, odt_bpp3d_plan **ou
             const double ibw = pf ? 1.0 / spline_bhat(order, w) : 1.0;
             const double sc = ibx * iby * ibw;
             G[k] = make_float2((float)(desc->filter[2 * k] * sc), (float)(desc->filter[2 * k + 1] * sc));
-            const float whi = (float)w;
-            W[k] = make_float2(whi, (float)(w - (double)whi));
+            const double wpi = w / M_PI;
+            const float whi = (float)wpi;
+            W[k] = make_float2(whi, (float)(wpi - (double)whi));
             S[k] = make_float2((float)std::cos(w), (float)std::sin(w));
             for (int i = 0; i < 2; ++i) {
                 AL[(size_t)i * K + k] = make_float2(0.f, 0.f);

@@ -177,6 +177,51 @@ struct Pow2Line {
     int n;  // == N, kept for a uniform interface with GenericLine
     __device__ __forceinline__ int size() const { return N; }
 
+    // One exchange: v written at the pass's output positions idxD + r*Ns,
+    // idxD = (j / Ns) 8 Ns + j mod Ns, Ns = 8^pass, and read back at j + r*TPL.
+    // The slots are a per-thread base and a compile-time offset or XOR mask
+    // per r (the compiler does not find these forms of xslot by itself: with
+    // plain xslot calls the index arithmetic was a quarter of the column
+    // kernel's instructions).
+    template <bool PAD>
+    __device__ __forceinline__ void exchange(float2 (&v)[8], int j, float2 *b, int es, int pass, int bar) const
+    {
+        const int Ns = pass == 0 ? 1 : (pass == 1 ? 8 : (pass == 2 ? 64 : 512));
+        const int idxD = (j / Ns) * Ns * 8 + (j & (Ns - 1));
+        if (PAD) {
+            // slot p + p/8: idxD + r Ns carries nothing into p/8 (pass 0: idxD
+            // is a multiple of 8; later passes: r Ns is)
+            float2 *w = b + (idxD + (idxD >> 3)) * es;
+            const int st = pass == 0 ? 1 : Ns + Ns / 8;
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                w[r * st * es] = v[r];
+        } else {
+            // slot p ^ (p/8 mod 16): r Ns occupies bits of p that idxD leaves
+            // zero, so its slot is the base's XOR a constant
+            const int w = xslot<false>(idxD);
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                b[(w ^ xslot<false>(r * Ns)) * es] = v[r];
+        }
+        if (bar > 0)
+            line_sync(bar, TPL);
+        else
+            __syncthreads();
+        if (PAD) {
+            const float2 *q = b + (j + (j >> 3)) * es;
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                v[r] = q[r * (TPL + TPL / 8) * es];
+        } else {
+            // j < TPL, a power of two: r TPL occupies bits that j leaves zero
+            const int q = xslot<false>(j);
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                v[r] = b[(q ^ xslot<false>(r * TPL)) * es];
+        }
+    }
+
     // v: positions j + r*TPL in, same positions out.  `line[0/1]` point at
     // element 0 of this line in the two exchange buffers; `es` is the
     // element stride.  `flip` alternates the buffers across exchanges.
@@ -215,17 +260,7 @@ struct Pow2Line {
                 break;
             float2 *b = flip ? line1 : line0;
             flip ^= 1;
-            const int idxD = (j / Ns) * Ns * 8 + (j & (Ns - 1));
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-                b[xslot<PAD>(idxD + r * Ns) * es] = v[r];
-            if (bar > 0)
-                line_sync(bar, TPL);
-            else
-                __syncthreads();
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-                v[r] = b[xslot<PAD>(j + r * TPL) * es];
+            exchange<PAD>(v, j, b, es, pass, bar);
             Ns *= 8;
         }
         if (TAIL == 4) {

@@ -41,7 +41,7 @@ constexpr int ZPOW_N = 24;
 
 struct FilterTables {
     const float2 *G;      // [lNy*lNx] filter * prefilter particular factors
-    const float2 *wsplit; // [lNy*lNx] propagator phase km*(M-1): (hi, lo)
+    const float2 *wsplit; // [lNy*lNx] propagator phase km*(M-1) / pi: (hi, lo)
     const float2 *step;   // [lNy*lNx] exp(i*km*(M-1))
     const float2 *alpha;  // [pole][lNy*lNx] z-prefilter boundary terms from p = 0
     const float2 *beta;   // [pole][lNy*lNx] z-prefilter boundary terms from p = nz-1

@@ -8,19 +8,18 @@
 
 namespace odt {
 
-// exp(i * w * z) with w held as (hi, lo) floats and z a small half-integer:
-// exact product hi*z via FMA, Cody-Waite reduction by 2*pi, then sincosf.
+// exp(i * w * z) with w/pi held as (hi, lo) floats and z a small
+// half-integer: exact product hi*z via FMA, whole turns taken off exactly
+// (ph is within one turn of an even integer, so the difference is exact),
+// then sincospif, which needs no reduction of its own (sincosf brings a slow
+// path for large arguments that the kernels never take, with its stack frame).
 __device__ __forceinline__ float2 expi_phase(float2 w, float z)
 {
     const float ph = w.x * z;
-    const float err = fmaf(w.x, z, -ph);
-    const float lo = fmaf(w.y, z, err);
-    const float k = rintf(ph * 0.15915494309189535f);
-    float r = fmaf(-k, 6.28125f, ph);
-    r = fmaf(-k, 1.9353071795864769253e-3f, r);
-    r += lo;
+    const float lo = fmaf(w.y, z, fmaf(w.x, z, -ph));
+    const float r = fmaf(-2.f, rintf(0.5f * ph), ph) + lo;
     float s, c;
-    sincosf(r, &s, &c);
+    sincospif(r, &s, &c);
     return make_float2(c, s);
 }
 
