@@ -124,10 +124,8 @@ odt_status odt_bpp3d_angle_batch(const odt_bpp3d_plan *plan, int32_t *batch);
  *   volume    device, (nx, ny, nx) complex64, or float32 when onlyreal;
  *             fully overwritten
  *   workspace device, odt_bpp3d_workspace_size bytes, 256-byte aligned
- * The row stage runs on a second stream that the plan owns, forked from and
- * joined back into `stream` with events (so the call also works inside
- * stream capture); a plan must not be executed by two host threads at
- * once. */
+ * Every launch goes to `stream` (the call also works inside stream capture);
+ * a plan must not be executed by two host threads at once. */
 odt_status odt_bpp3d_execute(const odt_bpp3d_plan *plan, const void *sino,
                              const double *weights, const double *geometry,
                              void *volume, void *workspace, void *stream);

@@ -321,9 +321,9 @@ def check(status):
 
 
 class Plan:
-    """Owns an ``odt_bpp3d_plan``.  A plan's executions fork onto the plan's
-    own second stream, so enqueueing them is serialised per plan (the C ABI
-    forbids concurrent execution of one plan from several host threads)."""
+    """Owns an ``odt_bpp3d_plan``.  Enqueueing executions is serialised per
+    plan (the C ABI forbids concurrent execution of one plan from several
+    host threads)."""
 
     def __init__(self, desc):
         self._lock = threading.Lock()

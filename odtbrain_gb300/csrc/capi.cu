@@ -45,11 +45,11 @@ uint64_t g_table_alloc_limit = 0;
 std::mutex g_debug_mutex;
 
 constexpr uint64_t kDefaultWorkspace = 16ull << 30;   // 16 GiB of slabs, chunk buffers etc.
-// column-stage output chunks: two buffers of half this size in total.  Large
-// chunks (1024 planes of a 512-wide spectrum per buffer) mean few launches
-// with full waves; measured on the 256^3 workload: 64 MB 92.8 ms, 256 MB
+// column-stage output chunk.  Large chunks (1024 planes of a 512-wide
+// spectrum) mean few launches with full waves; measured on the 256^3
+// workload (two chunk buffers of half the size each): 64 MB 92.8 ms, 256 MB
 // 84.2 ms, 1 GB 79.3 ms, 2 GB 78.7 ms, 4 GB 78.7 ms per reconstruction.
-constexpr uint64_t kPlaneBudget = 2048ull << 20;
+constexpr uint64_t kPlaneBudget = 1024ull << 20;
 constexpr size_t kAlign = 256;
 
 size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
@@ -212,7 +212,7 @@ struct Layout {
     int units, batch;  // slabs (angles, or units of opposite views), slabs per batch
     int spu;           // spectrum slots per slab: 1, or 2 with opposite views
     int jobs;          // (slab, plane) jobs per column/row launch
-    size_t off_rowspec, off_T, off_T2, off_Tab, off_slab, off_comp, off_rot, ws_bytes;
+    size_t off_rowspec, off_T, off_Tab, off_slab, off_comp, off_rot, ws_bytes;
     size_t off_Qg, off_W, off_Pg, off_vT, adj_ws_bytes;  // adjoint-only regions after ws_bytes
 };
 }  // namespace
@@ -233,11 +233,6 @@ struct odt_bpp3d_plan {
     void *d_tables;
     FilterTables tab;
     int *d_status;
-    // chunk pipeline: the row stage of chunk k runs on s2 while the column
-    // stage of chunk k+1 runs on the caller's stream (two column-stage
-    // output buffers, ordered by events)
-    cudaStream_t s2;
-    cudaEvent_t ev_fork, ev_join, ev_col[2], ev_row[2];
 };
 
 namespace {
@@ -257,16 +252,6 @@ odt_status check_device(const odt_bpp3d_plan *plan)
         return fail(ODT_ERR_INVALID_ARGUMENT, buf);
     }
     return ODT_OK;
-}
-
-void destroy_sync_objects(odt_bpp3d_plan *p)
-{
-    if (p->s2)
-        cudaStreamDestroy(p->s2);
-    for (cudaEvent_t ev : {p->ev_fork, p->ev_join, p->ev_col[0], p->ev_col[1], p->ev_row[0], p->ev_row[1]})
-        if (ev)
-            cudaEventDestroy(ev);
-    p->s2 = nullptr;
 }
 
 StageParams stage_params(const odt_bpp3d_plan *p)
@@ -326,12 +311,12 @@ Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
     const size_t tab_bytes = np ? (size_t)2 * np * d.ny * lNx * 8 : 0;  // one slab's z-boundary rows
     const size_t vol_bytes = (size_t)nz * d.ny * d.nx * 8;           // compensation buffer
     const uint64_t limit = d.workspace_limit ? d.workspace_limit : kDefaultWorkspace;
-    // chunk buffers take at most a quarter of the limit, so tight limits
+    // the chunk buffer takes at most an eighth of the limit, so tight limits
     // (save_memory) keep room for a batch of slabs
-    const uint64_t plane_budget = std::min<uint64_t>(kPlaneBudget, limit / 4);
+    const uint64_t plane_budget = std::min<uint64_t>(kPlaneBudget, limit / 8);
     // and at most 1024 planes (where the gain levels off), so small planes do
     // not take memory for nothing
-    const size_t jobs_cap = std::max<size_t>(16, std::min<size_t>(1024, plane_budget / 2 / plane_row_bytes));
+    const size_t jobs_cap = std::max<size_t>(16, std::min<size_t>(1024, plane_budget / plane_row_bytes));
     auto layout = [&](int batch, size_t jobs) -> Layout {
         Layout y{};
         y.units = units;
@@ -342,7 +327,6 @@ Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
         size_t w = 0;
         y.off_rowspec = w; w = align_up(w + (size_t)batch * rowspec_bytes);
         y.off_T = w; w = align_up(w + jobs * (plane_row_bytes + edge_row_bytes));
-        y.off_T2 = w; w = align_up(w + jobs * (plane_row_bytes + edge_row_bytes));
         y.off_Tab = w; w = align_up(w + (size_t)batch * tab_bytes);
         y.off_slab = w; w = align_up(w + (size_t)batch * slab_bytes);
         y.off_comp = w; w = align_up(w + (nbatches > 1 ? vol_bytes : 0));
@@ -683,13 +667,7 @@ odt_status odt_bpp3d_plan_create(const odt_bpp3d_desc *desc, odt_bpp3d_plan **ou
         e = odt::configure_adjoint_kernels(P);
     if (e == cudaSuccess && !tilted)
         e = odt::configure_rotate_adjoint_kernels();
-    if (e == cudaSuccess)
-        e = cudaStreamCreateWithFlags(&p->s2, cudaStreamNonBlocking);
-    for (cudaEvent_t *ev : {&p->ev_fork, &p->ev_join, &p->ev_col[0], &p->ev_col[1], &p->ev_row[0], &p->ev_row[1]})
-        if (e == cudaSuccess)
-            e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     if (e != cudaSuccess) {
-        destroy_sync_objects(p);
         cudaFree(p->d_tables);
         delete p;
         return cuda_fail(e, "kernel configuration");
@@ -828,8 +806,13 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *u
             if (e != cudaSuccess)
                 return cuda_fail(e, "rows_line launch");
             lt.end(ns * spec * 8.0 + (double)total * plane_in * 8.0);
-        } else if (timing) {
-            // per-stage timing: the stages one after the other on one stream
+        } else {
+            // column and row stage of a chunk one after the other.  Running
+            // the row stage of one chunk beside the column stage of the next
+            // (two chunk buffers, a second stream) gained 1-2 % on small
+            // planes and lost up to 16 % at 256^3 (step 28.3 ms like this,
+            // 28.7 to 33.0 ms overlapped): a column launch is one wave of
+            // long CTAs, and row CTAs that take its slots stretch it.
             for (int q0 = 0; q0 < total; q0 += lay.jobs) {
                 const int qn = std::min(lay.jobs, total - q0);
                 lt.begin(ODT_STAGE_COLUMNS_PROPAGATE);
@@ -843,34 +826,6 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *u
                     return cuda_fail(e, "rows_inverse launch");
                 lt.end((double)qn * plane_in * 8.0);
             }
-        } else {
-            // chunk pipeline: columns(k) on s into buffer k%2 after rows(k-2)
-            // released it; rows(k) on s2 after columns(k)
-            float2 *Tb[2] = {T, (float2 *)(ws + lay.off_T2)};
-            cudaStream_t s2 = plan->s2;
-            if ((e = cudaEventRecord(plan->ev_fork, s)) || (e = cudaStreamWaitEvent(s2, plan->ev_fork, 0)))
-                return cuda_fail(e, "stream fork");
-            int k = 0;
-            for (int q0 = 0; q0 < total; q0 += lay.jobs, ++k) {
-                const int qn = std::min(lay.jobs, total - q0);
-                const int buf = k & 1;
-                if (k >= 2 && (e = cudaStreamWaitEvent(s, plan->ev_row[buf], 0)))
-                    return cuda_fail(e, "stream wait");
-                e = odt::launch_columns_propagate(P, rowspec, Tb[buf], q0, qn, s);
-                if (e != cudaSuccess)
-                    return cuda_fail(e, "columns_propagate launch");
-                if ((e = cudaEventRecord(plan->ev_col[buf], s)) || (e = cudaStreamWaitEvent(s2, plan->ev_col[buf], 0)))
-                    return cuda_fail(e, "stream order");
-                e = odt::launch_rows_inverse(P, Tb[buf], Tab, slab, q0, qn, s2);
-                if (e != cudaSuccess)
-                    return cuda_fail(e, "rows_inverse launch");
-                if ((e = cudaEventRecord(plan->ev_row[buf], s2)))
-                    return cuda_fail(e, "stream order");
-            }
-            // join: everything after (the resampling, the next batch) waits
-            // for the row stage
-            if ((e = cudaEventRecord(plan->ev_join, s2)) || (e = cudaStreamWaitEvent(s, plan->ev_join, 0)))
-                return cuda_fail(e, "stream join");
         }
         RotParams R;
         R.ny = d.ny;
@@ -1198,7 +1153,6 @@ odt_status odt_bpp3d_plan_destroy(odt_bpp3d_plan *plan)
 {
     if (!plan)
         return ODT_OK;
-    destroy_sync_objects(plan);
     cudaError_t e = cudaFree(plan->d_tables);
     delete plan;
     if (e != cudaSuccess)
