@@ -44,8 +44,9 @@ _TABLE_CACHE_SIZE = 8
 
 
 # Units per angle up to which opposite views are paired.  A unit of two views
-# costs @@ of a single one (256^3 columns), so pairing pays from the first
-# few pairs; the share leaves out sets with stray accidental pairs.
+# costs 1.01 of a single one in the column stage and the same elsewhere (256^3:
+# 0.1176 and 0.1161 ms), so pairing pays from the first few pairs; the share
+# leaves out sets with stray accidental pairs.
 _PAIR_SHARE = 0.9
 
 

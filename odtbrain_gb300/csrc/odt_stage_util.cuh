@@ -211,10 +211,18 @@ constexpr int pow2_len()
 // threads) so that three CTAs of 85 registers fit an SM; measured on the
 // 256^3 workload, 8 per CTA at 64 registers took 27.1 ms for the column
 // stage against 25.7 ms (and 4 per CTA at 2 CTAs of 128 registers 28.7 ms).
+// 256-point columns run 8 per CTA for the same reason, with the propagator
+// steps in registers and long runs: column stage of 90 views of 128^2 1.01 ms
+// with 16, 0.79 with 8, 0.83 with 4; 75 tilted views of 90 x 111 1.22, 1.03,
+// 1.15; 121 views of 101 x 150 4.49, 4.51, 4.23.
 template <class L>
 struct Cfg {
     static constexpr int LPC = (L::TPL >= 256) ? 1 : 256 / L::TPL;
-    static constexpr int KX = (L::TPL == 64) ? 4 : ((L::TPL >= 512) ? 1 : ((512 / L::TPL) > 16 ? 16 : 512 / L::TPL));
+    static constexpr int KX = (L::TPL == 64)    ? 4
+                              : (L::TPL == 32)  ? 8
+                              : (L::TPL >= 512) ? 1
+                              : (512 / L::TPL) > 16 ? 16
+                                                    : 512 / L::TPL;
 };
 template <>
 struct Cfg<GenericLine> {

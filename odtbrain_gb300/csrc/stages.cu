@@ -34,7 +34,7 @@
 //   G X e^(i w z_p) + G X' e^(i w (2 zshift - 1 - z_p)).
 // Both terms are formed before the transforms, so one backward 2D transform
 // per plane and one resampling serve two views.  256^3 from 200 views of a
-// full circle: step 54.2 -> @@ ms.
+// full circle: step 54.2 -> 36.2 ms.
 #include <algorithm>
 #include <type_traits>
 
