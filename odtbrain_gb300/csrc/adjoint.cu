@@ -305,13 +305,8 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_spectrum(StageParams P, L l
                                                               const float2 *Qg, float *dgain, float2 *dagain,
                                                               float2 *W)
 {
-    if (!group_active<KX>(P, blockIdx.x * KX))
-        return;
     extern __shared__ float2 smem[];
     const int n = line.size();  // lNy
-    const int xs = xslots<true>(n);
-    float2 *buf0 = smem, *buf1 = smem + KX * xs, *tw = smem + 2 * KX * xs;
-    copy_twiddles<L>(tw, P.tab.twy, n);
     const int c = threadIdx.x % KX, j = threadIdx.x / KX;
     const int kx = blockIdx.x * KX + c;
     const bool colok = kx < P.lNx;
@@ -327,6 +322,18 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_spectrum(StageParams P, L l
             return;  // no opposite view (uniform over the CTA)
     }
     const int kg = (mirrored && kx) ? lNx - kx : kx;  // the gains' column
+    if (!group_active<KX>(P, blockIdx.x * KX)) {
+        // all-zero columns: nothing reads W there, and the angle gains'
+        // gradient is zero (the other gradients are cleared by the caller)
+        if (dagain && colok) {
+            for (int ky = j; ky < n; ky += L::TPL)
+                dagain[((size_t)a * n + ky) * lNx + kg] = make_float2(0.f, 0.f);
+        }
+        return;
+    }
+    const int xs = xslots<true>(n);
+    float2 *buf0 = smem, *buf1 = smem + KX * xs, *tw = smem + 2 * KX * xs;
+    copy_twiddles<L>(tw, P.tab.twy, n);
     __syncthreads();
     int flip = 0;
     float2 X[L::SLOTS];
