@@ -212,7 +212,7 @@ struct Layout {
     int units, batch;  // slabs (angles, or units of opposite views), slabs per batch
     int spu;           // spectrum slots per slab: 1, or 2 with opposite views
     int jobs;          // (slab, plane) jobs per column/row launch
-    size_t off_rowspec, off_T, off_Tab, off_slab, off_comp, off_rot, ws_bytes;
+    size_t off_spec, off_T, off_Tab, off_slab, off_comp, off_rot, ws_bytes;
     size_t off_Qg, off_W, off_Pg, off_vT, adj_ws_bytes;  // adjoint-only regions after ws_bytes
 };
 }  // namespace
@@ -221,17 +221,17 @@ struct odt_bpp3d_plan {
     odt_bpp3d_desc d;
     int device;      // CUDA device the tables, events and stream belong to
     int nz;
-    int ydefer;      // the row stage adds the y-prefilter terms (StageParams::ydefer)
     int even;        // filter and propagator phase are even in kx (opposite views can be paired)
     Layout lay;      // one angle per slab
     double bx_ca, bx_cb, by_ca, by_cb;  // one-pole solve in the adjoint's form
     int npoles;                         // prefilter poles: 0, 1 or 2
     float kx_solve[16], ky_solve[16];   // boundary_matrix of x and y lines
     int kx_zero_lo, kx_zero_hi;  // all-zero spectrum columns [lo, hi)
+    int ky_zero_lo, ky_zero_hi;  // all-zero spectrum rows [lo, hi)
     int col_slots;               // resident column-stage CTAs (occupancy x SMs)
     // device tables (one allocation)
     void *d_tables;
-    FilterTables tab;
+    FilterTables tab, tabt;
     int *d_status;
 };
 
@@ -273,6 +273,8 @@ StageParams stage_params(const odt_bpp3d_plan *p)
     P.in_c128 = d.input_dtype == ODT_INPUT_C128;
     P.kx_zero_lo = p->kx_zero_lo;
     P.kx_zero_hi = p->kx_zero_hi;
+    P.ky_zero_lo = p->ky_zero_lo;
+    P.ky_zero_hi = p->ky_zero_hi;
     P.bx_ca = (float)p->bx_ca;
     P.bx_cb = (float)p->bx_cb;
     P.by_ca = (float)p->by_ca;
@@ -286,12 +288,12 @@ StageParams stage_params(const odt_bpp3d_plan *p)
     P.col_slots = p->col_slots;
     P.zshift = (float)d.z_shift;
     P.tab = p->tab;
+    P.tabt = p->tabt;
     P.gain = nullptr;
     P.again = nullptr;
     P.status = p->d_status;
-    P.ydefer = p->ydefer;
     P.units = nullptr;
-    P.yedge_off = p->ydefer ? (long long)p->lay.jobs * d.ny * d.pad_nx : 0;
+    P.trow0 = P.trows = 0;
     return P;
 }
 
@@ -302,13 +304,17 @@ Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
     const odt_bpp3d_desc &d = p->d;
     const int lNy = d.pad_ny, lNx = d.pad_nx, nz = p->nz, np = p->npoles;
     const bool tilted = d.geometry == ODT_GEOM_AFFINE3D;
-    const size_t plane_row_bytes = (size_t)d.ny * lNx * 8;           // one job's column-stage output
-    const size_t edge_row_bytes = p->ydefer ? (size_t)4 * np * lNx * 8 : 0;  // its y-prefilter edge samples
+    // one job's column-stage output: transposed [row][lNy] in the forward
+    // execution, [y][lNx] in the adjoint
+    const size_t plane_row_bytes =
+        std::max((size_t)odt::transposed(stage_params(p)).trows * lNy, (size_t)d.ny * lNx) * 8;
+    const size_t spec_bytes = (size_t)spu * lNy * lNx * 8;           // one slab's spectra
     // one coefficient slab [z][x][ypitch] (the adjoint's slab gradients
-    // [y][z][x] fit too)
-    const size_t slab_bytes = (size_t)nz * odt::yaxis_slab_pitch(d.ny) * d.nx * 8;
-    const size_t rowspec_bytes = (size_t)spu * lNy * lNx * 8;        // one slab's row spectra
-    const size_t tab_bytes = np ? (size_t)2 * np * d.ny * lNx * 8 : 0;  // one slab's z-boundary rows
+    // [y][z][x] fit too).  The row spectra, dead before the slab is written,
+    // share its place.
+    const size_t slab_bytes = std::max((size_t)nz * odt::yaxis_slab_pitch(d.ny) * d.nx * 8, spec_bytes);
+    // one slab's z-boundary rows (not transposed for single-row planes)
+    const size_t tab_bytes = (size_t)2 * np * std::max((size_t)d.nx * lNy, (size_t)d.ny * lNx) * 8;
     const size_t vol_bytes = (size_t)nz * d.ny * d.nx * 8;           // compensation buffer
     const uint64_t limit = d.workspace_limit ? d.workspace_limit : kDefaultWorkspace;
     // the chunk buffer takes at most an eighth of the limit, so tight limits
@@ -325,15 +331,15 @@ Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
         y.jobs = (int)jobs;
         const int nbatches = (units + batch - 1) / batch;
         size_t w = 0;
-        y.off_rowspec = w; w = align_up(w + (size_t)batch * rowspec_bytes);
-        y.off_T = w; w = align_up(w + jobs * (plane_row_bytes + edge_row_bytes));
+        y.off_spec = w; w = align_up(w + (size_t)batch * spec_bytes);
+        y.off_T = w; w = align_up(w + jobs * plane_row_bytes);
         y.off_Tab = w; w = align_up(w + (size_t)batch * tab_bytes);
         y.off_slab = w; w = align_up(w + (size_t)batch * slab_bytes);
         y.off_comp = w; w = align_up(w + (nbatches > 1 ? vol_bytes : 0));
         y.off_rot = w;
         w = align_up(w + odt::rotate_scratch_bytes(batch, d.ny, d.nx, nz, tilted ? 1 : 0));
         y.ws_bytes = w;
-        const size_t spec_b = (size_t)batch * rowspec_bytes;
+        const size_t spec_b = (size_t)batch * spec_bytes;
         y.off_Qg = w; w = align_up(w + spec_b);
         y.off_W = w; w = align_up(w + spec_b);
         y.off_Pg = w; w = align_up(w + spec_b);
@@ -544,28 +550,34 @@ odt_status odt_bpp3d_plan_create(const odt_bpp3d_desc *desc, odt_bpp3d_plan **ou
             }
         }
     }
-    // largest run of all-zero filter columns around the Nyquist column
-    // (outside the |k| < km disc): neither computed nor read
-    {
-        auto zero_col = [&](int kx) {
-            for (int ky = 0; ky < lNy; ++ky) {
-                const size_t k = (size_t)ky * lNx + kx;
-                if (desc->filter[2 * k] != 0.0 || desc->filter[2 * k + 1] != 0.0)
-                    return false;
-            }
-            return true;
-        };
-        int lo = lNx / 2, hi = lNx / 2;
-        if (zero_col(lNx / 2)) {
-            hi = lNx / 2 + 1;
-            while (lo > 0 && zero_col(lo - 1))
-                --lo;
-            while (hi < lNx && zero_col(hi))
-                ++hi;
-        }
-        p->kx_zero_lo = lo;
-        p->kx_zero_hi = hi;
-    }
+    // largest runs of all-zero filter columns and rows around the Nyquist
+    // frequency (outside the |k| < km disc): neither computed nor read
+    auto zero_run = [](int n, auto &&zero, int *lo, int *hi) {
+        *lo = *hi = n / 2;
+        if (!zero(n / 2))
+            return;
+        *hi = n / 2 + 1;
+        while (*lo > 0 && zero(*lo - 1))
+            --*lo;
+        while (*hi < n && zero(*hi))
+            ++*hi;
+    };
+    auto zero_at = [&](int ky, int kx) {
+        const size_t k = (size_t)ky * lNx + kx;
+        return desc->filter[2 * k] == 0.0 && desc->filter[2 * k + 1] == 0.0;
+    };
+    zero_run(lNx, [&](int kx) {
+        for (int ky = 0; ky < lNy; ++ky)
+            if (!zero_at(ky, kx))
+                return false;
+        return true;
+    }, &p->kx_zero_lo, &p->kx_zero_hi);
+    zero_run(lNy, [&](int ky) {
+        for (int kx = 0; kx < lNx; ++kx)
+            if (!zero_at(ky, kx))
+                return false;
+        return true;
+    }, &p->ky_zero_lo, &p->ky_zero_hi);
     for (int m = 0; m < lNx; ++m)
         twx[m] = make_float2((float)std::cos(-2.0 * M_PI * m / lNx), (float)std::sin(-2.0 * M_PI * m / lNx));
     for (int m = 0; m < lNy; ++m)
@@ -577,6 +589,11 @@ odt_status odt_bpp3d_plan_create(const odt_bpp3d_desc *desc, odt_bpp3d_plan **ou
     const size_t oS = o; o = align_up(o + K * 8);
     const size_t oA = o; o = align_up(o + 2 * K * 8);
     const size_t oB = o; o = align_up(o + 2 * K * 8);
+    // the propagator and boundary tables in the transposed order
+    const size_t oWt = o; o = align_up(o + K * 8);
+    const size_t oSt_ = o; o = align_up(o + K * 8);
+    const size_t oAt = o; o = align_up(o + 2 * K * 8);
+    const size_t oBt = o; o = align_up(o + 2 * K * 8);
     const size_t oTx = o; o = align_up(o + (size_t)lNx * 8);
     const size_t oTy = o; o = align_up(o + (size_t)lNy * 8);
     const size_t oZ = o; o = align_up(o + 2 * odt::ZPOW_N * 4);
@@ -601,10 +618,20 @@ odt_status odt_bpp3d_plan_create(const odt_bpp3d_desc *desc, odt_bpp3d_plan **ou
                                               : cuda_fail(e, "cudaMalloc");
     }
     char *base = (char *)p->d_tables;
+    auto transpose = [&](const std::vector<float2> &src) {
+        std::vector<float2> t(src.size());
+        for (size_t i = 0; i < src.size(); i += K)
+            for (int ky = 0; ky < lNy; ++ky)
+                for (int kx = 0; kx < lNx; ++kx)
+                    t[i + (size_t)kx * lNy + ky] = src[i + (size_t)ky * lNx + kx];
+        return t;
+    };
+    const std::vector<float2> Wt = transpose(W), Stt = transpose(S), ALt = transpose(AL), BEt = transpose(BE);
     struct Up { size_t off; const void *src; size_t n; } ups[] = {
         {oG, G.data(), K * 8}, {oW, W.data(), K * 8}, {oS, S.data(), K * 8}, {oA, AL.data(), 2 * K * 8},
         {oB, BE.data(), 2 * K * 8}, {oTx, twx.data(), (size_t)lNx * 8}, {oTy, twy.data(), (size_t)lNy * 8},
-        {oZ, zp.data(), 2 * odt::ZPOW_N * 4}};
+        {oZ, zp.data(), 2 * odt::ZPOW_N * 4}, {oWt, Wt.data(), K * 8}, {oSt_, Stt.data(), K * 8},
+        {oAt, ALt.data(), 2 * K * 8}, {oBt, BEt.data(), 2 * K * 8}};
     for (const Up &u : ups) {
         e = cudaMemcpy(base + u.off, u.src, u.n, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
@@ -627,17 +654,15 @@ odt_status odt_bpp3d_plan_create(const odt_bpp3d_desc *desc, odt_bpp3d_plan **ou
     p->tab.twx = (const float2 *)(base + oTx);
     p->tab.twy = (const float2 *)(base + oTy);
     p->tab.zpow = (const float *)(base + oZ);
+    p->tabt = p->tab;
+    p->tabt.G = nullptr;
+    p->tabt.wsplit = (const float2 *)(base + oWt);
+    p->tabt.step = (const float2 *)(base + oSt_);
+    p->tabt.alpha = (const float2 *)(base + oAt);
+    p->tabt.beta = (const float2 *)(base + oBt);
+    std::swap(p->tabt.twx, p->tabt.twy);
     p->d_status = (int *)(base + oSt);
 
-    // tilted path, order >= 2: the column stage leaves the y-prefilter
-    // terms to the row stage and stores each job's raw edge samples (4 np
-    // rows) after the chunk's jobs
-    p->lay = Layout{};
-    p->ydefer = 0;
-    {
-        const StageParams G = stage_params(p);
-        p->ydefer = (tilted && pf && !odt::single_row_plan(G)) ? 1 : 0;
-    }
     p->lay = make_layout(p, d.num_angles, 1);
 
     // opposite views share a slab through the mirrored spectrum, which needs
@@ -657,7 +682,7 @@ odt_status odt_bpp3d_plan_create(const odt_bpp3d_desc *desc, odt_bpp3d_plan **ou
     StageParams P = stage_params(p);
     e = odt::configure_kernels(P);
     if (e == cudaSuccess) {
-        p->col_slots = odt::columns_slots(P);
+        p->col_slots = odt::columns_slots(odt::transposed(P));
         P.col_slots = p->col_slots;
     P.zshift = (float)d.z_shift;
     }
@@ -757,11 +782,14 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *u
     P.gain = gain;
     const size_t spec_elems = (size_t)plan->d.pad_ny * plan->d.pad_nx;
     char *ws = (char *)workspace;
-    float2 *rowspec = (float2 *)(ws + lay.off_rowspec);
+    float2 *fspec = (float2 *)(ws + lay.off_spec);
     float2 *T = (float2 *)(ws + lay.off_T);
     float2 *Tab = (float2 *)(ws + lay.off_Tab);
     float2 *slab = (float2 *)(ws + lay.off_slab);
     float2 *comp = (float2 *)(ws + lay.off_comp);
+    // row spectra: in the slab's place, in place of the filtered spectra for
+    // single-row planes
+    float2 *rowspec = odt::single_row_plan(P) ? fspec : slab;
     void *rot_scratch = ws + lay.off_rot;
     const size_t in_elem = d.input_dtype == ODT_INPUT_C128 ? 16 : 8;
     const int geo_stride = d.geometry == ODT_GEOM_AFFINE3D ? 12 : 6;
@@ -792,21 +820,32 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *u
         if (e != cudaSuccess)
             return cuda_fail(e, "rows_forward launch");
         lt.end(ns * (plane_in * in_elem + spec * 8.0));
+        const int total = nb * plan->nz;
         lt.begin(ODT_STAGE_COLUMNS_PROPAGATE);
-        e = odt::launch_columns_spectrum(P, rowspec, Tab, nb, s);
+        if (odt::single_row_plan(P))
+            e = odt::launch_spectrum_line(P, fspec, Tab, nb, s);
+        else
+            e = odt::launch_columns_spectrum(P, rowspec, fspec, ns, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "columns_spectrum launch");
         lt.end(0.0);
-        const int total = nb * plan->nz;
         if (odt::single_row_plan(P)) {
             // single-row planes: the column stage is the identity and runs
             // inside the row stage, one launch over the batch's jobs
             lt.begin(ODT_STAGE_ROWS_INVERSE);
-            e = odt::launch_rows_line(P, rowspec, Tab, slab, 0, total, s);
+            e = odt::launch_rows_line(P, fspec, Tab, slab, 0, total, s);
             if (e != cudaSuccess)
                 return cuda_fail(e, "rows_line launch");
             lt.end(ns * spec * 8.0 + (double)total * plane_in * 8.0);
         } else {
+            const StageParams Pt = odt::transposed(P);
+            if (d.intp_order >= 2) {
+                lt.begin(ODT_STAGE_COLUMNS_PROPAGATE);
+                e = odt::launch_columns_boundary(Pt, fspec, Tab, nb, s);
+                if (e != cudaSuccess)
+                    return cuda_fail(e, "columns_boundary launch");
+                lt.end(0.0);
+            }
             // column and row stage of a chunk one after the other.  Running
             // the row stage of one chunk beside the column stage of the next
             // (two chunk buffers, a second stream) gained 1-2 % on small
@@ -816,12 +855,12 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *u
             for (int q0 = 0; q0 < total; q0 += lay.jobs) {
                 const int qn = std::min(lay.jobs, total - q0);
                 lt.begin(ODT_STAGE_COLUMNS_PROPAGATE);
-                e = odt::launch_columns_propagate(P, rowspec, T, q0, qn, s);
+                e = odt::launch_columns_propagate(Pt, fspec, T, q0, qn, s);
                 if (e != cudaSuccess)
                     return cuda_fail(e, "columns_propagate launch");
                 lt.end((double)qn / plan->nz * lay.spu * spec * 8.0);
                 lt.begin(ODT_STAGE_ROWS_INVERSE);
-                e = odt::launch_rows_inverse(P, T, Tab, slab, q0, qn, s);
+                e = odt::launch_rows_inverse(Pt, T, Tab, slab, q0, qn, s);
                 if (e != cudaSuccess)
                     return cuda_fail(e, "rows_inverse launch");
                 lt.end((double)qn * plane_in * 8.0);
@@ -944,7 +983,7 @@ static odt_status run_adjoint(const odt_bpp3d_plan *plan, const Layout &lay, con
     StageParams P = stage_params(plan);
     P.gain = gain;
     char *ws = (char *)workspace;
-    float2 *rowspec = (float2 *)(ws + lay.off_rowspec);
+    float2 *rowspec = (float2 *)(ws + lay.off_spec);
     float2 *T = (float2 *)(ws + lay.off_T);
     float2 *slab = (float2 *)(ws + lay.off_slab);
     float2 *Qg = (float2 *)(ws + lay.off_Qg);
@@ -1071,7 +1110,7 @@ static int64_t count_launches(const odt_bpp3d_plan *plan, const Layout &lay)
         if (odt::single_row_plan(stage_params(plan)))
             n += 4;  // row spectra, filtered spectra, fused column + row stage, resampling
         else
-            n += 3 + 2 * ((total + lay.jobs - 1) / lay.jobs);
+            n += 3 + (plan->d.intp_order >= 2) + 2 * ((total + lay.jobs - 1) / lay.jobs);
         if (plan->d.geometry == ODT_GEOM_Y_AXIS)
             n += 1;  // per-(slab, tile) geometry setup
     }

@@ -60,6 +60,7 @@ struct StageParams {
     int in_c128;      // input sinogram is complex128
     int kx_zero_lo, kx_zero_hi;  // spectrum columns in [lo, hi) are all zero
                                  // (outside the |k| < km disc)
+    int ky_zero_lo, ky_zero_hi;  // the same for spectrum rows
     float bx_ca, bx_cb;  // x-prefilter boundary solve (n = nx), one pole (adjoint)
     float by_ca, by_cb;  // y-prefilter boundary solve (n = ny; zero for ny = 1)
     int npoles;          // prefilter poles: 1 (orders 2, 3), 2 (orders 4, 5)
@@ -69,7 +70,8 @@ struct StageParams {
                          // ny rounded up to a multiple of 32, 1 for ny == 1)
     int col_slots;       // resident CTAs of the column stage on the device
     float zshift;        // plane p sits at z = p - nz/2 + zshift
-    FilterTables tab;
+    FilterTables tab;   // [ky][kx]
+    FilterTables tabt;  // [kx][ky] (G is not kept in this order)
     const float *gain;   // optional real per-frequency gain [lNy*lNx] (NULL: 1)
     const float2 *again; // optional complex per-angle gain [A][lNy*lNx], this
                          // batch's first angle at again (NULL: 1); with
@@ -79,12 +81,9 @@ struct StageParams {
     // unit.  NULL: one angle per unit, numbered within the batch.
     const int2 *units;
     int *status;
-    // Tilted path, order >= 2 (ydefer = 1): the column stage leaves the
-    // y-prefilter boundary terms to the row stage and stores the raw y-line samples around the crop's ends, 4
-    // npoles rows of lNx per job (edge_row order), at T + yedge_off + (q -
-    // q0) * 4 npoles * lNx of the job chunk's buffer T.
-    int ydefer;
-    long long yedge_off;
+    int trow0, trows;    // transposed(): the column stage's output T holds
+                         // trows rows of a job, from padded row trow0 on
+    int tedge[8];        // transposed(): the T rows of the edge samples
 };
 
 // y pitch of the slab layout [a][z][x][y]
@@ -107,18 +106,26 @@ struct RotParams {
 // weights start at the batch's first angle, with units at angle 0.
 cudaError_t launch_rows_forward(const StageParams &P, const void *sino, const double *weights, int nslots,
                                 float2 *rowspec, cudaStream_t s);
-// Row spectra -> filtered spectra, in place, and (order >= 2) the
-// z-prefilter boundary rows Tab[unit][2 poles][ny][lNx].
-cudaError_t launch_columns_spectrum(const StageParams &P, float2 *rowspec, float2 *Tab, int nunits, cudaStream_t s);
+// Row spectra -> filtered spectra of the slots, transposed [slot][kx][ky].
+cudaError_t launch_columns_spectrum(const StageParams &P, const float2 *rowspec, float2 *spec, int nslots,
+                                    cudaStream_t s);
+// The parameters of the transposed plane: y and x exchange their roles in
+// every field.  The boundary, propagation and backward row stages take them.
+StageParams transposed(const StageParams &P);
+// Order >= 2: the z-prefilter boundary rows Tab[unit][2 poles][ny][lNx].
+cudaError_t launch_columns_boundary(const StageParams &P, const float2 *spec, float2 *Tab, int nunits,
+                                    cudaStream_t s);
 cudaError_t launch_columns_propagate(const StageParams &P, const float2 *spec, float2 *T, int q0, int qn,
                                      cudaStream_t s);
 // Single-row planes (lNy == ny == 1, slab pitch 1): the column and row
-// stages fused in one launch over jobs [q0, q0 + qn), from the filtered spectra.
+// stages fused in one launch over jobs [q0, q0 + qn), from the filtered spectra
+// (launch_spectrum_line: row spectra -> filtered spectra in place, and Tab).
 bool single_row_plan(const StageParams &P);
-// Square power-of-two padded planes (N >= 256) cropped to their centred
+// Square power-of-two padded planes (N >= 64) cropped to their centred
 // half (ny = nx = N/2 from N/4): the column and row stages then run
 // kernels whose crop and edge positions are compile-time constants.
 bool half_crop(const StageParams &P);
+cudaError_t launch_spectrum_line(const StageParams &P, float2 *spec, float2 *Tab, int nunits, cudaStream_t s);
 cudaError_t launch_rows_line(const StageParams &P, const float2 *spec, const float2 *Tab, float2 *slab, int q0,
                              int qn, cudaStream_t s);
 cudaError_t launch_rows_inverse(const StageParams &P, const float2 *T, const float2 *Tab, float2 *slab, int q0,

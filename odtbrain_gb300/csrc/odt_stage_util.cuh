@@ -91,13 +91,6 @@ __host__ __device__ constexpr bool edge_used(int slot, int np)
 {
     return ((slot & 3) >> 1) < np;
 }
-// Row of a used edge slot among the 4 np rows of the deferred y-prefilter's
-// edge samples (the slots at the crop's start, then those at its end).
-__host__ __device__ constexpr int edge_row(int slot, int np)
-{
-    return slot < 4 ? slot : 2 * np + (slot - 4);
-}
-
 // Coefficients of an NP-pole prefilter (NP = 1: orders 2, 3; NP = 2:
 // orders 4, 5) from the edge slots: c[i] = A_(i+1), c[NP + i] = B_(i+1).
 // K is the 2NP x 2NP boundary solve, row-major.  NP is a compile-time
@@ -235,15 +228,8 @@ inline size_t smem_rows(int n)
 {
     return (size_t)(2 * Cfg<L>::LPC * xslots<false>(n) + tw_slots(n) + EDGE_SLOTS * Cfg<L>::LPC) * sizeof(float2);
 }
-// k_rows_inverse_half: the exchange buffers, the twiddle table and the
-// edge samples.
-template <class L>
-inline size_t smem_rows_half(int n)
-{
-    return (size_t)(2 * Cfg<L>::LPC * xslots<false>(n) + tw_slots(n) + EDGE_SLOTS * Cfg<L>::LPC) * sizeof(float2);
-}
-// k_columns_spectrum: the exchange buffers, the twiddle table and the edge
-// samples.
+// k_columns_spectrum and k_columns_boundary: the exchange buffers, the twiddle
+// table and the edge samples.
 template <class L>
 inline size_t smem_cols(int n)
 {

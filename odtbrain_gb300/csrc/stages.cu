@@ -5,13 +5,22 @@
 //   pad -> forward 2D FFT -> *prefactor/(lNx*lNy) -> for every z plane p:
 //   *exp(i km (M-1) z_p) -> unnormalised backward 2D FFT -> crop.
 //
-// GB300 decomposition (four kernels, all lines in registers):
+// GB300 decomposition (all lines in registers):
 //   rows_forward       padded+weighted rows, forward FFT along x
-//   columns_spectrum   forward FFT along y, filter multiply (in place), and
-//                      the z-prefilter boundary rows
+//   columns_spectrum   forward FFT along y, filter multiply -> filtered
+//                      spectrum, stored transposed [kx][ky]
+//   columns_boundary   z-prefilter boundary rows (once per slab)
 //   columns_propagate  for a run of z planes: propagator (exact anchor +
-//                      complex recurrence), backward FFT along y, crop in y
-//   rows_inverse       backward FFT along x, crop in x -> coefficient slab
+//                      complex recurrence), backward FFT along x, crop in x
+//   rows_inverse       backward FFT along y, crop in y -> coefficient slab
+//
+// The last three work on the transposed plane (launched with the StageParams
+// of transposed()): their "columns" run along x and their "rows" along y, so
+// that a finished row lies along the slab's innermost axis and is stored from
+// registers, contiguously.  With the rows along x every row group had to be
+// transposed through shared memory behind three barriers and stored in runs
+// of 32 bytes: row stage of 256^3 from 200 views 10.4 -> 8.4 ms (whole step
+// 28.3 -> 27.0 ms), tilted 200^3 19.6 -> 16.1 ms.
 //
 // The B-spline prefilter that scipy.ndimage applies before resampling
 // (mirror boundaries, along z and x of every plane; along all three axes on
@@ -138,50 +147,18 @@ __global__ void __launch_bounds__(LPC * L::TPL) k_rows_forward(StageParams P, L 
 // Column helpers shared by the two column kernels.  A CTA owns KX adjacent
 // spectrum columns kx; thread (c, j) holds rows ky = j + r*TPL of column c.
 
-// Column kx of the row spectra of one slot, forward FFT along y, times the
-// filter table G (which includes the prefilter particular factors) and the
-// gains.  `kg` is the column whose gains apply (the mirrored one for an
-// opposite view), `again` the view's own gain map.
-template <class L, int KX>
-__device__ __forceinline__ void column_spectrum(const StageParams &P, const L &line, const float2 *spec, int kx,
-                                                int kg, const float2 *again, bool colok, int c, int j, float2 *buf0,
-                                                float2 *buf1, const float2 *tw, int &flip, float2 (&v)[L::SLOTS])
-{
-    const int n = line.size();
-#pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int ky = j + r * L::TPL;
-        v[r] = (colok && ky < n) ? spec[(size_t)ky * P.lNx + kx] : make_float2(0.f, 0.f);
-    }
-    line.template run<-1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
-#pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int ky = j + r * L::TPL;
-        if (colok && ky < n) {
-            const size_t row = (size_t)ky * P.lNx;
-            v[r] = cmul(v[r], P.tab.G[row + kx]);
-            if (P.gain)
-                v[r] = cscale(v[r], P.gain[row + kg]);
-            if (again)
-                v[r] = cmul(v[r], again[row + kg]);
-        } else {
-            v[r] = make_float2(0.f, 0.f);
-        }
-    }
-}
-
-// The edge samples of the y-prefilter solve that thread j holds after a
-// column's backward transform: bit 8 r + e is set when slot r holds the
-// sample of edge slot e (the same for every plane of the CTA, so it is
-// computed once).  Power-of-two lines (8 slots).
+// The edge samples of a prefilter's boundary solve that thread j holds after a
+// line's backward transform (crop of `len` samples from `pad`): bit 8 r + e
+// is set when slot r holds the sample of edge slot e (the same for every line
+// of the CTA, so it is computed once).  Power-of-two lines (8 slots).
 template <class L, int NP>
-__device__ __forceinline__ unsigned long long edge_holdings(const StageParams &P, int n, int j)
+__device__ __forceinline__ unsigned long long edge_holdings(int pad, int len, int n, int j)
 {
     unsigned long long m = 0;
 #pragma unroll
     for (int e = 0; e < EDGE_SLOTS; ++e) {
         if (edge_used(e, NP)) {
-            const int pos = (P.padyl + edge_offset(e, P.ny) + 2 * n) % n;
+            const int pos = (pad + edge_offset(e, len) + 2 * n) % n;
             if (pos % L::TPL == j)
                 m |= 1ull << (8 * (pos / L::TPL) + e);
         }
@@ -189,139 +166,118 @@ __device__ __forceinline__ unsigned long long edge_holdings(const StageParams &P
     return m;
 }
 
-// Backward FFT along y of v, then the y-prefilter boundary terms (YF > 0:
-// tilted path, order >= 2, YF poles) and the cropped store dst[yy * lNx]
-// for yy < ny.  DEFER (P.ydefer): the terms' coefficients need the line's
-// edge samples, held by a few other threads, so adding them here costs a
-// barrier per line; instead the raw edge samples go to yedge[row * lNx]
-// (rows edge_row(e)), the crop is stored raw, and the row stage adds the
-// terms.  `eheld`: edge_holdings of this thread (power-of-two lines).
-template <class L, int KX, int YF, bool TW2 = false, bool DEFER = false>
+// Backward FFT along the column of v, then the prefilter boundary terms (YF
+// poles) and the cropped store dst[yy * lNx] for yy < ny.
+template <class L, int KX, int YF>
 __device__ __forceinline__ void column_inverse_store(const StageParams &P, const L &line, float2 (&v)[L::SLOTS],
                                                      int c, int j, bool colok, float2 *buf0, float2 *buf1,
-                                                     const float2 *tw, float2 *edge, int &flip, float2 *dst,
-                                                     float2 *yedge = nullptr, unsigned long long eheld = 0)
+                                                     const float2 *tw, float2 *edge, int &flip, float2 *dst)
 {
     const int n = line.size();
     const int ny = P.ny, padyl = P.padyl;
-    line.template run<1, true, TW2>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
-    constexpr bool yfix = YF > 0 && !DEFER;
-    constexpr int NPY = YF > 0 ? YF : 1;
-    float2 cf[2 * NPY];
-    if constexpr (YF > 0 && DEFER) {
-        if constexpr (L::SLOTS <= 8) {
-            if (eheld && colok) {
+    line.template run<1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
+    // u around the crop's ends (periodic over the padded height)
 #pragma unroll
-                for (int r = 0; r < L::SLOTS; ++r) {
-                    const unsigned m = (unsigned)(eheld >> (8 * r)) & 0xffu;
-                    if (m) {
-#pragma unroll
-                        for (int e = 0; e < EDGE_SLOTS; ++e)
-                            if (edge_used(e, NPY) && (m & (1u << e)))
-                                yedge[(size_t)edge_row(e, NPY) * P.lNx] = v[r];
-                    }
-                }
-            }
-        } else if (colok) {
-#pragma unroll
-            for (int e = 0; e < EDGE_SLOTS; ++e) {
-                float2 t;
-                if (edge_used(e, NPY) && held<L>(v, j, (padyl + edge_offset(e, ny) + 2 * n) % n, t))
-                    yedge[(size_t)edge_row(e, NPY) * P.lNx] = t;
-            }
-        }
+    for (int e = 0; e < EDGE_SLOTS; ++e) {
+        float2 t;
+        if (edge_used(e, YF) && held<L>(v, j, (padyl + edge_offset(e, ny) + 2 * n) % n, t))
+            edge[c * EDGE_SLOTS + e] = t;
     }
-    if constexpr (yfix) {
-        // u around the crop's ends (periodic over the padded height)
-#pragma unroll
-        for (int e = 0; e < EDGE_SLOTS; ++e) {
-            float2 t;
-            if (edge_used(e, NPY) && held<L>(v, j, (padyl + edge_offset(e, ny) + 2 * n) % n, t))
-                edge[c * EDGE_SLOTS + e] = t;
-        }
-        __syncthreads();
-        pf_coefs<NPY>(P.kys, edge + c * EDGE_SLOTS, cf);
-    }
+    __syncthreads();
+    float2 cf[2 * YF];
+    pf_coefs<YF>(P.kys, edge + c * EDGE_SLOTS, cf);
     if (!colok)
         return;
 #pragma unroll
     for (int r = 0; r < L::SLOTS; ++r) {
         const int yy = j + r * L::TPL - padyl;
-        if (yy >= 0 && yy < ny) {
-            float2 o = v[r];
-            if constexpr (yfix)
-                o = pf_apply<NPY>(P, cf, yy, ny, o);
-            dst[(size_t)yy * P.lNx] = o;
-        }
+        if (yy >= 0 && yy < ny)
+            dst[(size_t)yy * P.lNx] = pf_apply<YF>(P, cf, yy, ny, v[r]);
     }
-}
-
-// Half-crop form of column_inverse_store (half_crop plans: ny = N/2 rows
-// starting at N/4 of a power-of-two column of N).  Thread j then holds the
-// cropped rows in slots 2..5, row j + TPL*(r-2), and the four edge samples
-// of the y-prefilter solve at compile-time slots, so the crop needs no
-// predicates and the stores use constant offsets from one row pointer.
-// dst points at row 0 of the job's T block, column kx (row stride N).
-// DEFER (P.ydefer): as in column_inverse_store, the raw edge samples go to
-// yedge[row * N] (their holders and slots are compile-time here) and the
-// row stage adds the y-prefilter terms.
-template <class L, int KX, int YF, bool TW2, bool DEFER = false>
-__device__ __forceinline__ void column_inverse_store_half(const StageParams &P, const L &line, float2 (&v)[L::SLOTS],
-                                                          int c, int j, float2 *buf0, float2 *buf1,
-                                                          const float2 *tw, float2 *edge, int &flip, float2 *dst,
-                                                          float2 *yedge = nullptr)
-{
-    constexpr int N = L::N, TPL = L::TPL, NY = N / 2, PAD = N / 4;
-    line.template run<1, true, TW2>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
-    if constexpr (YF > 0 && DEFER) {
-#pragma unroll
-        for (int e = 0; e < EDGE_SLOTS; ++e) {
-            if (edge_used(e, YF)) {
-                const int pos = PAD + edge_offset(e, NY);
-                if (j == pos % TPL)
-                    yedge[(size_t)edge_row(e, YF) * N] = v[pos / TPL];
-            }
-        }
-    } else if constexpr (YF > 0) {
-        // y-prefilter boundary terms from u around the crop's ends
-        // (compile-time positions)
-#pragma unroll
-        for (int e = 0; e < EDGE_SLOTS; ++e) {
-            float2 t;
-            if (edge_used(e, YF) && held<L>(v, j, PAD + edge_offset(e, NY), t))
-                edge[c * EDGE_SLOTS + e] = t;
-        }
-        __syncthreads();
-        float2 cf[2 * YF];
-        pf_coefs<YF>(P.kys, edge + c * EDGE_SLOTS, cf);
-#pragma unroll
-        for (int r = 2; r <= 5; ++r)
-            v[r] = pf_apply<YF>(P, cf, j + TPL * (r - 2), NY, v[r]);
-    }
-    float2 *d = dst + (size_t)j * N;
-#pragma unroll
-    for (int r = 2; r <= 5; ++r)
-        d[(r - 2) * TPL * N] = v[r];
 }
 
 // ---------------------------------------------------------------------------
-// (b0) filtered spectra, once per view: forward FFT along y of the row
-// spectra times the filter and the gains, written back in place, and (order
-// >= 2) the z-prefilter boundary rows of the unit.  The prefiltered
-// propagator of plane p is E_p + alpha z^p + beta z^(nz-1-p); by linearity
-// the alpha and beta parts are transformed once here (Tab[u][0] = column
-// transform of G X alpha, Tab[u][1] of G X beta) and the row stage adds
+// (a2) filtered spectra, once per slot: forward FFT along y of the row
+// spectra times the filter and the gains, stored transposed [kx][ky] (zero for
+// a unit without opposite view).  The column kernel used to redo this
+// transform at the head of every run of planes and keep its result in shared
+// memory for the re-anchoring; read from here (16 bytes per element and 32
+// planes) that shared memory is free.
+template <class L, int KX>
+__global__ void __launch_bounds__(KX * L::TPL) k_columns_spectrum(StageParams P, L line, const float2 *rowspec,
+                                                                  float2 *spec)
+{
+    extern __shared__ float2 smem[];
+    const int n = line.size();
+    const int ls = xslots<true>(n);
+    float2 *buf0 = smem, *buf1 = smem + KX * ls, *tw = smem + 2 * KX * ls;
+    const int c = threadIdx.x % KX, j = threadIdx.x / KX;
+    const int kx = blockIdx.x * KX + c;
+    const bool colok = kx < P.lNx;
+    const int slot = blockIdx.y;
+    const size_t K = (size_t)P.lNy * P.lNx;
+    int a = slot, kg = kx;
+    if (P.units) {
+        const int2 u = P.units[slot >> 1];
+        a = (slot & 1) ? u.y : u.x;
+        if ((slot & 1) && kx)
+            kg = P.lNx - kx;  // the gains' column of a mirrored view
+    }
+    float2 v[L::SLOTS];
+    // (the early cases are uniform over the CTA)
+    if (a < 0 || !group_active<KX>(P, blockIdx.x * KX)) {
+#pragma unroll
+        for (int r = 0; r < L::SLOTS; ++r)
+            v[r] = make_float2(0.f, 0.f);
+    } else {
+        copy_twiddles<L>(tw, P.tab.twy, n);
+        const float2 *src = rowspec + slot * K;
+#pragma unroll
+        for (int r = 0; r < L::SLOTS; ++r) {
+            const int ky = j + r * L::TPL;
+            v[r] = (colok && ky < n) ? src[(size_t)ky * P.lNx + kx] : make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+        int flip = 0;
+        line.template run<-1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
+#pragma unroll
+        for (int r = 0; r < L::SLOTS; ++r) {
+            const int ky = j + r * L::TPL;
+            if (colok && ky < n) {
+                const size_t row = (size_t)ky * P.lNx;
+                // (the zero band's row spectra do not reach the result)
+                v[r] = column_active(P, kx) ? cmul(v[r], P.tab.G[row + kx]) : make_float2(0.f, 0.f);
+                if (P.gain)
+                    v[r] = cscale(v[r], P.gain[row + kg]);
+                if (P.again)
+                    v[r] = cmul(v[r], P.again[a * K + row + kg]);
+            }
+        }
+    }
+    if (!colok)
+        return;
+    float2 *dst = spec + slot * K + (size_t)kx * n;
+#pragma unroll
+    for (int r = 0; r < L::SLOTS; ++r) {
+        const int ky = j + r * L::TPL;
+        if (ky < n)
+            dst[ky] = v[r];
+    }
+}
+
+// (b0) z-prefilter boundary rows, once per slab (order >= 2).  The
+// prefiltered propagator of plane p is E_p + alpha z^p + beta z^(nz-1-p); by
+// linearity the alpha and beta parts are transformed once here (Tab[u][0] =
+// column transform of G X alpha, Tab[u][1] of G X beta) and the row stage adds
 // z^p Tab[u][0] + z^(nz-1-p) Tab[u][1] to the first and last planes' rows.
 // The opposite view of a unit (PAIR) enters with alpha and beta exchanged:
 // its plane p is plane nz-1-p of its own slab.
-// The column kernel used to redo this transform at the head of every run of
-// planes and keep its result in shared memory for the re-anchoring; read
-// from here (16 bytes per element and 32 planes) that shared memory is free.
 template <class L, int KX, int YF, bool PAIR>
-__global__ void __launch_bounds__(KX * L::TPL) k_columns_spectrum(StageParams P, L line, float2 *rowspec, float2 *Tab)
+__global__ void __launch_bounds__(KX * L::TPL) k_columns_boundary(StageParams P, L line, const float2 *spec,
+                                                                  float2 *Tab)
 {
     if (!group_active<KX>(P, blockIdx.x * KX))
-        return;  // all-zero columns: no later stage reads them
+        return;  // all-zero columns: the row stage never reads them
     extern __shared__ float2 smem[];
     const int n = line.size();
     const int ls = xslots<true>(n);
@@ -334,46 +290,23 @@ __global__ void __launch_bounds__(KX * L::TPL) k_columns_spectrum(StageParams P,
     const size_t K = (size_t)P.lNy * P.lNx;
     __syncthreads();
     int flip = 0;
-    float2 g[L::SLOTS], h[L::SLOTS];
-    const int2 views = PAIR ? P.units[u] : make_int2(u, -1);
-    float2 *spec = rowspec + (size_t)(PAIR ? 2 * u : u) * K;
-    column_spectrum<L, KX>(P, line, spec, kx, kx, P.again ? P.again + views.x * K : nullptr, colok, c, j, buf0, buf1,
-                           tw, flip, g);
-    if constexpr (PAIR) {
-        if (views.y >= 0) {  // uniform over the CTA
-            column_spectrum<L, KX>(P, line, spec + K, kx, kx ? P.lNx - kx : 0,
-                                   P.again ? P.again + views.y * K : nullptr, colok, c, j, buf0, buf1, tw, flip, h);
-        } else {
-#pragma unroll
-            for (int r = 0; r < L::SLOTS; ++r)
-                h[r] = make_float2(0.f, 0.f);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int ky = j + r * L::TPL;
-        if (colok && ky < n) {
-            spec[(size_t)ky * P.lNx + kx] = g[r];
-            if (PAIR)
-                spec[K + (size_t)ky * P.lNx + kx] = h[r];
-        }
-    }
-    const int np = P.npoles;  // 0 below order 2
+    const float2 *su = spec + (size_t)(PAIR ? 2 * u : u) * K + kx;
+    const int np = P.npoles;
 #pragma unroll 1
     for (int t = 0; t < 2 * np; ++t) {
         const int i = t < np ? t : t - np;
-        const float2 *tab = (t < np ? P.tab.alpha : P.tab.beta) + i * K;
-        const float2 *opp = (t < np ? P.tab.beta : P.tab.alpha) + i * K;
+        const float2 *tab = (t < np ? P.tab.alpha : P.tab.beta) + i * K + kx;
+        const float2 *opp = (t < np ? P.tab.beta : P.tab.alpha) + i * K + kx;
         float2 v[L::SLOTS];
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
             const int ky = j + r * L::TPL;
             v[r] = make_float2(0.f, 0.f);
             if (colok && ky < n) {
-                const size_t k = (size_t)ky * P.lNx + kx;
-                v[r] = cmul(g[r], tab[k]);
+                const size_t k = (size_t)ky * P.lNx;
+                v[r] = cmul(su[k], tab[k]);
                 if (PAIR)
-                    v[r] = cfma(h[r], opp[k], v[r]);
+                    v[r] = cfma(su[K + k], opp[k], v[r]);
             }
         }
         column_inverse_store<L, KX, YF>(P, line, v, c, j, colok, buf0, buf1, tw, edge, flip,
@@ -383,10 +316,17 @@ __global__ void __launch_bounds__(KX * L::TPL) k_columns_spectrum(StageParams P,
 
 // (b1) columns: for the z planes of jobs q in [q0, q0+qn) (q = u*nz + p):
 // the filtered spectrum times the propagator (exact anchor, then a complex
-// recurrence), backward FFT along y, crop.  Output T[q-q0][y][kx], y over
-// the cropped height.  PAIR: the unit's opposite view is added with its own
-// propagator (the header comment), which the conjugate step advances.
-template <class L, int KX, bool HALF, int YF, bool PAIR>
+// recurrence), backward FFT along the column, crop.  PAIR: the unit's opposite
+// view is added with its own propagator (the header comment), which the
+// conjugate step advances.
+// Output T[q-q0][row][kx], the P.trows rows from padded row P.trow0 on: the
+// crop and, from order 2, the npoles samples before and after it, from which
+// the row stage solves the column axis' prefilter boundary terms.  (Adding
+// them here needs samples that a few other threads hold, a barrier per plane:
+// tilted 200^3 columns 30.4 ms against 24.8 ms.)
+// HALF (half_crop plans): the crop is slots 2..5 of every thread, without
+// predicates.
+template <class L, int KX, bool HALF, bool PAIR>
 __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX * L::TPL <= 512) ? 2 : 1))
     k_columns_propagate(StageParams P, L line, const float2 *spec, float2 *T, int q0, int qn, int ppc)
 {
@@ -410,7 +350,7 @@ __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX *
     const int c = threadIdx.x % KX, j = threadIdx.x / KX;
     const int kx = blockIdx.x * KX + c;
     const bool colok = kx < P.lNx;
-    const int lNx = P.lNx, nz = P.nz, ny = P.ny;
+    const int lNx = P.lNx, nz = P.nz;
     const size_t K = (size_t)n * lNx;
     const int qb = q0 + blockIdx.y * ppc;
     const int qe = min(q0 + qn, qb + ppc);
@@ -429,14 +369,13 @@ __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX *
     float2 V[L::SLOTS];                    // G X exp(i w z_p) for this thread's elements
     float2 W[PAIR ? L::SLOTS : 1];         // the opposite view's
     int flip = 0;
-    // tilted generic crops: the edge samples this thread holds (fixed)
-    unsigned long long eheld = 0;
-    if constexpr (!HALF && YF > 0 && L::SLOTS <= 8)
-        eheld = edge_holdings<L, YF>(P, n, j);
     int cur_u = -1;
     int since = 0;  // planes advanced by the recurrence since the last exact anchor
     int u = qb / nz, p = qb % nz;
-    for (int q = qb; q < qe; ++q, ++p) {
+    const long long tstep = (long long)P.trows * lNx;  // T elements per plane
+    float2 *d = T + (qb - q0) * tstep + (long long)(j - P.trow0) * lNx + kx;
+    const int t0 = j - P.trow0;
+    for (int q = qb; q < qe; ++q, ++p, d += tstep) {
         if (p == nz) {
             p = 0;
             ++u;
@@ -484,114 +423,134 @@ __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX *
                     W[r] = cmul_conj(W[r], st);
             }
         }
-        if constexpr (HALF)  // (tilted: the y-prefilter terms go to the row stage)
-            column_inverse_store_half<L, KX, YF, TW2, (YF > 0)>(
-                P, line, v, c, j, buf0, buf1, tw, nullptr, flip, T + (size_t)(q - q0) * (L::N / 2) * L::N + kx,
-                T + P.yedge_off + (size_t)(q - q0) * 4 * (YF > 0 ? YF : 1) * L::N + kx);
-        else if constexpr (YF > 0)  // (tilted: the y-prefilter terms go to the row stage)
-            column_inverse_store<L, KX, YF, TW2, true>(
-                P, line, v, c, j, colok, buf0, buf1, tw, nullptr, flip, T + (size_t)(q - q0) * ny * lNx + kx,
-                T + P.yedge_off + (size_t)(q - q0) * 4 * YF * lNx + kx, eheld);
-        else
-            column_inverse_store<L, KX, YF, TW2>(P, line, v, c, j, colok, buf0, buf1, tw, nullptr, flip,
-                                             T + (size_t)(q - q0) * ny * lNx + kx);
+        line.template run<1, true, TW2>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
+        if constexpr (HALF) {
+            constexpr int N = L::N, TPL = L::TPL;  // lNx is N too
+            const int np = P.npoles;
+#pragma unroll
+            for (int r = 2; r <= 5; ++r)
+                d[r * TPL * N] = v[r];
+            if (j >= TPL - np)
+                d[1 * TPL * N] = v[1];
+            if (j < np)
+                d[6 * TPL * N] = v[6];
+        } else if (colok) {
+#pragma unroll
+            for (int r = 0; r < L::SLOTS; ++r)
+                if ((unsigned)(t0 + r * L::TPL) < (unsigned)P.trows)
+                    d[r * L::TPL * lNx] = v[r];
+        }
     }
 }
 
 // ---------------------------------------------------------------------------
-// (b2) rows: (+ z-boundary rows), backward FFT along x, x-prefilter boundary
-// terms, crop -> slab.
-// Slab layout [a][z][x][y] (both geometries) with the y pitch P.ypitch (a
-// multiple of 32, or 1 for single-row planes).  A CTA owns RG consecutive y rows of one plane (job) and
-// transforms them in groups of LPC lines (one line per TPL threads); the T
-// values of the next group are loaded (evict-first) into registers while
-// the current group is transformed.  When a line is whole warps its FFT
-// exchanges sync only its own warps (named barrier).  The cropped rows of a
-// group are transposed through shared memory and stored as runs of LPC
-// consecutive y per x (rows y >= ny of a group are zero; groups and CTAs
-// wholly beyond ny are not run).
+// (b2) rows: (+ the column axis' prefilter terms, + z-boundary rows), backward
+// FFT along the row, the row axis' prefilter terms (ROWPF: tilted path), crop
+// -> slab [a][z][x][y] (y innermost, pitch P.ypitch: a multiple of 32, or 1 for
+// single-row planes).  P is transposed(): rows run along y, one per x, so
+// a row's crop is contiguous in the slab and is stored straight from
+// registers.  A CTA owns RG consecutive rows of one plane (job) and transforms
+// them in groups of LPC lines (one line per TPL threads); the T values of the
+// next group are loaded (evict-first) while the current one is transformed.
+// When a line is whole warps, its FFT exchanges sync only its own warps
+// (named barrier) and the lines never wait for each other.
+// HALF (half_crop plans): the cropped outputs are slots 2..5 of every
+// thread and the edge samples sit at compile-time slots.
+// NP: prefilter poles (0 below order 2).
 template <int LPC>
 constexpr int rows_per_cta()
 {
-    return LPC >= 8 ? LPC : 8;
+    // 16 rows share the CTA's set-up (twiddle table, boundary weights; 256^3
+    // row stage with 8 / 16 / 32 rows, before it stored rows directly: 21.7 /
+    // 20.9 / 21.2 ms for 200 single views)
+    return LPC >= 16 ? LPC : 16;
 }
 
-// YD (P.ydefer): the column stage left the tilted path's y-prefilter
-// boundary terms to this stage.  A CTA with rows within ZPOW_N of either end
-// of the crop solves each column's coefficients once, from the job's raw
-// edge samples, into shared memory (lines of up to 2048; longer lines solve
-// them per row), and those rows add the terms before the z-boundary rows:
-// the same values in the same order as in the column stage.
+// The column stage leaves its axis' prefilter boundary terms to this stage
+// (order >= 2).  A CTA with rows within ZPOW_N of either end of the crop
+// solves each column's coefficients once, from the job's samples around the
+// crop's ends, into shared memory (lines of up to 2048; longer lines solve them per row),
+// and those rows add the terms before the z-boundary rows.
 template <class L>
 constexpr bool ycoef_smem()
 {
     return pow2_len<L>() == 0 || pow2_len<L>() <= 2048;
 }
-template <class L, int NP, bool YD>
+template <class L, int NP>
 constexpr size_t smem_rows_y(int n)
 {
-    return (YD && ycoef_smem<L>()) ? (size_t)2 * NP * n * sizeof(float2) : 0;
+    return (NP > 0 && ycoef_smem<L>()) ? (size_t)2 * NP * n * sizeof(float2) : 0;
 }
-template <class L, int LPC, int NP, bool YD>
+template <class L, int LPC, int NP, bool ROWPF, bool HALF>
 __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
-    k_rows_inverse(StageParams P, L line, const float2 *T, const float2 *Tab, float2 *slab, int q0, int qn)
+    k_rows_inverse(StageParams P, L line, const float2 *T, const float2 *Tab, float2 *slab, int q0)
 {
     constexpr int RG = rows_per_cta<LPC>(), G = RG / LPC;
+    constexpr int NPA = NP > 0 ? NP : 1;  // array extents
     extern __shared__ float2 smem[];
-    const int n = line.size();  // lNx
+    const int n = line.size();  // the row's padded length
     const int ls = xslots<false>(n);
     float2 *buf0 = smem, *buf1 = smem + LPC * ls, *tw = smem + 2 * LPC * ls;
+    float2 *edge = tw + tw_slots(n);          // [LPC][EDGE_SLOTS]
+    float2 *ycs = edge + EDGE_SLOTS * LPC;    // [2 NP][n] column-axis coefficients
+    // (a third-pass twiddle table costs more to set up per CTA than its
+    // conflict-free reads save here)
     copy_twiddles<L>(tw, P.tab.twx, n);
     const int l = threadIdx.x / L::TPL, j = threadIdx.x % L::TPL;
     // lines of whole warps sync on named barrier 1 + l
     const int bar = (L::TPL % 32 == 0 && LPC < 15) ? 1 + l : 0;
-    const int ny = P.ny, nx = P.nx, nz = P.nz, padxl = P.padxl, yp = P.ypitch;
-    const int cpj = (ny + RG - 1) / RG;  // CTAs per job (rows y < ny only)
-    const int qrel = (int)blockIdx.x / cpj;
-    const int ybase = ((int)blockIdx.x - qrel * cpj) * RG;
-    // groups holding at least one row y < ny (the slab rows y >= ny are
-    // never read: the resampling lanes of those y store nothing)
-    const int GV = min(G, (ny - ybase + LPC - 1) / LPC);
-    const int qq = q0 + qrel;  // the grid covers exactly qn jobs
+    const int ny = P.ny, nx = P.nx, nz = P.nz, padxl = P.padxl;
+    const int cpj = (ny + RG - 1) / RG;  // CTAs per job
+    const int bid = (int)blockIdx.x;
+    const int qrel = bid / cpj;
+    const int ybase = (bid - qrel * cpj) * RG;
+    const int GV = min(G, (ny - ybase + LPC - 1) / LPC);  // groups holding a row
+    const int qq = q0 + qrel;  // the grid covers exactly the launch's jobs
     const int a = qq / nz, p = qq - a * nz;
-    const bool pf = P.order >= 2;
-    constexpr int np = NP;
     // z-boundary weights of this plane: z_i^p (alpha rows), z_i^(nz-1-p)
     // (beta rows), per pole
-    float zl[2], zh[2];
+    float zl[NPA], zh[NPA];
     bool zb_any = false;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        zl[i] = (pf && i < np && p < ZPOW_N) ? P.tab.zpow[i * ZPOW_N + p] : 0.f;
-        zh[i] = (pf && i < np && nz - 1 - p < ZPOW_N) ? P.tab.zpow[i * ZPOW_N + nz - 1 - p] : 0.f;
+    for (int i = 0; i < NP; ++i) {
+        zl[i] = p < ZPOW_N ? P.tab.zpow[i * ZPOW_N + p] : 0.f;
+        zh[i] = nz - 1 - p < ZPOW_N ? P.tab.zpow[i * ZPOW_N + nz - 1 - p] : 0.f;
         zb_any = zb_any || zl[i] != 0.f || zh[i] != 0.f;
     }
-    const float2 *Tq = T + (size_t)qrel * ny * n;
-    float2 *dst = slab + ((size_t)a * nz + p) * nx * yp + ybase;
+    // slots of this thread in the all-zero column band or beyond the line
+    unsigned zmask = 0;
+#pragma unroll
+    for (int r = 0; r < L::SLOTS; ++r)
+        if (!column_active(P, j + r * L::TPL))
+            zmask |= 1u << r;
+    unsigned long long eheld = 0;
+    if constexpr (ROWPF && !HALF && L::SLOTS <= 8)
+        eheld = edge_holdings<L, NPA>(padxl, nx, n, j);
+    // the job's T rows; crop row y is row y + crop0
+    const float2 *Tj = T + (size_t)qrel * P.trows * n;
+    const int crop0 = P.padyl - P.trow0;
+    const float2 *Tq = Tj + (size_t)crop0 * n + j;
+    auto edge_sample = [&](int e, int x) {
+        return Tj[(size_t)P.tedge[e] * n + x];
+    };
     // this thread's T values of row y (zeros for y >= ny or zero columns)
     auto load_row = [&](int y, float2 (&v)[L::SLOTS]) {
-        const bool valid = y < ny;
+        const bool valid = HALF || y < ny;
         const float2 *src = Tq + (size_t)(valid ? y : 0) * n;
 #pragma unroll
-        for (int r = 0; r < L::SLOTS; ++r) {
-            const int x = j + r * L::TPL;
-            v[r] = (valid && column_active(P, x)) ? __ldcs(src + x) : make_float2(0.f, 0.f);
-        }
+        for (int r = 0; r < L::SLOTS; ++r)
+            v[r] = (valid && !((zmask >> r) & 1u)) ? __ldcs(src + r * L::TPL) : make_float2(0.f, 0.f);
     };
-    // YD: the y-prefilter coefficient rows of this job, [2 NP][n] after the
-    // row buffers (CTAs with boundary rows)
-    float2 *ycs = smem + (2 * LPC * ls + tw_slots(n) + EDGE_SLOTS * LPC);
-    const float2 *yed = T + P.yedge_off + (size_t)qrel * 4 * NP * n;
-    if constexpr (YD && ycoef_smem<L>()) {
+    if constexpr (NP > 0 && ycoef_smem<L>()) {
         if (ybase < ZPOW_N || min(ybase + RG, ny) - 1 >= ny - ZPOW_N) {
             for (int x = threadIdx.x; x < n; x += LPC * L::TPL) {
-                float2 cy[2 * NP];
+                float2 cy[2 * NPA];
                 if (column_active(P, x)) {
                     float2 ed[EDGE_SLOTS];
 #pragma unroll
                     for (int e = 0; e < EDGE_SLOTS; ++e)
-                        ed[e] = edge_used(e, NP) ? yed[(size_t)edge_row(e, NP) * n + x] : make_float2(0.f, 0.f);
-                    pf_coefs<NP>(P.kys, ed, cy);
+                        ed[e] = edge_used(e, NP) ? edge_sample(e, x) : make_float2(0.f, 0.f);
+                    pf_coefs<NPA>(P.kys, ed, cy);
                 } else {
 #pragma unroll
                     for (int i = 0; i < 2 * NP; ++i)
@@ -606,19 +565,22 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
     float2 v[L::SLOTS], vn[L::SLOTS];
     load_row(ybase + l, v);
     __syncthreads();  // twiddles (and the coefficient rows)
+    // kept across groups: with an odd number of exchanges per transform the
+    // next group starts in the other buffer
+    int flip = 0;
 #pragma unroll 1
     for (int g = 0; g < GV; ++g) {
         const int y = ybase + g * LPC + l;
-        const bool valid = y < ny;
+        const bool valid = HALF || y < ny;
         if (g + 1 < GV)
             load_row(y + LPC, vn);
-        if constexpr (YD) {
+        if constexpr (NP > 0) {
             if (valid && (y < ZPOW_N || ny - 1 - y < ZPOW_N)) {
 #pragma unroll
                 for (int r = 0; r < L::SLOTS; ++r) {
-                    const int x = j + r * L::TPL;
-                    if (column_active(P, x)) {
-                        float2 cy[2 * NP];
+                    if (!((zmask >> r) & 1u)) {
+                        const int x = j + r * L::TPL;
+                        float2 cy[2 * NPA];
                         if constexpr (ycoef_smem<L>()) {
 #pragma unroll
                             for (int i = 0; i < 2 * NP; ++i)
@@ -627,26 +589,22 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
                             float2 ed[EDGE_SLOTS];
 #pragma unroll
                             for (int e = 0; e < EDGE_SLOTS; ++e)
-                                ed[e] = edge_used(e, NP) ? yed[(size_t)edge_row(e, NP) * n + x]
-                                                         : make_float2(0.f, 0.f);
-                            pf_coefs<NP>(P.kys, ed, cy);
+                                ed[e] = edge_used(e, NP) ? edge_sample(e, x) : make_float2(0.f, 0.f);
+                            pf_coefs<NPA>(P.kys, ed, cy);
                         }
-                        v[r] = pf_apply<NP>(P, cy, y, ny, v[r]);
+                        v[r] = pf_apply<NPA>(P, cy, y, ny, v[r]);
                     }
                 }
             }
-        }
-        if (valid && zb_any) {
+            if (valid && zb_any) {
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (i < np) {
-                    const float2 *ta = Tab + ((size_t)(a * 2 * np + i) * ny + y) * n;
-                    const float2 *tb = Tab + ((size_t)(a * 2 * np + np + i) * ny + y) * n;
+                for (int i = 0; i < NP; ++i) {
+                    const float2 *ta = Tab + ((size_t)(a * 2 * NP + i) * ny + y) * n + j;
+                    const float2 *tb = Tab + ((size_t)(a * 2 * NP + NP + i) * ny + y) * n + j;
 #pragma unroll
                     for (int r = 0; r < L::SLOTS; ++r) {
-                        const int x = j + r * L::TPL;
-                        if (column_active(P, x)) {
-                            const float2 u = ta[x], w = tb[x];
+                        if (!((zmask >> r) & 1u)) {
+                            const float2 u = ta[r * L::TPL], w = tb[r * L::TPL];
                             v[r] = make_float2(fmaf(zh[i], w.x, fmaf(zl[i], u.x, v[r].x)),
                                                fmaf(zh[i], w.y, fmaf(zl[i], u.y, v[r].y)));
                         }
@@ -654,255 +612,70 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
                 }
             }
         }
-        int flip = 0;
         line.template run<1>(v, j, buf0 + l * ls, buf1 + l * ls, 1, tw, flip, bar);
-        float2 cf[2 * NP];
-        if (pf) {
-            // the line's samples around the crop's ends (periodic): every
-            // thread writes its values to the exchange buffer the FFT's last
-            // exchange did not use (its reads ended before that exchange's
-            // barrier), then each thread reads the edge samples
-            // (plain positions 0..n-1: within the line's slots for every
-            // line type, and conflict-free for these stride-1 writes)
-            float2 *sc = (flip ? buf1 : buf0) + l * ls;
+        float2 cf[2 * NPA];
+        if constexpr (ROWPF) {
+            // the samples around the crop's ends, each held by one thread
+            // (its previous group's readers are past this transform's barriers)
+            if constexpr (HALF) {
 #pragma unroll
-            for (int r = 0; r < L::SLOTS; ++r) {
-                const int x = j + r * L::TPL;
-                if (x < n)
-                    sc[x] = v[r];
+                for (int e = 0; e < EDGE_SLOTS; ++e) {
+                    float2 t;
+                    if (edge_used(e, NP) && held<L>(v, j, n / 4 + edge_offset(e, n / 2), t))
+                        edge[l * EDGE_SLOTS + e] = t;
+                }
+            } else if constexpr (L::SLOTS <= 8) {
+                if (eheld) {
+#pragma unroll
+                    for (int r = 0; r < L::SLOTS; ++r) {
+                        const unsigned m = (unsigned)(eheld >> (8 * r)) & 0xffu;
+                        if (m) {
+#pragma unroll
+                            for (int e = 0; e < EDGE_SLOTS; ++e)
+                                if (edge_used(e, NP) && (m & (1u << e)))
+                                    edge[l * EDGE_SLOTS + e] = v[r];
+                        }
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < EDGE_SLOTS; ++e) {
+                    float2 t;
+                    if (edge_used(e, NP) && held<L>(v, j, (padxl + edge_offset(e, nx) + 2 * n) % n, t))
+                        edge[l * EDGE_SLOTS + e] = t;
+                }
             }
             if (bar > 0)
                 line_sync(bar, L::TPL);
             else
                 __syncthreads();
-            float2 ed[EDGE_SLOTS];
-#pragma unroll
-            for (int e = 0; e < EDGE_SLOTS; ++e)
-                ed[e] = edge_used(e, np) ? sc[(padxl + edge_offset(e, nx) + 2 * n) % n] : make_float2(0.f, 0.f);
-            pf_coefs<NP>(P.kxs, ed, cf);
+            pf_coefs<NPA>(P.kxs, edge + l * EDGE_SLOTS, cf);
         }
-        // stage[x][l] (pitch LPC+1) in buf0, then runs of LPC y per x
-        __syncthreads();  // every line is done with buf0
-        float2 *stage = buf0;
-        constexpr int SP = LPC + 1;
-#pragma unroll
-        for (int r = 0; r < L::SLOTS; ++r) {
-            const int xx = j + r * L::TPL - padxl;
-            if (xx >= 0 && xx < nx) {
-                float2 o = v[r];
-                if (pf)
-                    o = pf_apply<NP>(P, cf, xx, nx, o);
-                stage[xx * SP + l] = valid ? o : make_float2(0.f, 0.f);
-            }
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < nx * LPC; e += LPC * L::TPL) {
-            const int xx = e / LPC, ll = e - xx * LPC;
-            if (ybase + g * LPC + ll < ny)  // pitch 1 for single-row planes
-                __stcs(dst + (size_t)xx * yp + g * LPC + ll, stage[xx * SP + ll]);
-        }
-        if (g + 1 < GV) {
-            __syncthreads();  // stage reads done before buf0 is reused
-#pragma unroll
-            for (int r = 0; r < L::SLOTS; ++r)
-                v[r] = vn[r];
-        }
-    }
-}
-
-// (b2, half-crop plans) k_rows_inverse for square power-of-two planes
-// whose crop is the centred half (nx = ny = N/2 from N/4; the slab y pitch
-// is then N/2): every position the row needs -- the cropped outputs (slots
-// 2..5 of thread j, x = j + TPL*(r-2)), the x-prefilter edge samples and
-// the rows with boundary terms -- is a compile-time function of the thread
-// and slot, so the row runs without per-element index arithmetic or crop
-// predicates.  The all-zero spectrum columns (outside the |k| < km disc,
-// not written by the column stage) are a per-thread slot mask computed
-// once.  A CTA owns LPC*G consecutive rows of one job, LPC lines at a time.
-// YD (P.ydefer): the tilted path's y-prefilter terms, added as in
-// k_rows_inverse.
-template <class L, int LPC, int G, int NP, bool YD>
-__global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
-    k_rows_inverse_half(StageParams P, L line, const float2 *T, const float2 *Tab, float2 *slab, int q0)
-{
-    constexpr int N = L::N, TPL = L::TPL, NX = N / 2, PAD = N / 4, RG = LPC * G, CPJ = NX / RG;
-    static_assert(NX % RG == 0, "rows per CTA must divide the crop");
-    extern __shared__ float2 smem[];
-    constexpr int ls = xslots<false>(N);
-    float2 *buf0 = smem, *buf1 = smem + LPC * ls, *tw = smem + 2 * LPC * ls;
-    float2 *edge = tw + tw_slots(N);  // [LPC][EDGE_SLOTS]
-    // (the third-pass twiddle table costs more to set up per CTA than its
-    // conflict-free reads save here: +0.7 ms for the 256^3 row stage)
-    copy_twiddles<L>(tw, P.tab.twx, N);
-    const int l = threadIdx.x / TPL, j = threadIdx.x % TPL;
-    const int bar = 1 + l;  // each line is whole warps (TPL >= 32)
-    const int nz = P.nz;
-    const int qrel = (int)blockIdx.x / CPJ;
-    const int ybase = ((int)blockIdx.x - qrel * CPJ) * RG;
-    const int qq = q0 + qrel;
-    const int a = qq / nz, p = qq - a * nz;
-    const bool pf = P.order >= 2;
-    constexpr int np = NP;
-    float zl[2], zh[2];  // z-boundary weights of this plane, per pole
-    bool zb_any = false;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        zl[i] = (pf && i < np && p < ZPOW_N) ? P.tab.zpow[i * ZPOW_N + p] : 0.f;
-        zh[i] = (pf && i < np && nz - 1 - p < ZPOW_N) ? P.tab.zpow[i * ZPOW_N + nz - 1 - p] : 0.f;
-        zb_any = zb_any || zl[i] != 0.f || zh[i] != 0.f;
-    }
-    // slots of this thread in the all-zero column band
-    unsigned zmask = 0;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int x = j + r * TPL;
-        if (x >= P.kx_zero_lo && x < P.kx_zero_hi)
-            zmask |= 1u << r;
-    }
-    // x-prefilter boundary weights of this thread's cropped slots for the
-    // first pole: the A term (z^xx) for xx < ZPOW_N, the B term
-    // (z^(NX-1-xx)) near the end
-    float za[4], zb[4];
-#pragma unroll
-    for (int r = 2; r <= 5; ++r) {
-        const int xx = j + TPL * (r - 2);
-        za[r - 2] = (pf && xx < ZPOW_N) ? P.tab.zpow[xx] : 0.f;
-        zb[r - 2] = (pf && NX - 1 - xx < ZPOW_N) ? P.tab.zpow[NX - 1 - xx] : 0.f;
-    }
-    const float2 *Tq = T + (size_t)qrel * NX * N + j;
-    float2 *dst = slab + ((size_t)a * nz + p) * NX * NX + ybase;
-    auto load_row = [&](int y, float2 (&v)[L::SLOTS]) {
-        const float2 *src = Tq + (size_t)y * N;
-#pragma unroll
-        for (int r = 0; r < L::SLOTS; ++r)
-            v[r] = (zmask >> r) & 1u ? make_float2(0.f, 0.f) : __ldcs(src + r * TPL);
-    };
-    // YD: the y-prefilter coefficient rows of this job, [2 NP][N] after the
-    // edge slots (CTAs with boundary rows)
-    float2 *ycs = edge + EDGE_SLOTS * LPC;
-    const float2 *yed = T + P.yedge_off + (size_t)qrel * 4 * NP * N;
-    if constexpr (YD && ycoef_smem<L>()) {
-        if (ybase < ZPOW_N || ybase + RG - 1 >= NX - ZPOW_N) {
-            for (int x = threadIdx.x; x < N; x += LPC * TPL) {
-                float2 cy[2 * NP];
-                if (!(x >= P.kx_zero_lo && x < P.kx_zero_hi)) {
-                    float2 ed[EDGE_SLOTS];
-#pragma unroll
-                    for (int e = 0; e < EDGE_SLOTS; ++e)
-                        ed[e] = edge_used(e, NP) ? yed[(size_t)edge_row(e, NP) * N + x] : make_float2(0.f, 0.f);
-                    pf_coefs<NP>(P.kys, ed, cy);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 2 * NP; ++i)
-                        cy[i] = make_float2(0.f, 0.f);
-                }
-#pragma unroll
-                for (int i = 0; i < 2 * NP; ++i)
-                    ycs[i * N + x] = cy[i];
-            }
-        }
-    }
-    float2 v[L::SLOTS], vn[L::SLOTS];
-    load_row(ybase + l, v);
-    __syncthreads();  // twiddles (and the coefficient rows)
-#pragma unroll 1
-    for (int g = 0; g < G; ++g) {
-        const int y = ybase + g * LPC + l;
-        if (g + 1 < G)
-            load_row(y + LPC, vn);
-        if constexpr (YD) {
-            if (y < ZPOW_N || NX - 1 - y < ZPOW_N) {
-#pragma unroll
-                for (int r = 0; r < L::SLOTS; ++r) {
-                    if (!((zmask >> r) & 1u)) {
-                        const int x = j + r * TPL;
-                        float2 cy[2 * NP];
-                        if constexpr (ycoef_smem<L>()) {
-#pragma unroll
-                            for (int i = 0; i < 2 * NP; ++i)
-                                cy[i] = ycs[i * N + x];
-                        } else {
-                            float2 ed[EDGE_SLOTS];
-#pragma unroll
-                            for (int e = 0; e < EDGE_SLOTS; ++e)
-                                ed[e] = edge_used(e, NP) ? yed[(size_t)edge_row(e, NP) * N + x]
-                                                         : make_float2(0.f, 0.f);
-                            pf_coefs<NP>(P.kys, ed, cy);
-                        }
-                        v[r] = pf_apply<NP>(P, cy, y, NX, v[r]);
-                    }
-                }
-            }
-        }
-        if (zb_any) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (i < np) {
-                    const float2 *ta = Tab + ((size_t)(a * 2 * np + i) * NX + y) * N + j;
-                    const float2 *tb = Tab + ((size_t)(a * 2 * np + np + i) * NX + y) * N + j;
-#pragma unroll
-                    for (int r = 0; r < L::SLOTS; ++r) {
-                        if (!((zmask >> r) & 1u)) {
-                            const float2 u = ta[r * TPL], w = tb[r * TPL];
-                            v[r] = make_float2(fmaf(zh[i], w.x, fmaf(zl[i], u.x, v[r].x)),
-                                               fmaf(zh[i], w.y, fmaf(zl[i], u.y, v[r].y)));
-                        }
-                    }
-                }
-            }
-        }
-        int flip = 0;
-        line.template run<1>(v, j, buf0 + l * ls, buf1 + l * ls, 1, tw, flip, bar);
-        if (pf) {
-            // the samples around the crop's ends: each held by one thread,
-            // at a compile-time slot
-#pragma unroll
-            for (int e = 0; e < EDGE_SLOTS; ++e) {
-                float2 t;
-                if (edge_used(e, np) && held<L>(v, j, PAD + edge_offset(e, NX), t))
-                    edge[l * EDGE_SLOTS + e] = t;
-            }
-            line_sync(bar, TPL);
-            float2 cf[2 * NP];
-            pf_coefs<NP>(P.kxs, edge + l * EDGE_SLOTS, cf);
-            const float2 Ac = cf[0], Bc = cf[np];  // first pole
-#pragma unroll
-            for (int r = 2; r <= 5; ++r) {
-                v[r] = make_float2(fmaf(Bc.x, zb[r - 2], fmaf(Ac.x, za[r - 2], v[r].x)),
-                                   fmaf(Bc.y, zb[r - 2], fmaf(Ac.y, za[r - 2], v[r].y)));
-            }
-            if constexpr (NP == 2) {  // second pole (orders 4, 5)
-                const float2 A2 = cf[1], B2 = cf[3];
+        if (valid) {
+            float2 *dst = slab + (((size_t)a * nz + p) * ny + y) * P.ypitch;
+            if constexpr (HALF) {
+                dst += j;
 #pragma unroll
                 for (int r = 2; r <= 5; ++r) {
-                    const int xx = j + TPL * (r - 2);
-                    if (xx < ZPOW_N) {
-                        const float z = P.tab.zpow[ZPOW_N + xx];
-                        v[r] = make_float2(fmaf(A2.x, z, v[r].x), fmaf(A2.y, z, v[r].y));
-                    }
-                    if (NX - 1 - xx < ZPOW_N) {
-                        const float z = P.tab.zpow[ZPOW_N + NX - 1 - xx];
-                        v[r] = make_float2(fmaf(B2.x, z, v[r].x), fmaf(B2.y, z, v[r].y));
+                    float2 o = v[r];
+                    if constexpr (ROWPF)
+                        o = pf_apply<NPA>(P, cf, j + L::TPL * (r - 2), n / 2, o);
+                    __stcs(dst + (r - 2) * L::TPL, o);
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < L::SLOTS; ++r) {
+                    const int xx = j + r * L::TPL - padxl;
+                    if (xx >= 0 && xx < nx) {
+                        float2 o = v[r];
+                        if constexpr (ROWPF)
+                            o = pf_apply<NPA>(P, cf, xx, nx, o);
+                        __stcs(dst + xx, o);
                     }
                 }
             }
         }
-        // stage[x][l] (pitch LPC+1) in buf0, then runs of LPC y per x
-        __syncthreads();  // every line is done with buf0 (and edge)
-        float2 *stage = buf0;
-        constexpr int SP = LPC + 1;
-#pragma unroll
-        for (int r = 2; r <= 5; ++r)
-            stage[(j + TPL * (r - 2)) * SP + l] = v[r];
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < NX / TPL; ++k) {
-            const int e = threadIdx.x + k * LPC * TPL;
-            const int xx = e / LPC, ll = e % LPC;
-            __stcs(dst + (size_t)xx * NX + g * LPC + ll, stage[xx * SP + ll]);
-        }
-        if (g + 1 < G) {
-            __syncthreads();  // stage reads done before buf0 is reused
+        if (g + 1 < GV) {
 #pragma unroll
             for (int r = 0; r < L::SLOTS; ++r)
                 v[r] = vn[r];
@@ -922,11 +695,16 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
 // group every line is anchored exactly.  Then per line the z-boundary rows
 // of its plane, the backward FFT along x, the x-prefilter boundary terms,
 // and the cropped row stored contiguously at slab[a][p][x].
+template <int LPC>
+constexpr int line_jobs_per_cta()
+{
+    return LPC >= 8 ? LPC : 8;
+}
 template <class L, int LPC, int NP, bool PAIR>
 __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 3 : 1)
     k_rows_line(StageParams P, L line, const float2 *spec, const float2 *Tab, float2 *slab, int q0, int qn)
 {
-    constexpr int RG = rows_per_cta<LPC>(), G = RG / LPC;
+    constexpr int RG = line_jobs_per_cta<LPC>(), G = RG / LPC;
     extern __shared__ float2 smem[];
     const int n = line.size();  // lNx
     const int ls = xslots<false>(n);
@@ -1048,8 +826,8 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 3 : 1)
     }
 }
 
-// (b0) k_columns_spectrum for single-row planes, whose column transforms are
-// the identity.  One thread per (unit, kx).
+// (a2, b0) the filtered spectra (in place) and z-boundary rows of single-row
+// planes, whose column transforms are the identity.  One thread per (unit, kx).
 __global__ void __launch_bounds__(256) k_spectrum_line(StageParams P, float2 *rowspec, float2 *Tab, int nunits)
 {
     const int lNx = P.lNx;
@@ -1130,16 +908,10 @@ static cudaError_t with_poles(int v, F &&fn)
     default: return cudaErrorInvalidValue;
     }
 }
-// Poles of the y-prefilter the column stage applies (tilted path, order
-// >= 2), 0 for none; poles of the x- and z-prefilters of the row stages
-// (1 also for orders 0 and 1, where the row stages skip the prefilter).
-static int column_poles(const StageParams &P)
+// Prefilter poles of the transposed stages (0 below order 2).
+static int stage_poles(const StageParams &P)
 {
-    return (P.tilted && P.order >= 2) ? P.npoles : 0;
-}
-static int row_poles(const StageParams &P)
-{
-    return P.order >= 4 ? 2 : 1;
+    return P.order >= 2 ? P.npoles : 0;
 }
 
 template <class L>
@@ -1154,110 +926,30 @@ static cudaError_t rows_forward_impl(const StageParams &P, L line, const void *s
 }
 
 template <class L>
-static cudaError_t spectrum_impl(const StageParams &P, L line, float2 *rowspec, float2 *Tab, int nunits,
+static cudaError_t spectrum_impl(const StageParams &P, L line, const float2 *rowspec, float2 *spec, int nslots,
+                                 cudaStream_t s)
+{
+    constexpr int KX = Cfg<L>::KX;
+    dim3 grid((P.lNx + KX - 1) / KX, nslots);
+    k_columns_spectrum<L, KX><<<grid, KX * L::TPL, smem_cols<L>(line.n), s>>>(P, line, rowspec, spec);
+    return cudaGetLastError();
+}
+
+template <class L>
+static cudaError_t boundary_impl(const StageParams &P, L line, const float2 *spec, float2 *Tab, int nunits,
                                  cudaStream_t s)
 {
     constexpr int KX = Cfg<L>::KX;
     dim3 grid((P.lNx + KX - 1) / KX, nunits);
-    return with_poles(column_poles(P), [&](auto yf) {
+    return with_poles(stage_poles(P), [&](auto yf) {
         constexpr int YF = decltype(yf)::value;
-        if constexpr (YF == 0) {  // (units: y-axis plans only, no y-prefilter)
-            if (P.units) {
-                k_columns_spectrum<L, KX, YF, true>
-                    <<<grid, KX * L::TPL, smem_cols<L>(line.n), s>>>(P, line, rowspec, Tab);
-                return cudaGetLastError();
-            }
-        }
-        if (P.units)
-            return cudaErrorInvalidValue;
-        k_columns_spectrum<L, KX, YF, false>
-            <<<grid, KX * L::TPL, smem_cols<L>(line.n), s>>>(P, line, rowspec, Tab);
-        return cudaGetLastError();
-    });
-}
-
-// Lines of a half-crop row kernel: whole warps (the line barriers are
-// per line).
-template <class L>
-constexpr bool half_line()
-{
-    return pow2_len<L>() >= 256;
-}
-// Groups of lines per half-crop row CTA (LPC * G rows): 16 rows, so that
-// the CTA's set-up (twiddle table, boundary weights, zero-column mask) is
-// shared by more lines (256^3 workload: 8 rows 21.7 ms, 16 rows 20.9 ms,
-// 32 rows 21.2 ms for the row stage).
-template <class L>
-constexpr int half_groups()
-{
-    return Cfg<L>::LPC >= 16 ? 1 : 16 / Cfg<L>::LPC;
-}
-template <class L, bool HALF, int YF, bool PAIR>
-static cudaError_t columns_launch(const StageParams &P, L line, const float2 *spec, float2 *T, int q0, int qn,
-                                  cudaStream_t s)
-{
-    constexpr int KX = Cfg<L>::KX;
-    const int ppc = planes_per_cta<KX>(P, qn, long_runs<L, KX, HALF>());
-    dim3 grid((P.lNx + KX - 1) / KX, (qn + ppc - 1) / ppc);
-    k_columns_propagate<L, KX, HALF, YF, PAIR>
-        <<<grid, KX * L::TPL, smem_cols_prop<L, HALF>(line.n), s>>>(P, line, spec, T, q0, qn, ppc);
-    return cudaGetLastError();
-}
-template <class L>
-static cudaError_t columns_impl(const StageParams &P, L line, const float2 *spec, float2 *T, int q0, int qn,
-                                cudaStream_t s)
-{
-    return with_poles(column_poles(P), [&](auto yf) {
-        constexpr int YF = decltype(yf)::value;
-        if constexpr (half_line<L>()) {
-            if (half_crop(P)) {
-                if constexpr (YF == 0) {
-                    if (P.units)
-                        return columns_launch<L, true, YF, true>(P, line, spec, T, q0, qn, s);
-                }
-                return P.units ? cudaErrorInvalidValue
-                               : columns_launch<L, true, YF, false>(P, line, spec, T, q0, qn, s);
-            }
-        }
-        if constexpr (YF == 0) {
+        if constexpr (YF > 0) {
             if (P.units)
-                return columns_launch<L, false, YF, true>(P, line, spec, T, q0, qn, s);
-        }
-        return P.units ? cudaErrorInvalidValue : columns_launch<L, false, YF, false>(P, line, spec, T, q0, qn, s);
-    });
-}
-
-template <class L>
-static cudaError_t rows_inverse_impl(const StageParams &P, L line, const float2 *T, const float2 *Tab,
-                                     float2 *slab, int q0, int qn, cudaStream_t s)
-{
-    constexpr int LPC = Cfg<L>::LPC;
-    return with_poles(row_poles(P), [&](auto np) {
-        constexpr int NP = decltype(np)::value;
-        if constexpr (NP >= 1) {
-            if constexpr (half_line<L>()) {
-                if (half_crop(P)) {
-                    constexpr int G = half_groups<L>();
-                    const unsigned grid = (unsigned)((long long)qn * (L::N / 2 / (LPC * G)));
-                    if (P.ydefer)
-                        k_rows_inverse_half<L, LPC, G, NP, true>
-                            <<<grid, LPC * L::TPL, smem_rows_half<L>(line.n) + smem_rows_y<L, NP, true>(line.n),
-                               s>>>(P, line, T, Tab, slab, q0);
-                    else
-                        k_rows_inverse_half<L, LPC, G, NP, false>
-                            <<<grid, LPC * L::TPL, smem_rows_half<L>(line.n), s>>>(P, line, T, Tab, slab, q0);
-                    return cudaGetLastError();
-                }
-            }
-            const unsigned grid =
-                (unsigned)((long long)qn * ((P.ny + rows_per_cta<LPC>() - 1) / rows_per_cta<LPC>()));
-            if (P.ydefer)
-                k_rows_inverse<L, LPC, NP, true>
-                    <<<grid, LPC * L::TPL, smem_rows<L>(line.n) + smem_rows_y<L, NP, true>(line.n), s>>>(
-                        P, line, T, Tab, slab, q0, qn);
+                k_columns_boundary<L, KX, YF, true>
+                    <<<grid, KX * L::TPL, smem_cols<L>(line.n), s>>>(P, line, spec, Tab);
             else
-                k_rows_inverse<L, LPC, NP, false>
-                    <<<grid, LPC * L::TPL, smem_rows<L>(line.n), s>>>(P, line, T, Tab, slab, q0, qn);
+                k_columns_boundary<L, KX, YF, false>
+                    <<<grid, KX * L::TPL, smem_cols<L>(line.n), s>>>(P, line, spec, Tab);
             return cudaGetLastError();
         } else {
             return cudaErrorInvalidValue;
@@ -1265,73 +957,120 @@ static cudaError_t rows_inverse_impl(const StageParams &P, L line, const float2 
     });
 }
 
+// Lines of the half-crop kernels.
+template <class L>
+constexpr bool half_line()
+{
+    return pow2_len<L>() > 0;
+}
+template <class L, bool HALF, bool PAIR>
+static cudaError_t columns_launch(const StageParams &P, L line, const float2 *spec, float2 *T, int q0, int qn,
+                                  cudaStream_t s)
+{
+    constexpr int KX = Cfg<L>::KX;
+    const int ppc = planes_per_cta<KX>(P, qn, long_runs<L, KX, HALF>());
+    dim3 grid((P.lNx + KX - 1) / KX, (qn + ppc - 1) / ppc);
+    k_columns_propagate<L, KX, HALF, PAIR>
+        <<<grid, KX * L::TPL, smem_cols_prop<L, HALF>(line.n), s>>>(P, line, spec, T, q0, qn, ppc);
+    return cudaGetLastError();
+}
+template <class L>
+static cudaError_t columns_impl(const StageParams &P, L line, const float2 *spec, float2 *T, int q0, int qn,
+                                cudaStream_t s)
+{
+    if constexpr (half_line<L>()) {
+        if (half_crop(P))
+            return P.units ? columns_launch<L, true, true>(P, line, spec, T, q0, qn, s)
+                           : columns_launch<L, true, false>(P, line, spec, T, q0, qn, s);
+    }
+    return P.units ? columns_launch<L, false, true>(P, line, spec, T, q0, qn, s)
+                   : columns_launch<L, false, false>(P, line, spec, T, q0, qn, s);
+}
+
+template <class L, int NP, bool ROWPF, bool HALF>
+static size_t smem_rows_inverse(int n)
+{
+    return smem_rows<L>(n) + smem_rows_y<L, NP>(n);
+}
+template <class L, int NP, bool ROWPF, bool HALF>
+static cudaError_t rows_launch(const StageParams &P, L line, const float2 *T, const float2 *Tab, float2 *slab, int q0,
+                               int qn, cudaStream_t s)
+{
+    constexpr int LPC = Cfg<L>::LPC, RG = rows_per_cta<LPC>();
+    const unsigned grid = (unsigned)((long long)qn * ((P.ny + RG - 1) / RG));
+    k_rows_inverse<L, LPC, NP, ROWPF, HALF>
+        <<<grid, LPC * L::TPL, smem_rows_inverse<L, NP, ROWPF, HALF>(line.n), s>>>(P, line, T, Tab, slab, q0);
+    return cudaGetLastError();
+}
+template <class L>
+static cudaError_t rows_inverse_impl(const StageParams &P, L line, const float2 *T, const float2 *Tab,
+                                     float2 *slab, int q0, int qn, cudaStream_t s)
+{
+    // scipy prefilters the row axis on the tilted path only, and leaves an
+    // axis of length 1 alone
+    return with_poles(stage_poles(P), [&](auto np) {
+        constexpr int NP = decltype(np)::value;
+        const bool rowpf = NP > 0 && P.tilted && P.nx >= 2;
+        if constexpr (half_line<L>()) {
+            if (half_crop(P)) {
+                if constexpr (NP > 0) {
+                    if (rowpf)
+                        return rows_launch<L, NP, true, true>(P, line, T, Tab, slab, q0, qn, s);
+                }
+                return rows_launch<L, NP, false, true>(P, line, T, Tab, slab, q0, qn, s);
+            }
+        }
+        if constexpr (NP > 0) {
+            if (rowpf)
+                return rows_launch<L, NP, true, false>(P, line, T, Tab, slab, q0, qn, s);
+        }
+        return rows_launch<L, NP, false, false>(P, line, T, Tab, slab, q0, qn, s);
+    });
+}
+
 // The attribute is per kernel and process-wide, so it is always set to the
 // largest size the instantiation can need (the generic line serves every
 // length up to its maximum).
+template <class F>
+static cudaError_t allow_smem(F *kernel, size_t bytes)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+template <class L, int NP, bool HALF>
+static cudaError_t set_smem_attrs_crop(int n)
+{
+    constexpr int KX = Cfg<L>::KX, LPC = Cfg<L>::LPC;
+    cudaError_t e = allow_smem(k_columns_propagate<L, KX, HALF, false>, smem_cols_prop<L, HALF>(n));
+    if (e == cudaSuccess)
+        e = allow_smem(k_columns_propagate<L, KX, HALF, true>, smem_cols_prop<L, HALF>(n));
+    if (e == cudaSuccess)
+        e = allow_smem(k_rows_inverse<L, LPC, NP, false, HALF>, smem_rows_inverse<L, NP, false, HALF>(n));
+    if constexpr (NP > 0) {
+        if (e == cudaSuccess)
+            e = allow_smem(k_rows_inverse<L, LPC, NP, true, HALF>, smem_rows_inverse<L, NP, true, HALF>(n));
+    }
+    return e;
+}
 template <class L, int NP>
 static cudaError_t set_smem_attrs_np(int n)
 {
-    cudaError_t e;
-    if constexpr (NP >= 1) {
-        e = cudaFuncSetAttribute(k_rows_inverse<L, Cfg<L>::LPC, NP, false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows<L>(n));
-        if (e != cudaSuccess)
-            return e;
-        e = cudaFuncSetAttribute(k_rows_inverse<L, Cfg<L>::LPC, NP, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(smem_rows<L>(n) + smem_rows_y<L, NP, true>(n)));
-        if (e != cudaSuccess)
-            return e;
-        e = cudaFuncSetAttribute(k_rows_line<L, Cfg<L>::LPC, NP, false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows<L>(n));
-        if (e != cudaSuccess)
-            return e;
-        e = cudaFuncSetAttribute(k_rows_line<L, Cfg<L>::LPC, NP, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows<L>(n));
-        if (e != cudaSuccess)
-            return e;
-    }
+    constexpr int KX = Cfg<L>::KX, LPC = Cfg<L>::LPC;
+    cudaError_t e = set_smem_attrs_crop<L, NP, false>(n);
     if constexpr (half_line<L>()) {
-        e = cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, true, NP, false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols_prop<L, true>(n));
-        if (e != cudaSuccess)
-            return e;
-        if constexpr (NP == 0) {
-            e = cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, true, NP, true>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_cols_prop<L, true>(n));
-            if (e != cudaSuccess)
-                return e;
-        }
-        if constexpr (NP >= 1) {
-            e = cudaFuncSetAttribute(k_rows_inverse_half<L, Cfg<L>::LPC, half_groups<L>(), NP, false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows_half<L>(n));
-            if (e != cudaSuccess)
-                return e;
-            e = cudaFuncSetAttribute(k_rows_inverse_half<L, Cfg<L>::LPC, half_groups<L>(), NP, true>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(smem_rows_half<L>(n) + smem_rows_y<L, NP, true>(n)));
-            if (e != cudaSuccess)
-                return e;
-        }
+        if (e == cudaSuccess)
+            e = set_smem_attrs_crop<L, NP, true>(n);
     }
-    if constexpr (NP == 0) {
-        e = cudaFuncSetAttribute(k_columns_spectrum<L, Cfg<L>::KX, NP, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols<L>(n));
-        if (e != cudaSuccess)
-            return e;
-        e = cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, false, NP, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_cols_prop<L, false>(n));
-        if (e != cudaSuccess)
-            return e;
+    if constexpr (NP > 0) {
+        if (e == cudaSuccess)
+            e = allow_smem(k_rows_line<L, LPC, NP, false>, smem_rows<L>(n));
+        if (e == cudaSuccess)
+            e = allow_smem(k_rows_line<L, LPC, NP, true>, smem_rows<L>(n));
+        if (e == cudaSuccess)
+            e = allow_smem(k_columns_boundary<L, KX, NP, false>, smem_cols<L>(n));
+        if (e == cudaSuccess)
+            e = allow_smem(k_columns_boundary<L, KX, NP, true>, smem_cols<L>(n));
     }
-    e = cudaFuncSetAttribute(k_columns_spectrum<L, Cfg<L>::KX, NP, false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols<L>(n));
-    if (e != cudaSuccess)
-        return e;
-    return cudaFuncSetAttribute(k_columns_propagate<L, Cfg<L>::KX, false, NP, false>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols_prop<L, false>(n));
+    return e;
 }
 
 template <class L>
@@ -1340,8 +1079,9 @@ static cudaError_t set_smem_attrs(int n)
     if (std::is_same<L, GenericLine>::value)
         n = GenericLine::TPL * GenericLine::SLOTS;
     cudaError_t e;
-    e = cudaFuncSetAttribute(k_rows_forward<L, Cfg<L>::LPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_rows<L>(n));
+    e = allow_smem(k_rows_forward<L, Cfg<L>::LPC>, smem_rows<L>(n));
+    if (e == cudaSuccess)
+        e = allow_smem(k_columns_spectrum<L, Cfg<L>::KX>, smem_cols<L>(n));
     if (e != cudaSuccess)
         return e;
     for (int np = 0; np <= 2; ++np) {
@@ -1361,7 +1101,7 @@ int columns_slots(const StageParams &P)
     const cudaError_t e = with_line(P.lNy, [&](auto line) {
         using L = decltype(line);
         constexpr int KX = Cfg<L>::KX;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_columns_propagate<L, KX, false, 0, false>,
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_columns_propagate<L, KX, false, false>,
                                                              KX * L::TPL, smem_cols_prop<L, false>(line.n));
     });
     return e == cudaSuccess ? per * sms : 0;
@@ -1400,7 +1140,7 @@ cudaError_t launch_columns_propagate(const StageParams &P, const float2 *spec, f
 bool half_crop(const StageParams &P)
 {
     const int N = P.lNx;
-    return P.lNy == N && N >= 256 && N <= 4096 && (N & (N - 1)) == 0 && 2 * P.ny == N && 2 * P.nx == N &&
+    return P.lNy == N && N >= 64 && N <= 4096 && (N & (N - 1)) == 0 && 2 * P.ny == N && 2 * P.nx == N &&
            4 * P.padyl == N && 4 * P.padxl == N && P.nz == P.nx && P.ypitch == P.ny;
 }
 
@@ -1415,8 +1155,9 @@ cudaError_t launch_rows_line(const StageParams &P, const float2 *spec, const flo
     return with_line(P.lNx, [&](auto line) {
         using L = decltype(line);
         constexpr int LPC = Cfg<L>::LPC;
-        const unsigned grid = (unsigned)((qn + rows_per_cta<LPC>() - 1) / rows_per_cta<LPC>());
-        return with_poles(row_poles(P), [&](auto np) {
+        const unsigned grid = (unsigned)((qn + line_jobs_per_cta<LPC>() - 1) / line_jobs_per_cta<LPC>());
+        // (one pole's kernel also runs orders 0 and 1, without prefilter terms)
+        return with_poles(std::max(1, stage_poles(P)), [&](auto np) {
             constexpr int NP = decltype(np)::value;
             if constexpr (NP >= 1) {
                 if (P.units)
@@ -1433,14 +1174,46 @@ cudaError_t launch_rows_line(const StageParams &P, const float2 *spec, const flo
     });
 }
 
-cudaError_t launch_columns_spectrum(const StageParams &P, float2 *rowspec, float2 *Tab, int nunits, cudaStream_t s)
+cudaError_t launch_columns_spectrum(const StageParams &P, const float2 *rowspec, float2 *spec, int nslots,
+                                    cudaStream_t s)
 {
-    if (single_row_plan(P)) {
-        const long long n = (long long)nunits * P.lNx;
-        k_spectrum_line<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, rowspec, Tab, nunits);
-        return cudaGetLastError();
+    return with_line(P.lNy, [&](auto line) { return spectrum_impl(P, line, rowspec, spec, nslots, s); });
+}
+
+cudaError_t launch_columns_boundary(const StageParams &P, const float2 *spec, float2 *Tab, int nunits, cudaStream_t s)
+{
+    return with_line(P.lNy, [&](auto line) { return boundary_impl(P, line, spec, Tab, nunits, s); });
+}
+
+cudaError_t launch_spectrum_line(const StageParams &P, float2 *spec, float2 *Tab, int nunits, cudaStream_t s)
+{
+    const long long n = (long long)nunits * P.lNx;
+    k_spectrum_line<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, spec, Tab, nunits);
+    return cudaGetLastError();
+}
+
+StageParams transposed(const StageParams &P)
+{
+    StageParams t = P;
+    std::swap(t.ny, t.nx);
+    std::swap(t.lNy, t.lNx);
+    std::swap(t.padyl, t.padxl);
+    std::swap(t.kx_zero_lo, t.ky_zero_lo);
+    std::swap(t.kx_zero_hi, t.ky_zero_hi);
+    std::swap(t.kxs, t.kys);
+    t.tab = P.tabt;
+    t.tabt = P.tab;
+    // T rows: the crop and npoles samples on either side, or the whole column
+    // where those would wrap around its ends
+    t.trow0 = t.padyl - t.npoles;
+    t.trows = t.ny + 2 * t.npoles;
+    if (t.trow0 < 0 || t.trow0 + t.trows > t.lNy) {
+        t.trow0 = 0;
+        t.trows = t.lNy;
     }
-    return with_line(P.lNy, [&](auto line) { return spectrum_impl(P, line, rowspec, Tab, nunits, s); });
+    for (int e = 0; e < EDGE_SLOTS; ++e)
+        t.tedge[e] = (t.padyl + edge_offset(e, t.ny) + 2 * t.lNy) % t.lNy - t.trow0;
+    return t;
 }
 
 cudaError_t launch_rows_inverse(const StageParams &P, const float2 *T, const float2 *Tab, float2 *slab, int q0,
