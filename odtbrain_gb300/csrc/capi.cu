@@ -45,11 +45,12 @@ uint64_t g_table_alloc_limit = 0;
 std::mutex g_debug_mutex;
 
 constexpr uint64_t kDefaultWorkspace = 16ull << 30;   // 16 GiB of slabs, chunk buffers etc.
-// column-stage output chunk.  Large chunks (1024 planes of a 512-wide
-// spectrum) mean few launches with full waves; measured on the 256^3
-// workload (two chunk buffers of half the size each): 64 MB 92.8 ms, 256 MB
-// 84.2 ms, 1 GB 79.3 ms, 2 GB 78.7 ms, 4 GB 78.7 ms per reconstruction.
-constexpr uint64_t kPlaneBudget = 1024ull << 20;
+// Column-stage output chunk: planes and bytes at most.  Large chunks mean few
+// launches with full waves.  Step with 256 / 512 / 1024 / 2048 / 4096 planes:
+// 256^3 from 200 views 28.6 / 27.8 / 27.0 / 26.6 / 26.6 ms, 128^3 from 90
+// 2.15 / 2.03 / 1.88 / 1.82 / 1.92 ms.
+constexpr size_t kMaxJobs = 2048;
+constexpr uint64_t kPlaneBudget = 2048ull << 20;
 constexpr size_t kAlign = 256;
 
 size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
@@ -320,9 +321,7 @@ Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
     // the chunk buffer takes at most an eighth of the limit, so tight limits
     // (save_memory) keep room for a batch of slabs
     const uint64_t plane_budget = std::min<uint64_t>(kPlaneBudget, limit / 8);
-    // and at most 1024 planes (where the gain levels off), so small planes do
-    // not take memory for nothing
-    const size_t jobs_cap = std::max<size_t>(16, std::min<size_t>(1024, plane_budget / plane_row_bytes));
+    const size_t jobs_cap = std::max<size_t>(16, std::min<size_t>(kMaxJobs, plane_budget / plane_row_bytes));
     auto layout = [&](int batch, size_t jobs) -> Layout {
         Layout y{};
         y.units = units;
@@ -852,8 +851,10 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *u
             // planes and lost up to 16 % at 256^3 (step 28.3 ms like this,
             // 28.7 to 33.0 ms overlapped): a column launch is one wave of
             // long CTAs, and row CTAs that take its slots stretch it.
-            for (int q0 = 0; q0 < total; q0 += lay.jobs) {
-                const int qn = std::min(lay.jobs, total - q0);
+            // (chunks of equal size, so that the last one fills its waves too)
+            const int nchunks = (total + lay.jobs - 1) / lay.jobs, chunk = (total + nchunks - 1) / nchunks;
+            for (int q0 = 0; q0 < total; q0 += chunk) {
+                const int qn = std::min(chunk, total - q0);
                 lt.begin(ODT_STAGE_COLUMNS_PROPAGATE);
                 e = odt::launch_columns_propagate(Pt, fspec, T, q0, qn, s);
                 if (e != cudaSuccess)

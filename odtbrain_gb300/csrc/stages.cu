@@ -501,7 +501,8 @@ __global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
     const int bar = (L::TPL % 32 == 0 && LPC < 15) ? 1 + l : 0;
     const int ny = P.ny, nx = P.nx, nz = P.nz, padxl = P.padxl;
     const int cpj = (ny + RG - 1) / RG;  // CTAs per job
-    const int bid = (int)blockIdx.x;
+    // (last jobs first: their T rows are the ones still in L2)
+    const int bid = (int)gridDim.x - 1 - (int)blockIdx.x;
     const int qrel = bid / cpj;
     const int ybase = (bid - qrel * cpj) * RG;
     const int GV = min(G, (ny - ybase + LPC - 1) / LPC);  // groups holding a row
@@ -866,11 +867,10 @@ __global__ void __launch_bounds__(256) k_spectrum_line(StageParams P, float2 *ro
 }
 
 // ---------------------------------------------------------------------------
-// Planes per column-stage CTA: enough CTAs for one full wave of the
-// resident slots over the active column groups (the forward column FFT of a
-// CTA is amortised over its planes, so fewer, longer CTAs are better as long
-// as every slot is busy), at least 4 and at most 256 for long runs
-// (long_runs), else at most kReanchorPlanes.
+// Planes per column-stage CTA: the run length that takes the fewest plane
+// times, whole waves of the resident CTAs over the active column groups, with
+// a start-up (tables, exact anchor) counted as four planes.  At most 256 for
+// long runs (long_runs), else at most kReanchorPlanes.
 template <int KX>
 static int planes_per_cta(const StageParams &P, int qn, bool long_run)
 {
@@ -879,9 +879,18 @@ static int planes_per_cta(const StageParams &P, int qn, bool long_run)
     for (int g = 0; g < groups; ++g)
         if (!(g * KX >= P.kx_zero_lo && g * KX + KX <= P.kx_zero_hi))
             ++active;
-    const int per = P.col_slots > 0 ? std::max(1, P.col_slots / std::max(1, active)) : 4;
-    const int ppc = (qn + per - 1) / per;
-    return std::min(long_run ? 256 : kReanchorPlanes, std::max(4, ppc));
+    const int slots = std::max(1, P.col_slots), cap = std::min(long_run ? 256 : kReanchorPlanes, qn);
+    int best = cap;
+    long long least = -1;
+    for (int ppc = cap; ppc >= std::min(4, cap); --ppc) {
+        const long long ctas = (long long)active * ((qn + ppc - 1) / ppc);
+        const long long t = (ctas + slots - 1) / slots * (ppc + 4);
+        if (least < 0 || t < least) {
+            least = t;
+            best = ppc;
+        }
+    }
+    return best;
 }
 
 // Shared memory of the column kernel: the exchange buffers, the twiddle
