@@ -548,15 +548,11 @@ def _run(uSin, angles, res, nm, lD, tilted_axis, weight_angles, onlyreal,
          count):
     torch = _torch()
     dev = _device_for(uSin)
-    weights = None
     flat = np.squeeze(angles) if tilted_axis is not None else angles
-    if weight_angles and len(np.shape(flat)) == 1:
-        weights = geom.compute_angle_weights_1d(flat)
     with torch.cuda.device(dev):
-        if weights is not None and not copy:
+        if weight_angles and not copy and len(np.shape(flat)) == 1:
             # the caller's array now carries the weights; none on the GPU
-            _apply_weights_inplace(uSin, weights)
-            weights = None
+            _apply_weights_inplace(uSin, geom.compute_angle_weights_1d(flat))
             weight_angles = False
         t = _upload(uSin, dev)
         rec = Backprop3D(tuple(t.shape), angles, res, nm, lD=lD,
@@ -565,7 +561,7 @@ def _run(uSin, angles, res, nm, lD, tilted_axis, weight_angles, onlyreal,
                          padding=padding, padfac=padfac, padval=padval,
                          intp_order=intp_order, save_memory=save_memory,
                          input_dtype=str(t.dtype).replace("torch.", ""),
-                         device=dev, weights=weights)
+                         device=dev)
         if count is not None:
             count.value += 2
         vol = rec(t)
