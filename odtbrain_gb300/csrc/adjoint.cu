@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(LPC * L::TPL) k_adj_rows(StageParams P, L line
 // Columns: forward FFT along y of the zero-padded cotangent column of every
 // plane, accumulated against the conjugate propagator into Qg[slot][ky][kx].
 template <class L, int KX, bool PAIR>
-__global__ void __launch_bounds__(KX * L::TPL) k_adj_columns(StageParams P, L line, const float2 *Tg, float2 *Qg,
+__global__ void __launch_bounds__(KX * L::TPL, KX * L::TPL <= 256 ? 3 : 1) k_adj_columns(StageParams P, L line, const float2 *Tg, float2 *Qg,
                                                              int q0, int qn, int ppc)
 {
     if (!group_active<KX>(P, blockIdx.x * KX))
