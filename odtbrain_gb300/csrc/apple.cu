@@ -388,27 +388,50 @@ __global__ void k_apple_tables(int n0, int n1, int n2, double km, double shell_w
     }
 }
 
-__global__ void k_apple_flags(int n0, int n1, int n2, double km, int use_shell, FlagTables T, const uint8_t *mask,
-                              const uint8_t *shell, uint8_t *flags)
+// kr > sqrt(2) km, kr = 2 pi sqrt(s), decided from s alone: both roundings
+// are monotonic, so the largest s for which it does not hold is found once, by
+// bisection over the doubles (an FP64 square root per voxel was most of the
+// flag kernel's time: 256^3 0.66 ms with it).
+double core_limit(double km)
 {
-    // grid (ceil(n2/32), ceil(n1/8), n0), blocks of 32 x 8
-    const double twopi = 6.283185307179586;
-    const double sqrt2km = __dmul_rn(1.4142135623730951, km);
-    {
-        const int i2 = (int)(blockIdx.x * 32 + threadIdx.x), i1 = (int)(blockIdx.y * 8 + threadIdx.y);
-        const int i0 = (int)blockIdx.z;
-        if (i2 >= n2 || i1 >= n1)
-            return;
-        const long long v = ((long long)i0 * n1 + i1) * n2 + i2;
-        bool core = fabs(T.ky[i1]) > T.sroot[(long long)i0 * n2 + i2];
-        const double kr = __dmul_rn(twopi, sqrt(__dadd_rn(__dadd_rn(T.sq[0][i0], T.sq[1][i1]), T.sq[2][i2])));
+    const double sqrt2km = 1.4142135623730951 * km;
+    auto value = [](int64_t bits) {
+        double d;
+        memcpy(&d, &bits, 8);
+        return d;
+    };
+    double top = 1e300;
+    int64_t lo = 0, hi;  // non-negative doubles order like their bits
+    memcpy(&hi, &top, 8);
+    while (lo < hi) {
+        const int64_t mid = lo + (hi - lo + 1) / 2;
+        const double kr = 6.283185307179586 * sqrt(value(mid));
         if (kr > sqrt2km)
-            core = false;
+            hi = mid - 1;
+        else
+            lo = mid;
+    }
+    return value(lo);
+}
+
+__global__ void __launch_bounds__(256) k_apple_flags(int n0, int n1, int n2, double limit, int use_shell,
+                                                     FlagTables T, const uint8_t *mask, const uint8_t *shell, uint8_t *flags)
+{
+    // grid (ceil(n1/8), n0): a warp per (i0, i1) row
+    const int i1 = (int)(blockIdx.x * 8 + threadIdx.x / 32), i0 = (int)blockIdx.y;
+    if (i1 >= n1)
+        return;
+    const double s01 = __dadd_rn(T.sq[0][i0], T.sq[1][i1]), eo01 = __dadd_rn(T.eo[0][i0], T.eo[1][i1]);
+    const double ei01 = use_shell ? __dadd_rn(T.ei[0][i0], T.ei[1][i1]) : 0.0;
+    const double ky = fabs(T.ky[i1]);
+    for (int i2 = threadIdx.x % 32; i2 < n2; i2 += 32) {
+        const long long v = ((long long)i0 * n1 + i1) * n2 + i2;
+        const bool core = ky > T.sroot[(long long)i0 * n2 + i2] && !(__dadd_rn(s01, T.sq[2][i2]) > limit);
         uint8_t f = core ? F_CORE : 0;
-        const bool outer = __dadd_rn(__dadd_rn(T.eo[0][i0], T.eo[1][i1]), T.eo[2][i2]) > 1.0;
+        const bool outer = __dadd_rn(eo01, T.eo[2][i2]) > 1.0;
         if (outer)
             f |= F_SPOV;
-        if (use_shell && outer != (__dadd_rn(__dadd_rn(T.ei[0][i0], T.ei[1][i1]), T.ei[2][i2]) > 1.0))
+        if (use_shell && outer != (__dadd_rn(ei01, T.ei[2][i2]) > 1.0))
             f |= F_SHELL;
         if (shell && shell[v])
             f |= F_SHELL;
@@ -447,8 +470,8 @@ cudaError_t compute_flags(int n0, int n1, int n2, double km, int use_shell, doub
     const int mx = std::max(n0, std::max(n1, n2));
     const unsigned tg = (unsigned)std::max<long long>((mx + 255) / 256, std::min<long long>((q + 255) / 256, 1024));
     k_apple_tables<<<tg, 256, 0, s>>>(n0, n1, n2, km, shell_width, T);
-    const dim3 fg((unsigned)((n2 + 31) / 32), (unsigned)((n1 + 7) / 8), (unsigned)n0), fb(32, 8);
-    k_apple_flags<<<fg, fb, 0, s>>>(n0, n1, n2, km, use_shell, T, mask, shell, flags);
+    const dim3 fg((unsigned)((n1 + 7) / 8), (unsigned)n0);
+    k_apple_flags<<<fg, 256, 0, s>>>(n0, n1, n2, core_limit(km), use_shell, T, mask, shell, flags);
     return cudaGetLastError();
 }
 
@@ -632,22 +655,77 @@ __global__ void k_edt_gather(long long M, const int *ft, const double *in, doubl
 // 32 consecutive x2 positions (the filtered axis) and 8 x1 rows.
 constexpr int GAUSS_RMAX = 64;  // radius limit (sigma <= 15.9, volumes <= 1590)
 
+// One axis of the Gaussian over staged samples x[k * st], k = -r..r, in
+// scipy's order x[0] w0 + sum_{j=r..1} (x[j] + x[-j]) w_j.
+// float64 data: FP64.
+__device__ __forceinline__ double gauss_sum(const double *x, int st, const double *w, int r)
+{
+    double acc = __dmul_rn(x[0], w[r]);
+    for (int j = r; j >= 1; --j)
+        acc = __dadd_rn(acc, __dmul_rn(__dadd_rn(x[j * st], x[-j * st]), w[r + j]));
+    return acc;
+}
+// float32 data: the FP64 sum rounded to float32 is what scipy stores.  FP64
+// runs at 1/64 of the FP32 rate here, so the sum is carried as an unevaluated
+// pair of floats (error-free sums after Knuth, products with FMA; the weights
+// split into two floats): all terms are non-negative, so its relative error
+// stays below 2^-44 and the rounded result is the FP64 one's except for
+// values that close to a rounding boundary.  Sums outside the range where the
+// products are exact (or not finite) are formed again in FP64.
+__device__ __forceinline__ float gauss_sum(const float *x, int st, const float2 *ws, const double *w, int r)
+{
+    float2 wj = ws[0];
+    float hi = x[0] * wj.x, lo = fmaf(x[0], wj.x, -hi) + x[0] * wj.y;
+    const float c0h = hi, c0l = lo;
+    hi = lo = 0.f;
+    auto add = [&](float ph, float pl) {
+        const float t = hi + ph, z = t - hi;
+        lo += ((hi - (t - z)) + (ph - z)) + pl;
+        hi = t;
+    };
+    add(c0h, c0l);
+    for (int j = r; j >= 1; --j) {
+        wj = ws[j];
+        const float a = x[j * st], b = x[-j * st];
+        const float sum = a + b, z = sum - a, err = (a - (sum - z)) + (b - z);
+        const float ph = sum * wj.x;
+        add(ph, fmaf(sum, wj.x, -ph) + fmaf(sum, wj.y, err * wj.x));
+    }
+    if (!(hi >= 1e-24f && hi <= 1e37f)) {
+        double acc = __dmul_rn((double)x[0], w[r]);
+        for (int j = r; j >= 1; --j)
+            acc = __dadd_rn(acc, __dmul_rn(__dadd_rn((double)x[j * st], (double)x[-j * st]), w[r + j]));
+        return (float)acc;
+    }
+    return __fadd_rn(hi, lo);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_env_gauss(EnvGeom G, int axis, const double *hp, const T *in, T *out,
                                                    const double *w, int r)
 {
-    extern __shared__ double gx[];  // the staged inputs with halo
+    extern __shared__ double gauss_smem[];
+    T *gx = reinterpret_cast<T *>(gauss_smem);  // the staged inputs with halo
+    __shared__ float2 ws[GAUSS_RMAX + 1];       // float32: w_j as (hi, lo)
     const int n[3] = {G.n0, G.n1, G.n2};
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
     int ii[3];
-    auto input = [&](int a0, int a1, int a2) -> double {
+    auto input = [&](int a0, int a1, int a2) -> T {
         if (a0 < 0 || a0 >= G.n0 || a1 < 0 || a1 >= G.n1 || a2 < 0 || a2 >= G.n2)
-            return 0.0;
+            return T(0);
         if (axis == 0)
-            return (double)(T)hp[((long long)(a0 + G.off0) * G.msh + (a1 + G.off1)) * G.msh + (a2 + G.off2)];
-        return (double)in[((long long)a0 * G.n1 + a1) * G.n2 + a2];
+            return (T)hp[((long long)(a0 + G.off0) * G.msh + (a1 + G.off1)) * G.msh + (a2 + G.off2)];
+        return in[((long long)a0 * G.n1 + a1) * G.n2 + a2];
     };
-    double acc;
+    if constexpr (sizeof(T) == 4) {
+        if (tid <= r) {
+            const double v = w[r + tid];
+            const float h = (float)v;
+            ws[tid] = make_float2(h, (float)(v - (double)h));
+        }
+    }
+    const T *x;
+    int st;
     if (axis < 2) {
         // grid (ceil(n2/32), ceil(n_axis/8), n_other); smem [(8 + 2r)][32]
         const int a2 = (int)blockIdx.x * 32 + tx;
@@ -665,10 +743,8 @@ __global__ void __launch_bounds__(256) k_env_gauss(EnvGeom G, int axis, const do
         ii[axis] = k;
         ii[axis == 0 ? 1 : 0] = other;
         ii[2] = a2;
-        const double *col = gx + (ty + r) * 32 + tx;
-        acc = __dmul_rn(col[0], w[r]);
-        for (int j = r; j >= 1; --j)
-            acc = __dadd_rn(acc, __dmul_rn(__dadd_rn(col[j * 32], col[-j * 32]), w[r + j]));
+        x = gx + (ty + r) * 32 + tx;
+        st = 32;
     } else {
         // grid (ceil(n2/32), ceil(n1/8), n0); smem [8][32 + 2r]
         const int wdt = 32 + 2 * r;
@@ -684,18 +760,21 @@ __global__ void __launch_bounds__(256) k_env_gauss(EnvGeom G, int axis, const do
         ii[0] = (int)blockIdx.z;
         ii[1] = a1;
         ii[2] = a2;
-        const double *row = gx + ty * wdt + tx + r;
-        acc = __dmul_rn(row[0], w[r]);
-        for (int j = r; j >= 1; --j)
-            acc = __dadd_rn(acc, __dmul_rn(__dadd_rn(row[j], row[-j]), w[r + j]));
+        x = gx + ty * wdt + tx + r;
+        st = 1;
     }
+    T acc;
+    if constexpr (sizeof(T) == 4)
+        acc = gauss_sum(x, st, ws, w, r);
+    else
+        acc = gauss_sum(x, st, w, r);
     long long o = ((long long)ii[0] * G.n1 + ii[1]) * G.n2 + ii[2];
     if (axis == 2) {  // ifftshift: out[k] = g[(k + n/2) mod n]  =>  g[i] -> out[i - n/2]
         const int s0 = wrapi(ii[0] - G.n0 / 2, G.n0), s1 = wrapi(ii[1] - G.n1 / 2, G.n1),
                   s2 = wrapi(ii[2] - G.n2 / 2, G.n2);
         o = ((long long)s0 * G.n1 + s1) * G.n2 + s2;
     }
-    out[o] = (T)acc;
+    out[o] = acc;
 }
 
 // envelope_gauss (apple.py:289-350) of the spectrum `orig` (n0 == n2; C2 =
@@ -756,7 +835,7 @@ cudaError_t run_envelope(int n0, int n1, int n2, int gr, const C2 *orig, const u
     const dim3 vb(32, 8);
     const dim3 g0g((unsigned)((n2 + 31) / 32), (unsigned)((n0 + 7) / 8), (unsigned)n1);
     const dim3 g1g((unsigned)((n2 + 31) / 32), (unsigned)((n1 + 7) / 8), (unsigned)n0);
-    const size_t sm01 = (size_t)(8 + 2 * gr) * 32 * 8, sm2 = (size_t)8 * (32 + 2 * gr) * 8;
+    const size_t sm01 = (size_t)(8 + 2 * gr) * 32 * sizeof(T), sm2 = (size_t)8 * (32 + 2 * gr) * sizeof(T);
     const size_t smx = std::max(sm01, sm2);
     if (smx > 48 * 1024 &&
         (e = cudaFuncSetAttribute(k_env_gauss<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx)))
