@@ -877,6 +877,9 @@ odt_status run_plan(const odt_bpp3d_plan *plan, const Layout &lay, const int2 *u
         R.last_pass = b == nbatches - 1;
         R.onlyreal = d.onlyreal;
         R.status = plan->d_status;
+        // the column stage's output is dead here: room for partial sums
+        R.part = (float4 *)T;
+        R.part_bytes = lay.off_Tab - lay.off_T;
         lt.begin(ODT_STAGE_ROTATE);
         e = odt::launch_rotate(R, d.intp_order, d.geometry == ODT_GEOM_AFFINE3D, slab,
                                geometry + (size_t)a0 * geo_stride, volume, comp, rot_scratch, s);
@@ -1024,6 +1027,8 @@ static odt_status run_adjoint(const odt_bpp3d_plan *plan, const Layout &lay, con
         R.last_pass = 1;
         R.onlyreal = 0;
         R.status = plan->d_status;
+        R.part = nullptr;
+        R.splits = 1;
         e = odt::launch_rotate_adjoint(R, d.intp_order, tilted ? 1 : 0, vg,
                                        geometry + (size_t)u0 * geo_stride, slab, ws + lay.off_rot, s);
         if (e != cudaSuccess)

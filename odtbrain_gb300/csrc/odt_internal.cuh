@@ -99,6 +99,12 @@ struct RotParams {
     int last_pass;    // this launch ends the sum (drop the compensation)
     int onlyreal;
     int *status;
+    // split sums (y axis; rotate.cu): room for partial sums (NULL: no
+    // splitting); the rest is filled in by launch_rotate
+    float4 *part;
+    size_t part_bytes;
+    int splits, per_split, ncta;  // splits, angles per split, tiles x y blocks
+    int *done;
 };
 
 // Launchers (stream-ordered; return cudaGetLastError()).
@@ -131,7 +137,7 @@ cudaError_t launch_rows_line(const StageParams &P, const float2 *spec, const flo
 cudaError_t launch_rows_inverse(const StageParams &P, const float2 *T, const float2 *Tab, float2 *slab, int q0,
                                 int qn, cudaStream_t s);
 // Scratch (device bytes) the rotation stage needs for a batch: per-(angle,
-// tile) geometry records of the y-axis path.
+// tile) geometry records of the y-axis path and its split counters.
 size_t rotate_scratch_bytes(int nbatch_angles, int ny, int nx, int nz, int tilted);
 cudaError_t launch_rotate(const RotParams &R, int order, int tilted, const float2 *slab, const double *geo,
                           void *volume, float2 *comp, void *scratch, cudaStream_t s);

@@ -24,6 +24,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "odt_fft.cuh"
@@ -211,6 +212,57 @@ __device__ __forceinline__ void kahan_add(float2 &s, float2 &c, float2 v)
     s.y = t;
 }
 
+// (S, C) + (s, c), compensated: (S - C) + (s - c)
+__device__ __forceinline__ void merge_sums(float2 &S, float2 &C, float2 s, float2 c)
+{
+    float y = (s.x - c.x) - C.x;
+    float t = S.x + y;
+    C.x = (t - S.x) - y;
+    S.x = t;
+    y = (s.y - c.y) - C.y;
+    t = S.y + y;
+    C.y = (t - S.y) - y;
+    S.y = t;
+}
+
+// Split sums: with R.splits > 1 the batch's angles are divided among `splits`
+// CTAs per tile, so that small volumes fill the device.  Each leaves its
+// compensated sums (one float4 per thread and sum, R.part), and the CTA that
+// finishes last merges all of them in the order of the angles.  Returns true
+// in that CTA, with the merged sums in s, c.
+template <int N>
+__device__ __forceinline__ bool merge_splits(float4 *part, int *done, int splits, int cta, int ncta, int split,
+                                             float2 (&s)[N], float2 (&c)[N])
+{
+    const int nt = blockDim.x;
+    float4 *mine = part + ((size_t)split * ncta + cta) * N * nt + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+        mine[q * nt] = make_float4(s[q].x, s[q].y, c[q].x, c[q].y);
+    __threadfence();
+    __syncthreads();
+    __shared__ int before;
+    if (threadIdx.x == 0)
+        before = atomicAdd(done + cta, 1);
+    __syncthreads();
+    if (before != splits - 1)
+        return false;
+    __threadfence();
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+        s[q] = c[q] = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int t = 0; t < splits; ++t) {
+        const float4 *p = part + ((size_t)t * ncta + cta) * N * nt + threadIdx.x;
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            const float4 v = __ldcg(p + q * nt);
+            merge_sums(s[q], c[q], make_float2(v.x, v.y), make_float2(v.z, v.w));
+        }
+    }
+    return true;
+}
+
 // Store the compensated partial sum of this launch (s, c) for voxel `idx`.
 template <bool ONLYREAL>
 __device__ __forceinline__ void store_sum(const RotParams &R, void *volume, float2 *comp, size_t idx, float2 s,
@@ -226,15 +278,9 @@ __device__ __forceinline__ void store_sum(const RotParams &R, void *volume, floa
             S1 = make_float2(reinterpret_cast<float *>(volume)[idx], 0.f);
         else
             S1 = reinterpret_cast<float2 *>(volume)[idx];
-        // (S1 - C1) + (s - c), compensated
-        float y = (s.x - c.x) - C1.x;
-        float t = S1.x + y;
-        C.x = (t - S1.x) - y;
-        S.x = t;
-        y = (s.y - c.y) - C1.y;
-        t = S1.y + y;
-        C.y = (t - S1.y) - y;
-        S.y = t;
+        merge_sums(S1, C1, s, c);
+        S = S1;
+        C = C1;
     }
     if (R.last_pass) {
         S = make_float2(S.x - C.x, S.y - C.y);
@@ -348,6 +394,9 @@ __global__ void k_rotate_y_setup(RotParams R, const double *__restrict__ geo, Ti
 {
     const int ntz = (R.nz + R2_T - 1) / R2_T, ntx = (R.nx + R2_T - 1) / R2_T;
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (R.splits > 1)
+        for (int i = id; i < R.ncta; i += gridDim.x * blockDim.x)
+            R.done[i] = 0;
     if (id >= R.nbatch_angles * ntz * ntx)
         return;
     const int a = id / (ntz * ntx), t = id % (ntz * ntx);
@@ -590,10 +639,17 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_rotate_y(RotParams R, const f
     const int hw = tid / LPO, yl = (tid % LPO) * 2;
     const int ntx = (R.nx + R2_T - 1) / R2_T, ntz = (R.nz + R2_T - 1) / R2_T;
     const int tile = blockIdx.y * ntx + blockIdx.x;
-    const int ox0 = blockIdx.x * R2_T, oz0 = blockIdx.y * R2_T, y0 = blockIdx.z * R2_Y;
+    const int nyb = (R.ny + R2_Y - 1) / R2_Y, split = blockIdx.z / nyb, yblk = blockIdx.z - split * nyb;
+    const int ox0 = blockIdx.x * R2_T, oz0 = blockIdx.y * R2_T, y0 = yblk * R2_Y;
     const int nx = R.nx, nz = R.nz, ny = R.ny, yp = R.ypitch;
-    const int nb = R.nbatch_angles;
     const size_t aslab_stride = (size_t)nz * nx * yp;
+    // this CTA's angles (all of the batch's, or its split's share of them)
+    // (no division: the records' addresses stay block-uniform)
+    const int abase = split * R.per_split;
+    const int nb = min(R.per_split, R.nbatch_angles - abase);
+    geo += 6 * (size_t)abase;
+    tiles += (size_t)abase * ntz * ntx;
+    slab += abase * aslab_stride;
     // this thread's outputs: x = ox0 + (hw & 15), z = oz0 + (hw >> 4) * OUTW + i
     const int hx = hw & 15, hz0 = (hw >> 4) * OUTW;
     float2 s[R2_OUT], cp[R2_OUT], part[R2_OUT];  // [output q][y pair]: 2q, 2q+1
@@ -625,7 +681,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_rotate_y(RotParams R, const f
                 const unsigned bytes = (unsigned)t.box_zn * t.box_xn * R2_Y * sizeof(float2);
                 fence_proxy_async_smem();
                 mbar_arrive_expect_tx(bar + b, bytes);
-                tma_load_4d(box + b * R2_BOXE, &maps.m[mi], bar + b, y0, t.box_x0, t.box_z0, aa);
+                tma_load_4d(box + b * R2_BOXE, &maps.m[mi], bar + b, y0, t.box_x0, t.box_z0, abase + aa);
             }
         } else if (t.box_zn > 0) {
             stage_box<R2_Y>(t, slab + (size_t)aa * aslab_stride, nz, nx, yp, y0, box + b * R2_BOXE);
@@ -747,6 +803,8 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_rotate_y(RotParams R, const f
         if (a + 1 < nb)
             cur = load_tile(ring + (a + 1) % R2_RING);
     }
+    if (R.splits > 1 && !merge_splits<R2_OUT>(R.part, R.done, R.splits, tile * nyb + yblk, R.ncta, split, s, cp))
+        return;
     const int ox = ox0 + hx;
     if (ox < nx) {
 #pragma unroll
@@ -795,7 +853,9 @@ __device__ __forceinline__ void stage_plane(const BoxDesc &b, const float2 *asla
     }
 }
 
-template <int ORDER, bool ONLYREAL>
+// SPLIT: a share of the angles per CTA (merge_splits), for few tiles; the
+// whole loop keeps its 48 registers (5 CTAs per SM) in a kernel of its own.
+template <int ORDER, bool ONLYREAL, bool SPLIT>
 __global__ void __launch_bounds__(R2_T * R2_T) k_rotate_plane(RotParams R, const float2 *__restrict__ slab,
                                                               const double *__restrict__ geo,
                                                               const TileGeo *__restrict__ tiles, void *volume,
@@ -808,10 +868,19 @@ __global__ void __launch_bounds__(R2_T * R2_T) k_rotate_plane(RotParams R, const
     const int tile = blockIdx.y * ntx + blockIdx.x;
     const int ox0 = blockIdx.x * R2_T, oz0 = blockIdx.y * R2_T;
     const int ox = ox0 + (tid & (R2_T - 1)), oz = oz0 + tid / R2_T;
-    const int nx = R.nx, nz = R.nz, nb = R.nbatch_angles;
+    const int nx = R.nx, nz = R.nz, split = SPLIT ? blockIdx.z : 0;
     const size_t astride = (size_t)nz * nx, rstride = (size_t)ntz * ntx;
+    // this CTA's angles (all of the batch's, or its split's share of them)
+    // (no division: the records' addresses stay block-uniform)
+    const int abase = SPLIT ? split * R.per_split : 0;
+    const int nb = SPLIT ? min(R.per_split, R.nbatch_angles - abase) : R.nbatch_angles;
+    if (SPLIT) {
+        geo += 6 * (size_t)abase;
+        slab += abase * astride;
+        tiles += abase * rstride;
+    }
     const TileGeo *trec = tiles + tile;
-    float2 s = make_float2(0.f, 0.f), c = s, part = s;
+    float2 s[1] = {make_float2(0.f, 0.f)}, c[1] = {make_float2(0.f, 0.f)}, part = make_float2(0.f, 0.f);
     // angles 0 and 1 staged; records: cur = 0, nxt = 1; box d2 = angle 2
     TileGeo cur = load_tile(trec);
     TileGeo nxt = cur;
@@ -862,7 +931,7 @@ __global__ void __launch_bounds__(R2_T * R2_T) k_rotate_plane(RotParams R, const
             part = acc;
         }
         if ((a % R2_KAHAN) == R2_KAHAN - 1 || a == nb - 1) {
-            kahan_add(s, c, part);
+            kahan_add(s[0], c[0], part);
             part = make_float2(0.f, 0.f);
         }
         __syncthreads();  // box[a % 3] is refilled with angle a + 3 next
@@ -870,8 +939,10 @@ __global__ void __launch_bounds__(R2_T * R2_T) k_rotate_plane(RotParams R, const
         nxt = nxt2;
         d2 = d3;
     }
+    if (SPLIT && !merge_splits<1>(R.part, R.done, R.splits, tile, R.ncta, split, s, c))
+        return;
     if (oz < nz && ox < nx)
-        store_sum<ONLYREAL>(R, volume, comp, (size_t)oz * nx + ox, s, c);
+        store_sum<ONLYREAL>(R, volume, comp, (size_t)oz * nx + ox, s[0], c[0]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1149,21 +1220,84 @@ static bool rotate_tma_ok(const RotParams &R, const float2 *slab)
            tensor_map_encoder() != nullptr;
 }
 
+// Angle splits of the y-axis resampling of `ncta` tiles with `angles` angles
+// each and `slots` resident CTAs (one per SM): the count with the fewest
+// angle times over whole waves, where a CTA's start and merge count as two
+// angles; at most 16, and `most` (the room for partial sums).  64^3 from 30
+// units, 64 tiles on 152 SMs: step 0.36 -> 0.32 ms; 101 x 150^2 from 121 views,
+// 700 tiles: 8.80 -> 8.66 ms.
+static int angle_splits(int ncta, int angles, int slots, size_t most)
+{
+    int best = 1;
+    long long least = -1;
+    for (int n = 1; n <= 16 && n <= angles && (n == 1 || (size_t)n <= most); ++n) {
+        const long long waves = ((long long)ncta * n + slots - 1) / slots;
+        const long long t = waves * ((angles + n - 1) / n + 2);
+        if (least < 0 || t < least) {
+            least = t;
+            best = n;
+        }
+    }
+    return best;
+}
+// ... and of the single-row path, whose CTAs share an SM: only as many as fit
+// beside each other (a second wave's CTAs run faster for having the SM to
+// fewer, so splitting full waves gains nothing: 512^2 from 202 units 1.94 ->
+// 1.96 ms), with at least 3 angles each.  128^2 from 30 units, 64 tiles on 608
+// slots: 0.125 -> 0.090 ms.
+static int plane_splits(int ncta, int angles, int slots, size_t most)
+{
+    int n = std::min(std::min(16, angles / 3), slots / std::max(1, ncta));
+    if ((size_t)n > most)
+        n = (int)most;
+    return std::max(1, n);
+}
+static int resident_ctas(const void *kernel, int threads, size_t smem)
+{
+    int dev = 0, sms = 0, per = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess)
+        return 1;
+    return std::max(1, per * sms);
+}
+
 template <int ORDER, bool ONLYREAL>
-static cudaError_t rotate_impl(const RotParams &R, int tilted, const float2 *slab, const double *geo, void *volume,
+static cudaError_t rotate_impl(RotParams R, int tilted, const float2 *slab, const double *geo, void *volume,
                                float2 *comp, void *scratch, cudaStream_t s)
 {
+    R.splits = 1;
     if (!tilted) {
         const int ntiles = ((R.nx + R2_T - 1) / R2_T) * ((R.nz + R2_T - 1) / R2_T);
         const int nset = R.nbatch_angles * ntiles;
         TileGeo *tiles = reinterpret_cast<TileGeo *>(scratch);
-        if (R.ny == 1 && R.ypitch == 1) {
+        R.done = reinterpret_cast<int *>(tiles + nset);
+        const bool plane = R.ny == 1 && R.ypitch == 1;
+        const int nyb = plane ? 1 : (R.ny + RotY<ORDER>::Y - 1) / RotY<ORDER>::Y;
+        const int per_cta = plane ? R2_T * R2_T : RotY<ORDER>::SUMS * R2_THREADS;  // sums
+        R.ncta = ntiles * nyb;
+        if (R.part && (uintptr_t)R.part % 16 == 0) {
+            const size_t most = R.part_bytes / ((size_t)R.ncta * per_cta * sizeof(float4));
+            R.splits =
+                plane ? plane_splits(R.ncta, R.nbatch_angles,
+                                     resident_ctas((const void *)k_rotate_plane<ORDER, ONLYREAL, true>, R2_T * R2_T, 0),
+                                     most)
+                      : angle_splits(R.ncta, R.nbatch_angles,
+                                     resident_ctas((const void *)k_rotate_y<ORDER, ONLYREAL, true>, R2_THREADS,
+                                                   RotY<ORDER>::SMEM),
+                                     most);
+        }
+        R.per_split = (R.nbatch_angles + R.splits - 1) / R.splits;
+        R.splits = (R.nbatch_angles + R.per_split - 1) / R.per_split;  // none without angles
+        if (plane) {
             k_rotate_y_setup<ORDER, false><<<(nset + 127) / 128, 128, 0, s>>>(R, geo, tiles);
-            dim3 grid((R.nx + R2_T - 1) / R2_T, (R.nz + R2_T - 1) / R2_T);
-            k_rotate_plane<ORDER, ONLYREAL><<<grid, R2_T * R2_T, 0, s>>>(R, slab, geo, tiles, volume, comp);
+            dim3 grid((R.nx + R2_T - 1) / R2_T, (R.nz + R2_T - 1) / R2_T, R.splits);
+            if (R.splits > 1)
+                k_rotate_plane<ORDER, ONLYREAL, true><<<grid, R2_T * R2_T, 0, s>>>(R, slab, geo, tiles, volume, comp);
+            else
+                k_rotate_plane<ORDER, ONLYREAL, false><<<grid, R2_T * R2_T, 0, s>>>(R, slab, geo, tiles, volume, comp);
         } else {
-            constexpr int Y = RotY<ORDER>::Y;
-            dim3 grid((R.nx + R2_T - 1) / R2_T, (R.nz + R2_T - 1) / R2_T, (R.ny + Y - 1) / Y);
+            dim3 grid((R.nx + R2_T - 1) / R2_T, (R.nz + R2_T - 1) / R2_T, nyb * R.splits);
             RotMaps maps;
             std::memset(&maps, 0, sizeof maps);
             if (rotate_tma_ok<ORDER>(R, slab) && encode_slab_maps<ORDER>(R, slab, maps) == cudaSuccess) {
@@ -1185,11 +1319,11 @@ static cudaError_t rotate_impl(const RotParams &R, int tilted, const float2 *sla
 
 size_t rotate_scratch_bytes(int nbatch_angles, int ny, int nx, int nz, int tilted)
 {
-    (void)ny;
     if (tilted)
         return 0;
+    // tile records, then one counter per tile and y block of at least 8
     const size_t ntiles = (size_t)((nx + R2_T - 1) / R2_T) * ((nz + R2_T - 1) / R2_T);
-    return (size_t)nbatch_angles * ntiles * sizeof(TileGeo);
+    return (size_t)nbatch_angles * ntiles * sizeof(TileGeo) + ntiles * ((ny + 7) / 8) * sizeof(int);
 }
 
 template <int ORDER>
