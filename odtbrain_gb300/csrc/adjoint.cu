@@ -32,93 +32,130 @@
 
 namespace odt {
 
-// (a^T... ) rows: crop_x/xfix transpose + forward FFT along x.
-template <class L, int LPC>
-__global__ void __launch_bounds__(LPC * L::TPL) k_adj_rows(StageParams P, L line, const float2 *sgrad, float2 *Tg,
-                                                           int q0, int qn)
+// Rows: crop_x/xfix transpose + forward FFT along x.  A CTA transforms G
+// groups of LPC consecutive rows: they share its twiddle table, and the next
+// group's loads are in flight while the current one is transformed.  The
+// boundary sums are formed with shuffles: shared-memory float atomics on one
+// address are compare-and-swap loops, and 24 lanes of every line met on them
+// (128^3 from 90 views: 1.13 ms with the atomics, 0.60 ms like this).
+template <int LPC>
+constexpr int adj_row_groups()
 {
+    return LPC >= 32 ? 1 : 32 / LPC;
+}
+template <class L, int LPC>
+__global__ void __launch_bounds__(LPC * L::TPL, (LPC * L::TPL <= 256) ? 4 : 1)
+    k_adj_rows(StageParams P, L line, const float2 *sgrad, float2 *Tg, int q0, int qn)
+{
+    constexpr int G = adj_row_groups<LPC>();
     extern __shared__ float2 smem[];
     const int n = line.size();  // lNx
     const int xs = xslots<false>(n);
     float2 *buf0 = smem, *buf1 = smem + LPC * xs, *tw = smem + 2 * LPC * xs;
-    float2 *red = tw + tw_slots(n);  // [LPC][2] boundary sums
+    constexpr int WPL = L::TPL / 32;  // warps per line (0: less than one)
+    float4 *red = reinterpret_cast<float4 *>(tw + (tw_slots(n) + 1) / 2 * 2);  // [LPC][WPL] partial boundary sums
     copy_twiddles<L>(tw, P.tab.twx, n);
     const int l = threadIdx.x / L::TPL, j = threadIdx.x % L::TPL;
+    // lines of whole warps sync on named barrier 1 + l
+    const int bar = (L::TPL % 32 == 0 && LPC < 15) ? 1 + l : 0;
     const int ny = P.ny, nx = P.nx, nz = P.nz, padxl = P.padxl;
-    const long long rid = (long long)blockIdx.x * LPC + l;
-    const bool valid = rid < (long long)qn * ny;
-    const int qq = q0 + (int)((valid ? rid : 0) / ny);
-    const int y = (int)((valid ? rid : 0) % ny);
-    const int a = qq / nz, p = qq % nz;
-    // slab gradient of (a, y, p, xx): [a][y][z][x] from the y-axis
-    // resampling transpose, the forward slab layout [a][z][x][ypitch] from
-    // the tilted one
+    const long long rows = (long long)qn * ny, row0 = (long long)blockIdx.x * LPC * G;
+    const int GV = (int)min((long long)G, (rows - row0 + LPC - 1) / LPC);  // groups holding a row
     const bool tl = P.tilted != 0;
-    const float2 *src = tl ? sgrad + ((size_t)a * nz + p) * nx * P.ypitch + y
-                           : sgrad + (((size_t)a * ny + y) * nz + p) * nx;
-    const size_t xstep = tl ? (size_t)P.ypitch : 1;
-    if (threadIdx.x < 2 * LPC)
-        red[threadIdx.x] = make_float2(0.f, 0.f);
-    __syncthreads();
-    float2 v[L::SLOTS];
-    float2 gA = make_float2(0.f, 0.f), gB = make_float2(0.f, 0.f);
     const bool pf = P.order >= 2;
-#pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int x = j + r * L::TPL;
-        const int xx = x - padxl;
-        float2 t = make_float2(0.f, 0.f);
-        if (valid && x < n && xx >= 0 && xx < nx) {
-            t = src[xx * xstep];
-            if (pf && xx < ZPOW_N) {
-                const float zz = P.tab.zpow[xx];
-                gA.x = fmaf(zz, t.x, gA.x);
-                gA.y = fmaf(zz, t.y, gA.y);
-            }
-            if (pf && nx - 1 - xx < ZPOW_N) {
-                const float zz = P.tab.zpow[nx - 1 - xx];
-                gB.x = fmaf(zz, t.x, gB.x);
-                gB.y = fmaf(zz, t.y, gB.y);
-            }
-        }
-        v[r] = t;
-    }
-    if (pf) {
-        if (gA.x != 0.f || gA.y != 0.f) {
-            atomicAdd(&red[l * 2].x, gA.x);
-            atomicAdd(&red[l * 2].y, gA.y);
-        }
-        if (gB.x != 0.f || gB.y != 0.f) {
-            atomicAdd(&red[l * 2 + 1].x, gB.x);
-            atomicAdd(&red[l * 2 + 1].y, gB.y);
-        }
-        __syncthreads();
-        const float2 A = red[l * 2], B = red[l * 2 + 1];
-        // d0 = u[e0] - u[e1] and d1 = u[e3] - u[e2] enter as
-        // A_coef = ca d0 + cb d1, B_coef = ca d1 + cb d0
-        const float2 d0g = make_float2(P.bx_ca * A.x + P.bx_cb * B.x, P.bx_ca * A.y + P.bx_cb * B.y);
-        const float2 d1g = make_float2(P.bx_cb * A.x + P.bx_ca * B.x, P.bx_cb * A.y + P.bx_ca * B.y);
-        const int e0 = (padxl - 1 + n) % n, e1 = (padxl + 1) % n;
-        const int e2 = (padxl + nx - 2 + n) % n, e3 = (padxl + nx) % n;
+    // this thread's cotangents of row rid.  Slab gradient of (a, y, p, xx):
+    // [a][y][z][x] from the y-axis resampling transpose, the forward slab
+    // layout [a][z][x][ypitch] from the tilted one
+    auto load_row = [&](long long rid, float2 (&v)[L::SLOTS]) {
+        const bool valid = rid < rows;
+        const int qq = q0 + (int)((valid ? rid : 0) / ny), y = (int)((valid ? rid : 0) % ny);
+        const int a = qq / nz, p = qq % nz;
+        const float2 *src = tl ? sgrad + ((size_t)a * nz + p) * nx * P.ypitch + y
+                               : sgrad + (((size_t)a * ny + y) * nz + p) * nx;
+        const size_t xstep = tl ? (size_t)P.ypitch : 1;
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
-            const int x = j + r * L::TPL;
-            if (x == e0) v[r] = v[r] + d0g;
-            if (x == e1) v[r] = v[r] - d0g;
-            if (x == e3) v[r] = v[r] + d1g;
-            if (x == e2) v[r] = v[r] - d1g;
+            const int xx = j + r * L::TPL - padxl;
+            v[r] = (valid && j + r * L::TPL < n && xx >= 0 && xx < nx) ? src[xx * xstep] : make_float2(0.f, 0.f);
         }
-    }
+    };
+    float2 v[L::SLOTS], vn[L::SLOTS];
+    load_row(row0 + l, v);
+    __syncthreads();
     int flip = 0;
-    line.template run<-1>(v, j, buf0 + l * xs, buf1 + l * xs, 1, tw, flip);
-    if (!valid)
-        return;
-    float2 *dst = Tg + (size_t)rid * n;
+#pragma unroll 1
+    for (int g = 0; g < GV; ++g) {
+        const long long rid = row0 + g * LPC + l;
+        if (g + 1 < GV)
+            load_row(rid + LPC, vn);
+        if (pf) {
+            float2 gA = make_float2(0.f, 0.f), gB = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int x = j + r * L::TPL;
-        if (x < n && column_active(P, x))
-            dst[x] = v[r];
+            for (int r = 0; r < L::SLOTS; ++r) {
+                const int xx = j + r * L::TPL - padxl;
+                if (xx >= 0 && xx < ZPOW_N && xx < nx) {
+                    const float zz = P.tab.zpow[xx];
+                    gA = make_float2(fmaf(zz, v[r].x, gA.x), fmaf(zz, v[r].y, gA.y));
+                }
+                if (xx >= 0 && xx < nx && nx - 1 - xx < ZPOW_N) {
+                    const float zz = P.tab.zpow[nx - 1 - xx];
+                    gB = make_float2(fmaf(zz, v[r].x, gB.x), fmaf(zz, v[r].y, gB.y));
+                }
+            }
+            float4 sum = make_float4(gA.x, gA.y, gB.x, gB.y);
+#pragma unroll
+            for (int d = 1; d < (L::TPL < 32 ? L::TPL : 32); d <<= 1) {
+                sum.x += __shfl_xor_sync(0xffffffffu, sum.x, d);
+                sum.y += __shfl_xor_sync(0xffffffffu, sum.y, d);
+                sum.z += __shfl_xor_sync(0xffffffffu, sum.z, d);
+                sum.w += __shfl_xor_sync(0xffffffffu, sum.w, d);
+            }
+            if constexpr (WPL > 1) {
+                if ((j & 31) == 0)
+                    red[l * WPL + j / 32] = sum;
+                if (bar > 0)
+                    line_sync(bar, L::TPL);
+                else
+                    __syncthreads();
+                sum = red[l * WPL];
+#pragma unroll
+                for (int w = 1; w < WPL; ++w) {
+                    const float4 t = red[l * WPL + w];
+                    sum = make_float4(sum.x + t.x, sum.y + t.y, sum.z + t.z, sum.w + t.w);
+                }
+            }
+            const float2 A = make_float2(sum.x, sum.y), B = make_float2(sum.z, sum.w);
+            // d0 = u[e0] - u[e1] and d1 = u[e3] - u[e2] enter as
+            // A_coef = ca d0 + cb d1, B_coef = ca d1 + cb d0
+            const float2 d0g = make_float2(P.bx_ca * A.x + P.bx_cb * B.x, P.bx_ca * A.y + P.bx_cb * B.y);
+            const float2 d1g = make_float2(P.bx_cb * A.x + P.bx_ca * B.x, P.bx_cb * A.y + P.bx_ca * B.y);
+            const int e0 = (padxl - 1 + n) % n, e1 = (padxl + 1) % n;
+            const int e2 = (padxl + nx - 2 + n) % n, e3 = (padxl + nx) % n;
+#pragma unroll
+            for (int r = 0; r < L::SLOTS; ++r) {
+                const int x = j + r * L::TPL;
+                if (x == e0) v[r] = v[r] + d0g;
+                if (x == e1) v[r] = v[r] - d0g;
+                if (x == e3) v[r] = v[r] + d1g;
+                if (x == e2) v[r] = v[r] - d1g;
+            }
+        }
+        // (the transform's barriers also end the reads of the partial sums)
+        line.template run<-1>(v, j, buf0 + l * xs, buf1 + l * xs, 1, tw, flip, bar);
+        if (rid < rows) {
+            float2 *dst = Tg + (size_t)rid * n;
+#pragma unroll
+            for (int r = 0; r < L::SLOTS; ++r) {
+                const int x = j + r * L::TPL;
+                if (x < n && column_active(P, x))
+                    dst[x] = v[r];
+            }
+        }
+        if (g + 1 < GV) {
+#pragma unroll
+            for (int r = 0; r < L::SLOTS; ++r)
+                v[r] = vn[r];
+        }
     }
 }
 
@@ -136,6 +173,9 @@ __global__ void __launch_bounds__(KX * L::TPL, KX * L::TPL <= 256 ? 3 : 1) k_adj
     float2 *buf0 = smem, *buf1 = smem + KX * xs, *tw = smem + 2 * KX * xs;
     float2 *stp = tw + tw_slots(n);  // [n][KX]
     float2 *red = stp + n * KX;      // [KX][2] y-prefilter boundary sums
+    // [SLOTS][threads], each thread its own: sum over the boundary planes of
+    // one end of pole^m Z_p
+    float2 *bsum = red + 2 * KX + threadIdx.x;
     copy_twiddles<L>(tw, P.tab.twy, n);
     const int c = threadIdx.x % KX, j = threadIdx.x / KX;
     const int kx = blockIdx.x * KX + c;
@@ -174,15 +214,46 @@ __global__ void __launch_bounds__(KX * L::TPL, KX * L::TPL <= 256 ? 3 : 1) k_adj
             }
         }
     };
+    // Boundary planes.  Where the two ends do not overlap, the terms
+    // zl conj(alpha) Z_p + zh conj(beta) Z_p are collected as the sum over the
+    // planes of one end (kind 1: zl, 2: zh) and multiplied by the table when
+    // the end's planes are over: a fused multiply-add per element and plane
+    // instead of table reads and, with opposite views, a sine and cosine
+    // (48 of 128 planes: 90 views of 128^2 1.95 -> 1.47 ms).
+    const bool split = pf && nz >= 2 * ZPOW_N;
+    int kind = 0;  // of the planes in bsum, 0: none
+    auto fold = [&]() {
+#pragma unroll
+        for (int r = 0; r < L::SLOTS; ++r) {
+            const int ky = j + r * L::TPL;
+            if (colok && ky < n) {
+                const size_t k = (size_t)ky * lNx + kx;
+                const float2 t = bsum[r * KX * L::TPL];
+                const float2 al = P.tab.alpha[k], be = P.tab.beta[k];
+                Q[r] = Q[r] + cmul_conj(t, kind == 1 ? al : be);
+                if (PAIR)  // the opposite view's, alpha and beta exchanged
+                    R[r] = cfma(cmul_conj(t, kind == 1 ? be : al), expi_phase(P.tab.wsplit[k], copp), R[r]);
+            }
+        }
+        kind = 0;
+    };
     int a = qb / nz, p = qb % nz;
-    for (int q = qb; q < qe; ++q, ++p) {
+    // (one more turn than planes: sums are folded and flushed in one place)
+    for (int q = qb;; ++q, ++p) {
         if (p == nz) {
             p = 0;
             ++a;
         }
+        float zl = (pf && p < ZPOW_N) ? P.tab.zpow[p] : 0.f;
+        float zh = (pf && nz - 1 - p < ZPOW_N) ? P.tab.zpow[nz - 1 - p] : 0.f;
+        const int now = !split ? 0 : (zl != 0.f ? 1 : (zh != 0.f ? 2 : 0));
+        if (kind && (now != kind || a != cur_a || q == qe))
+            fold();
+        if (cur_a >= 0 && (a != cur_a || q == qe))
+            flush(cur_a);
+        if (q >= qe)
+            break;
         if (a != cur_a) {
-            if (cur_a >= 0)
-                flush(cur_a);
             const float zp = (float)p - 0.5f * (float)nz + P.zshift;
 #pragma unroll
             for (int r = 0; r < L::SLOTS; ++r) {
@@ -257,8 +328,18 @@ __global__ void __launch_bounds__(KX * L::TPL, KX * L::TPL <= 256 ? 3 : 1) k_adj
             }
         }
         line.template run<-1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
-        const float zl = (pf && p < ZPOW_N) ? P.tab.zpow[p] : 0.f;
-        const float zh = (pf && nz - 1 - p < ZPOW_N) ? P.tab.zpow[nz - 1 - p] : 0.f;
+        if (split) {
+            if (now) {
+                const float z = zl + zh;  // (one of them is zero)
+#pragma unroll
+                for (int r = 0; r < L::SLOTS; ++r) {
+                    float2 *b = bsum + r * KX * L::TPL;
+                    *b = kind ? sfma2(z, v[r], *b) : cscale(v[r], z);
+                }
+                kind = now;
+            }
+            zl = zh = 0.f;
+        }
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
             const int ky = j + r * L::TPL;
@@ -294,8 +375,6 @@ __global__ void __launch_bounds__(KX * L::TPL, KX * L::TPL <= 256 ? 3 : 1) k_adj
                 E[r] = cmul(E[r], stp[ky * KX + c]);
         }
     }
-    if (cur_a >= 0)
-        flush(cur_a);
 }
 
 // Spectrum: gain gradient dg += Re(conj(G X) Q) (X recomputed from the row
@@ -385,7 +464,25 @@ __global__ void __launch_bounds__(KX * L::TPL) k_adj_spectrum(StageParams P, L l
     }
 }
 
-// Rows: full backward FFT along x of W -> the cotangent of the padded plane.
+// Transpose of the padding along one axis: padded position X contributes to
+// source position pad_source with weight `c` (1 for data and edge padding, the
+// ramp fraction for linear_ramp).
+__device__ __forceinline__ int pad_source(int X, int n, int pad_l, int pad_r, int mode, float &c)
+{
+    const int i = X - pad_l;
+    c = 1.f;
+    if (i >= 0 && i < n)
+        return i;
+    if (mode == 2)
+        c = i < 0 ? (float)X / (float)pad_l : (float)(pad_r - 1 - (i - n)) / (float)pad_r;
+    return i < 0 ? 0 : n - 1;
+}
+
+// Rows: full backward FFT along x of W -> the cotangent of the padded plane,
+// with the x padding transposed (and an opposite view's mirroring undone):
+// Pg[slot][padded y][x].  (The padding's whole transpose in k_adj_pad left
+// the 65 x 65 corner sums of a 128^2 view to single threads: 0.36 ms for 90
+// views; 0.02 ms there and 0.03 ms more here with the x sums formed here.)
 template <class L, int LPC>
 __global__ void __launch_bounds__(LPC * L::TPL) k_adj_rows_full(StageParams P, L line, const float2 *W, float2 *Pg,
                                                                 int nslots)
@@ -394,6 +491,7 @@ __global__ void __launch_bounds__(LPC * L::TPL) k_adj_rows_full(StageParams P, L
     const int n = line.size();  // lNx
     const int xs = xslots<false>(n);
     float2 *buf0 = smem, *buf1 = smem + LPC * xs, *tw = smem + 2 * LPC * xs;
+    float2 *red = tw + tw_slots(n);  // [LPC][2] sums at the first and last column
     copy_twiddles<L>(tw, P.tab.twx, n);
     const int l = threadIdx.x / L::TPL, j = threadIdx.x % L::TPL;
     const long long lid = (long long)blockIdx.x * LPC + l;
@@ -405,43 +503,47 @@ __global__ void __launch_bounds__(LPC * L::TPL) k_adj_rows_full(StageParams P, L
         const int x = j + r * L::TPL;
         v[r] = (valid && x < n && column_active(P, x)) ? src[x] : make_float2(0.f, 0.f);
     }
+    if (threadIdx.x < 2 * LPC)
+        red[threadIdx.x] = make_float2(0.f, 0.f);
     __syncthreads();
     int flip = 0;
     line.template run<1>(v, j, buf0 + l * xs, buf1 + l * xs, 1, tw, flip);
-    if (!valid)
-        return;
-    float2 *dst = Pg + (size_t)lid * n;
+    const int nx = P.nx, padxr = P.lNx - P.nx - P.padxl;
+    const bool mirrored = P.units && ((valid ? lid : 0) / P.lNy & 1);
+    float2 first = make_float2(0.f, 0.f), last = first;
 #pragma unroll
     for (int r = 0; r < L::SLOTS; ++r) {
-        const int x = j + r * L::TPL;
-        if (x < n)
-            dst[x] = v[r];
+        int X = j + r * L::TPL;
+        if (X >= n)
+            continue;
+        if (mirrored) {
+            X = 2 * P.padxl + nx - 1 - X;
+            X += X < 0 ? n : 0;
+            X -= X >= n ? n : 0;
+        }
+        float c;
+        const int x = pad_source(X, nx, P.padxl, padxr, P.pad_mode, c);
+        if (x == 0)
+            first = sfma2(c, v[r], first);
+        else if (x == nx - 1)
+            last = sfma2(c, v[r], last);
+        else if (valid)
+            Pg[(size_t)lid * nx + x] = v[r];
     }
+    if (first.x != 0.f || first.y != 0.f) {
+        atomicAdd(&red[2 * l].x, first.x);
+        atomicAdd(&red[2 * l].y, first.y);
+    }
+    if (last.x != 0.f || last.y != 0.f) {
+        atomicAdd(&red[2 * l + 1].x, last.x);
+        atomicAdd(&red[2 * l + 1].y, last.y);
+    }
+    __syncthreads();
+    if (valid && j < 2)
+        Pg[(size_t)lid * nx + (j ? nx - 1 : 0)] = red[2 * l + j];
 }
 
-// Transpose of the padding along one axis: the padded positions that a
-// source index contributes to, with their coefficients (1 for data and
-// edge padding, the ramp fraction for linear_ramp).
-struct PadAxis {
-    int n, pad_l, pad_r, mode;  // mode: 0 none, 1 edge, 2 ramp
-};
-
-template <class F>
-__device__ __forceinline__ void pad_transpose_axis(const PadAxis &ax, int i, F &&emit)
-{
-    emit(i + ax.pad_l, 1.f);
-    if (ax.mode == 0)
-        return;
-    if (i == 0) {
-        for (int q = 0; q < ax.pad_l; ++q)
-            emit(q, ax.mode == 1 ? 1.f : (float)q / (float)ax.pad_l);
-    }
-    if (i == ax.n - 1) {
-        for (int jj = 0; jj < ax.pad_r; ++jj)
-            emit(ax.pad_l + ax.n + jj, ax.mode == 1 ? 1.f : (float)(ax.pad_r - 1 - jj) / (float)ax.pad_r);
-    }
-}
-
+// The y padding's transpose and the angle weight.
 __global__ void k_adj_pad(StageParams P, const float2 *Pg, const double *weights, int nslots, float2 *dsino)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -450,31 +552,28 @@ __global__ void k_adj_pad(StageParams P, const float2 *Pg, const double *weights
     if (x >= P.nx || sl >= nslots)
         return;
     int a = sl;
-    bool mirrored = false;
     if (P.units) {
         const int2 u = P.units[sl >> 1];
-        mirrored = sl & 1;
-        a = mirrored ? u.y : u.x;
+        a = (sl & 1) ? u.y : u.x;
         if (a < 0)
             return;
     }
-    const PadAxis ay{P.ny, P.padyl, P.lNy - P.ny - P.padyl, P.pad_mode};
-    const PadAxis axx{P.nx, P.padxl, P.lNx - P.nx - P.padxl, P.pad_mode};
-    const float2 *plane = Pg + (size_t)sl * P.lNy * P.lNx;
-    float2 acc = make_float2(0.f, 0.f);
-    pad_transpose_axis(ay, y, [&](int Y, float cy) {
-        pad_transpose_axis(axx, x, [&](int X, float cx) {
-            if (mirrored) {
-                X = 2 * P.padxl + P.nx - 1 - X;
-                X += X < 0 ? P.lNx : 0;
-                X -= X >= P.lNx ? P.lNx : 0;
-            }
-            const float2 g = plane[(size_t)Y * P.lNx + X];
-            const float cc = cy * cx;
-            acc.x = fmaf(cc, g.x, acc.x);
-            acc.y = fmaf(cc, g.y, acc.y);
-        });
-    });
+    const int padyr = P.lNy - P.ny - P.padyl;
+    const float2 *col = Pg + (size_t)sl * P.lNy * P.nx + x;
+    float2 acc = col[(size_t)(y + P.padyl) * P.nx];
+    if (P.pad_mode != 0) {
+        if (y == 0) {
+#pragma unroll 8
+            for (int Y = 0; Y < P.padyl; ++Y)
+                acc = sfma2(P.pad_mode == 1 ? 1.f : (float)Y / (float)P.padyl, col[(size_t)Y * P.nx], acc);
+        }
+        if (y == P.ny - 1) {
+#pragma unroll 8
+            for (int q = 0; q < padyr; ++q)
+                acc = sfma2(P.pad_mode == 1 ? 1.f : (float)(padyr - 1 - q) / (float)padyr,
+                            col[(size_t)(P.padyl + P.ny + q) * P.nx], acc);
+        }
+    }
     const float w = weights ? (float)weights[a] : 1.f;
     dsino[((size_t)a * P.ny + y) * P.nx + x] = make_float2(w * acc.x, w * acc.y);
 }
@@ -485,13 +584,22 @@ constexpr int kAdjPlanesPerBlock = 16;
 template <class L>
 static size_t smem_adj_rows(int n)
 {
-    return (size_t)(2 * Cfg<L>::LPC * xslots<false>(n) + tw_slots(n) + 2 * Cfg<L>::LPC) * sizeof(float2);
+    // (the last terms: partial sums, 2 float2 per line in k_adj_rows_full, one
+    // 16-byte aligned float4 per warp of a line in k_adj_rows)
+    constexpr int WPL = L::TPL > 32 ? L::TPL / 32 : 1;
+    return (size_t)(2 * Cfg<L>::LPC * xslots<false>(n) + tw_slots(n) + 1 + 2 * Cfg<L>::LPC * WPL) * sizeof(float2);
 }
 template <class L>
 static size_t smem_adj_cols(int n)
 {
-    return (size_t)(2 * Cfg<L>::KX * xslots<true>(n) + Cfg<L>::KX * n + tw_slots(n) + 2 * Cfg<L>::KX) *
+    constexpr int KX = Cfg<L>::KX;
+    return (size_t)(2 * KX * xslots<true>(n) + KX * n + tw_slots(n) + 2 * KX + L::SLOTS * KX * L::TPL) *
            sizeof(float2);
+}
+template <class L>
+static size_t smem_adj_spectrum(int n)
+{
+    return (size_t)(2 * Cfg<L>::KX * xslots<true>(n) + tw_slots(n)) * sizeof(float2);
 }
 
 template <class L>
@@ -517,7 +625,7 @@ static cudaError_t set_adj_attrs(int n)
     if (e != cudaSuccess)
         return e;
     return cudaFuncSetAttribute(k_adj_spectrum<L, Cfg<L>::KX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem_adj_cols<L>(n));
+                                (int)smem_adj_spectrum<L>(n));
 }
 
 cudaError_t configure_adjoint_kernels(const StageParams &P)
@@ -533,8 +641,9 @@ cudaError_t launch_adj_rows(const StageParams &P, const float2 *sgrad, float2 *T
     return with_line(P.lNx, [&](auto line) {
         using L = decltype(line);
         constexpr int LPC = Cfg<L>::LPC;
+        constexpr int rpc = LPC * adj_row_groups<LPC>();
         const long long lines = (long long)qn * P.ny;
-        k_adj_rows<L, LPC><<<(unsigned)((lines + LPC - 1) / LPC), LPC * L::TPL, smem_adj_rows<L>(line.n), s>>>(
+        k_adj_rows<L, LPC><<<(unsigned)((lines + rpc - 1) / rpc), LPC * L::TPL, smem_adj_rows<L>(line.n), s>>>(
             P, line, sgrad, Tg, q0, qn);
         return cudaGetLastError();
     });
@@ -563,7 +672,7 @@ cudaError_t launch_adj_spectrum(const StageParams &P, const float2 *rowspec, con
         using L = decltype(line);
         constexpr int KX = Cfg<L>::KX;
         dim3 grid((P.lNx + KX - 1) / KX, nslots);
-        k_adj_spectrum<L, KX><<<grid, KX * L::TPL, smem_adj_cols<L>(line.n), s>>>(P, line, rowspec, Qg, dgain,
+        k_adj_spectrum<L, KX><<<grid, KX * L::TPL, smem_adj_spectrum<L>(line.n), s>>>(P, line, rowspec, Qg, dgain,
                                                                                  dagain, W);
         return cudaGetLastError();
     });
