@@ -29,6 +29,14 @@
 //                      k_uw_hook     root -> neighbouring root, turn offset
 //                      k_uw_jump     pointer jumping among this round's roots
 //                      k_uw_flatten  every pixel -> its new root
+//                    A frame without residues (no 2 x 2 loop of pixels whose
+//                    wrapped steps do not cancel) needs no tree: the turns
+//                    between two pixels are then the same along every path,
+//                    so running sums along the first column and the rows give
+//                    the tree's (k_uf_scan .. k_uf_apply), and only the pixel
+//                    the tree starts from has to be found.  200 residue-free
+//                    frames of 256^2: 4.25 -> 1.69 ms; the kernels below leave
+//                    such frames out.
 //                    (at most ceil(log2(pixels)) + 2 rounds; a round with no
 //                    hook ends the work of the following ones), with
 //                      k_uw_anchor   first edge of each frame (after round 0's
@@ -190,6 +198,7 @@ struct Frames {
     int H, W;
     long long P;  // H * W
     long long N;  // A * P
+    const uint32_t *bad;  // per frame: nonzero where the tree is needed
 };
 
 // The per-pixel kernels run on blocks of 32 x 8 pixels over a grid
@@ -241,20 +250,21 @@ __global__ void k_phase(const C2<T> *sino, const C2<T> *u0arr, C2<T> u0s, long l
     }
 }
 
-// numpy.unwrap along each line of `len` values (period 2 pi, discont pi), in
-// T arithmetic and NumPy's order: dd = p[i] - p[i-1];
-// ddmod = mod(dd + pi, 2 pi) - pi, set to +pi where ddmod == -pi and dd > 0;
-// correction ddmod - dd (0 where |dd| < pi), accumulated sequentially.
+// numpy.unwrap along a line (period 2 pi, discont pi), in T arithmetic and
+// NumPy's order: dd = p[i] - p[i-1]; ddmod = mod(dd + pi, 2 pi) - pi, set to
+// +pi where ddmod == -pi and dd > 0; correction ddmod - dd (0 where |dd| < pi),
+// accumulated sequentially.
 template <class T>
-__device__ __forceinline__ void unwrap_line(T *p, long long len, long long stride, double *steps_out)
-{
-    const T pi = (T)PI_D, twopi = (T)TWOPI_D;
-    T prev = p[0];
-    T cum = T(0);
-    if (steps_out)
-        steps_out[0] = (double)sub_rn(prev, prev);
-    for (long long i = 1; i < len; ++i) {
-        const T cur = p[i * stride];
+struct LineUnwrap {
+    T prev, cum;
+    __device__ __forceinline__ void start(T first)
+    {
+        prev = first;
+        cum = T(0);
+    }
+    __device__ __forceinline__ T next(T cur)  // the unwrapped value
+    {
+        const T pi = (T)PI_D, twopi = (T)TWOPI_D;
         const T dd = sub_rn(cur, prev);
         T ddmod = add_rn(np_mod_pos<T>(add_rn(dd, pi), twopi), -pi);
         if (ddmod == -pi && dd > T(0))
@@ -263,21 +273,335 @@ __device__ __forceinline__ void unwrap_line(T *p, long long len, long long strid
         if (fabs(dd) < pi)
             pc = T(0);
         cum = add_rn(cum, pc);
-        const T up = add_rn(cur, cum);
-        if (steps_out)
-            steps_out[i] = (double)sub_rn(cur, up);  // sample - unwrapped
-        else
-            p[i * stride] = up;
         prev = cur;
+        return add_rn(cur, cum);
     }
-}
+};
 
 template <class T>
 __global__ void k_unwrap_rows(T *phi, long long rows, int len)
 {
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < rows)
-        unwrap_line<T>(phi + r * len, len, 1, nullptr);
+    if (r >= rows)
+        return;
+    T *p = phi + r * len;
+    LineUnwrap<T> u;
+    u.start(p[0]);
+    for (int i = 1; i < len; ++i)
+        p[i] = u.next(p[i]);
+}
+
+// ---- 3D frames without residues -------------------------------------------
+// Turns of v minus turns of u across the edge u - v: the wrapped step's whole
+// turns (the reference's find_wrap), decided in FP64 where FP32 is too close.
+template <class T>
+__device__ __forceinline__ int turn_step(T u, T v)
+{
+    const float df = (float)u - (float)v;  // (off by less than 2e-6: |u|, |v| <= UF_MAX)
+    if (fabsf(df) < 3.1415f)
+        return 0;
+    if (fabsf(df) > 3.1417f)
+        return df > 0.f ? 1 : -1;
+    const double d = (double)u - (double)v;
+    return d > PI_D ? 1 : (d < -PI_D ? -1 : 0);
+}
+
+// Frames with a phase beyond this (phases of complex data are within pi) or a
+// NaN go through the tree: the FP32 estimates below rely on it.
+constexpr float UF_MAX = 8.f;
+
+// Tile of phases of a 32 x 8 block with two positions of halo on the right
+// and below and one on the left and above.
+constexpr int UF_TW = 35, UF_TH = 11;
+
+template <class T>
+__device__ __forceinline__ void uf_load_tile(const T *frame, const Frames &F, T (&ph)[UF_TH][UF_TW])
+{
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    const int i0 = (int)blockIdx.y * 8 - 1, j0 = (int)blockIdx.x * 32 - 1;
+    for (int t = tid; t < UF_TH * UF_TW; t += 256) {
+        const int ti = t / UF_TW, tj = t - ti * UF_TW;
+        const int gi = i0 + ti, gj = j0 + tj;
+        ph[ti][tj] = (gi >= 0 && gi < F.H && gj >= 0 && gj < F.W) ? frame[(size_t)gi * F.W + gj] : T(0);
+    }
+}
+
+// Wrapped difference, NaN where FP32 cannot tell on which side of pi it is.
+__device__ __forceinline__ float wrapf(float d)
+{
+    const float m = fabsf(d);
+    if (m < 3.1415f)
+        return d;
+    return m > 3.1417f ? d - copysignf(6.28318531f, d) : __int_as_float(0x7fffffff);
+}
+
+// FP32 estimate of the reliability (k_uw_init) of the pixel at tile position
+// (ti, tj), image position (i, j); NaN where it may be off by a wrap.
+template <class T>
+__device__ __forceinline__ float rel_estimate(const T (&ph)[UF_TH][UF_TW], const Frames &F, uint32_t seed, int ti, int tj,
+                                              int i, int j)
+{
+    if (i < 1 || i > F.H - 2 || j < 1 || j > F.W - 2)
+        return (float)(BORDER_BASE + border_noise(seed, (unsigned long long)((uint32_t)i * (uint32_t)F.W + j)));
+    auto at = [&](int a, int b) { return (float)ph[ti + a][tj + b]; };
+    const float c = at(0, 0);
+    const float h = wrapf(at(0, -1) - c) - wrapf(c - at(0, 1)), v = wrapf(at(-1, 0) - c) - wrapf(c - at(1, 0));
+    const float d1 = wrapf(at(-1, -1) - c) - wrapf(c - at(1, 1)), d2 = wrapf(at(-1, 1) - c) - wrapf(c - at(1, -1));
+    return h * h + v * v + d1 * d1 + d2 * d2;
+}
+
+// The reliability itself, with k_uw_init's operations.
+template <class T>
+__device__ double rel_exact(const T (&ph)[UF_TH][UF_TW], const Frames &F, uint32_t seed, int ti, int tj, int i, int j)
+{
+    if (i < 1 || i > F.H - 2 || j < 1 || j > F.W - 2)
+        return __dadd_rn(BORDER_BASE, border_noise(seed, (unsigned long long)((uint32_t)i * (uint32_t)F.W + j)));
+    auto at = [&](int a, int b) { return (double)ph[ti + a][tj + b]; };
+    const T c0 = ph[ti][tj];
+    bool flat = true;  // nine equal phases: zero without any FP64 work
+#pragma unroll
+    for (int a = -1; a <= 1; ++a)
+#pragma unroll
+        for (int b = -1; b <= 1; ++b)
+            flat = flat && ph[ti + a][tj + b] == c0;
+    if (flat)
+        return 0.0;
+    const double c = at(0, 0);
+    auto second = [&](double p, double q) { return __dsub_rn(wrapd(__dsub_rn(p, c)), wrapd(__dsub_rn(c, q))); };
+    const double h = second(at(0, -1), at(0, 1)), v = second(at(-1, 0), at(1, 0));
+    const double d1 = second(at(-1, -1), at(1, 1)), d2 = second(at(-1, 1), at(1, -1));
+    return __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(h, h), __dmul_rn(v, v)), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
+}
+
+// Steps of every pixel (right: bits 0-1, down: bits 2-3, two's complement),
+// whether the frame has a residue (bad), and the smallest estimated edge
+// weight of the frame (bits of a non-negative float; ~0, a NaN, if there is
+// none).
+template <class T>
+__global__ void __launch_bounds__(256) k_uf_scan(const T *phi, Frames F, uint32_t seed, uint8_t *steps, uint32_t *bad,
+                                                 uint32_t *wmin)
+{
+    __shared__ T ph[UF_TH][UF_TW];
+    __shared__ float re[9][33];
+    const Px x = pixel(F);
+    uf_load_tile(phi + (size_t)x.a * (size_t)F.P, F, ph);
+    __syncthreads();
+    const int i0 = (int)blockIdx.y * 8, j0 = (int)blockIdx.x * 32;
+    for (int t = threadIdx.y * 32 + threadIdx.x; t < 9 * 33; t += 256) {
+        const int ti = t / 33, tj = t - ti * 33;
+        if (i0 + ti < F.H && j0 + tj < F.W)
+            re[ti][tj] = rel_estimate(ph, F, seed, ti + 1, tj + 1, i0 + ti, j0 + tj);
+    }
+    __syncthreads();
+    bool residue = false;  // or a phase that the estimates do not cover
+    float w = 3e38f;
+    if (x.ok) {
+        const int ti = threadIdx.y + 1, tj = threadIdx.x + 1;
+        const bool right = x.j + 1 < F.W, down = x.i + 1 < F.H;
+        const T c = ph[ti][tj];
+        residue = !(fabs(c) <= T(UF_MAX));
+        const int sr = right ? turn_step(c, ph[ti][tj + 1]) : 0, sd = down ? turn_step(c, ph[ti + 1][tj]) : 0;
+        steps[x.p] = (uint8_t)((sr & 3) | ((sd & 3) << 2));
+        if (right && down) {
+            const T q = ph[ti + 1][tj + 1];
+            residue |= sr + turn_step(ph[ti][tj + 1], q) != sd + turn_step(ph[ti + 1][tj], q);
+        }
+        const float r = re[ti - 1][tj - 1];
+        if (right)
+            w = fminf(w, r + re[ti - 1][tj]);
+        if (down)
+            w = fminf(w, r + re[ti][tj - 1]);
+    }
+    if (__syncthreads_or(residue) && threadIdx.x == 0 && threadIdx.y == 0)
+        atomicOr(bad + x.a, 1u);
+    for (int o = 16; o > 0; o >>= 1)
+        w = fminf(w, __shfl_xor_sync(0xffffffffu, w, o));
+    if (threadIdx.x == 0 && w < 3e38f)
+        atomicMin(wmin + x.a, __float_as_uint(w));
+}
+
+// The first edge in (weight, index) order among a block's edges; the weight in
+// FP64, only of edges whose estimate can be the frame's smallest.  A second
+// difference's estimate is off by less than 6e-6 (two wrapped differences of
+// phases up to UF_MAX: conversions 2 x 2.4e-7, subtraction 4.8e-7, turn 1.8e-7
+// and its subtraction 2.4e-7 each, and the last subtraction), so the root of a
+// weight, the norm of eight of them, by less than 1.7e-5; the relative margin
+// covers the sums and border weights.
+template <class T>
+__global__ void __launch_bounds__(256) k_uf_first(const T *phi, Frames F, uint32_t seed, const uint32_t *bad,
+                                                  const uint32_t *wmin, ulonglong2 *first)
+{
+    __shared__ T ph[UF_TH][UF_TW];
+    __shared__ unsigned long long sw[8];
+    __shared__ uint32_t se[8];
+    const Px x = pixel(F);
+    if (bad[x.a])
+        return;
+    uf_load_tile(phi + (size_t)x.a * (size_t)F.P, F, ph);
+    __syncthreads();
+    unsigned long long mw = NONE64;
+    uint32_t me = NONE32;
+    if (x.ok) {
+        const int ti = threadIdx.y + 1, tj = threadIdx.x + 1;
+        const float root = sqrtf(__uint_as_float(wmin[x.a])) + 4e-5f, lim = root * root * 1.0001f;
+        const float r = rel_estimate(ph, F, seed, ti, tj, x.i, x.j);
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            const int di = d, dj = 1 - d;
+            if (x.i + di >= F.H || x.j + dj >= F.W)
+                continue;
+            // (a NaN estimate is a candidate)
+            if (r + rel_estimate(ph, F, seed, ti + di, tj + dj, x.i + di, x.j + dj) > lim)
+                continue;
+            const unsigned long long wb = dbits(__dadd_rn(rel_exact(ph, F, seed, ti, tj, x.i, x.j),
+                                                          rel_exact(ph, F, seed, ti + di, tj + dj, x.i + di, x.j + dj)));
+            const uint32_t le = d == 0 ? (uint32_t)(x.i * (F.W - 1) + x.j)
+                                       : (uint32_t)(F.H * (F.W - 1)) + (uint32_t)x.i * (uint32_t)F.W + (uint32_t)x.j;
+            if (wb < mw || (wb == mw && le < me)) {
+                mw = wb;
+                me = le;
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long w = __shfl_xor_sync(0xffffffffu, mw, o);
+        const uint32_t e = __shfl_xor_sync(0xffffffffu, me, o);
+        if (w < mw || (w == mw && e < me)) {
+            mw = w;
+            me = e;
+        }
+    }
+    if (threadIdx.x == 0) {
+        sw[threadIdx.y] = mw;
+        se[threadIdx.y] = me;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        for (int i = 1; i < 8; ++i)
+            if (sw[i] < mw || (sw[i] == mw && se[i] < me)) {
+                mw = sw[i];
+                me = se[i];
+            }
+        first[((size_t)x.a * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = make_ulonglong2(mw, me);
+    }
+}
+
+__device__ __forceinline__ int step_right(uint8_t b) { return (int)((uint32_t)b << 30) >> 30; }
+__device__ __forceinline__ int step_down(uint8_t b) { return (int)((uint32_t)b << 28) >> 30; }
+
+// Per frame: its first edge, the turns of the first column, and those of the
+// edge's pixel 1 (kan).  One CTA of 256 threads per frame.
+__global__ void __launch_bounds__(256) k_uf_frame(Frames F, const uint8_t *steps, const uint32_t *bad,
+                                                  const ulonglong2 *first, int nblk, int32_t *col, int32_t *kan)
+{
+    const int a = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (bad[a])
+        return;
+    __shared__ unsigned long long sw[8];
+    __shared__ uint32_t se[8];
+    __shared__ int32_t ssum[8];
+    unsigned long long mw = NONE64;
+    uint32_t me = NONE32;
+    for (int b = tid; b < nblk; b += 256) {
+        const ulonglong2 f = first[(size_t)a * nblk + b];
+        if (f.x < mw || (f.x == mw && (uint32_t)f.y < me)) {
+            mw = f.x;
+            me = (uint32_t)f.y;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long w = __shfl_xor_sync(0xffffffffu, mw, o);
+        const uint32_t e = __shfl_xor_sync(0xffffffffu, me, o);
+        if (w < mw || (w == mw && e < me)) {
+            mw = w;
+            me = e;
+        }
+    }
+    if (lane == 0) {
+        sw[wid] = mw;
+        se[wid] = me;
+    }
+    __syncthreads();
+    for (int i = 0; i < 8; ++i)
+        if (sw[i] < mw || (sw[i] == mw && se[i] < me)) {
+            mw = sw[i];
+            me = se[i];
+        }
+    // first column
+    const uint8_t *fs = steps + (size_t)a * F.P;
+    int32_t carry = 0;
+    for (int i0 = 0; i0 < F.H; i0 += 256) {
+        const int i = i0 + tid;
+        const int32_t st = (i > 0 && i < F.H) ? step_down(fs[(size_t)(i - 1) * F.W]) : 0;
+        int32_t incl = st;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d)
+                incl += t;
+        }
+        if (lane == 31)
+            ssum[wid] = incl;
+        __syncthreads();
+        int32_t before = carry, total = carry;
+        for (int w = 0; w < 8; ++w) {
+            if (w < wid)
+                before += ssum[w];
+            total += ssum[w];
+        }
+        if (i < F.H)
+            col[(size_t)a * F.H + i] = before + incl;
+        carry = total;
+        __syncthreads();
+    }
+    // turns of the first edge's pixel 1
+    int iu = 0, ju = 0;
+    if (me != NONE32) {
+        uint32_t u, v;
+        edge_ends(F, 0u, me, u, v);
+        iu = (int)(u / (uint32_t)F.W);
+        ju = (int)(u - (uint32_t)iu * (uint32_t)F.W);
+    }
+    int32_t sum = 0;
+    for (int j = tid; j < ju; j += 256)
+        sum += step_right(fs[(size_t)iu * F.W + j]);
+    for (int o = 16; o > 0; o >>= 1)
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0)
+        ssum[wid] = sum;
+    __syncthreads();
+    if (tid == 0) {
+        int32_t k = col[(size_t)a * F.H + iu];
+        for (int w = 0; w < 8; ++w)
+            k += ssum[w];
+        kan[a] = me == NONE32 ? 0 : k;
+    }
+}
+
+// phi + 2 pi k of a residue-free frame, k relative to pixel 1 of its first
+// edge.  A warp per row.
+template <class T>
+__global__ void __launch_bounds__(256) k_uf_apply(T *phi, Frames F, const uint8_t *steps, const uint32_t *bad,
+                                                  const int32_t *col, const int32_t *kan)
+{
+    const int a = blockIdx.y, i = (int)(blockIdx.x * 8 + threadIdx.x / 32), lane = threadIdx.x & 31;
+    if (bad[a] || i >= F.H)
+        return;
+    const size_t row = (size_t)a * F.P + (size_t)i * F.W;
+    int32_t k = col[(size_t)a * F.H + i] - kan[a];  // of column j0
+    for (int j0 = 0; j0 < F.W; j0 += 32) {
+        const int j = j0 + lane;
+        const int32_t st = j < F.W ? step_right(steps[row + j]) : 0;  // step from j to j + 1
+        int32_t incl = st;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d)
+                incl += t;
+        }
+        const int32_t kj = k + incl - st;
+        if (j < F.W && kj != 0)
+            phi[row + j] = (T)__dadd_rn((double)phi[row + j], __dmul_rn(TWOPI_D, (double)kj));
+        k += __shfl_sync(0xffffffffu, incl, 31);
+    }
 }
 
 // ---- 3D frames: reliability-sorted unwrapping as a Boruvka MST ------------
@@ -343,6 +667,8 @@ __global__ void __launch_bounds__(256) k_uw_init(const T *phi, Frames F, uint32_
     __shared__ double ph[UI_TH][UI_TW];
     __shared__ double dR[UI_TH][UI_TW], dD[UI_TH][UI_TW], dDR[UI_TH][UI_TW], dDL[UI_TH][UI_TW];
     const Px x = pixel(F);
+    if (!F.bad[x.a])
+        return;
     const int tid = threadIdx.y * 32 + threadIdx.x;
     const int i0 = (int)blockIdx.y * 8 - 1, j0 = (int)blockIdx.x * 32 - 1;
     const T *frame = phi + (size_t)x.a * (size_t)F.P;
@@ -398,6 +724,8 @@ __global__ void k_uw_minw(Frames F, const double *rel, const unsigned long long 
     if (round > 0 && flags[round - 1] == 0)
         return;
     const Px x = pixel(F);
+    if (!F.bad[x.a])
+        return;
     const uint32_t p = x.p;
     const int i = x.i, j = x.j;
     const uint32_t rp = x.ok ? par_of(word[p]) : 0u;
@@ -436,7 +764,7 @@ __global__ void k_uw_mine(Frames F, const double *rel, const unsigned long long 
     if (round > 0 && flags[round - 1] == 0)
         return;
     const Px x = pixel(F);
-    if (!x.ok)
+    if (!x.ok || !F.bad[x.a])
         return;
     const uint32_t p = x.p;
     const int i = x.i, j = x.j;
@@ -470,6 +798,8 @@ __global__ void k_uw_hook(Frames F, const T *phi, const unsigned long long *word
     if (round > 0 && flags[round - 1] == 0)
         return;
     const Px x = pixel(F);
+    if (!F.bad[x.a])
+        return;
     const uint32_t r = x.p;
     bool keep = false;  // a root after this round with an outgoing edge left
     if (x.ok && par_of(word[r]) == r) {
@@ -511,7 +841,7 @@ __global__ void k_uw_jump(Frames F, const unsigned long long *word, unsigned lon
     if (flags[round] == 0)
         return;
     const Px x = pixel(F);
-    if (!x.ok)
+    if (!x.ok || !F.bad[x.a])
         return;
     const uint32_t r = x.p;
     if (par_of(word[r]) != r)
@@ -539,7 +869,7 @@ __global__ void k_uw_flatten(Frames F, unsigned long long *word, const unsigned 
     if (flags[round] == 0)
         return;
     const Px x = pixel(F);
-    if (!x.ok)
+    if (!x.ok || !F.bad[x.a])
         return;
     const uint32_t p = x.p;
     const unsigned long long w = word[p];
@@ -710,6 +1040,8 @@ __global__ void __launch_bounds__(1024) k_uw_anchor(Frames F, const unsigned lon
     __shared__ unsigned long long sw[32];
     __shared__ uint32_t se[32];
     const long long a = blockIdx.x;
+    if (!F.bad[a])
+        return;
     const long long base = a * F.P;
     unsigned long long mw = NONE64;
     uint32_t me = NONE32;
@@ -749,7 +1081,7 @@ template <class T>
 __global__ void k_uw_finish(Frames F, T *phi, unsigned long long *word, const uint32_t *fe, uint32_t *status)
 {
     const Px x = pixel(F);
-    if (!x.ok)
+    if (!x.ok || !F.bad[x.a])
         return;
     const uint32_t p = x.p;
     const int a = x.a;
@@ -813,18 +1145,33 @@ __global__ void k_align(const T *phi, long long A, int ny, int nx, int three_d, 
                         const uint32_t *nan_seen, double *steps, double *remove)
 {
     const long long fr = three_d ? (long long)ny * nx : nx;
-    if (threadIdx.x < 5) {
-        long long off;
-        const int s = threadIdx.x;
-        if (three_d) {
-            const long long last = (long long)(ny - 1) * nx;
-            const long long offs[5] = {0, nx - 1, last, last + nx - 1, 1};
-            off = offs[s];
-        } else {
-            const long long offs[5] = {0, 1, 2, nx - 1, nx - 2};
-            off = offs[s];
+    const long long last = (long long)(ny - 1) * nx;
+    const long long off3[5] = {0, nx - 1, last, last + nx - 1, 1}, off2[5] = {0, 1, 2, nx - 1, nx - 2};
+    // the samples come through shared memory, 256 angles at a time (read one
+    // by one by the five threads that unwrap them, 200 angles took 0.13 ms)
+    __shared__ T smp[5][256];
+    LineUnwrap<T> u;
+    for (long long a0 = 0; a0 < A; a0 += 256) {
+        __syncthreads();
+        if (a0 + threadIdx.x < A) {
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+                smp[i][threadIdx.x] = phi[(a0 + threadIdx.x) * fr + (three_d ? off3[i] : off2[i])];
         }
-        unwrap_line<T>(const_cast<T *>(phi) + off, A, fr, steps + s * A);
+        __syncthreads();
+        if (threadIdx.x < 5) {
+            double *st = steps + threadIdx.x * A + a0;
+            const int n = (int)(A - a0 < 256 ? A - a0 : 256);
+            for (int k = 0; k < n; ++k) {
+                const T cur = smp[threadIdx.x][k];
+                if (a0 + k == 0) {
+                    u.start(cur);
+                    st[0] = (double)sub_rn(cur, cur);
+                } else {
+                    st[k] = (double)sub_rn(cur, u.next(cur));  // sample - unwrapped
+                }
+            }
+        }
     }
     __syncthreads();
     // whole turns of the minimum, in T like the reference's scalar divmod
@@ -891,7 +1238,8 @@ __global__ void k_compose(const T *phi, const double *remove, long long per_angl
 
 // ---------------------------------------------------------------------------
 struct Layout {
-    size_t phi, rel, word, rw, bw, be, fe, flags, status, minkey, nan, steps, remove, elist[2], rlist[2], cnt, total;
+    size_t phi, rel, word, rw, bw, be, fe, flags, status, minkey, nan, steps, remove, elist[2], rlist[2], cnt, bad, wmin,
+        kan, total;
 };
 
 int num_rounds(long long P)
@@ -927,7 +1275,8 @@ Layout layout_of(const odt_sino_desc &d)
         L.rel = take((size_t)N * 8);
         L.word = take((size_t)N * 8);
         L.rw = take((size_t)N * 8);
-        L.bw = take((size_t)N * 8);
+        // also 16 bytes per 32 x 8 block of k_uf_first
+        L.bw = take(std::max<size_t>((size_t)N * 8, (size_t)A * ((d.ny + 7) / 8) * ((d.nx + 31) / 32) * 16));
         L.be = take((size_t)N * 4);
         L.fe = take((size_t)A * 4);
         for (int k = 0; k < 2; ++k) {
@@ -935,6 +1284,9 @@ Layout layout_of(const odt_sino_desc &d)
             L.rlist[k] = take((size_t)N * 4);
         }
         L.cnt = take(4 * 4);
+        L.bad = take((size_t)A * 4);
+        L.wmin = take((size_t)A * 4);
+        L.kan = take((size_t)A * 4);
     }
     L.total = o;
     return L;
@@ -1008,7 +1360,8 @@ odt_status run(const odt_sino_desc &d, const void *sino, void *out, char *ws, cu
     } else if (!three_d) {
         k_unwrap_rows<T><<<(unsigned)((A + 127) / 128), 128, 0, s>>>(phi, A, d.nx);
     } else {
-        Frames F{d.ny, d.nx, P, N};
+        uint32_t *bad = (uint32_t *)(ws + L.bad), *wmin = (uint32_t *)(ws + L.wmin);
+        Frames F{d.ny, d.nx, P, N, bad};
         double *rel = (double *)(ws + L.rel);
         unsigned long long *word = (unsigned long long *)(ws + L.word);
         unsigned long long *rw = (unsigned long long *)(ws + L.rw);
@@ -1025,6 +1378,18 @@ odt_status run(const odt_sino_desc &d, const void *sino, void *out, char *ws, cu
         uint32_t *ecnt = (uint32_t *)(ws + L.cnt), *rcnt = ecnt + 2;
         if (cudaMemsetAsync(ecnt, 0, 16, s) != cudaSuccess)
             return launched("unwrap workspace reset");
+        // frames without residues; steps, first edges and first columns in the
+        // places of rel, bw and rw, which the tree needs only afterwards
+        if (cudaMemsetAsync(bad, 0, (size_t)A * 4, s) != cudaSuccess ||
+            cudaMemsetAsync(wmin, 0xff, (size_t)A * 4, s) != cudaSuccess)
+            return launched("unwrap workspace reset");
+        uint8_t *steps = (uint8_t *)rel;
+        int32_t *col = (int32_t *)rw, *kan = (int32_t *)(ws + L.kan);
+        ulonglong2 *first = (ulonglong2 *)bw;
+        k_uf_scan<T><<<pg, pb, 0, s>>>(phi, F, d.seed, steps, bad, wmin);
+        k_uf_first<T><<<pg, pb, 0, s>>>(phi, F, d.seed, bad, wmin, first);
+        k_uf_frame<<<(unsigned)A, 256, 0, s>>>(F, steps, bad, first, (int)(pg.x * pg.y), col, kan);
+        k_uf_apply<T><<<dim3((unsigned)((d.ny + 7) / 8), (unsigned)A), 256, 0, s>>>(phi, F, steps, bad, col, kan);
         k_uw_init<T><<<pg, pb, 0, s>>>(phi, F, d.seed, rel, word, bw, be);
         // rounds 0 and 1 over the pixel grid; round 1 also lists the edges
         // that cross components and the roots that stay
@@ -1077,7 +1442,7 @@ int launches_of(const odt_sino_desc &d)
         return 3;  // min, align, compose
     int n = (d.kind == ODT_SINO_UNWRAP ? 1 : 2) + (d.align ? 2 : 0);  // (phase,) compose (+ min, align)
     if (d.ny > 0)
-        n += 3 + 5 * num_rounds((long long)d.ny * d.nx);  // init, anchor, rounds, finish
+        n += 7 + 5 * num_rounds((long long)d.ny * d.nx);  // residue-free frames (4), init, anchor, rounds, finish
     else
         n += 1;
     return n;
