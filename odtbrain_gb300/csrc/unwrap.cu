@@ -29,20 +29,21 @@
 //                      k_uw_hook     root -> neighbouring root, turn offset
 //                      k_uw_jump     pointer jumping among this round's roots
 //                      k_uw_flatten  every pixel -> its new root
+//                    (at most ceil(log2(pixels)) + 2 rounds; a round with no
+//                    hook ends the work of the following ones; from the third
+//                    round on all steps are in k_ul_rounds), with
+//                      k_uw_anchor   first edge of each frame (after round 0's
+//                                    k_uw_mine), then
+//                      k_uw_finish   phi + 2 pi k, k relative to pixel 1 of
+//                                    the frame's first edge
 //                    A frame without residues (no 2 x 2 loop of pixels whose
 //                    wrapped steps do not cancel) needs no tree: the turns
 //                    between two pixels are then the same along every path,
 //                    so running sums along the first column and the rows give
 //                    the tree's (k_uf_scan .. k_uf_apply), and only the pixel
 //                    the tree starts from has to be found.  200 residue-free
-//                    frames of 256^2: 4.25 -> 1.69 ms; the kernels below leave
+//                    frames of 256^2: 4.3 -> 0.56 ms; the kernels below leave
 //                    such frames out.
-//                    (at most ceil(log2(pixels)) + 2 rounds; a round with no
-//                    hook ends the work of the following ones), with
-//                      k_uw_anchor   first edge of each frame (after round 0's
-//                                    k_uw_mine), then
-//                      k_uw_finish   phi + 2 pi k, k relative to pixel 1 of
-//                                    the frame's first edge
 //   align            k_phase_min (global minimum), k_align (one CTA: the
 //                    five border samples unwrapped along the angle axis,
 //                    per-angle majority step, whole turns of the minimum)
@@ -51,8 +52,9 @@
 // ODT_SINO_UNWRAP takes a real wrapped phase and skips k_phase;
 // ODT_SINO_ALIGN takes an unwrapped real phase and runs the last three steps.
 //
-// Every wait is bounded: k_uw_jump's loop stops after a fixed number of
-// steps and records ODT_ERR_DEVICE_CHECK in the status word.
+// Every wait is bounded: pointer jumping stops after a fixed number of steps,
+// the barrier of k_ul_rounds after a fixed time; both record
+// ODT_ERR_DEVICE_CHECK in the status word.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -71,7 +73,7 @@ constexpr double BORDER_BASE = 9999999.0;
 constexpr unsigned long long NONE64 = ~0ull;
 constexpr uint32_t NONE32 = ~0u;
 constexpr int JUMP_LIMIT = 1 << 22;
-constexpr int STATUS_JUMP = 1, STATUS_SPLIT = 2;
+constexpr int STATUS_JUMP = 1, STATUS_SPLIT = 2, STATUS_BARRIER = 4;
 
 template <class T>
 struct C2 {
@@ -198,23 +200,25 @@ struct Frames {
     int H, W;
     long long P;  // H * W
     long long N;  // A * P
-    const uint32_t *bad;  // per frame: nonzero where the tree is needed
+    const uint32_t *bad;            // per frame: nonzero where the tree is needed
+    const uint32_t *list, *nlist;  // those frames, their number
 };
 
-// The per-pixel kernels run on blocks of 32 x 8 pixels over a grid
-// (ceil(W/32), ceil(H/8), frames): frame, row and column come from the
-// block and thread indices (no divisions); p = (a*H + i)*W + j < 2^31.
+// The tree's per-pixel kernels run on blocks of 32 x 8 pixels over a grid
+// (ceil(W/32), ceil(H/8), z), the z layers striding over the listed frames
+// (a grid of all frames costs 0.03 ms per kernel for 200 frames of 256^2 that
+// need no tree, 12 kernels); p = (a*H + i)*W + j < 2^31.
 struct Px {
     int a, i, j;
     uint32_t p;
     bool ok;
 };
-__device__ __forceinline__ Px pixel(const Frames &F)
+__device__ __forceinline__ Px pixel(const Frames &F, uint32_t z)
 {
     Px x;
     x.j = (int)(blockIdx.x * 32 + threadIdx.x);
     x.i = (int)(blockIdx.y * 8 + threadIdx.y);
-    x.a = (int)blockIdx.z;
+    x.a = (int)F.list[z];
     x.ok = x.i < F.H && x.j < F.W;
     x.p = ((uint32_t)x.a * (uint32_t)F.H + (uint32_t)x.i) * (uint32_t)F.W + (uint32_t)x.j;
     return x;
@@ -291,198 +295,236 @@ __global__ void k_unwrap_rows(T *phi, long long rows, int len)
         p[i] = u.next(p[i]);
 }
 
-// ---- 3D frames without residues -------------------------------------------
-// Turns of v minus turns of u across the edge u - v: the wrapped step's whole
-// turns (the reference's find_wrap), decided in FP64 where FP32 is too close.
-template <class T>
-__device__ __forceinline__ int turn_step(T u, T v)
+// ---- whole turns and shifts added in FP64 ----------------------------------
+// float(double(x) + c) for c = hi + lo (to 2^-46 of |hi|) in FP32: the sum as
+// an unevaluated pair is good to 2^-45 (|x| + |hi|); r is the result if both
+// ends of that interval round to it, else (about one sum in 2^20, and zeros,
+// infinities and NaN) the caller adds in FP64.  The FP64 conversions and sums
+// were what bounded k_uf_apply and k_compose: 0.124 -> 0.020 and 0.076 -> 0.049 ms
+// for 200 frames of 256^2.
+__device__ __forceinline__ bool add_pair(float x, float hi, float lo, float &r)
 {
-    const float df = (float)u - (float)v;  // (off by less than 2e-6: |u|, |v| <= UF_MAX)
-    if (fabsf(df) < 3.1415f)
-        return 0;
-    if (fabsf(df) > 3.1417f)
-        return df > 0.f ? 1 : -1;
-    const double d = (double)u - (double)v;
-    return d > PI_D ? 1 : (d < -PI_D ? -1 : 0);
+    const float m = fabsf(x) + fabsf(hi), d = m * 0x1p-44f;
+    const float s = __fadd_rn(x, hi), b = __fsub_rn(s, x);
+    const float e = __fadd_rn(__fsub_rn(x, __fsub_rn(s, b)), __fsub_rn(hi, b));  // x + hi = s + e
+    const float t = __fadd_rn(e, lo);
+    r = __fadd_rn(s, __fadd_rn(t, d));
+    return r == __fadd_rn(s, __fsub_rn(t, d)) && m > 1e-10f;
 }
 
+// x + 2 pi k, the FP64 product and sum rounded to T.
+template <class T>
+__device__ __forceinline__ T add_turns(T x, int32_t k)
+{
+    if constexpr (sizeof(T) == 4) {
+        constexpr float A = (float)TWOPI_D, B = (float)(TWOPI_D - (double)(float)TWOPI_D);
+        const float kf = (float)k, hi = __fmul_rn(kf, A);
+        float r;
+        if (abs(k) < (1 << 24) && add_pair((float)x, hi, __fmaf_rn(kf, B, __fmaf_rn(kf, A, -hi)), r))
+            return (T)r;
+    }
+    return (T)__dadd_rn((double)x, __dmul_rn(TWOPI_D, (double)k));
+}
+
+// ---- 3D frames without residues -------------------------------------------
 // Frames with a phase beyond this (phases of complex data are within pi) or a
 // NaN go through the tree: the FP32 estimates below rely on it.
 constexpr float UF_MAX = 8.f;
 
-// Tile of phases of a 32 x 8 block with two positions of halo on the right
-// and below and one on the left and above.
-constexpr int UF_TW = 35, UF_TH = 11;
+// A warp marches down a strip of 32 columns, of which it owns the 29 in lanes
+// 1 to 29, UF_ROWS rows at a time: neighbours in a row come by shuffle, the
+// differences to the row above stay in registers, so a pixel costs one load,
+// four wrapped differences and no shared memory (as 32 x 8 tiles in shared
+// memory with the eight differences per pixel formed anew, 200 frames of
+// 256^2 took 0.24 ms, like this 0.09 ms).
+constexpr int UF_COLS = 29, UF_ROWS = 16;
+__host__ __device__ inline int uf_tiles_x(int W) { return (W + UF_COLS - 1) / UF_COLS; }
+__host__ __device__ inline int uf_tiles(int H, int W) { return uf_tiles_x(W) * ((H + UF_ROWS - 1) / UF_ROWS); }
 
+// Turns of v minus turns of u across the edge u - v: the wrapped step's whole
+// turns (the reference's find_wrap).
 template <class T>
-__device__ __forceinline__ void uf_load_tile(const T *frame, const Frames &F, T (&ph)[UF_TH][UF_TW])
+__device__ __forceinline__ int turn_exact(T u, T v)
 {
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    const int i0 = (int)blockIdx.y * 8 - 1, j0 = (int)blockIdx.x * 32 - 1;
-    for (int t = tid; t < UF_TH * UF_TW; t += 256) {
-        const int ti = t / UF_TW, tj = t - ti * UF_TW;
-        const int gi = i0 + ti, gj = j0 + tj;
-        ph[ti][tj] = (gi >= 0 && gi < F.H && gj >= 0 && gj < F.W) ? frame[(size_t)gi * F.W + gj] : T(0);
-    }
+    const double d = (double)u - (double)v;
+    return d > PI_D ? 1 : (d < -PI_D ? -1 : 0);
 }
+
+// FP32 differences of phases within UF_MAX are off by less than 1e-6: those
+// outside this band are on the same side of pi in FP64.
+__device__ __forceinline__ bool near_pi(float d) { return fabsf(fabsf(d) - 3.1416f) <= 1e-4f; }
+__device__ __forceinline__ int turn_of(float d) { return fabsf(d) < 3.1416f ? 0 : (d > 0.f ? 1 : -1); }
 
 // Wrapped difference, NaN where FP32 cannot tell on which side of pi it is.
 __device__ __forceinline__ float wrapf(float d)
 {
     const float m = fabsf(d);
-    if (m < 3.1415f)
-        return d;
-    return m > 3.1417f ? d - copysignf(6.28318531f, d) : __int_as_float(0x7fffffff);
+    if (near_pi(d))
+        return __int_as_float(0x7fffffff);
+    return m < 3.1416f ? d : d - copysignf(6.28318531f, d);
 }
 
-// FP32 estimate of the reliability (k_uw_init) of the pixel at tile position
-// (ti, tj), image position (i, j); NaN where it may be off by a wrap.
+// The reliability of pixel (i, j) with k_uw_init's operations.
 template <class T>
-__device__ __forceinline__ float rel_estimate(const T (&ph)[UF_TH][UF_TW], const Frames &F, uint32_t seed, int ti, int tj,
-                                              int i, int j)
-{
-    if (i < 1 || i > F.H - 2 || j < 1 || j > F.W - 2)
-        return (float)(BORDER_BASE + border_noise(seed, (unsigned long long)((uint32_t)i * (uint32_t)F.W + j)));
-    auto at = [&](int a, int b) { return (float)ph[ti + a][tj + b]; };
-    const float c = at(0, 0);
-    const float h = wrapf(at(0, -1) - c) - wrapf(c - at(0, 1)), v = wrapf(at(-1, 0) - c) - wrapf(c - at(1, 0));
-    const float d1 = wrapf(at(-1, -1) - c) - wrapf(c - at(1, 1)), d2 = wrapf(at(-1, 1) - c) - wrapf(c - at(1, -1));
-    return h * h + v * v + d1 * d1 + d2 * d2;
-}
-
-// The reliability itself, with k_uw_init's operations.
-template <class T>
-__device__ double rel_exact(const T (&ph)[UF_TH][UF_TW], const Frames &F, uint32_t seed, int ti, int tj, int i, int j)
+__device__ double rel_exact(const T *frame, const Frames &F, uint32_t seed, int i, int j)
 {
     if (i < 1 || i > F.H - 2 || j < 1 || j > F.W - 2)
         return __dadd_rn(BORDER_BASE, border_noise(seed, (unsigned long long)((uint32_t)i * (uint32_t)F.W + j)));
-    auto at = [&](int a, int b) { return (double)ph[ti + a][tj + b]; };
-    const T c0 = ph[ti][tj];
-    bool flat = true;  // nine equal phases: zero without any FP64 work
-#pragma unroll
-    for (int a = -1; a <= 1; ++a)
-#pragma unroll
-        for (int b = -1; b <= 1; ++b)
-            flat = flat && ph[ti + a][tj + b] == c0;
-    if (flat)
-        return 0.0;
-    const double c = at(0, 0);
-    auto second = [&](double p, double q) { return __dsub_rn(wrapd(__dsub_rn(p, c)), wrapd(__dsub_rn(c, q))); };
-    const double h = second(at(0, -1), at(0, 1)), v = second(at(-1, 0), at(1, 0));
-    const double d1 = second(at(-1, -1), at(1, 1)), d2 = second(at(-1, 1), at(1, -1));
+    const T *q = frame + (size_t)i * F.W + j;
+    const long long W = F.W;
+    const T c0 = q[0];
+    if (q[-1] == c0 && q[1] == c0 && q[-W] == c0 && q[W] == c0 && q[-W - 1] == c0 && q[W + 1] == c0 &&
+        q[-W + 1] == c0 && q[W - 1] == c0)
+        return 0.0;  // without any FP64 work
+    const double c = (double)c0;
+    auto second = [&](T a, T b) {
+        return __dsub_rn(wrapd(__dsub_rn((double)a, c)), wrapd(__dsub_rn(c, (double)b)));
+    };
+    const double h = second(q[-1], q[1]), v = second(q[-W], q[W]);
+    const double d1 = second(q[-W - 1], q[W + 1]), d2 = second(q[-W + 1], q[W - 1]);
     return __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(h, h), __dmul_rn(v, v)), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
 }
 
-// Steps of every pixel (right: bits 0-1, down: bits 2-3, two's complement),
-// whether the frame has a residue (bad), and the smallest estimated edge
-// weight of the frame (bits of a non-negative float; ~0, a NaN, if there is
-// none).
-template <class T>
-__global__ void __launch_bounds__(256) k_uf_scan(const T *phi, Frames F, uint32_t seed, uint8_t *steps, uint32_t *bad,
-                                                 uint32_t *wmin)
+// FIRST = false: the steps of every pixel (right: bits 0-1, down: bits 2-3,
+// two's complement), whether the frame has a residue (bad), the smallest
+// estimated edge weight of the tile (tmin; 0 if FP32 cannot tell) and of the
+// frame (wmin: bits of a non-negative float; ~0, a NaN, if there is none).
+//
+// FIRST = true, of frames without residues: the first edge of the tile in
+// (weight, index) order, the weight in FP64, only of edges whose estimate can
+// be the frame's smallest.  A second difference's estimate is off by less than
+// 6e-6 (two wrapped differences of phases up to UF_MAX: conversions 2 x
+// 2.4e-7, subtraction 4.8e-7, turn 1.8e-7 and its subtraction 2.4e-7 each, and
+// the last subtraction), so the root of a weight, the norm of eight of them,
+// by less than 1.7e-5; the relative margin covers the sums and the border
+// weights.
+template <class T, bool FIRST>
+__global__ void __launch_bounds__(256) k_uf_scan(const T *phi, Frames F, uint32_t seed, int tiles, uint8_t *steps,
+                                                 uint32_t *bad, uint32_t *wmin, float *tmin, ulonglong2 *first)
 {
-    __shared__ T ph[UF_TH][UF_TW];
-    __shared__ float re[9][33];
-    const Px x = pixel(F);
-    uf_load_tile(phi + (size_t)x.a * (size_t)F.P, F, ph);
-    __syncthreads();
-    const int i0 = (int)blockIdx.y * 8, j0 = (int)blockIdx.x * 32;
-    for (int t = threadIdx.y * 32 + threadIdx.x; t < 9 * 33; t += 256) {
-        const int ti = t / 33, tj = t - ti * 33;
-        if (i0 + ti < F.H && j0 + tj < F.W)
-            re[ti][tj] = rel_estimate(ph, F, seed, ti + 1, tj + 1, i0 + ti, j0 + tj);
-    }
-    __syncthreads();
-    bool residue = false;  // or a phase that the estimates do not cover
-    float w = 3e38f;
-    if (x.ok) {
-        const int ti = threadIdx.y + 1, tj = threadIdx.x + 1;
-        const bool right = x.j + 1 < F.W, down = x.i + 1 < F.H;
-        const T c = ph[ti][tj];
-        residue = !(fabs(c) <= T(UF_MAX));
-        const int sr = right ? turn_step(c, ph[ti][tj + 1]) : 0, sd = down ? turn_step(c, ph[ti + 1][tj]) : 0;
-        steps[x.p] = (uint8_t)((sr & 3) | ((sd & 3) << 2));
-        if (right && down) {
-            const T q = ph[ti + 1][tj + 1];
-            residue |= sr + turn_step(ph[ti][tj + 1], q) != sd + turn_step(ph[ti + 1][tj], q);
-        }
-        const float r = re[ti - 1][tj - 1];
-        if (right)
-            w = fminf(w, r + re[ti - 1][tj]);
-        if (down)
-            w = fminf(w, r + re[ti][tj - 1]);
-    }
-    if (__syncthreads_or(residue) && threadIdx.x == 0 && threadIdx.y == 0)
-        atomicOr(bad + x.a, 1u);
-    for (int o = 16; o > 0; o >>= 1)
-        w = fminf(w, __shfl_xor_sync(0xffffffffu, w, o));
-    if (threadIdx.x == 0 && w < 3e38f)
-        atomicMin(wmin + x.a, __float_as_uint(w));
-}
-
-// The first edge in (weight, index) order among a block's edges; the weight in
-// FP64, only of edges whose estimate can be the frame's smallest.  A second
-// difference's estimate is off by less than 6e-6 (two wrapped differences of
-// phases up to UF_MAX: conversions 2 x 2.4e-7, subtraction 4.8e-7, turn 1.8e-7
-// and its subtraction 2.4e-7 each, and the last subtraction), so the root of a
-// weight, the norm of eight of them, by less than 1.7e-5; the relative margin
-// covers the sums and border weights.
-template <class T>
-__global__ void __launch_bounds__(256) k_uf_first(const T *phi, Frames F, uint32_t seed, const uint32_t *bad,
-                                                  const uint32_t *wmin, ulonglong2 *first)
-{
-    __shared__ T ph[UF_TH][UF_TW];
-    __shared__ unsigned long long sw[8];
-    __shared__ uint32_t se[8];
-    const Px x = pixel(F);
-    if (bad[x.a])
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, a = blockIdx.y, t = (int)(blockIdx.x * 8 + threadIdx.x / 32);
+    if (t >= tiles || (FIRST && bad[a]))
         return;
-    uf_load_tile(phi + (size_t)x.a * (size_t)F.P, F, ph);
-    __syncthreads();
+    const size_t tile = (size_t)a * tiles + t;
+    float lim = 0.f;
+    if (FIRST) {
+        const float root = sqrtf(__uint_as_float(wmin[a])) + 4e-5f;
+        lim = root * root * 1.0001f;
+        if (tmin[tile] > lim) {
+            if (lane == 0)
+                first[tile] = make_ulonglong2(NONE64, NONE32);
+            return;
+        }
+    }
+    const int gx = uf_tiles_x(F.W), ty = t / gx;
+    const int i0 = ty * UF_ROWS, i1 = i0 + UF_ROWS < F.H ? i0 + UF_ROWS : F.H, j = (t - ty * gx) * UF_COLS - 1 + lane;
+    const bool col = j >= 0 && j < F.W, own = lane >= 1 && lane <= UF_COLS && j < F.W, right = j + 1 < F.W;
+    const T *frame = phi + (size_t)a * (size_t)F.P;
+    auto row = [&](int i) -> T { return (col && i >= 0 && i < F.H) ? frame[(size_t)i * F.W + j] : T(0); };
+
+    float dD = 0.f, dDR = 0.f, dDL = 0.f;  // wrapped differences of a row and the one below
+    auto below = [&](float c, float n) {
+        const float nr = __shfl_down_sync(FULL, n, 1), nl = __shfl_up_sync(FULL, n, 1);
+        dD = wrapf(c - n);
+        dDR = wrapf(c - nr);
+        dDL = wrapf(c - nl);
+    };
+    T c = row(i0), n = row(i0 + 1);
+    below((float)row(i0 - 1), (float)c);
+    float rup = 0.f, w = 3e38f;
+    int srup = 0, sdup = 0, sdrup = 0;
+    bool residue = false, unsure = false;  // (residue: or a phase that the estimates do not cover)
     unsigned long long mw = NONE64;
     uint32_t me = NONE32;
-    if (x.ok) {
-        const int ti = threadIdx.y + 1, tj = threadIdx.x + 1;
-        const float root = sqrtf(__uint_as_float(wmin[x.a])) + 4e-5f, lim = root * root * 1.0001f;
-        const float r = rel_estimate(ph, F, seed, ti, tj, x.i, x.j);
-#pragma unroll
-        for (int d = 0; d < 2; ++d) {
-            const int di = d, dj = 1 - d;
-            if (x.i + di >= F.H || x.j + dj >= F.W)
-                continue;
-            // (a NaN estimate is a candidate)
-            if (r + rel_estimate(ph, F, seed, ti + di, tj + dj, x.i + di, x.j + dj) > lim)
-                continue;
-            const unsigned long long wb = dbits(__dadd_rn(rel_exact(ph, F, seed, ti, tj, x.i, x.j),
-                                                          rel_exact(ph, F, seed, ti + di, tj + dj, x.i + di, x.j + dj)));
-            const uint32_t le = d == 0 ? (uint32_t)(x.i * (F.W - 1) + x.j)
-                                       : (uint32_t)(F.H * (F.W - 1)) + (uint32_t)x.i * (uint32_t)F.W + (uint32_t)x.j;
+    auto edge = [&](float est, int i, bool vertical) {
+        if (FIRST) {
+            if (est > lim)  // (NaN: a candidate)
+                return;
+            const int iv = vertical ? i + 1 : i, jv = vertical ? j : j + 1;
+            const uint32_t le = vertical ? (uint32_t)(F.H * (F.W - 1)) + (uint32_t)i * (uint32_t)F.W + (uint32_t)j
+                                         : (uint32_t)(i * (F.W - 1) + j);
+            if (mw == 0 && le > me)  // (flat backgrounds: nothing is before a zero with a lower index)
+                return;
+            const unsigned long long wb =
+                dbits(__dadd_rn(rel_exact(frame, F, seed, i, j), rel_exact(frame, F, seed, iv, jv)));
             if (wb < mw || (wb == mw && le < me)) {
                 mw = wb;
                 me = le;
             }
+        } else {
+            unsure |= est != est;
+            w = fminf(w, est);
         }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(0xffffffffu, mw, o);
-        const uint32_t e = __shfl_xor_sync(0xffffffffu, me, o);
-        if (w < mw || (w == mw && e < me)) {
-            mw = w;
-            me = e;
-        }
-    }
-    if (threadIdx.x == 0) {
-        sw[threadIdx.y] = mw;
-        se[threadIdx.y] = me;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        for (int i = 1; i < 8; ++i)
-            if (sw[i] < mw || (sw[i] == mw && se[i] < me)) {
-                mw = sw[i];
-                me = se[i];
+    };
+    for (int i = i0; i <= i1 && i < F.H; ++i) {
+        const T nn = row(i + 2);
+        const float cf = (float)c, nf = (float)n, df = cf - __shfl_down_sync(FULL, cf, 1);
+        // the pixel's reliability
+        const float uD = dD, uDR = __shfl_up_sync(FULL, dDR, 1), uDL = __shfl_down_sync(FULL, dDL, 1);
+        const float dR = wrapf(df), lR = __shfl_up_sync(FULL, dR, 1);
+        below(cf, nf);
+        const float h = lR - dR, v = uD - dD, d1 = uDR - dDR, d2 = uDL - dDL;
+        float r = h * h + v * v + d1 * d1 + d2 * d2;
+        if (col && (i < 1 || i > F.H - 2 || j < 1 || j > F.W - 2))
+            r = (float)(BORDER_BASE + border_noise(seed, (unsigned long long)((uint32_t)i * (uint32_t)F.W + j)));
+        const float rr = __shfl_down_sync(FULL, r, 1);
+        if (own && i > i0)
+            edge(rup + r, i - 1, true);
+        if (own && right && i < i1)
+            edge(r + rr, i, false);
+        rup = r;
+        if (!FIRST) {
+            int sr = turn_of(df), sd = turn_of(cf - nf);
+            if (__any_sync(FULL, near_pi(df) || near_pi(cf - nf))) {
+                sr = turn_exact(c, __shfl_down_sync(FULL, c, 1));
+                sd = turn_exact(c, n);
             }
-        first[((size_t)x.a * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = make_ulonglong2(mw, me);
+            sr = right ? sr : 0;
+            sd = i + 1 < F.H ? sd : 0;
+            if (own) {
+                residue |= !(fabs(c) <= T(UF_MAX));
+                if (i > i0 && right)
+                    residue |= srup + sdrup != sdup + sr;
+                if (i < i1)
+                    steps[(size_t)a * F.P + (size_t)i * F.W + j] = (uint8_t)((sr & 3) | ((sd & 3) << 2));
+            }
+            srup = sr;
+            sdup = sd;
+            sdrup = __shfl_down_sync(FULL, sd, 1);
+        }
+        if (FIRST) {  // every lane at a horizontal edge of weight zero: nothing below is before those
+            const unsigned need = __ballot_sync(FULL, own && right);
+            const unsigned zero = __ballot_sync(FULL, mw == 0 && me < (uint32_t)(F.H * (F.W - 1)));
+            if (need && (zero & need) == need)
+                break;
+        }
+        c = n;
+        n = nn;
+    }
+    if (FIRST) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long ow = __shfl_xor_sync(FULL, mw, o);
+            const uint32_t oe = __shfl_xor_sync(FULL, me, o);
+            if (ow < mw || (ow == mw && oe < me)) {
+                mw = ow;
+                me = oe;
+            }
+        }
+        if (lane == 0)
+            first[tile] = make_ulonglong2(mw, me);
+    } else {
+        for (int o = 16; o > 0; o >>= 1)
+            w = fminf(w, __shfl_xor_sync(FULL, w, o));
+        residue = __any_sync(FULL, residue);
+        unsure = __any_sync(FULL, unsure);
+        if (lane == 0) {
+            if (residue)
+                atomicOr(bad + a, 1u);
+            if (w < 3e38f)
+                atomicMin(wmin + a, __float_as_uint(w));
+            tmin[tile] = unsure ? 0.f : w;
+        }
     }
 }
 
@@ -490,13 +532,18 @@ __device__ __forceinline__ int step_right(uint8_t b) { return (int)((uint32_t)b 
 __device__ __forceinline__ int step_down(uint8_t b) { return (int)((uint32_t)b << 28) >> 30; }
 
 // Per frame: its first edge, the turns of the first column, and those of the
-// edge's pixel 1 (kan).  One CTA of 256 threads per frame.
+// edge's pixel 1 (kan); the frames that need the tree are listed.  One CTA of
+// 256 threads per frame.
 __global__ void __launch_bounds__(256) k_uf_frame(Frames F, const uint8_t *steps, const uint32_t *bad,
-                                                  const ulonglong2 *first, int nblk, int32_t *col, int32_t *kan)
+                                                  const ulonglong2 *first, int nblk, int32_t *col, int32_t *kan,
+                                                  uint32_t *list, uint32_t *nlist)
 {
     const int a = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (bad[a])
+    if (bad[a]) {
+        if (tid == 0)
+            list[atomicAdd(nlist, 1u)] = (uint32_t)a;
         return;
+    }
     __shared__ unsigned long long sw[8];
     __shared__ uint32_t se[8];
     __shared__ int32_t ssum[8];
@@ -588,19 +635,25 @@ __global__ void __launch_bounds__(256) k_uf_apply(T *phi, Frames F, const uint8_
         return;
     const size_t row = (size_t)a * F.P + (size_t)i * F.W;
     int32_t k = col[(size_t)a * F.H + i] - kan[a];  // of column j0
-    for (int j0 = 0; j0 < F.W; j0 += 32) {
-        const int j = j0 + lane;
-        const int32_t st = j < F.W ? step_right(steps[row + j]) : 0;  // step from j to j + 1
-        int32_t incl = st;
-        for (int d = 1; d < 32; d <<= 1) {
-            const int32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d)
-                incl += t;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int j0 = 0; j0 < F.W; j0 += 128) {
+        int st[4];
+        T v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // step from j to j + 1
+            const int j = j0 + 32 * q + lane;
+            st[q] = j < F.W ? step_right(steps[row + j]) : 0;
+            v[q] = j < F.W ? phi[row + j] : T(0);
         }
-        const int32_t kj = k + incl - st;
-        if (j < F.W && kj != 0)
-            phi[row + j] = (T)__dadd_rn((double)phi[row + j], __dmul_rn(TWOPI_D, (double)kj));
-        k += __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = j0 + 32 * q + lane;
+            const unsigned up = __ballot_sync(0xffffffffu, st[q] > 0), dn = __ballot_sync(0xffffffffu, st[q] < 0);
+            const int32_t kj = k + __popc(up & lt) - __popc(dn & lt);
+            if (j < F.W && kj != 0)
+                phi[row + j] = add_turns(v[q], kj);
+            k += __popc(up) - __popc(dn);
+        }
     }
 }
 
@@ -666,51 +719,52 @@ __global__ void __launch_bounds__(256) k_uw_init(const T *phi, Frames F, uint32_
 {
     __shared__ double ph[UI_TH][UI_TW];
     __shared__ double dR[UI_TH][UI_TW], dD[UI_TH][UI_TW], dDR[UI_TH][UI_TW], dDL[UI_TH][UI_TW];
-    const Px x = pixel(F);
-    if (!F.bad[x.a])
-        return;
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    const int i0 = (int)blockIdx.y * 8 - 1, j0 = (int)blockIdx.x * 32 - 1;
-    const T *frame = phi + (size_t)x.a * (size_t)F.P;
-    for (int t = tid; t < UI_TH * UI_TW; t += 256) {
-        const int ti = t / UI_TW, tj = t - ti * UI_TW;
-        const int gi = i0 + ti, gj = j0 + tj;
-        ph[ti][tj] = (gi >= 0 && gi < F.H && gj >= 0 && gj < F.W) ? (double)frame[(size_t)gi * F.W + gj] : 0.0;
-    }
-    __syncthreads();
-    for (int t = tid; t < UI_TH * UI_TW; t += 256) {
-        const int ti = t / UI_TW, tj = t - ti * UI_TW;
-        const double c = ph[ti][tj];
-        if (tj + 1 < UI_TW)
-            dR[ti][tj] = wrapd(__dsub_rn(c, ph[ti][tj + 1]));
-        if (ti + 1 < UI_TH) {
-            dD[ti][tj] = wrapd(__dsub_rn(c, ph[ti + 1][tj]));
-            if (tj + 1 < UI_TW)
-                dDR[ti][tj] = wrapd(__dsub_rn(c, ph[ti + 1][tj + 1]));
-            if (tj >= 1)
-                dDL[ti][tj] = wrapd(__dsub_rn(c, ph[ti + 1][tj - 1]));
+    for (uint32_t z = blockIdx.z, nz = *F.nlist; z < nz; z += gridDim.z) {
+        const Px x = pixel(F, z);
+        const int tid = threadIdx.y * 32 + threadIdx.x;
+        const int i0 = (int)blockIdx.y * 8 - 1, j0 = (int)blockIdx.x * 32 - 1;
+        __syncthreads();  // (the previous frame's tile)
+        const T *frame = phi + (size_t)x.a * (size_t)F.P;
+        for (int t = tid; t < UI_TH * UI_TW; t += 256) {
+            const int ti = t / UI_TW, tj = t - ti * UI_TW;
+            const int gi = i0 + ti, gj = j0 + tj;
+            ph[ti][tj] = (gi >= 0 && gi < F.H && gj >= 0 && gj < F.W) ? (double)frame[(size_t)gi * F.W + gj] : 0.0;
         }
+        __syncthreads();
+        for (int t = tid; t < UI_TH * UI_TW; t += 256) {
+            const int ti = t / UI_TW, tj = t - ti * UI_TW;
+            const double c = ph[ti][tj];
+            if (tj + 1 < UI_TW)
+                dR[ti][tj] = wrapd(__dsub_rn(c, ph[ti][tj + 1]));
+            if (ti + 1 < UI_TH) {
+                dD[ti][tj] = wrapd(__dsub_rn(c, ph[ti + 1][tj]));
+                if (tj + 1 < UI_TW)
+                    dDR[ti][tj] = wrapd(__dsub_rn(c, ph[ti + 1][tj + 1]));
+                if (tj >= 1)
+                    dDL[ti][tj] = wrapd(__dsub_rn(c, ph[ti + 1][tj - 1]));
+            }
+        }
+        __syncthreads();
+        if (!x.ok)
+            continue;
+        const uint32_t p = x.p;
+        const int i = x.i, j = x.j;
+        double r;
+        if (i >= 1 && i <= F.H - 2 && j >= 1 && j <= F.W - 2) {
+            const int ti = threadIdx.y + 1, tj = threadIdx.x + 1;
+            const double h = __dsub_rn(dR[ti][tj - 1], dR[ti][tj]);         // wrap(l - c) - wrap(c - r)
+            const double v = __dsub_rn(dD[ti - 1][tj], dD[ti][tj]);         // wrap(u - c) - wrap(c - d)
+            const double d1 = __dsub_rn(dDR[ti - 1][tj - 1], dDR[ti][tj]);  // wrap(ul - c) - wrap(c - dr)
+            const double d2 = __dsub_rn(dDL[ti - 1][tj + 1], dDL[ti][tj]);  // wrap(ur - c) - wrap(c - dl)
+            r = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(h, h), __dmul_rn(v, v)), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
+        } else {
+            r = __dadd_rn(BORDER_BASE, border_noise(seed, (unsigned long long)((uint32_t)i * (uint32_t)F.W + j)));
+        }
+        rel[p] = r;
+        word[p] = pack(p, 0);
+        bw[p] = NONE64;
+        be[p] = NONE32;
     }
-    __syncthreads();
-    if (!x.ok)
-        return;
-    const uint32_t p = x.p;
-    const int i = x.i, j = x.j;
-    double r;
-    if (i >= 1 && i <= F.H - 2 && j >= 1 && j <= F.W - 2) {
-        const int ti = threadIdx.y + 1, tj = threadIdx.x + 1;
-        const double h = __dsub_rn(dR[ti][tj - 1], dR[ti][tj]);         // wrap(l - c) - wrap(c - r)
-        const double v = __dsub_rn(dD[ti - 1][tj], dD[ti][tj]);         // wrap(u - c) - wrap(c - d)
-        const double d1 = __dsub_rn(dDR[ti - 1][tj - 1], dDR[ti][tj]);  // wrap(ul - c) - wrap(c - dr)
-        const double d2 = __dsub_rn(dDL[ti - 1][tj + 1], dDL[ti][tj]);  // wrap(ur - c) - wrap(c - dl)
-        r = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(h, h), __dmul_rn(v, v)), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
-    } else {
-        r = __dadd_rn(BORDER_BASE, border_noise(seed, (unsigned long long)((uint32_t)i * (uint32_t)F.W + j)));
-    }
-    rel[p] = r;
-    word[p] = pack(p, 0);
-    bw[p] = NONE64;
-    be[p] = NONE32;
 }
 
 // Lightest outgoing edge weight of every component root (edges handled by
@@ -723,36 +777,36 @@ __global__ void k_uw_minw(Frames F, const double *rel, const unsigned long long 
 {
     if (round > 0 && flags[round - 1] == 0)
         return;
-    const Px x = pixel(F);
-    if (!F.bad[x.a])
-        return;
-    const uint32_t p = x.p;
-    const int i = x.i, j = x.j;
-    const uint32_t rp = x.ok ? par_of(word[p]) : 0u;
-    const double relp = x.ok ? rel[p] : 0.0;
+    for (uint32_t z = blockIdx.z, nz = *F.nlist; z < nz; z += gridDim.z) {
+        const Px x = pixel(F, z);
+        const uint32_t p = x.p;
+        const int i = x.i, j = x.j;
+        const uint32_t rp = x.ok ? par_of(word[p]) : 0u;
+        const double relp = x.ok ? rel[p] : 0.0;
 #pragma unroll
-    for (int d = 0; d < 2; ++d) {
-        bool cross = false;
-        uint32_t le = 0;
-        if (x.ok && (d == 0 ? (j + 1 < F.W) : (i + 1 < F.H))) {
-            const uint32_t q = p + (d == 0 ? 1u : (uint32_t)F.W);
-            const uint32_t rq = par_of(word[q]);
-            if (rp != rq) {
-                cross = true;
-                le = d == 0 ? (uint32_t)(i * (F.W - 1) + j)
-                            : (uint32_t)(F.H * (F.W - 1)) + (uint32_t)i * (uint32_t)F.W + (uint32_t)j;
-                const unsigned long long wb = dbits(__dadd_rn(relp, rel[q]));
-                if (wb < bw[rp])
-                    atomicMin(bw + rp, wb);
-                if (wb < bw[rq])
-                    atomicMin(bw + rq, wb);
+        for (int d = 0; d < 2; ++d) {
+            bool cross = false;
+            uint32_t le = 0;
+            if (x.ok && (d == 0 ? (j + 1 < F.W) : (i + 1 < F.H))) {
+                const uint32_t q = p + (d == 0 ? 1u : (uint32_t)F.W);
+                const uint32_t rq = par_of(word[q]);
+                if (rp != rq) {
+                    cross = true;
+                    le = d == 0 ? (uint32_t)(i * (F.W - 1) + j)
+                                : (uint32_t)(F.H * (F.W - 1)) + (uint32_t)i * (uint32_t)F.W + (uint32_t)j;
+                    const unsigned long long wb = dbits(__dadd_rn(relp, rel[q]));
+                    if (wb < bw[rp])
+                        atomicMin(bw + rp, wb);
+                    if (wb < bw[rq])
+                        atomicMin(bw + rq, wb);
+                }
             }
-        }
-        if (elist) {
-            // list entry: (pixel 1, local edge index | vertical flag)
-            const uint32_t slot = append_slot(ecnt, cross);
-            if (cross)
-                elist[slot] = make_uint2(p, d == 0 ? le : (le | 0x80000000u));
+            if (elist) {
+                // list entry: (pixel 1, local edge index | vertical flag)
+                const uint32_t slot = append_slot(ecnt, cross);
+                if (cross)
+                    elist[slot] = make_uint2(p, d == 0 ? le : (le | 0x80000000u));
+            }
         }
     }
 }
@@ -763,28 +817,30 @@ __global__ void k_uw_mine(Frames F, const double *rel, const unsigned long long 
 {
     if (round > 0 && flags[round - 1] == 0)
         return;
-    const Px x = pixel(F);
-    if (!x.ok || !F.bad[x.a])
-        return;
-    const uint32_t p = x.p;
-    const int i = x.i, j = x.j;
-    const uint32_t lp = (uint32_t)i * (uint32_t)F.W + (uint32_t)j;
-    const uint32_t rp = par_of(word[p]);
-    const double relp = rel[p];
+    for (uint32_t z = blockIdx.z, nz = *F.nlist; z < nz; z += gridDim.z) {
+        const Px x = pixel(F, z);
+        if (!x.ok)
+            continue;
+        const uint32_t p = x.p;
+        const int i = x.i, j = x.j;
+        const uint32_t lp = (uint32_t)i * (uint32_t)F.W + (uint32_t)j;
+        const uint32_t rp = par_of(word[p]);
+        const double relp = rel[p];
 #pragma unroll
-    for (int d = 0; d < 2; ++d) {
-        if (d == 0 ? (j + 1 >= F.W) : (i + 1 >= F.H))
-            continue;
-        const uint32_t q = p + (d == 0 ? 1u : (uint32_t)F.W);
-        const uint32_t rq = par_of(word[q]);
-        if (rp == rq)
-            continue;
-        const unsigned long long wb = dbits(__dadd_rn(relp, rel[q]));
-        const uint32_t le = d == 0 ? (uint32_t)(i * (F.W - 1) + j) : (uint32_t)(F.H * (F.W - 1)) + lp;
-        if (wb == bw[rp])
-            atomicMin(be + rp, le);
-        if (wb == bw[rq])
-            atomicMin(be + rq, le);
+        for (int d = 0; d < 2; ++d) {
+            if (d == 0 ? (j + 1 >= F.W) : (i + 1 >= F.H))
+                continue;
+            const uint32_t q = p + (d == 0 ? 1u : (uint32_t)F.W);
+            const uint32_t rq = par_of(word[q]);
+            if (rp == rq)
+                continue;
+            const unsigned long long wb = dbits(__dadd_rn(relp, rel[q]));
+            const uint32_t le = d == 0 ? (uint32_t)(i * (F.W - 1) + j) : (uint32_t)(F.H * (F.W - 1)) + lp;
+            if (wb == bw[rp])
+                atomicMin(be + rp, le);
+            if (wb == bw[rq])
+                atomicMin(be + rq, le);
+        }
     }
 }
 
@@ -797,41 +853,41 @@ __global__ void k_uw_hook(Frames F, const T *phi, const unsigned long long *word
 {
     if (round > 0 && flags[round - 1] == 0)
         return;
-    const Px x = pixel(F);
-    if (!F.bad[x.a])
-        return;
-    const uint32_t r = x.p;
-    bool keep = false;  // a root after this round with an outgoing edge left
-    if (x.ok && par_of(word[r]) == r) {
-        const uint32_t le = be[r];
-        if (le == NONE32) {
-            rw[r] = pack(r, 0);
-        } else {
-            const uint32_t base = (uint32_t)x.a * (uint32_t)F.P;
-            uint32_t u, v;
-            edge_ends(F, base, le, u, v);
-            const unsigned long long wu = word[u], wv = word[v];
-            const bool u_in_r = par_of(wu) == r;
-            const uint32_t s = u_in_r ? par_of(wv) : par_of(wu);
-            if (be[s] == le && r < s) {
+    for (uint32_t z = blockIdx.z, nz = *F.nlist; z < nz; z += gridDim.z) {
+        const Px x = pixel(F, z);
+        const uint32_t r = x.p;
+        bool keep = false;  // a root after this round with an outgoing edge left
+        if (x.ok && par_of(word[r]) == r) {
+            const uint32_t le = be[r];
+            if (le == NONE32) {
                 rw[r] = pack(r, 0);
-                keep = true;
             } else {
-                // turns: k(v) - k(u) = -e with e = +1 / -1 / 0 as
-                // phi[u] - phi[v] is below -pi / above pi / neither (the
-                // reference's find_wrap)
-                const double d = (double)phi[u] - (double)phi[v];
-                const int e = d > PI_D ? -1 : (d < -PI_D ? 1 : 0);
-                const int32_t ou = off_of(wu), ov = off_of(wv);
-                rw[r] = pack(s, u_in_r ? (e + ov - ou) : (-e + ou - ov));
-                flags[round] = 1;
+                const uint32_t base = (uint32_t)x.a * (uint32_t)F.P;
+                uint32_t u, v;
+                edge_ends(F, base, le, u, v);
+                const unsigned long long wu = word[u], wv = word[v];
+                const bool u_in_r = par_of(wu) == r;
+                const uint32_t s = u_in_r ? par_of(wv) : par_of(wu);
+                if (be[s] == le && r < s) {
+                    rw[r] = pack(r, 0);
+                    keep = true;
+                } else {
+                    // turns: k(v) - k(u) = -e with e = +1 / -1 / 0 as
+                    // phi[u] - phi[v] is below -pi / above pi / neither (the
+                    // reference's find_wrap)
+                    const double d = (double)phi[u] - (double)phi[v];
+                    const int e = d > PI_D ? -1 : (d < -PI_D ? 1 : 0);
+                    const int32_t ou = off_of(wu), ov = off_of(wv);
+                    rw[r] = pack(s, u_in_r ? (e + ov - ou) : (-e + ou - ov));
+                    flags[round] = 1;
+                }
             }
         }
-    }
-    if (rlist) {
-        const uint32_t slot = append_slot(rcnt, keep);
-        if (keep)
-            rlist[slot] = r;
+        if (rlist) {
+            const uint32_t slot = append_slot(rcnt, keep);
+            if (keep)
+                rlist[slot] = r;
+        }
     }
 }
 
@@ -840,162 +896,13 @@ __global__ void k_uw_jump(Frames F, const unsigned long long *word, unsigned lon
 {
     if (flags[round] == 0)
         return;
-    const Px x = pixel(F);
-    if (!x.ok || !F.bad[x.a])
-        return;
-    const uint32_t r = x.p;
-    if (par_of(word[r]) != r)
-        return;
-    unsigned long long w = __ldcg(rw + r);
-    for (int it = 0;; ++it) {
-        const uint32_t pp = par_of(w);
-        if (pp == r)
-            break;
-        const unsigned long long wp = __ldcg(rw + pp);
-        if (par_of(wp) == pp)
-            break;
-        w = pack(par_of(wp), off_of(w) + off_of(wp));
-        __stcg(rw + r, w);
-        if (it >= JUMP_LIMIT) {
-            atomicOr(status, STATUS_JUMP);
-            break;
-        }
-    }
-}
-
-__global__ void k_uw_flatten(Frames F, unsigned long long *word, const unsigned long long *rw,
-                             unsigned long long *bw, uint32_t *be, const uint32_t *flags, int round)
-{
-    if (flags[round] == 0)
-        return;
-    const Px x = pixel(F);
-    if (!x.ok || !F.bad[x.a])
-        return;
-    const uint32_t p = x.p;
-    const unsigned long long w = word[p];
-    const unsigned long long wr = rw[par_of(w)];
-    word[p] = pack(par_of(wr), off_of(w) + off_of(wr));
-    bw[p] = NONE64;
-    be[p] = NONE32;
-}
-
-// ---- rounds >= 2 on lists ---------------------------------------------------
-// From round 2 on, only the edges that crossed components in the previous
-// round and the roots that are left are visited (lists compacted every
-// round); pixel roots are found by following the (parent, offset) words,
-// which only the roots update (k_ul_update), with path compression.  Grids
-// are fixed; the kernels stride over the device-side counts.
-constexpr int UL_GRID = 152 * 8, UL_BLOCK = 256;
-
-__global__ void __launch_bounds__(UL_BLOCK) k_ul_edges_w(const double *rel, unsigned long long *word,
-                                                         unsigned long long *bw, const uint2 *ein,
-                                                         const uint32_t *ecnt_in, uint2 *eout, uint32_t *ecnt_out,
-                                                         int W, const uint32_t *flags, int round, uint32_t *status)
-{
-    if (flags[round - 1] == 0)
-        return;
-    const uint32_t n = *ecnt_in;
-    for (uint32_t b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
-        const uint32_t k = b + threadIdx.x;
-        bool cross = false;
-        uint2 e = make_uint2(0, 0);
-        if (k < n) {
-            e = ein[k];
-            const uint32_t u = e.x;
-            const uint32_t v = u + ((e.y & 0x80000000u) ? (uint32_t)W : 1u);
-            int32_t ou, ov;
-            const uint32_t ru = resolve(word, u, ou, status), rv = resolve(word, v, ov, status);
-            if (ru != rv) {
-                cross = true;
-                const unsigned long long wb = dbits(__dadd_rn(rel[u], rel[v]));
-                if (wb < bw[ru])
-                    atomicMin(bw + ru, wb);
-                if (wb < bw[rv])
-                    atomicMin(bw + rv, wb);
-            }
-        }
-        const uint32_t slot = append_slot(ecnt_out, cross);
-        if (cross)
-            eout[slot] = e;
-    }
-}
-
-__global__ void __launch_bounds__(UL_BLOCK) k_ul_edges_e(const double *rel, unsigned long long *word,
-                                                         const unsigned long long *bw, uint32_t *be, const uint2 *el,
-                                                         const uint32_t *ecnt, int W, const uint32_t *flags,
-                                                         int round, uint32_t *status)
-{
-    if (flags[round - 1] == 0)
-        return;
-    const uint32_t n = *ecnt;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint2 e = el[k];
-        const uint32_t u = e.x;
-        const uint32_t v = u + ((e.y & 0x80000000u) ? (uint32_t)W : 1u);
-        const uint32_t le = e.y & 0x7fffffffu;
-        int32_t ou, ov;
-        const uint32_t ru = resolve(word, u, ou, status), rv = resolve(word, v, ov, status);
-        if (ru == rv)
+    for (uint32_t z = blockIdx.z, nz = *F.nlist; z < nz; z += gridDim.z) {
+        const Px x = pixel(F, z);
+        if (!x.ok)
             continue;
-        const unsigned long long wb = dbits(__dadd_rn(rel[u], rel[v]));
-        if (wb == bw[ru])
-            atomicMin(be + ru, le);
-        if (wb == bw[rv])
-            atomicMin(be + rv, le);
-    }
-}
-
-template <class T>
-__global__ void __launch_bounds__(UL_BLOCK) k_ul_hook(Frames F, const T *phi, unsigned long long *word,
-                                                      const uint32_t *be, unsigned long long *rw, const uint32_t *rin,
-                                                      const uint32_t *rcnt_in, uint32_t *rout, uint32_t *rcnt_out,
-                                                      uint32_t *flags, int round, uint32_t *status)
-{
-    if (flags[round - 1] == 0)
-        return;
-    const uint32_t n = *rcnt_in;
-    for (uint32_t b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
-        const uint32_t k = b + threadIdx.x;
-        bool keep = false;
-        uint32_t r = 0;
-        if (k < n) {
-            r = rin[k];
-            const uint32_t le = be[r];
-            if (le == NONE32) {
-                rw[r] = pack(r, 0);
-            } else {
-                const uint32_t base = r / (uint32_t)F.P * (uint32_t)F.P;
-                uint32_t u, v;
-                edge_ends(F, base, le, u, v);
-                int32_t ou, ov;
-                const uint32_t ru = resolve(word, u, ou, status), rv = resolve(word, v, ov, status);
-                const bool u_in_r = ru == r;
-                const uint32_t s = u_in_r ? rv : ru;
-                if (be[s] == le && r < s) {
-                    rw[r] = pack(r, 0);
-                    keep = true;
-                } else {
-                    const double d = (double)phi[u] - (double)phi[v];
-                    const int e = d > PI_D ? -1 : (d < -PI_D ? 1 : 0);
-                    rw[r] = pack(s, u_in_r ? (e + ov - ou) : (-e + ou - ov));
-                    flags[round] = 1;
-                }
-            }
-        }
-        const uint32_t slot = append_slot(rcnt_out, keep);
-        if (keep)
-            rout[slot] = r;
-    }
-}
-
-__global__ void __launch_bounds__(UL_BLOCK) k_ul_jump(unsigned long long *rw, const uint32_t *rl, const uint32_t *rcnt,
-                                                      const uint32_t *flags, int round, uint32_t *status)
-{
-    if (flags[round] == 0)
-        return;
-    const uint32_t n = *rcnt;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t r = rl[k];
+        const uint32_t r = x.p;
+        if (par_of(word[r]) != r)
+            continue;
         unsigned long long w = __ldcg(rw + r);
         for (int it = 0;; ++it) {
             const uint32_t pp = par_of(w);
@@ -1014,19 +921,202 @@ __global__ void __launch_bounds__(UL_BLOCK) k_ul_jump(unsigned long long *rw, co
     }
 }
 
-// the roots of this round take their new parent word; per-root minima reset
-__global__ void __launch_bounds__(UL_BLOCK) k_ul_update(unsigned long long *word, const unsigned long long *rw,
-                                                        unsigned long long *bw, uint32_t *be, const uint32_t *rl,
-                                                        const uint32_t *rcnt, const uint32_t *flags, int round)
+__global__ void k_uw_flatten(Frames F, unsigned long long *word, const unsigned long long *rw,
+                             unsigned long long *bw, uint32_t *be, const uint32_t *flags, int round)
 {
     if (flags[round] == 0)
         return;
-    const uint32_t n = *rcnt;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t r = rl[k];
-        word[r] = rw[r];
-        bw[r] = NONE64;
-        be[r] = NONE32;
+    for (uint32_t z = blockIdx.z, nz = *F.nlist; z < nz; z += gridDim.z) {
+        const Px x = pixel(F, z);
+        if (!x.ok)
+            continue;
+        const uint32_t p = x.p;
+        const unsigned long long w = word[p];
+        const unsigned long long wr = rw[par_of(w)];
+        word[p] = pack(par_of(wr), off_of(w) + off_of(wr));
+        bw[p] = NONE64;
+        be[p] = NONE32;
+    }
+}
+
+// ---- rounds >= 2 on lists ---------------------------------------------------
+// From round 2 on, only the edges that crossed components in the previous
+// round and the roots that are left are visited (lists compacted every
+// round); pixel roots are found by following the (parent, offset) words,
+// which only the roots update, with path compression.  All these rounds are
+// one cooperative launch with a barrier between the steps: as five launches
+// and two resets per round they cost 0.35 ms for 256^2 frames even when there
+// was nothing to do (@L).
+constexpr int UL_BLOCK = 256;
+constexpr unsigned long long UL_WAIT_NS = 10000000000ull;
+
+// Barrier of the whole (cooperative) grid: every block counts up to `target`.
+// A block that waits longer than UL_WAIT_NS records it and gives up, as do the
+// blocks that see the record; returns false then.
+__device__ __forceinline__ bool grid_barrier(uint32_t *count, uint32_t target, uint32_t *status)
+{
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ok = 1;
+        __threadfence();
+        atomicAdd(count, 1u);
+        unsigned long long t0, t1;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+        for (;;) {
+            uint32_t v;
+            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            if (v >= target)
+                break;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+            if (t1 - t0 > UL_WAIT_NS || (__ldcg(status) & STATUS_BARRIER)) {
+                atomicOr(status, (uint32_t)STATUS_BARRIER);
+                ok = 0;
+                break;
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+struct ListRounds {
+    const double *rel;
+    unsigned long long *word, *rw, *bw;
+    uint32_t *be;
+    uint2 *el[2];       // edges in, out (alternating; round 1 wrote 0)
+    uint32_t *rl[2];    // roots, likewise
+    uint32_t *ecnt, *rcnt;  // per round: entries of the lists that it wrote
+    uint32_t *flags;    // per round: some root hooked
+    uint32_t *bar, *status;
+    int rounds;
+};
+
+template <class T>
+__global__ void __launch_bounds__(UL_BLOCK) k_ul_rounds(Frames F, const T *phi, ListRounds R)
+{
+    const uint32_t t0 = blockIdx.x * blockDim.x, stride = gridDim.x * blockDim.x;
+    uint32_t *status = R.status;
+    uint32_t target = 0;
+    for (int r = 2; r < R.rounds && __ldcg(R.flags + r - 1); ++r) {
+        const int in = r & 1 ? 1 : 0, out = in ^ 1;
+        const uint2 *ein = R.el[in];
+        uint2 *eout = R.el[out];
+        const uint32_t *rin = R.rl[in];
+        uint32_t *rout = R.rl[out];
+        const uint32_t ne = __ldcg(R.ecnt + r - 1), nr = __ldcg(R.rcnt + r - 1);
+        // lightest outgoing edge weight of every root; the edges that cross
+        for (uint32_t b = t0; b < ne; b += stride) {
+            const uint32_t k = b + threadIdx.x;
+            bool cross = false;
+            uint2 e = make_uint2(0, 0);
+            if (k < ne) {
+                e = __ldcg(ein + k);
+                const uint32_t u = e.x;
+                const uint32_t v = u + ((e.y & 0x80000000u) ? (uint32_t)F.W : 1u);
+                int32_t ou, ov;
+                const uint32_t ru = resolve(R.word, u, ou, status), rv = resolve(R.word, v, ov, status);
+                if (ru != rv) {
+                    cross = true;
+                    const unsigned long long wb = dbits(__dadd_rn(R.rel[u], R.rel[v]));
+                    if (wb < __ldcg(R.bw + ru))
+                        atomicMin(R.bw + ru, wb);
+                    if (wb < __ldcg(R.bw + rv))
+                        atomicMin(R.bw + rv, wb);
+                }
+            }
+            const uint32_t slot = append_slot(R.ecnt + r, cross);
+            if (cross)
+                eout[slot] = e;
+        }
+        if (!grid_barrier(R.bar, target += gridDim.x, status))
+            return;
+        // its lowest edge index
+        const uint32_t nx = __ldcg(R.ecnt + r);
+        for (uint32_t k = t0 + threadIdx.x; k < nx; k += stride) {
+            const uint2 e = __ldcg(eout + k);
+            const uint32_t u = e.x;
+            const uint32_t v = u + ((e.y & 0x80000000u) ? (uint32_t)F.W : 1u);
+            const uint32_t le = e.y & 0x7fffffffu;
+            int32_t ou, ov;
+            const uint32_t ru = resolve(R.word, u, ou, status), rv = resolve(R.word, v, ov, status);
+            if (ru == rv)
+                continue;
+            const unsigned long long wb = dbits(__dadd_rn(R.rel[u], R.rel[v]));
+            if (wb == __ldcg(R.bw + ru))
+                atomicMin(R.be + ru, le);
+            if (wb == __ldcg(R.bw + rv))
+                atomicMin(R.be + rv, le);
+        }
+        if (!grid_barrier(R.bar, target += gridDim.x, status))
+            return;
+        // hooks
+        for (uint32_t b = t0; b < nr; b += stride) {
+            const uint32_t k = b + threadIdx.x;
+            bool keep = false;
+            uint32_t rt = 0;
+            if (k < nr) {
+                rt = __ldcg(rin + k);
+                const uint32_t le = __ldcg(R.be + rt);
+                if (le == NONE32) {
+                    R.rw[rt] = pack(rt, 0);
+                } else {
+                    const uint32_t base = rt / (uint32_t)F.P * (uint32_t)F.P;
+                    uint32_t u, v;
+                    edge_ends(F, base, le, u, v);
+                    int32_t ou, ov;
+                    const uint32_t ru = resolve(R.word, u, ou, status), rv = resolve(R.word, v, ov, status);
+                    const bool u_in_r = ru == rt;
+                    const uint32_t s = u_in_r ? rv : ru;
+                    if (__ldcg(R.be + s) == le && rt < s) {
+                        R.rw[rt] = pack(rt, 0);
+                        keep = true;
+                    } else {
+                        const int e = -turn_exact(phi[u], phi[v]);
+                        R.rw[rt] = pack(s, u_in_r ? (e + ov - ou) : (-e + ou - ov));
+                        R.flags[r] = 1;
+                    }
+                }
+            }
+            const uint32_t slot = append_slot(R.rcnt + r, keep);
+            if (keep)
+                rout[slot] = rt;
+        }
+        if (!grid_barrier(R.bar, target += gridDim.x, status))
+            return;
+        if (__ldcg(R.flags + r) == 0)
+            return;
+        // pointer jumping among this round's roots
+        for (uint32_t k = t0 + threadIdx.x; k < nr; k += stride) {
+            const uint32_t rt = __ldcg(rin + k);
+            unsigned long long w = __ldcg(R.rw + rt);
+            for (int it = 0;; ++it) {
+                const uint32_t pp = par_of(w);
+                if (pp == rt)
+                    break;
+                const unsigned long long wp = __ldcg(R.rw + pp);
+                if (par_of(wp) == pp)
+                    break;
+                w = pack(par_of(wp), off_of(w) + off_of(wp));
+                __stcg(R.rw + rt, w);
+                if (it >= JUMP_LIMIT) {
+                    atomicOr(status, STATUS_JUMP);
+                    break;
+                }
+            }
+        }
+        if (!grid_barrier(R.bar, target += gridDim.x, status))
+            return;
+        // the roots take their new parent word; per-root minima reset
+        for (uint32_t k = t0 + threadIdx.x; k < nr; k += stride) {
+            const uint32_t rt = __ldcg(rin + k);
+            __stcg(R.word + rt, __ldcg(R.rw + rt));
+            R.bw[rt] = NONE64;
+            R.be[rt] = NONE32;
+        }
+        if (!grid_barrier(R.bar, target += gridDim.x, status))
+            return;
     }
 }
 
@@ -1080,26 +1170,28 @@ __global__ void __launch_bounds__(1024) k_uw_anchor(Frames F, const unsigned lon
 template <class T>
 __global__ void k_uw_finish(Frames F, T *phi, unsigned long long *word, const uint32_t *fe, uint32_t *status)
 {
-    const Px x = pixel(F);
-    if (!x.ok || !F.bad[x.a])
-        return;
-    const uint32_t p = x.p;
-    const int a = x.a;
-    int32_t op;
-    const uint32_t rp = resolve(word, p, op, status);
-    int32_t ka = 0;
-    if (fe[a] != NONE32) {
-        uint32_t u, v;
-        edge_ends(F, (uint32_t)a * (uint32_t)F.P, fe[a], u, v);
-        const uint32_t ra = resolve(word, u, ka, status);
-        if (ra != rp) {
-            atomicOr(status, STATUS_SPLIT);
-            return;
+    for (uint32_t z = blockIdx.z, nz = *F.nlist; z < nz; z += gridDim.z) {
+        const Px x = pixel(F, z);
+        if (!x.ok)
+            continue;
+        const uint32_t p = x.p;
+        const int a = x.a;
+        int32_t op;
+        const uint32_t rp = resolve(word, p, op, status);
+        int32_t ka = 0;
+        if (fe[a] != NONE32) {
+            uint32_t u, v;
+            edge_ends(F, (uint32_t)a * (uint32_t)F.P, fe[a], u, v);
+            const uint32_t ra = resolve(word, u, ka, status);
+            if (ra != rp) {
+                atomicOr(status, STATUS_SPLIT);
+                continue;
+            }
         }
+        const int32_t k = op - ka;
+        if (k != 0)
+            phi[p] = add_turns(phi[p], k);
     }
-    const int32_t k = op - ka;
-    if (k != 0)
-        phi[p] = (T)__dadd_rn((double)phi[p], __dmul_rn(TWOPI_D, (double)k));
 }
 
 // ---- align_unwrapped -------------------------------------------------------
@@ -1120,13 +1212,29 @@ __global__ void k_phase_min(const T *phi, long long n, unsigned long long *minke
 {
     unsigned long long m = NONE64;
     bool nan = false;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const double v = (double)phi[i];
-        if (v != v)
-            nan = true;
-        else
-            m = min(m, okey(v));
+    if constexpr (sizeof(T) == 4) {  // keys of the floats: no FP64 per sample (0.052 -> 0.021 ms for 200 x 256^2)
+        uint32_t k = NONE32;
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+             i += (long long)gridDim.x * blockDim.x) {
+            const float v = (float)phi[i];
+            const uint32_t b = __float_as_uint(v);
+            if (v != v)
+                nan = true;
+            else
+                k = min(k, (b >> 31) ? ~b : (b | 0x80000000u));
+        }
+        k = __reduce_min_sync(0xffffffffu, k);
+        if (k != NONE32)
+            m = okey((double)__uint_as_float((k >> 31) ? (k & 0x7fffffffu) : ~k));
+    } else {
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+             i += (long long)gridDim.x * blockDim.x) {
+            const double v = (double)phi[i];
+            if (v != v)
+                nan = true;
+            else
+                m = min(m, okey(v));
+        }
     }
     for (int o = 16; o > 0; o >>= 1)
         m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -1217,12 +1325,19 @@ __global__ void k_compose(const T *phi, const double *remove, long long per_angl
 {
     const long long a = blockIdx.y;
     const double rm = remove ? remove[a] : 0.0;
+    const bool shifted = __double_as_longlong(rm) != 0;  // (x - 0.0 is x, also for -0.0)
+    const float hi = (float)-rm, lo = (float)(-rm - (double)hi);
     for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < per_angle;
          k += (long long)gridDim.x * blockDim.x) {
         const long long i = a * per_angle + k;
         T ph = phi[i];
-        if (remove)
-            ph = (T)__dsub_rn((double)ph, rm);
+        if (shifted) {
+            float r;
+            if (sizeof(T) == 4 && add_pair((float)ph, hi, lo, r))
+                ph = (T)r;
+            else
+                ph = (T)__dsub_rn((double)ph, rm);
+        }
         if (!rytov) {
             outr[i] = ph;
             continue;
@@ -1238,8 +1353,8 @@ __global__ void k_compose(const T *phi, const double *remove, long long per_angl
 
 // ---------------------------------------------------------------------------
 struct Layout {
-    size_t phi, rel, word, rw, bw, be, fe, flags, status, minkey, nan, steps, remove, elist[2], rlist[2], cnt, bad, wmin,
-        kan, total;
+    size_t phi, rel, word, rw, bw, be, fe, flags, status, minkey, nan, steps, remove, elist[2], rlist[2], bad, wmin,
+        kan, list, total;
 };
 
 int num_rounds(long long P)
@@ -1271,22 +1386,23 @@ Layout layout_of(const odt_sino_desc &d)
     L.steps = take((size_t)5 * A * 8);
     L.remove = take((size_t)A * 8);
     if (three_d) {
-        L.flags = take((size_t)(num_rounds(P) + 1) * 4);
+        // zeroed together: flags, list counts (edges, roots) per round; barrier,
+        // number of listed frames; bad
+        L.flags = take((size_t)(num_rounds(P) + 1) * 12 + 8 + (size_t)A * 4);
         L.rel = take((size_t)N * 8);
         L.word = take((size_t)N * 8);
         L.rw = take((size_t)N * 8);
-        // also 16 bytes per 32 x 8 block of k_uf_first
-        L.bw = take(std::max<size_t>((size_t)N * 8, (size_t)A * ((d.ny + 7) / 8) * ((d.nx + 31) / 32) * 16));
+        // also 16 bytes per tile of k_uf_scan
+        L.bw = take(std::max<size_t>((size_t)N * 8, (size_t)A * uf_tiles(d.ny, d.nx) * 16));
         L.be = take((size_t)N * 4);
         L.fe = take((size_t)A * 4);
         for (int k = 0; k < 2; ++k) {
             L.elist[k] = take((size_t)N * 2 * 8);
             L.rlist[k] = take((size_t)N * 4);
         }
-        L.cnt = take(4 * 4);
-        L.bad = take((size_t)A * 4);
         L.wmin = take((size_t)A * 4);
         L.kan = take((size_t)A * 4);
+        L.list = take((size_t)A * 4);
     }
     L.total = o;
     return L;
@@ -1360,63 +1476,61 @@ odt_status run(const odt_sino_desc &d, const void *sino, void *out, char *ws, cu
     } else if (!three_d) {
         k_unwrap_rows<T><<<(unsigned)((A + 127) / 128), 128, 0, s>>>(phi, A, d.nx);
     } else {
-        uint32_t *bad = (uint32_t *)(ws + L.bad), *wmin = (uint32_t *)(ws + L.wmin);
-        Frames F{d.ny, d.nx, P, N, bad};
+        const int rounds = num_rounds(P), tiles = uf_tiles(d.ny, d.nx);
+        uint32_t *flags = (uint32_t *)(ws + L.flags), *ecnt = flags + rounds + 1, *rcnt = ecnt + rounds + 1;
+        uint32_t *bar = rcnt + rounds + 1, *nlist = bar + 1, *bad = nlist + 1;
+        uint32_t *wmin = (uint32_t *)(ws + L.wmin), *list = (uint32_t *)(ws + L.list);
+        Frames F{d.ny, d.nx, P, N, bad, list, nlist};
         double *rel = (double *)(ws + L.rel);
         unsigned long long *word = (unsigned long long *)(ws + L.word);
         unsigned long long *rw = (unsigned long long *)(ws + L.rw);
         unsigned long long *bw = (unsigned long long *)(ws + L.bw);
         uint32_t *be = (uint32_t *)(ws + L.be);
         uint32_t *fe = (uint32_t *)(ws + L.fe);
-        uint32_t *flags = (uint32_t *)(ws + L.flags);
-        const int rounds = num_rounds(P);
-        if (cudaMemsetAsync(flags, 0, (size_t)(rounds + 1) * 4, s) != cudaSuccess)
-            return launched("unwrap workspace reset");
-        const dim3 pg((unsigned)((d.nx + 31) / 32), (unsigned)((d.ny + 7) / 8), (unsigned)A), pb(32, 8);
         uint2 *el[2] = {(uint2 *)(ws + L.elist[0]), (uint2 *)(ws + L.elist[1])};
         uint32_t *rl[2] = {(uint32_t *)(ws + L.rlist[0]), (uint32_t *)(ws + L.rlist[1])};
-        uint32_t *ecnt = (uint32_t *)(ws + L.cnt), *rcnt = ecnt + 2;
-        if (cudaMemsetAsync(ecnt, 0, 16, s) != cudaSuccess)
-            return launched("unwrap workspace reset");
-        // frames without residues; steps, first edges and first columns in the
-        // places of rel, bw and rw, which the tree needs only afterwards
-        if (cudaMemsetAsync(bad, 0, (size_t)A * 4, s) != cudaSuccess ||
+        if (cudaMemsetAsync(flags, 0, (size_t)(rounds + 1) * 12 + 8 + (size_t)A * 4, s) != cudaSuccess ||
             cudaMemsetAsync(wmin, 0xff, (size_t)A * 4, s) != cudaSuccess)
             return launched("unwrap workspace reset");
+        // frames without residues; steps, first edges, first columns and tile
+        // minima in the places of rel, bw, rw and be, which the tree needs
+        // only afterwards
         uint8_t *steps = (uint8_t *)rel;
         int32_t *col = (int32_t *)rw, *kan = (int32_t *)(ws + L.kan);
         ulonglong2 *first = (ulonglong2 *)bw;
-        k_uf_scan<T><<<pg, pb, 0, s>>>(phi, F, d.seed, steps, bad, wmin);
-        k_uf_first<T><<<pg, pb, 0, s>>>(phi, F, d.seed, bad, wmin, first);
-        k_uf_frame<<<(unsigned)A, 256, 0, s>>>(F, steps, bad, first, (int)(pg.x * pg.y), col, kan);
+        float *tmin = (float *)be;
+        const dim3 tg((unsigned)((tiles + 7) / 8), (unsigned)A);
+        k_uf_scan<T, false><<<tg, 256, 0, s>>>(phi, F, d.seed, tiles, steps, bad, wmin, tmin, nullptr);
+        k_uf_scan<T, true><<<tg, 256, 0, s>>>(phi, F, d.seed, tiles, nullptr, bad, wmin, tmin, first);
+        k_uf_frame<<<(unsigned)A, 256, 0, s>>>(F, steps, bad, first, tiles, col, kan, list, nlist);
         k_uf_apply<T><<<dim3((unsigned)((d.ny + 7) / 8), (unsigned)A), 256, 0, s>>>(phi, F, steps, bad, col, kan);
+        // the other frames
+        const unsigned gx = (unsigned)((d.nx + 31) / 32), gy = (unsigned)((d.ny + 7) / 8);
+        const unsigned gz = (unsigned)std::min<long long>(A, std::max<long long>(1, 152ll * 16 / ((long long)gx * gy)));
+        const dim3 pg(gx, gy, gz), pb(32, 8);
         k_uw_init<T><<<pg, pb, 0, s>>>(phi, F, d.seed, rel, word, bw, be);
         // rounds 0 and 1 over the pixel grid; round 1 also lists the edges
         // that cross components and the roots that stay
         for (int r = 0; r < std::min(rounds, 2); ++r) {
-            k_uw_minw<<<pg, pb, 0, s>>>(F, rel, word, bw, flags, r, r == 1 ? el[0] : nullptr, ecnt);
+            k_uw_minw<<<pg, pb, 0, s>>>(F, rel, word, bw, flags, r, r == 1 ? el[0] : nullptr, ecnt + 1);
             k_uw_mine<<<pg, pb, 0, s>>>(F, rel, word, bw, be, flags, r);
             if (r == 0)
                 k_uw_anchor<<<(unsigned)A, 1024, 0, s>>>(F, bw, be, fe);
-            k_uw_hook<T><<<pg, pb, 0, s>>>(F, phi, word, be, rw, flags, r, r == 1 ? rl[0] : nullptr, rcnt);
+            k_uw_hook<T><<<pg, pb, 0, s>>>(F, phi, word, be, rw, flags, r, r == 1 ? rl[0] : nullptr, rcnt + 1);
             k_uw_jump<<<pg, pb, 0, s>>>(F, word, rw, flags, r, status);
             k_uw_flatten<<<pg, pb, 0, s>>>(F, word, rw, bw, be, flags, r);
         }
-        // rounds >= 2 on the lists, in and out alternating (round 2 reads
-        // the lists round 1 wrote into slot 0)
-        for (int r = 2; r < rounds; ++r) {
-            const int in = r & 1 ? 1 : 0, out = in ^ 1;
-            if (cudaMemsetAsync(ecnt + out, 0, 4, s) != cudaSuccess ||
-                cudaMemsetAsync(rcnt + out, 0, 4, s) != cudaSuccess)
-                return launched("unwrap list reset");
-            k_ul_edges_w<<<UL_GRID, UL_BLOCK, 0, s>>>(rel, word, bw, el[in], ecnt + in, el[out], ecnt + out, d.nx,
-                                                      flags, r, status);
-            k_ul_edges_e<<<UL_GRID, UL_BLOCK, 0, s>>>(rel, word, bw, be, el[out], ecnt + out, d.nx, flags, r,
-                                                      status);
-            k_ul_hook<T><<<UL_GRID, UL_BLOCK, 0, s>>>(F, phi, word, be, rw, rl[in], rcnt + in, rl[out], rcnt + out,
-                                                      flags, r, status);
-            k_ul_jump<<<UL_GRID, UL_BLOCK, 0, s>>>(rw, rl[in], rcnt + in, flags, r, status);
-            k_ul_update<<<UL_GRID, UL_BLOCK, 0, s>>>(word, rw, bw, be, rl[in], rcnt + in, flags, r);
+        if (rounds > 2) {
+            ListRounds R{rel, word, rw, bw, be, {el[0], el[1]}, {rl[0], rl[1]}, ecnt, rcnt, flags, bar, status, rounds};
+            int dev = 0, sms = 0, occ = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ul_rounds<T>, UL_BLOCK, 0) != cudaSuccess)
+                return launched("unwrap occupancy");
+            void *args[] = {(void *)&F, (void *)&phi, (void *)&R};
+            if (cudaLaunchCooperativeKernel((const void *)k_ul_rounds<T>, dim3((unsigned)(sms * std::max(occ, 1))),
+                                            dim3(UL_BLOCK), args, 0, s) != cudaSuccess)
+                return launched("unwrap rounds");
         }
         k_uw_finish<T><<<pg, pb, 0, s>>>(F, phi, word, fe, status);
     }
@@ -1442,7 +1556,11 @@ int launches_of(const odt_sino_desc &d)
         return 3;  // min, align, compose
     int n = (d.kind == ODT_SINO_UNWRAP ? 1 : 2) + (d.align ? 2 : 0);  // (phase,) compose (+ min, align)
     if (d.ny > 0)
-        n += 7 + 5 * num_rounds((long long)d.ny * d.nx);  // residue-free frames (4), init, anchor, rounds, finish
+    {
+        // residue-free frames (4), init, anchor, two rounds, the others, finish
+        const int rounds = num_rounds((long long)d.ny * d.nx);
+        n += 7 + 5 * (rounds < 2 ? rounds : 2) + (rounds > 2 ? 1 : 0);
+    }
     else
         n += 1;
     return n;
@@ -1512,6 +1630,8 @@ odt_status odt_sino_read_status(const void *workspace, void *stream)
         return (odt_status)set_error(ODT_ERR_DEVICE_CHECK, "phase unwrap: pointer jumping exceeded its step limit");
     if (v & STATUS_SPLIT)
         return (odt_status)set_error(ODT_ERR_DEVICE_CHECK, "phase unwrap: a frame did not join into one tree");
+    if (v & STATUS_BARRIER)
+        return (odt_status)set_error(ODT_ERR_DEVICE_CHECK, "phase unwrap: a grid barrier exceeded its time limit");
     return ODT_OK;
 }
 

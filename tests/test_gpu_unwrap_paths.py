@@ -59,3 +59,27 @@ def test_nan_frame_leaves_the_others(cuda_ready):
     for a in (1, 2, 4, 5):
         assert np.array_equal(got[a], clean[a])
     assert np.array_equal(np.isnan(got), np.isnan(v))
+
+
+@pytest.mark.parametrize("low", [-13.0, -40.0, 21.0, -0.5])
+def test_alignment_shift_rounds_like_fp64(cuda_ready, low):
+    """float32 phases minus the FP64 shift, through FP32 pairs: the same
+    rounding as the FP64 difference, zeros and cancelling sums included.
+    Equal angles have no steps between them, so the shift is the minimum's
+    whole turns, a float32 product."""
+    from odtbrain_gb300 import _prepare_sino as ps
+    rng = np.random.default_rng(11)
+    base = (low + rng.gamma(2, 3, size=(40, 33))).astype(np.float32)
+    turn = np.float32(2 * np.pi)
+    base[0, :8] = [max(low, 0), 1e-30, turn, -turn, -3 * turn, 1e8, 0.5, 30]
+    base[1] = np.float32(low)
+    base[2] = np.linspace(0, 1e-6, 33)
+    base = np.maximum(base, np.float32(low))
+    w = np.repeat(base[None], 5, axis=0)
+    got = w.copy()
+    ps.align_unwrapped(got)
+    q = np.float32(np.round(np.median(w - got) / (2 * np.pi)))
+    ref = (w.astype(np.float64) - np.float64(q * turn)).astype(np.float32)
+    assert abs(q) >= (low < -1 or low > 7)
+    assert np.array_equal(got, ref)
+    assert np.array_equal(np.signbit(got), np.signbit(ref))
