@@ -7,13 +7,13 @@
 // 3D FFTs (single precision, unnormalised, like the reference's pyFFTW
 // plans) are line transforms in registers (odt_fft.cuh), one kernel per
 // axis.  One iteration of the reference's loop is five kernels:
-//   k_apple_s (axis 1, forward)
-//   k_apple_s (axis 0, forward; then per voxel: envelope suppression,
+//   k_apple_s1 (axis 1, forward)
+//   k_apple_s0 (axis 0, forward; then per voxel: envelope suppression,
 //              DC update (method "sh"), restore of the non-core spectrum,
 //              sum of |spectrum| over the core; then axis 0 inverse)
 //   k_apple_dec  stopping criterion, one thread, in float32 like the
 //              reference's NumPy scalars
-//   k_apple_s (axis 1, inverse)
+//   k_apple_s1 (axis 1, inverse)
 //   k_apple_x (axis 2 inverse, times fl32(1/N) -> result; for "nn" and a
 //              following iteration also the constraint and the axis 2
 //              forward transform of the next iteration)
@@ -139,11 +139,14 @@ __device__ __forceinline__ float2 constrain(const AP &P, float2 d, uint8_t fl, f
 // ---- axis 2 (contiguous lines) --------------------------------------------
 // mode 0: f.real -> forward -> buf (the original spectrum's first axis)
 // mode 1: constrain(f.real) -> forward -> buf (iteration 0's first axis)
-// mode 2: buf -> inverse -> * scale -> data; for "nn" with a following
-//         iteration: constrain -> forward -> buf
+// mode 2: buf -> inverse -> * scale; with a following iteration (not "sh"):
+//         constrain -> forward -> buf, else -> data (k_apple_dec has decided;
+//         data written by every iteration and the flags read after the
+//         transform: 0.078 ms at 256^3, like this 0.07, 0.042 at the copy rate)
 // mode 3: constrain(data) -> forward -> buf (method "sh")
 template <class L, int LPC>
-__global__ void __launch_bounds__(LPC *L::TPL) k_apple_x(AP P, L line, int mode, int it)
+__global__ void __launch_bounds__(LPC *L::TPL, LPC *L::TPL <= 256 ? 5 : 1)
+    k_apple_x(AP P, L line, int mode, int it, int groups)
 {
     if (mode >= 2 && ran_out(P, it))
         return;
@@ -153,9 +156,6 @@ __global__ void __launch_bounds__(LPC *L::TPL) k_apple_x(AP P, L line, int mode,
     float2 *buf0 = smem, *buf1 = smem + LPC * ls, *tw = smem + 2 * LPC * ls;
     copy_twiddles<L>(tw, P.tw2, n);
     const int l = threadIdx.x / L::TPL, j = threadIdx.x % L::TPL;
-    const long long lid = (long long)blockIdx.x * LPC + l;
-    const bool valid = lid < (long long)P.n0 * P.n1;
-    const long long base = valid ? lid * n : 0;
     float fmin = 0.f, fmax = 0.f, lo = 0.f, hi = 0.f;
     if (P.method == 1) {
         fmin = P.ctl->fmin;
@@ -163,143 +163,225 @@ __global__ void __launch_bounds__(LPC *L::TPL) k_apple_x(AP P, L line, int mode,
         lo = P.ctl->lo;
         hi = P.ctl->hi;
     }
-    float2 v[L::SLOTS];
-#pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int x = j + r * L::TPL;
-        float2 a = make_float2(0.f, 0.f);
-        if (valid && x < n) {
-            if (mode <= 1)
-                a = make_float2(P.freal[base + x], 0.f);
-            else if (mode == 2)
-                a = P.buf[base + x];
-            else
-                a = P.data[base + x];
-            if (mode == 1 || mode == 3)
-                a = constrain(P, a, P.flags[base + x], fmin, fmax, lo, hi);
-        }
-        v[r] = a;
-    }
-    __syncthreads();
-    int flip = 0;
-    if (mode == 2) {
-        line.template run<1>(v, j, buf0 + l * ls, buf1 + l * ls, 1, tw, flip);
-        const bool next = P.method != 1 && it + 1 < P.max_iter && !ran_out(P, it + 1);
+    // (of mode 2; uniform over the grid)
+    const bool next = P.method != 1 && it + 1 < P.max_iter && !ran_out(P, it + 1);
+    for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+        const long long lid = (long long)g * LPC + l;
+        const bool valid = lid < (long long)P.n0 * P.n1;
+        const long long base = valid ? lid * n : 0;
+        float2 v[L::SLOTS];
+        uint8_t fl[L::SLOTS];  // read ahead of the transform
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
             const int x = j + r * L::TPL;
-            v[r] = make_float2(__fmul_rn(v[r].x, P.scale), __fmul_rn(v[r].y, P.scale));
+            fl[r] = (valid && x < n && mode != 0 && (mode != 2 || next)) ? P.flags[base + x] : (uint8_t)0;
+            float2 a = make_float2(0.f, 0.f);
             if (valid && x < n) {
-                P.data[base + x] = v[r];
-                if (next)
-                    v[r] = constrain(P, v[r], P.flags[base + x], 0.f, 0.f, 0.f, 0.f);
+                if (mode <= 1)
+                    a = make_float2(P.freal[base + x], 0.f);
+                else if (mode == 2)
+                    a = P.buf[base + x];
+                else
+                    a = P.data[base + x];
+                if (mode == 1 || mode == 3)
+                    a = constrain(P, a, fl[r], fmin, fmax, lo, hi);
             }
+            v[r] = a;
         }
-        if (!next)
-            return;  // uniform over the CTA
         __syncthreads();
-    }
-    line.template run<-1>(v, j, buf0 + l * ls, buf1 + l * ls, 1, tw, flip);
-    if (!valid)
-        return;
+        int flip = 0;
+        if (mode == 2) {
+            line.template run<1>(v, j, buf0 + l * ls, buf1 + l * ls, 1, tw, flip);
 #pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int x = j + r * L::TPL;
-        if (x < n)
-            P.buf[base + x] = v[r];
+            for (int r = 0; r < L::SLOTS; ++r) {
+                const int x = j + r * L::TPL;
+                v[r] = make_float2(__fmul_rn(v[r].x, P.scale), __fmul_rn(v[r].y, P.scale));
+                if (valid && x < n) {
+                    if (next)
+                        v[r] = constrain(P, v[r], fl[r], 0.f, 0.f, 0.f, 0.f);
+                    else
+                        P.data[base + x] = v[r];
+                }
+            }
+            if (!next)
+                continue;  // uniform over the CTA
+            __syncthreads();
+        }
+        line.template run<-1>(v, j, buf0 + l * ls, buf1 + l * ls, 1, tw, flip);
+        if (!valid)
+            continue;
+#pragma unroll
+        for (int r = 0; r < L::SLOTS; ++r) {
+            const int x = j + r * L::TPL;
+            if (x < n)
+                P.buf[base + x] = v[r];
+        }
     }
 }
 
-// ---- axes 1 and 0 (strided lines, KX adjacent lines per CTA) --------------
-// mode 0: forward (axis 1) ; mode 1: inverse (axis 1)
-// mode 2: axis 0 forward -> orig (the original spectrum) + core sum
-// mode 3: axis 0 forward -> frequency-domain step -> inverse (iteration)
+// ---- axes 1 and 0 (strided lines, KX adjacent lines per group) ------------
+// As many CTAs as are resident stride over the groups, so the twiddle table
+// is filled once per CTA and neighbouring groups, which share 128-byte lines,
+// are in flight together.  (256^3, all 25 iterations: 4 CTAs per SM on axis 1
+// and 3 on axis 0 8.4 ms; 5 on axis 1 9.2, 3 8.6, 2 9.0; 4 on axis 0 9.1,
+// 2 9.0; the next group's loads ahead of the transforms 8.5 on axis 1 and 8.9
+// on axis 0; groups of 4 or 16 columns 9.6, 9.2.)
+// axis 1, forward or inverse (256^3: one
+// group per CTA 0.080 ms, like this 0.048)
 template <class L, int KX>
-__global__ void __launch_bounds__(KX *L::TPL) k_apple_s(AP P, L line, int axis, int mode, int it)
+__global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 4 : KX *L::TPL <= 512 ? 2 : 1)
+    k_apple_s1(AP P, L line, int inverse, int it, int groups)
 {
-    if (mode != 2 && ran_out(P, it))
+    if (ran_out(P, it))
+        return;
+    extern __shared__ float2 smem[];
+    const int n = line.size();
+    const int ls = xslots<true>(n);
+    float2 *buf0 = smem, *buf1 = smem + KX * ls, *tw = smem + 2 * KX * ls;
+    copy_twiddles<L>(tw, P.tw1, n);
+    const int c = threadIdx.x % KX, j = threadIdx.x / KX, stride = P.n2;
+    const int gpo = (P.n2 + KX - 1) / KX;
+    auto column = [&](int g) -> float2 * {  // NULL past the last column
+        const int o = g / gpo, q = (g - o * gpo) * KX + c;
+        return q < P.n2 ? P.buf + (long long)o * P.n1 * P.n2 + q : nullptr;
+    };
+    auto load = [&](const float2 *col, float2 (&v)[L::SLOTS]) {
+#pragma unroll
+        for (int r = 0; r < L::SLOTS; ++r) {
+            const int k = j + r * L::TPL;
+            v[r] = (col && k < n) ? col[(long long)k * stride] : make_float2(0.f, 0.f);
+        }
+    };
+    float2 v[L::SLOTS];
+    float2 *col = column(blockIdx.x);
+    load(col, v);
+    __syncthreads();
+    int flip = 0;
+    for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+        if (inverse)
+            line.template run<1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
+        else
+            line.template run<-1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
+        if (col) {
+#pragma unroll
+            for (int r = 0; r < L::SLOTS; ++r) {
+                const int k = j + r * L::TPL;
+                if (k < n)
+                    col[(long long)k * stride] = v[r];
+            }
+        }
+        if (g + (int)gridDim.x < groups) {
+            col = column(g + gridDim.x);
+            load(col, v);
+        }
+        __syncthreads();  // the exchange buffers are the next group's
+    }
+}
+
+// axis 0: forward; original: -> orig and the core sum (the original
+// spectrum), else the frequency-domain step and back.  The step's operands are
+// read ahead of the transform, and only the one that the voxel's flag asks for
+// (256^3: one group per CTA and all operands after the transform 0.126 ms,
+// like this 0.100).
+template <class L, int KX>
+__global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 3 : KX *L::TPL <= 512 ? 2 : 1)
+    k_apple_s0(AP P, L line, int original, int it, int groups)
+{
+    if (!original && ran_out(P, it))
         return;
     extern __shared__ float2 smem[];
     __shared__ double red[32];
     const int n = line.size();
     const int ls = xslots<true>(n);
     float2 *buf0 = smem, *buf1 = smem + KX * ls, *tw = smem + 2 * KX * ls;
-    copy_twiddles<L>(tw, axis == 0 ? P.tw0 : P.tw1, n);
-    const long long inner = axis == 0 ? (long long)P.n1 * P.n2 : P.n2;
-    const long long stride = inner;
-    const long long ostride = (long long)P.n1 * P.n2;
-    const unsigned gpo = (unsigned)((inner + KX - 1) / KX);
-    const long long o = blockIdx.x / gpo;
-    const long long q0 = (long long)(blockIdx.x - (unsigned)o * gpo) * KX;
+    copy_twiddles<L>(tw, P.tw0, n);
     const int c = threadIdx.x % KX, j = threadIdx.x / KX;
-    const long long q = q0 + c;
-    const bool colok = q < inner;
-    const long long base = (axis == 0 ? 0 : o * ostride) + (colok ? q : 0);
-    float2 v[L::SLOTS];
-#pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int k = j + r * L::TPL;
-        v[r] = (colok && k < n) ? P.buf[base + k * stride] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    int flip = 0;
-    if (mode == 1)
-        line.template run<1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
-    else
-        line.template run<-1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
-    double part = 0.0;
-    if (mode >= 2) {
+    const long long stride = (long long)P.n1 * P.n2;
+    auto load = [&](long long q, float2 (&v)[L::SLOTS], uint8_t (&fl)[L::SLOTS]) {
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
             const int k = j + r * L::TPL;
-            if (!(colok && k < n))
-                continue;
-            const long long vox = base + k * stride;
-            const uint8_t fl = P.flags[vox];
-            float2 ft = v[r];
-            if (mode == 2) {
-                P.orig[vox] = ft;
-            } else {
-                if (P.evlp && hypotf(ft.x, ft.y) > P.evlp[vox])
-                    ft = make_float2(__fmul_rn(ft.x, P.ee), __fmul_rn(ft.y, P.ee));
-                if (!(fl & F_CORE)) {
-                    float2 og = P.orig[vox];
-                    if (P.method == 1 && vox == 0) {  // (orig + ft) / 2 at the DC term
-                        og = make_float2(__fmul_rn(__fadd_rn(og.x, ft.x), 0.5f),
-                                         __fmul_rn(__fadd_rn(og.y, ft.y), 0.5f));
-                        P.orig[0] = og;
-                    }
-                    ft = og;
-                }
+            const bool in = q < stride && k < n;
+            v[r] = in ? P.buf[q + k * stride] : make_float2(0.f, 0.f);
+            fl[r] = in ? P.flags[q + k * stride] : (uint8_t)0;
+        }
+    };
+    float2 v[L::SLOTS];
+    uint8_t fl[L::SLOTS];
+    long long q = (long long)blockIdx.x * KX + c;
+    load(q, v, fl);
+    __syncthreads();
+    int flip = 0;
+    double part = 0.0;
+    for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+        float2 og[L::SLOTS];
+        float ev[L::SLOTS];
+        if (!original) {
+#pragma unroll
+            for (int r = 0; r < L::SLOTS; ++r) {
+                const int k = j + r * L::TPL;
+                const bool in = q < stride && k < n;
+                og[r] = (in && !(fl[r] & F_CORE)) ? P.orig[q + k * stride] : make_float2(0.f, 0.f);
+                ev[r] = (in && (fl[r] & F_CORE) && P.evlp) ? P.evlp[q + k * stride] : 0.f;
             }
-            if (fl & F_CORE)
-                part += (double)hypotf(ft.x, ft.y);
+        }
+        line.template run<-1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
+#pragma unroll
+        for (int r = 0; r < L::SLOTS; ++r) {
+            const int k = j + r * L::TPL;
+            if (!(q < stride && k < n))
+                continue;
+            const long long vox = q + k * stride;
+            float2 ft = v[r];
+            if (original) {
+                P.orig[vox] = ft;
+                if (fl[r] & F_CORE)
+                    part += (double)hypotf(ft.x, ft.y);
+            } else if (fl[r] & F_CORE) {
+                float h = hypotf(ft.x, ft.y);
+                if (P.evlp && h > ev[r]) {
+                    ft = make_float2(__fmul_rn(ft.x, P.ee), __fmul_rn(ft.y, P.ee));
+                    h = hypotf(ft.x, ft.y);
+                }
+                part += (double)h;
+            } else {
+                if (P.method == 1 && vox == 0) {  // (orig + ft) / 2 at the DC term
+                    if (P.evlp && hypotf(ft.x, ft.y) > P.evlp[0])
+                        ft = make_float2(__fmul_rn(ft.x, P.ee), __fmul_rn(ft.y, P.ee));
+                    og[r] = make_float2(__fmul_rn(__fadd_rn(og[r].x, ft.x), 0.5f),
+                                        __fmul_rn(__fadd_rn(og[r].y, ft.y), 0.5f));
+                    P.orig[0] = og[r];
+                }
+                ft = og[r];
+            }
             v[r] = ft;
         }
-        // block sum of the core magnitudes
-        for (int s = 16; s > 0; s >>= 1)
-            part += __shfl_xor_sync(0xffffffffu, part, s);
-        if ((threadIdx.x & 31) == 0)
-            red[threadIdx.x >> 5] = part;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
-                t += red[w];
-            atomicAdd(P.state + (mode == 2 ? 0 : it + 1), t);
-        }
-        if (mode == 2)
-            return;
-        __syncthreads();
-        line.template run<1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
-    }
-    if (!colok)
-        return;
+        if (!original) {
+            line.template run<1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
 #pragma unroll
-    for (int r = 0; r < L::SLOTS; ++r) {
-        const int k = j + r * L::TPL;
-        if (k < n)
-            P.buf[base + k * stride] = v[r];
+            for (int r = 0; r < L::SLOTS; ++r) {
+                const int k = j + r * L::TPL;
+                if (q < stride && k < n)
+                    P.buf[q + k * stride] = v[r];
+            }
+            __syncthreads();  // the exchange buffers are the next group's
+        }
+        q += (long long)gridDim.x * KX;
+        if (g + (int)gridDim.x < groups)
+            load(q, v, fl);
+    }
+    // sum of the core magnitudes
+    for (int s = 16; s > 0; s >>= 1)
+        part += __shfl_xor_sync(0xffffffffu, part, s);
+    if ((threadIdx.x & 31) == 0)
+        red[threadIdx.x >> 5] = part;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w)
+            t += red[w];
+        atomicAdd(P.state + (original ? 0 : it + 1), t);
     }
 }
 
@@ -1121,12 +1203,20 @@ cudaError_t launch_x(const AP &P, int mode, int it, cudaStream_t s)
         constexpr int LPC = Cfg<L>::LPC;
         const size_t sm = smem_x<L>(P.n2);
         cudaFuncSetAttribute(k_apple_x<L, LPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        const long long lines = (long long)P.n0 * P.n1;
-        k_apple_x<L, LPC><<<(unsigned)((lines + LPC - 1) / LPC), LPC * L::TPL, sm, s>>>(P, line, mode, it);
+        const int groups = (int)(((long long)P.n0 * P.n1 + LPC - 1) / LPC);
+        int dev = 0, sms = 0, occ = 0;
+        cudaError_t e;
+        if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
+            (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_apple_x<L, LPC>, LPC * L::TPL, sm)))
+            return e;
+        const int grid = std::min(groups, sms * std::max(occ, 1));
+        k_apple_x<L, LPC><<<(unsigned)grid, LPC * L::TPL, sm, s>>>(P, line, mode, it, groups);
         return cudaGetLastError();
     });
 }
 
+// mode 0: axis 1 forward, 1: axis 1 inverse, 2: axis 0 forward -> orig (the
+// original spectrum) + core sum, 3: axis 0 of an iteration
 cudaError_t launch_s(const AP &P, int axis, int mode, int it, cudaStream_t s)
 {
     const int n = axis == 0 ? P.n0 : P.n1;
@@ -1134,11 +1224,17 @@ cudaError_t launch_s(const AP &P, int axis, int mode, int it, cudaStream_t s)
         using L = decltype(line);
         constexpr int KX = Cfg<L>::KX;
         const size_t sm = smem_s<L>(n);
-        cudaFuncSetAttribute(k_apple_s<L, KX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        int dev = 0, sms = 0, occ = 0;
+        cudaError_t e;
+        const auto kernel = axis == 0 ? k_apple_s0<L, KX> : k_apple_s1<L, KX>;
         const long long inner = axis == 0 ? (long long)P.n1 * P.n2 : P.n2;
-        const long long outer = axis == 0 ? 1 : P.n0;
-        const long long grid = outer * ((inner + KX - 1) / KX);
-        k_apple_s<L, KX><<<(unsigned)grid, KX * L::TPL, sm, s>>>(P, line, axis, mode, it);
+        const long long groups = (axis == 0 ? 1 : P.n0) * ((inner + KX - 1) / KX);
+        if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) ||
+            (e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
+            (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, KX * L::TPL, sm)))
+            return e;
+        const long long grid = std::min<long long>(groups, (long long)sms * std::max(occ, 1));
+        kernel<<<(unsigned)grid, KX * L::TPL, sm, s>>>(P, line, axis == 0 ? mode == 2 : mode == 1, it, (int)groups);
         return cudaGetLastError();
     });
 }
