@@ -83,3 +83,30 @@ def test_alignment_shift_rounds_like_fp64(cuda_ready, low):
     assert abs(q) >= (low < -1 or low > 7)
     assert np.array_equal(got, ref)
     assert np.array_equal(np.signbit(got), np.signbit(ref))
+
+
+def test_capture_and_replay(cuda_ready):
+    """The whole preparation in a CUDA graph, replayed on other data (frames
+    with residues where the captured ones had none)."""
+    import torch
+    from odtbrain_gb300 import _prepare_sino as ps
+    rng = np.random.default_rng(21)
+    field = [torch.tensor(np.exp(1j * np.array(
+        [_frames(k, 40, 70, rng) for k in kinds])), device="cuda")
+        for kinds in (("smooth",) * 4, ("noise", "smooth", "noise", "noise"))]
+    run = ps.SinogramPrep((4, 40, 70), kind="rytov", single=False)
+    want = [run(f).clone() for f in field]
+    static, out = field[0].clone(), torch.empty_like(field[0])
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        run(static, out=out, check=False)
+    torch.cuda.current_stream().wait_stream(stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(static, out=out, check=False)
+    for f, ref in ((field[1], want[1]), (field[0], want[0])):
+        static.copy_(f)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
