@@ -33,3 +33,20 @@ def test_lines_in_turn(cuda_ready, shape, kw):
     scale = np.abs(ref).max()
     tol = max(2e-5, 4 * np.abs(other - ref).max() / scale)
     assert np.abs(got - ref).max() <= tol * scale
+
+
+@pytest.mark.parametrize("scale", [1e-30, 1e-18, 1.0, 1e18, 1e30])
+def test_envelope_over_the_float_range(cuda_ready, scale):
+    """The envelope's Gaussian sums in float pairs hand over to FP64 where the
+    pairs are not exact: magnitudes near both ends of float32."""
+    import odtbrain_gb300 as odt
+    rng = np.random.default_rng(3)
+    shape = (36, 40, 36)
+    ft = ((rng.standard_normal(shape) + 1j * rng.standard_normal(shape))
+          * np.exp(rng.uniform(-3, 3, shape)) * scale).astype(np.complex64)
+    core = odt.apple.apple_core_3d(shape, 3.0, 1.333)
+    ref = ao.envelope_gauss(ft.copy(), core)
+    got = np.asarray(odt.apple.envelope_gauss(ft.copy(), core))
+    assert np.isfinite(ref).all() and ref.max() > 0
+    # one rounding of the magnitudes and of each axis's float32 result
+    assert np.abs(got - ref).max() <= 2e-6 * ref.max()
