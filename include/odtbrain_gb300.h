@@ -207,8 +207,10 @@ odt_status odt_bpp3d_launch_count(const odt_bpp3d_plan *plan,
  * The caller pairs only views whose in/out decisions agree: for every output
  * (z, x), inside the domain for the second view exactly where the first
  * view's coordinates are inside it.
- * ODT_ERR_UNSUPPORTED for plans about a tilted axis, filter or kz_phase tables
- * that are not even in kx, and workspace limits too small for one unit. */
+ * ODT_ERR_UNSUPPORTED for plans about a tilted axis, spline order 0 (the
+ * nearest sample is a decision of every view's own: coordinates c and n-1-c
+ * round halves to different samples), filter or kz_phase tables that are not
+ * even in kx, and workspace limits too small for one unit. */
 typedef struct odt_bpp3d_units {
     int32_t num_units;
     int32_t reserved;

@@ -96,7 +96,8 @@ def opposite_units(geometry, n):
     FP64 coordinates with 0 and n-1; c and n-1-c agree to about 1e-13, so
     views are paired when no output's coordinate lies within 1e-9 of the
     boundary, or when both matrices' entries are 0 or +-1 and the coordinates
-    therefore exact.
+    therefore exact.  This is for interpolation that is continuous in the
+    coordinate (spline orders 1 and up); plans of order 0 refuse units.
     """
     geometry = np.asarray(geometry)
     A = geometry.shape[0]

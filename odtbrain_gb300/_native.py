@@ -384,7 +384,7 @@ class Plan:
     def pair_workspace_bytes(self, num_units):
         """(workspace, adjoint workspace) bytes of an execution over
         `num_units` units of opposite views, or None if the plan cannot pair
-        views (its tables, or a workspace limit too small)."""
+        views (its tables, spline order 0, or a workspace limit too small)."""
         ws, adj = ctypes.c_uint64(), ctypes.c_uint64()
         st = lib().odt_bpp3d_pair_workspace_size(
             self._h, int(num_units), ctypes.byref(ws), ctypes.byref(adj))
