@@ -298,6 +298,10 @@ StageParams stage_params(const odt_bpp3d_plan *p)
     return P;
 }
 
+// Spectrum slots per batch: the spectrum, boundary and padding kernels have them
+// on a grid's y or z extent.
+constexpr int kMaxSlots = 65535;
+
 // The largest batch of slabs (and column-stage chunk) whose workspace fits
 // the plan's limit; one slab per batch with a shrunken chunk where none does.
 Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
@@ -351,8 +355,9 @@ Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
         size_t jobs = std::min((size_t)batch * nz, jobs_cap);
         return jobs >= 16 ? jobs / 16 * 16 : jobs;
     };
+    const int most = std::min(units, kMaxSlots / spu);
     int best = 0;
-    for (int lo = 1, hi = units; lo <= hi;) {  // ws grows with the batch
+    for (int lo = 1, hi = most; lo <= hi;) {  // ws grows with the batch
         const int mid = lo + (hi - lo) / 2;
         if (layout(mid, jobs_for(mid)).ws_bytes <= limit) {
             best = mid;
@@ -363,7 +368,7 @@ Layout make_layout(const odt_bpp3d_plan *p, int units, int spu)
     }
     // a single batch needs no compensation buffer, so it can fit when a
     // slightly smaller batch does not
-    if (best < units && layout(units, jobs_for(units)).ws_bytes <= limit)
+    if (best < units && most == units && layout(units, jobs_for(units)).ws_bytes <= limit)
         best = units;
     if (best > 0)
         return layout(best, jobs_for(best));
