@@ -750,36 +750,41 @@ __device__ __forceinline__ double gauss_sum(const double *x, int st, const doubl
 // float32 data: the FP64 sum rounded to float32 is what scipy stores.  FP64
 // runs at 1/64 of the FP32 rate here, so the sum is carried as an unevaluated
 // pair of floats (error-free sums after Knuth, products with FMA; the weights
-// split into two floats): all terms are non-negative, so its relative error
-// stays below 2^-44 and the rounded result is the FP64 one's except for
-// values that close to a rounding boundary.  Sums outside the range where the
-// products are exact (or not finite) are formed again in FP64.
-__device__ __forceinline__ float gauss_sum(const float *x, int st, const float2 *ws, const double *w, int r)
+// split into two floats).  With S the sum, all terms non-negative and t_j a
+// term, in units of 2^-48: a term's low part is off by 7 t_j (weight 1, two FMAs
+// 5, dropped product 1); the low part lo is below 2^-24 (k + 3) S after k terms,
+// so adding term k to it is off by (k + 4) S + 3 t_k; the last sum adds (r + 5)
+// S, and the FP64 sum's own error is below S for r <= 29, 2.2 S at 64.  Together
+// r^2 / 2 + 6.5 r + 24 at most: (r + 8)^2 covers it.  Where both ends of that
+// interval round alike, the result is the FP64 one; else (about one sum in 2^15
+// at r = 10), and outside the range where the products are exact, FP64 decides.
+__device__ __forceinline__ float gauss_sum(const float *x, int st, const float2 *ws, const double *w, int r,
+                                           bool exact)
 {
-    float2 wj = ws[0];
-    float hi = x[0] * wj.x, lo = fmaf(x[0], wj.x, -hi) + x[0] * wj.y;
-    const float c0h = hi, c0l = lo;
-    hi = lo = 0.f;
-    auto add = [&](float ph, float pl) {
-        const float t = hi + ph, z = t - hi;
-        lo += ((hi - (t - z)) + (ph - z)) + pl;
-        hi = t;
-    };
-    add(c0h, c0l);
-    for (int j = r; j >= 1; --j) {
-        wj = ws[j];
-        const float a = x[j * st], b = x[-j * st];
-        const float sum = a + b, z = sum - a, err = (a - (sum - z)) + (b - z);
-        const float ph = sum * wj.x;
-        add(ph, fmaf(sum, wj.x, -ph) + fmaf(sum, wj.y, err * wj.x));
+    if (!exact) {
+        float2 wj = ws[0];
+        float hi = __fmul_rn(x[0], wj.x), lo = __fmaf_rn(x[0], wj.y, __fmaf_rn(x[0], wj.x, -hi));
+        for (int j = r; j >= 1; --j) {
+            wj = ws[j];
+            const float a = x[j * st], b = x[-j * st];
+            const float sum = __fadd_rn(a, b), z = __fsub_rn(sum, a);
+            const float err = __fadd_rn(__fsub_rn(a, __fsub_rn(sum, z)), __fsub_rn(b, z));
+            const float ph = __fmul_rn(sum, wj.x);
+            const float pl = __fmaf_rn(sum, wj.y, __fmaf_rn(err, wj.x, __fmaf_rn(sum, wj.x, -ph)));
+            const float t = __fadd_rn(hi, ph), y = __fsub_rn(t, hi);
+            const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, y)), __fsub_rn(ph, y));
+            lo = __fadd_rn(lo, __fadd_rn(e, pl));
+            hi = t;
+        }
+        const float d = __fmul_rn(hi, (float)((r + 8) * (r + 8)) * 0x1p-48f);
+        const float up = __fadd_rn(hi, __fadd_rn(lo, d));
+        if (hi >= 1e-24f && hi <= 1e37f && up == __fadd_rn(hi, __fsub_rn(lo, d)))
+            return up;
     }
-    if (!(hi >= 1e-24f && hi <= 1e37f)) {
-        double acc = __dmul_rn((double)x[0], w[r]);
-        for (int j = r; j >= 1; --j)
-            acc = __dadd_rn(acc, __dmul_rn(__dadd_rn((double)x[j * st], (double)x[-j * st]), w[r + j]));
-        return (float)acc;
-    }
-    return __fadd_rn(hi, lo);
+    double acc = __dmul_rn((double)x[0], w[r]);
+    for (int j = r; j >= 1; --j)
+        acc = __dadd_rn(acc, __dmul_rn(__dadd_rn((double)x[j * st], (double)x[-j * st]), w[r + j]));
+    return (float)acc;
 }
 
 template <typename T>
@@ -799,13 +804,16 @@ __global__ void __launch_bounds__(256) k_env_gauss(EnvGeom G, int axis, const do
             return (T)hp[((long long)(a0 + G.off0) * G.msh + (a1 + G.off1)) * G.msh + (a2 + G.off2)];
         return in[((long long)a0 * G.n1 + a1) * G.n2 + a2];
     };
+    int odd = 0;  // float32: weights outside what the pairs' bound covers
     if constexpr (sizeof(T) == 4) {
         if (tid <= r) {
             const double v = w[r + tid];
             const float h = (float)v;
             ws[tid] = make_float2(h, (float)(v - (double)h));
+            odd = !(h >= 1e-30f && h <= 1e30f) && (__double_as_longlong(v) << 1) != 0;  // (no FP64 compares)
         }
     }
+    bool exact;
     const T *x;
     int st;
     if (axis < 2) {
@@ -818,7 +826,7 @@ __global__ void __launch_bounds__(256) k_env_gauss(EnvGeom G, int axis, const do
             const int k = s0 + t / 32, c = (int)blockIdx.x * 32 + (t & 31);
             gx[t] = axis == 0 ? input(k, other, c) : input(other, k, c);
         }
-        __syncthreads();
+        exact = __syncthreads_or(odd);
         const int k = (int)blockIdx.y * 8 + ty;
         if (k >= n[axis] || a2 >= G.n2)
             return;
@@ -835,7 +843,7 @@ __global__ void __launch_bounds__(256) k_env_gauss(EnvGeom G, int axis, const do
             const int row = t / wdt, c = t - row * wdt;
             gx[t] = input((int)blockIdx.z, (int)blockIdx.y * 8 + row, s2 + c);
         }
-        __syncthreads();
+        exact = __syncthreads_or(odd);
         const int a1 = (int)blockIdx.y * 8 + ty, a2 = (int)blockIdx.x * 32 + tx;
         if (a1 >= G.n1 || a2 >= G.n2)
             return;
@@ -847,7 +855,7 @@ __global__ void __launch_bounds__(256) k_env_gauss(EnvGeom G, int axis, const do
     }
     T acc;
     if constexpr (sizeof(T) == 4)
-        acc = gauss_sum(x, st, ws, w, r);
+        acc = gauss_sum(x, st, ws, w, r, exact);
     else
         acc = gauss_sum(x, st, w, r);
     long long o = ((long long)ii[0] * G.n1 + ii[1]) * G.n2 + ii[2];
