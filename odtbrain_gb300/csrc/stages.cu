@@ -60,18 +60,16 @@ namespace odt {
 // 24.1 ms with both).
 constexpr bool kColumnStepRegs = true;
 constexpr bool kColumnTw2 = true;
-// Planes between exact propagator anchors within a column CTA's run.
+// Planes between exact propagator anchors within a column CTA's run, at most
+// (anchor_planes has the rule).
 constexpr int kReanchorPlanes = 32;
 // Column CTAs that run through up to 256 planes of an angle, re-anchoring
-// the propagator every kReanchorPlanes planes: power-of-two columns of
-// 64-thread lines with the steps in registers (4 columns per CTA, the
-// 512-point planes).  256^3 workload,
-// cap on the planes per CTA against the column stage: 32 planes 24.1 ms,
-// 64 22.8, 128 22.4, 256 22.2 ms.  The other column kernels keep runs of
-// at most kReanchorPlanes planes (one exact anchor each): the 512-thread
-// CTAs of 256-point columns lost 30 % with longer runs (one wave of long
-// CTAs).
-template <class L, int KX, bool HALF>
+// the propagator on the way: power-of-two columns in CTAs of at most 256
+// threads, with the steps in registers (64 to 512 points).  256^3 from 200
+// single views, cap on the planes per CTA against the column stage: 32 planes
+// 24.1 ms, 64 22.8, 128 22.4, 256 22.2 ms.  The other column kernels keep runs
+// of at most kReanchorPlanes planes.
+template <class L, int KX>
 constexpr bool long_runs()
 {
     return pow2_len<L>() > 0 && kColumnStepRegs && KX * L::TPL <= 256;
@@ -328,7 +326,7 @@ __global__ void __launch_bounds__(KX * L::TPL) k_columns_boundary(StageParams P,
 // predicates.
 template <class L, int KX, bool HALF, bool PAIR>
 __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX * L::TPL <= 512) ? 2 : 1))
-    k_columns_propagate(StageParams P, L line, const float2 *spec, float2 *T, int q0, int qn, int ppc)
+    k_columns_propagate(StageParams P, L line, const float2 *spec, float2 *T, int q0, int qn, int ppc, int anchor)
 {
     if (!group_active<KX>(P, blockIdx.x * KX))
         return;  // all-zero columns: the row stage never reads them
@@ -380,9 +378,9 @@ __global__ void __launch_bounds__(KX * L::TPL, (KX * L::TPL <= 256) ? 3 : ((KX *
             p = 0;
             ++u;
         }
-        if (u != cur_u || since == kReanchorPlanes) {
+        if (u != cur_u || since == anchor) {
             // exact anchor at the first plane of a unit, and again every
-            // kReanchorPlanes planes: the FP32 recurrence drifts by about one
+            // `anchor` planes: the FP32 recurrence drifts by about one
             // rounding per plane (measured on the 256^3 workload: rel-L2 to
             // the FP64 oracle 3.5e-7 with anchors every 32 planes, 1.6e-6
             // with one anchor per 256-plane run)
@@ -872,13 +870,19 @@ __global__ void __launch_bounds__(256) k_spectrum_line(StageParams P, float2 *ro
 // a start-up (tables, exact anchor) counted as four planes.  At most 256 for
 // long runs (long_runs), else at most kReanchorPlanes.
 template <int KX>
-static int planes_per_cta(const StageParams &P, int qn, bool long_run)
+static int active_groups(const StageParams &P)
 {
     const int groups = (P.lNx + KX - 1) / KX;
     int active = 0;
     for (int g = 0; g < groups; ++g)
         if (!(g * KX >= P.kx_zero_lo && g * KX + KX <= P.kx_zero_hi))
             ++active;
+    return active;
+}
+template <int KX>
+static int planes_per_cta(const StageParams &P, int qn, bool long_run)
+{
+    const int active = active_groups<KX>(P);
     const int slots = std::max(1, P.col_slots), cap = std::min(long_run ? 256 : kReanchorPlanes, qn);
     int best = cap;
     long long least = -1;
@@ -891,6 +895,26 @@ static int planes_per_cta(const StageParams &P, int qn, bool long_run)
         }
     }
     return best;
+}
+
+// Planes between anchors: what one wave of up to 1024 planes gives a CTA, 4 to
+// 32, in equal parts of a slab.  Few column groups make long runs of small
+// planes, whose anchors cost little: 64^3 from 60 views with anchors every 32 /
+// 16 / 8 planes 323 / 320 / 333 us at rel-L2 2.0 / 1.7 / 1.6e-7, 256^3 from 200
+// views 26.6 / 27.3 / 28.7 ms at 2.6 / 2.4 / 2.4e-7.  Opposite views drift
+// together from one anchor where single ones do so apart, so below 512 points,
+// where that shows (128^3 2.71e-7 against 2.60e-7 for single views), units
+// take three quarters of it.
+template <int KX>
+static int anchor_planes(const StageParams &P, int qn)
+{
+    const int slots = std::max(1, P.col_slots);
+    const int wave = (std::min(qn, 1024) * active_groups<KX>(P) + slots - 1) / slots;
+    int most = std::min(kReanchorPlanes, std::max(4, wave));
+    if (P.units && P.lNy < 512)
+        most = std::max(4, most * 3 / 4);
+    const int parts = (P.nz + most - 1) / most;
+    return (P.nz + parts - 1) / parts;
 }
 
 // Shared memory of the column kernel: the exchange buffers, the twiddle
@@ -977,10 +1001,10 @@ static cudaError_t columns_launch(const StageParams &P, L line, const float2 *sp
                                   cudaStream_t s)
 {
     constexpr int KX = Cfg<L>::KX;
-    const int ppc = planes_per_cta<KX>(P, qn, long_runs<L, KX, HALF>());
+    const int ppc = planes_per_cta<KX>(P, qn, long_runs<L, KX>());
     dim3 grid((P.lNx + KX - 1) / KX, (qn + ppc - 1) / ppc);
     k_columns_propagate<L, KX, HALF, PAIR>
-        <<<grid, KX * L::TPL, smem_cols_prop<L, HALF>(line.n), s>>>(P, line, spec, T, q0, qn, ppc);
+        <<<grid, KX * L::TPL, smem_cols_prop<L, HALF>(line.n), s>>>(P, line, spec, T, q0, qn, ppc, anchor_planes<KX>(P, qn));
     return cudaGetLastError();
 }
 template <class L>
