@@ -68,14 +68,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
     return *reinterpret_cast<uint32_t *>(&v);
 }
 
-__device__ __forceinline__ uint32_t pair_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi)
-{
-    __nv_bfloat162 v;
-    v.x = lo;
-    v.y = hi;
-    return *reinterpret_cast<uint32_t *>(&v);
-}
-
 // fast reciprocal: the activations are rounded to BF16 next (C5 gain
 // inference: 0.37 -> 0.18 ms with the IEEE division replaced)
 __device__ __forceinline__ float sigmoid(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }

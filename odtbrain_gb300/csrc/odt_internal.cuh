@@ -86,7 +86,6 @@ struct StageParams {
     int tedge[8];        // transposed(): the T rows of the edge samples
 };
 
-// y pitch of the slab layout [a][z][x][y]
 // y pitch of the y-axis coefficient slab [a][z][x][y]: a multiple of 32,
 // except for single-row planes (the 2D reconstruction), stored as [a][z][x]
 inline int yaxis_slab_pitch(int ny) { return ny == 1 ? 1 : (ny + 31) / 32 * 32; }

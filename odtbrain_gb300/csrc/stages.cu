@@ -1020,7 +1020,7 @@ static cudaError_t columns_impl(const StageParams &P, L line, const float2 *spec
                    : columns_launch<L, false, false>(P, line, spec, T, q0, qn, s);
 }
 
-template <class L, int NP, bool ROWPF, bool HALF>
+template <class L, int NP>
 static size_t smem_rows_inverse(int n)
 {
     return smem_rows<L>(n) + smem_rows_y<L, NP>(n);
@@ -1032,7 +1032,7 @@ static cudaError_t rows_launch(const StageParams &P, L line, const float2 *T, co
     constexpr int LPC = Cfg<L>::LPC, RG = rows_per_cta<LPC>();
     const unsigned grid = (unsigned)((long long)qn * ((P.ny + RG - 1) / RG));
     k_rows_inverse<L, LPC, NP, ROWPF, HALF>
-        <<<grid, LPC * L::TPL, smem_rows_inverse<L, NP, ROWPF, HALF>(line.n), s>>>(P, line, T, Tab, slab, q0);
+        <<<grid, LPC * L::TPL, smem_rows_inverse<L, NP>(line.n), s>>>(P, line, T, Tab, slab, q0);
     return cudaGetLastError();
 }
 template <class L>
@@ -1077,10 +1077,10 @@ static cudaError_t set_smem_attrs_crop(int n)
     if (e == cudaSuccess)
         e = allow_smem(k_columns_propagate<L, KX, HALF, true>, smem_cols_prop<L, HALF>(n));
     if (e == cudaSuccess)
-        e = allow_smem(k_rows_inverse<L, LPC, NP, false, HALF>, smem_rows_inverse<L, NP, false, HALF>(n));
+        e = allow_smem(k_rows_inverse<L, LPC, NP, false, HALF>, smem_rows_inverse<L, NP>(n));
     if constexpr (NP > 0) {
         if (e == cudaSuccess)
-            e = allow_smem(k_rows_inverse<L, LPC, NP, true, HALF>, smem_rows_inverse<L, NP, true, HALF>(n));
+            e = allow_smem(k_rows_inverse<L, LPC, NP, true, HALF>, smem_rows_inverse<L, NP>(n));
     }
     return e;
 }

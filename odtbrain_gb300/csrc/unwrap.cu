@@ -768,8 +768,6 @@ __global__ void __launch_bounds__(256) k_uw_init(const T *phi, Frames F, uint32_
 }
 
 // Lightest outgoing edge weight of every component root (edges handled by
-// their pixel 1: right and down neighbours).
-// Lightest outgoing edge weight of every component root (edges handled by
 // their pixel 1: right and down neighbours).  With `elist`, the crossing
 // edges are also appended to it as (pixel 1, frame-local edge index).
 __global__ void k_uw_minw(Frames F, const double *rel, const unsigned long long *word, unsigned long long *bw,
