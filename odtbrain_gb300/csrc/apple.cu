@@ -136,6 +136,33 @@ __device__ __forceinline__ float2 constrain(const AP &P, float2 d, uint8_t fl, f
     return make_float2(constrain_re<float>(P.method, P.has_mask, d.x, fl, fmin, fmax, lo, hi), 0.f);
 }
 
+// CTAs per SM that the line kernels' registers are bounded for: power-of-two
+// lines `small` at up to 256 threads, `mid` at up to 512; direct transforms (any
+// other length; 16 slots, addressed by a run-time index) `direct`, the most
+// without spills, each group's loads and operands where they are used.  (With the
+// registers of the power-of-two lines and their reading ahead 12 iterations of
+// 45^3 took 1.08 ms, of 101^3 6.0 and of 130^3 14.6; like this 0.88, 5.0, 12.5.)
+template <class L>
+constexpr int line_ctas(int threads, int direct, int small, int mid)
+{
+    return pow2_len<L>() == 0 ? direct : threads <= 256 ? small : threads <= 512 ? mid : 1;
+}
+template <class L>
+constexpr bool reads_ahead()
+{
+    return pow2_len<L>() > 0;
+}
+
+// CTAs of a line kernel over `groups`: the resident ones, striding.  A direct
+// transform's time is its n^2 products, not the set-up that striding saves, and
+// beyond one and a half waves one group per CTA balances better (12 iterations of
+// 101^3 5.5 -> 5.0 ms; 45^3, 1.1 waves, 0.88 against 0.90 ms).
+template <class L>
+int line_grid(long long groups, long long resident)
+{
+    return (int)(pow2_len<L>() == 0 && 2 * groups > 3 * resident ? groups : std::min(groups, resident));
+}
+
 // ---- axis 2 (contiguous lines) --------------------------------------------
 // mode 0: f.real -> forward -> buf (the original spectrum's first axis)
 // mode 1: constrain(f.real) -> forward -> buf (iteration 0's first axis)
@@ -145,7 +172,7 @@ __device__ __forceinline__ float2 constrain(const AP &P, float2 d, uint8_t fl, f
 //         transform: 0.078 ms at 256^3, like this 0.07, 0.042 at the copy rate)
 // mode 3: constrain(data) -> forward -> buf (method "sh")
 template <class L, int LPC>
-__global__ void __launch_bounds__(LPC *L::TPL, LPC *L::TPL <= 256 ? 5 : 1)
+__global__ void __launch_bounds__(LPC *L::TPL, line_ctas<L>(LPC *L::TPL, 4, 5, 1))
     k_apple_x(AP P, L line, int mode, int it, int groups)
 {
     if (mode >= 2 && ran_out(P, it))
@@ -165,16 +192,23 @@ __global__ void __launch_bounds__(LPC *L::TPL, LPC *L::TPL <= 256 ? 5 : 1)
     }
     // (of mode 2; uniform over the grid)
     const bool next = P.method != 1 && it + 1 < P.max_iter && !ran_out(P, it + 1);
+    auto flag = [&](const auto &fl, int r, long long vox) -> uint8_t {
+        if constexpr (reads_ahead<L>())
+            return fl[r];
+        else
+            return P.flags[vox];
+    };
     for (int g = blockIdx.x; g < groups; g += gridDim.x) {
         const long long lid = (long long)g * LPC + l;
         const bool valid = lid < (long long)P.n0 * P.n1;
         const long long base = valid ? lid * n : 0;
         float2 v[L::SLOTS];
-        uint8_t fl[L::SLOTS];  // read ahead of the transform
+        uint8_t fl[reads_ahead<L>() ? L::SLOTS : 1];
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
             const int x = j + r * L::TPL;
-            fl[r] = (valid && x < n && mode != 0 && (mode != 2 || next)) ? P.flags[base + x] : (uint8_t)0;
+            if constexpr (reads_ahead<L>())
+                fl[r] = (valid && x < n && mode != 0 && (mode != 2 || next)) ? P.flags[base + x] : (uint8_t)0;
             float2 a = make_float2(0.f, 0.f);
             if (valid && x < n) {
                 if (mode <= 1)
@@ -184,7 +218,7 @@ __global__ void __launch_bounds__(LPC *L::TPL, LPC *L::TPL <= 256 ? 5 : 1)
                 else
                     a = P.data[base + x];
                 if (mode == 1 || mode == 3)
-                    a = constrain(P, a, fl[r], fmin, fmax, lo, hi);
+                    a = constrain(P, a, flag(fl, r, base + x), fmin, fmax, lo, hi);
             }
             v[r] = a;
         }
@@ -198,7 +232,7 @@ __global__ void __launch_bounds__(LPC *L::TPL, LPC *L::TPL <= 256 ? 5 : 1)
                 v[r] = make_float2(__fmul_rn(v[r].x, P.scale), __fmul_rn(v[r].y, P.scale));
                 if (valid && x < n) {
                     if (next)
-                        v[r] = constrain(P, v[r], fl[r], 0.f, 0.f, 0.f, 0.f);
+                        v[r] = constrain(P, v[r], flag(fl, r, base + x), 0.f, 0.f, 0.f, 0.f);
                     else
                         P.data[base + x] = v[r];
                 }
@@ -229,7 +263,7 @@ __global__ void __launch_bounds__(LPC *L::TPL, LPC *L::TPL <= 256 ? 5 : 1)
 // axis 1, forward or inverse (256^3: one
 // group per CTA 0.080 ms, like this 0.048)
 template <class L, int KX>
-__global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 4 : KX *L::TPL <= 512 ? 2 : 1)
+__global__ void __launch_bounds__(KX *L::TPL, line_ctas<L>(KX *L::TPL, 3, 4, 2))
     k_apple_s1(AP P, L line, int inverse, int it, int groups)
 {
     if (ran_out(P, it))
@@ -253,11 +287,18 @@ __global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 4 : KX *L::TPL
         }
     };
     float2 v[L::SLOTS];
-    float2 *col = column(blockIdx.x);
-    load(col, v);
+    float2 *col;
+    if constexpr (reads_ahead<L>()) {
+        col = column(blockIdx.x);
+        load(col, v);
+    }
     __syncthreads();
     int flip = 0;
     for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+        if constexpr (!reads_ahead<L>()) {
+            col = column(g);
+            load(col, v);
+        }
         if (inverse)
             line.template run<1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
         else
@@ -270,9 +311,11 @@ __global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 4 : KX *L::TPL
                     col[(long long)k * stride] = v[r];
             }
         }
-        if (g + (int)gridDim.x < groups) {
-            col = column(g + gridDim.x);
-            load(col, v);
+        if constexpr (reads_ahead<L>()) {
+            if (g + (int)gridDim.x < groups) {
+                col = column(g + gridDim.x);
+                load(col, v);
+            }
         }
         __syncthreads();  // the exchange buffers are the next group's
     }
@@ -284,7 +327,7 @@ __global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 4 : KX *L::TPL
 // (256^3: one group per CTA and all operands after the transform 0.126 ms,
 // like this 0.100).
 template <class L, int KX>
-__global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 3 : KX *L::TPL <= 512 ? 2 : 1)
+__global__ void __launch_bounds__(KX *L::TPL, line_ctas<L>(KX *L::TPL, 4, 3, 2))
     k_apple_s0(AP P, L line, int original, int it, int groups)
 {
     if (!original && ran_out(P, it))
@@ -297,32 +340,40 @@ __global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 3 : KX *L::TPL
     copy_twiddles<L>(tw, P.tw0, n);
     const int c = threadIdx.x % KX, j = threadIdx.x / KX;
     const long long stride = (long long)P.n1 * P.n2;
-    auto load = [&](long long q, float2 (&v)[L::SLOTS], uint8_t (&fl)[L::SLOTS]) {
+    constexpr bool AHEAD = reads_ahead<L>();
+    constexpr int NA = AHEAD ? L::SLOTS : 1;
+    auto load = [&](long long q, float2 (&v)[L::SLOTS], uint8_t (&fl)[NA]) {
 #pragma unroll
         for (int r = 0; r < L::SLOTS; ++r) {
             const int k = j + r * L::TPL;
             const bool in = q < stride && k < n;
             v[r] = in ? P.buf[q + k * stride] : make_float2(0.f, 0.f);
-            fl[r] = in ? P.flags[q + k * stride] : (uint8_t)0;
+            if constexpr (AHEAD)
+                fl[r] = in ? P.flags[q + k * stride] : (uint8_t)0;
         }
     };
     float2 v[L::SLOTS];
-    uint8_t fl[L::SLOTS];
+    uint8_t fl[NA];
     long long q = (long long)blockIdx.x * KX + c;
-    load(q, v, fl);
+    if constexpr (AHEAD)
+        load(q, v, fl);
     __syncthreads();
     int flip = 0;
     double part = 0.0;
     for (int g = blockIdx.x; g < groups; g += gridDim.x) {
-        float2 og[L::SLOTS];
-        float ev[L::SLOTS];
-        if (!original) {
+        if constexpr (!AHEAD)
+            load(q, v, fl);
+        float2 og[NA];
+        float ev[NA];
+        if constexpr (AHEAD) {
+            if (!original) {
 #pragma unroll
-            for (int r = 0; r < L::SLOTS; ++r) {
-                const int k = j + r * L::TPL;
-                const bool in = q < stride && k < n;
-                og[r] = (in && !(fl[r] & F_CORE)) ? P.orig[q + k * stride] : make_float2(0.f, 0.f);
-                ev[r] = (in && (fl[r] & F_CORE) && P.evlp) ? P.evlp[q + k * stride] : 0.f;
+                for (int r = 0; r < L::SLOTS; ++r) {
+                    const int k = j + r * L::TPL;
+                    const bool in = q < stride && k < n;
+                    og[r] = (in && !(fl[r] & F_CORE)) ? P.orig[q + k * stride] : make_float2(0.f, 0.f);
+                    ev[r] = (in && (fl[r] & F_CORE) && P.evlp) ? P.evlp[q + k * stride] : 0.f;
+                }
             }
         }
         line.template run<-1, true>(v, j, buf0 + c, buf1 + c, KX, tw, flip);
@@ -333,26 +384,27 @@ __global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 3 : KX *L::TPL
                 continue;
             const long long vox = q + k * stride;
             float2 ft = v[r];
+            const bool core = (AHEAD ? fl[AHEAD ? r : 0] : P.flags[vox]) & F_CORE;
             if (original) {
                 P.orig[vox] = ft;
-                if (fl[r] & F_CORE)
+                if (core)
                     part += (double)hypotf(ft.x, ft.y);
-            } else if (fl[r] & F_CORE) {
+            } else if (core) {
                 float h = hypotf(ft.x, ft.y);
-                if (P.evlp && h > ev[r]) {
+                if (P.evlp && h > (AHEAD ? ev[AHEAD ? r : 0] : P.evlp[vox])) {
                     ft = make_float2(__fmul_rn(ft.x, P.ee), __fmul_rn(ft.y, P.ee));
                     h = hypotf(ft.x, ft.y);
                 }
                 part += (double)h;
             } else {
+                float2 o = AHEAD ? og[AHEAD ? r : 0] : P.orig[vox];
                 if (P.method == 1 && vox == 0) {  // (orig + ft) / 2 at the DC term
                     if (P.evlp && hypotf(ft.x, ft.y) > P.evlp[0])
                         ft = make_float2(__fmul_rn(ft.x, P.ee), __fmul_rn(ft.y, P.ee));
-                    og[r] = make_float2(__fmul_rn(__fadd_rn(og[r].x, ft.x), 0.5f),
-                                        __fmul_rn(__fadd_rn(og[r].y, ft.y), 0.5f));
-                    P.orig[0] = og[r];
+                    o = make_float2(__fmul_rn(__fadd_rn(o.x, ft.x), 0.5f), __fmul_rn(__fadd_rn(o.y, ft.y), 0.5f));
+                    P.orig[0] = o;
                 }
-                ft = og[r];
+                ft = o;
             }
             v[r] = ft;
         }
@@ -368,8 +420,10 @@ __global__ void __launch_bounds__(KX *L::TPL, KX *L::TPL <= 256 ? 3 : KX *L::TPL
             __syncthreads();  // the exchange buffers are the next group's
         }
         q += (long long)gridDim.x * KX;
-        if (g + (int)gridDim.x < groups)
-            load(q, v, fl);
+        if constexpr (AHEAD) {
+            if (g + (int)gridDim.x < groups)
+                load(q, v, fl);
+        }
     }
     // sum of the core magnitudes
     for (int s = 16; s > 0; s >>= 1)
@@ -1204,45 +1258,91 @@ size_t smem_s(int n)
     return (size_t)(2 * Cfg<L>::KX * xslots<true>(n) + tw_slots(n)) * sizeof(float2);
 }
 
-cudaError_t launch_x(const AP &P, int mode, int it, cudaStream_t s)
+// CTAs of the line kernels, found once per call: a query and an attribute per
+// launch were 2 % of a 32^3 call.
+struct LineGrids {
+    int x, s1, s0;
+};
+
+// Allows the kernel its shared memory (per kernel and process, so the most its
+// line type can need) and returns its CTAs over `groups`.
+template <class L, class F>
+cudaError_t line_setup(F *kernel, int threads, size_t sm, size_t sm_most, long long groups, int *grid)
+{
+    int dev = 0, sms = 0, occ = 0;
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_most)) ||
+        (e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, sm)))
+        return e;
+    *grid = line_grid<L>(groups, sms * std::max(occ, 1));
+    return cudaSuccess;
+}
+template <class L>
+constexpr int longest()
+{
+    return pow2_len<L>() > 0 ? pow2_len<L>() : GenericLine::TPL * GenericLine::SLOTS;
+}
+template <class L>
+long long groups_x(const AP &P)
+{
+    return ((long long)P.n0 * P.n1 + Cfg<L>::LPC - 1) / Cfg<L>::LPC;
+}
+template <class L>
+long long groups_s(const AP &P, int axis)
+{
+    const long long inner = axis == 0 ? (long long)P.n1 * P.n2 : P.n2;
+    return (axis == 0 ? 1 : P.n0) * ((inner + Cfg<L>::KX - 1) / Cfg<L>::KX);
+}
+
+cudaError_t line_grids(const AP &P, LineGrids *G)
+{
+    cudaError_t e = with_line(P.n2, [&](auto line) {
+        using L = decltype(line);
+        constexpr int LPC = Cfg<L>::LPC;
+        return line_setup<L>(k_apple_x<L, LPC>, LPC * L::TPL, smem_x<L>(P.n2), smem_x<L>(longest<L>()),
+                             groups_x<L>(P), &G->x);
+    });
+    if (e == cudaSuccess)
+        e = with_line(P.n1, [&](auto line) {
+            using L = decltype(line);
+            constexpr int KX = Cfg<L>::KX;
+            return line_setup<L>(k_apple_s1<L, KX>, KX * L::TPL, smem_s<L>(P.n1), smem_s<L>(longest<L>()),
+                                 groups_s<L>(P, 1), &G->s1);
+        });
+    if (e == cudaSuccess)
+        e = with_line(P.n0, [&](auto line) {
+            using L = decltype(line);
+            constexpr int KX = Cfg<L>::KX;
+            return line_setup<L>(k_apple_s0<L, KX>, KX * L::TPL, smem_s<L>(P.n0), smem_s<L>(longest<L>()),
+                                 groups_s<L>(P, 0), &G->s0);
+        });
+    return e;
+}
+
+cudaError_t launch_x(const AP &P, const LineGrids &G, int mode, int it, cudaStream_t s)
 {
     return with_line(P.n2, [&](auto line) {
         using L = decltype(line);
         constexpr int LPC = Cfg<L>::LPC;
-        const size_t sm = smem_x<L>(P.n2);
-        cudaFuncSetAttribute(k_apple_x<L, LPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        const int groups = (int)(((long long)P.n0 * P.n1 + LPC - 1) / LPC);
-        int dev = 0, sms = 0, occ = 0;
-        cudaError_t e;
-        if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
-            (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_apple_x<L, LPC>, LPC * L::TPL, sm)))
-            return e;
-        const int grid = std::min(groups, sms * std::max(occ, 1));
-        k_apple_x<L, LPC><<<(unsigned)grid, LPC * L::TPL, sm, s>>>(P, line, mode, it, groups);
+        k_apple_x<L, LPC><<<(unsigned)G.x, LPC * L::TPL, smem_x<L>(P.n2), s>>>(P, line, mode, it, (int)groups_x<L>(P));
         return cudaGetLastError();
     });
 }
 
 // mode 0: axis 1 forward, 1: axis 1 inverse, 2: axis 0 forward -> orig (the
 // original spectrum) + core sum, 3: axis 0 of an iteration
-cudaError_t launch_s(const AP &P, int axis, int mode, int it, cudaStream_t s)
+cudaError_t launch_s(const AP &P, const LineGrids &G, int axis, int mode, int it, cudaStream_t s)
 {
     const int n = axis == 0 ? P.n0 : P.n1;
     return with_line(n, [&](auto line) {
         using L = decltype(line);
         constexpr int KX = Cfg<L>::KX;
-        const size_t sm = smem_s<L>(n);
-        int dev = 0, sms = 0, occ = 0;
-        cudaError_t e;
-        const auto kernel = axis == 0 ? k_apple_s0<L, KX> : k_apple_s1<L, KX>;
-        const long long inner = axis == 0 ? (long long)P.n1 * P.n2 : P.n2;
-        const long long groups = (axis == 0 ? 1 : P.n0) * ((inner + KX - 1) / KX);
-        if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) ||
-            (e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
-            (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, KX * L::TPL, sm)))
-            return e;
-        const long long grid = std::min<long long>(groups, (long long)sms * std::max(occ, 1));
-        kernel<<<(unsigned)grid, KX * L::TPL, sm, s>>>(P, line, axis == 0 ? mode == 2 : mode == 1, it, (int)groups);
+        const int groups = (int)groups_s<L>(P, axis);
+        if (axis == 0)
+            k_apple_s0<L, KX><<<(unsigned)G.s0, KX * L::TPL, smem_s<L>(n), s>>>(P, line, mode == 2, it, groups);
+        else
+            k_apple_s1<L, KX><<<(unsigned)G.s1, KX * L::TPL, smem_s<L>(n), s>>>(P, line, mode == 1, it, groups);
         return cudaGetLastError();
     });
 }
@@ -1561,7 +1661,9 @@ odt_status odt_apple_correct(const odt_apple_desc *desc, const float *f_real, co
                            (uint8_t *)(ws + L.flags), (double *)(ws + L.ftab), s)))
         return cuda_fail("apple flags", e);
     // original spectrum: axis 2, 1 from f.real into buf, axis 0 into orig
-    if ((e = launch_x(P, 0, -1, s)) || (e = launch_s(P, 1, 0, -1, s)) || (e = launch_s(P, 0, 2, -1, s)))
+    LineGrids G;
+    if ((e = line_grids(P, &G)) || (e = launch_x(P, G, 0, -1, s)) || (e = launch_s(P, G, 1, 0, -1, s)) ||
+        (e = launch_s(P, G, 0, 2, -1, s)))
         return cuda_fail("apple spectrum", e);
     k_apple_dec<<<1, 1, 0, s>>>(P, -1);
     if (P.evlp) {
@@ -1587,7 +1689,7 @@ odt_status odt_apple_correct(const odt_apple_desc *desc, const float *f_real, co
         const int it1 = std::min(d.max_iter, it0 + CHUNK);
         for (int it = it0; it < it1; ++it) {
             if (d.method != ODT_APPLE_SH) {
-                if (it == 0 && (e = launch_x(P, 1, 0, s)))
+                if (it == 0 && (e = launch_x(P, G, 1, 0, s)))
                     return cuda_fail("apple iteration", e);
             } else {
                 // constraint_sh: min / max over the spillover region, the
@@ -1609,13 +1711,13 @@ odt_status odt_apple_correct(const odt_apple_desc *desc, const float *f_real, co
                     return cuda_fail("apple sh", e);
                 if (stopped)
                     break;
-                if ((e = launch_x(P, 3, it, s)))
+                if ((e = launch_x(P, G, 3, it, s)))
                     return cuda_fail("apple iteration", e);
             }
-            if ((e = launch_s(P, 1, 0, it, s)) || (e = launch_s(P, 0, 3, it, s)))
+            if ((e = launch_s(P, G, 1, 0, it, s)) || (e = launch_s(P, G, 0, 3, it, s)))
                 return cuda_fail("apple iteration", e);
             k_apple_dec<<<1, 1, 0, s>>>(P, it);
-            if ((e = launch_s(P, 1, 1, it, s)) || (e = launch_x(P, 2, it, s)))
+            if ((e = launch_s(P, G, 1, 1, it, s)) || (e = launch_x(P, G, 2, it, s)))
                 return cuda_fail("apple iteration", e);
         }
         if ((e = cudaMemcpyAsync(&host_ctl, P.ctl, sizeof(AppleCtl), cudaMemcpyDeviceToHost, s)) ||
